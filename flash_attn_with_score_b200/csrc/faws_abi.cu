@@ -63,6 +63,13 @@ FwdParams make_fwd(const faws_problem* p) {
   return f;
 }
 
+// Whether the tcgen05 kernels may take this problem.  Head dims 16 and 32 run on their D = 64 instances (the TMA
+// boxes' missing columns are filled with zeros on loads and clipped on stores); a caller that forces the family
+// is refused there, as ever: FAWS_BACKEND_TCGEN05 stands for D in {64, 128}.
+bool tc_allowed(const faws_problem* p) {
+  return p->backend != FAWS_BACKEND_GENERIC && !(p->backend == FAWS_BACKEND_TCGEN05 && p->D < 64);
+}
+
 // Scratch must start on a 256-byte boundary (faws_workspace_bytes says so): the kernels read and write it with
 // 16-byte vectors, TMA stores and bulk copies.
 bool misaligned_ws(const void* ws) { return reinterpret_cast<uintptr_t>(ws) % 256 != 0; }
@@ -85,7 +92,7 @@ ColSoftmaxParams make_cs(const faws_problem* p, const float* L, float* out, int 
 int run_fwd(const faws_problem* p, FwdParams& f, cudaStream_t s, int* block_m, int* block_n) {
   if (f.v == nullptr || f.o == nullptr) return FAWS_EINVAL;
   bool use_tc = false;
-  if (p->backend != FAWS_BACKEND_GENERIC) use_tc = tc_fwd_supported(f, p->dtype);
+  if (tc_allowed(p)) use_tc = tc_fwd_supported(f, p->dtype);
   if (p->backend == FAWS_BACKEND_TCGEN05 && !use_tc) return FAWS_EBACKEND;
   if (!use_tc) f.col_lin = 0;
   *block_m = use_tc ? kTcBlockM : kGenericBlockM;
@@ -111,7 +118,7 @@ int run_fwd(const faws_problem* p, FwdParams& f, cudaStream_t s, int* block_m, i
 int run_colsoftmax(const faws_problem* p, ColSoftmaxParams& c, float* final_out, float* per_head_ws,
                    int group_sum, cudaStream_t s) {
   bool use_tc = false;
-  if (p->backend != FAWS_BACKEND_GENERIC) use_tc = tc_colsoftmax_supported(c, p->dtype);
+  if (tc_allowed(p)) use_tc = tc_colsoftmax_supported(c, p->dtype);
   if (p->backend == FAWS_BACKEND_TCGEN05 && !use_tc && c.s_scratch == nullptr) return FAWS_EBACKEND;
   cudaError_t e;
   if (c.s_scratch != nullptr) {  // buffered variant: stream the stored scores back
@@ -308,7 +315,7 @@ int faws_attention(const faws_problem* p, void* stream) {
   int st = validate(p);
   if (st != FAWS_OK) return st;
   faws_problem packed;
-  if (p->backend != FAWS_BACKEND_GENERIC && pack_gqa(p, &packed)) {
+  if (tc_allowed(p) && pack_gqa(p, &packed)) {
     FwdParams fp = make_fwd(&packed);
     if (fp.v != nullptr && tc_fwd_supported(fp, packed.dtype)) p = &packed;
   }
@@ -333,7 +340,7 @@ int faws_attention_with_scores(const faws_problem* p, void* scores, int32_t scor
 
 int32_t faws_split_kv_plan(const faws_problem* p) {
   if (validate(p) != FAWS_OK) return 1;
-  if (p->dropout_p > 0.f || p->m_begin != 0 || p->m_end != p->M || p->backend == FAWS_BACKEND_GENERIC) return 1;
+  if (p->dropout_p > 0.f || p->m_begin != 0 || p->m_end != p->M || !tc_allowed(p)) return 1;
   if (p->v.ptr == nullptr || p->out.ptr == nullptr) return 1;
   faws_problem packed;
   if (pack_gqa(p, &packed)) {
@@ -360,12 +367,12 @@ int faws_attention_split_kv(const faws_problem* p, int32_t n_splits, void* works
     return FAWS_EWORKSPACE;
   if (p->out.ptr == nullptr || p->v.ptr == nullptr) return FAWS_EINVAL;
   faws_problem packed;  // same bytes of workspace either way: B*Hq*M is unchanged by the packing
-  if (p->backend != FAWS_BACKEND_GENERIC && pack_gqa(p, &packed)) {
+  if (tc_allowed(p) && pack_gqa(p, &packed)) {
     FwdParams fp = make_fwd(&packed);
     if (tc_fwd_supported(fp, packed.dtype)) p = &packed;
   }
   FwdParams f = make_fwd(p);
-  if (p->backend == FAWS_BACKEND_GENERIC || !tc_fwd_supported(f, p->dtype)) return FAWS_EBACKEND;
+  if (!tc_allowed(p) || !tc_fwd_supported(f, p->dtype)) return FAWS_EBACKEND;
   float* L_part = static_cast<float*>(workspace);
   char* o_part = static_cast<char*>(workspace) + align256((size_t)p->B * p->Hq * n_splits * p->M * 4);
   f.o = o_part;
@@ -398,7 +405,7 @@ int faws_compute_attention_scores(const faws_problem* p, void* scores, int32_t s
   sp.B = p->B; sp.Hq = p->Hq; sp.Hk = p->Hk; sp.M = p->M; sp.N = p->N; sp.D = p->D;
   sp.sm_scale = p->sm_scale;
   bool use_tc = false;
-  if (p->backend != FAWS_BACKEND_GENERIC) use_tc = tc_scores_only_supported(sp, p->dtype);
+  if (tc_allowed(p)) use_tc = tc_scores_only_supported(sp, p->dtype);
   if (p->backend == FAWS_BACKEND_TCGEN05 && !use_tc) return FAWS_EBACKEND;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const cudaError_t e = use_tc ? launch_tc_scores_only(sp, p->dtype, s) : launch_generic_scores_only(sp, p->dtype, s);
@@ -501,7 +508,7 @@ int faws_attention_backward(const faws_problem* p, const faws_grads* g, void* wo
   b.drop = make_drop(p);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   bool use_tc = false;
-  if (p->backend != FAWS_BACKEND_GENERIC) use_tc = tc_bwd_supported(b, p->dtype);
+  if (tc_allowed(p)) use_tc = tc_bwd_supported(b, p->dtype);
   if (p->backend == FAWS_BACKEND_TCGEN05 && !use_tc) return FAWS_EBACKEND;
   // the tcgen05 path has its own pre-pass (delta and L into tile-padded arrays in the workspace)
   if (!use_tc && launch_bwd_delta(b, p->dtype, s) != cudaSuccess) return FAWS_ECUDA;

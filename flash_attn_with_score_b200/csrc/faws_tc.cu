@@ -1030,7 +1030,8 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
         T* orow = reinterpret_cast<T*>(p.o) + b * p.o_sb + ho * p.o_sh + (int64_t)i * p.o_ss;
         const uint4 z = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
-        for (int g = 0; g < D / 8; ++g) *reinterpret_cast<uint4*>(orow + g * 8) = z;
+        for (int g = 0; g < D / 8; ++g)
+          if (g * 8 < p.D) *reinterpret_cast<uint4*>(orow + g * 8) = z;
       }
       if (row_ok) {
         if (p.L != nullptr)
@@ -1610,7 +1611,7 @@ cudaError_t launch_fwd_t(const TcMaps& maps, const FwdParams& p, cudaStream_t s)
 
 bool tc_fwd_supported(const FwdParams& p, int dtype) {
   (void)dtype;
-  if (p.D != 64 && p.D != 128) return false;
+  if (!tc_head_dim(p.D)) return false;
   if (p.drop.p > 0.f && (p.s_scratch != nullptr || (p.scores != nullptr && !p.scores_f32)))
     return false;  // no dropout variant of the scratch and 16-bit-score hooks: CUDA-core kernels
   if (!(p.sm_scale > 0.f)) return false;  // the row max is taken on unscaled scores
@@ -1706,7 +1707,7 @@ bool tc_colsoftmax_group_in_kernel(const ColSoftmaxParams& p) {
 
 bool tc_colsoftmax_supported(const ColSoftmaxParams& p, int dtype) {
   (void)dtype;
-  if (p.D != 64 && p.D != 128) return false;
+  if (!tc_head_dim(p.D)) return false;
   if (p.s_scratch != nullptr) return false;  // the buffered pass reads stored scores, no MMA
   if (p.drop.p > 0.f) return false;
   if (p.m_begin % BM != 0 || !(p.sm_scale > 0.f)) return false;

@@ -490,13 +490,13 @@ cudaError_t launch_bwd_td(const BwdParams& p, cudaStream_t s) {
     void* dv_dst = per_head ? static_cast<void*>(part + part_bytes) : p.dv;
     void* dk_dst = per_head ? static_cast<void*>(part) : p.dk;
     const int64_t ph_ss = p.D, ph_sh = (int64_t)p.N * p.D, ph_sb = (int64_t)p.Hq * p.N * p.D;
-    if (!make_map_bhsd(&m.x, p.k, D, p.N, p.Hk, p.B, p.k_ss, p.k_sh, p.k_sb, 128) ||
-        !make_map_bhsd(&m.y, p.v, D, p.N, p.Hk, p.B, p.v_ss, p.v_sh, p.v_sb, 128) ||
-        !make_map_bhsd(&m.a, p.q, D, p.M, p.Hq, p.B, p.q_ss, p.q_sh, p.q_sb, 128) ||
-        !make_map_bhsd(&m.b, p.dout, D, p.M, p.Hq, p.B, p.do_ss, p.do_sh, p.do_sb, 128) ||
-        !make_map_bhsd(&m.o0, dv_dst, D, p.N, p.Hq, p.B, per_head ? ph_ss : p.dv_ss, per_head ? ph_sh : p.dv_sh,
+    if (!make_map_bhsd(&m.x, p.k, p.D, p.N, p.Hk, p.B, p.k_ss, p.k_sh, p.k_sb, 128) ||
+        !make_map_bhsd(&m.y, p.v, p.D, p.N, p.Hk, p.B, p.v_ss, p.v_sh, p.v_sb, 128) ||
+        !make_map_bhsd(&m.a, p.q, p.D, p.M, p.Hq, p.B, p.q_ss, p.q_sh, p.q_sb, 128) ||
+        !make_map_bhsd(&m.b, p.dout, p.D, p.M, p.Hq, p.B, p.do_ss, p.do_sh, p.do_sb, 128) ||
+        !make_map_bhsd(&m.o0, dv_dst, p.D, p.N, p.Hq, p.B, per_head ? ph_ss : p.dv_ss, per_head ? ph_sh : p.dv_sh,
                        per_head ? ph_sb : p.dv_sb, 32) ||
-        !make_map_bhsd(&m.o1, dk_dst, D, p.N, p.Hq, p.B, per_head ? ph_ss : p.dk_ss, per_head ? ph_sh : p.dk_sh,
+        !make_map_bhsd(&m.o1, dk_dst, p.D, p.N, p.Hq, p.B, per_head ? ph_ss : p.dk_ss, per_head ? ph_sh : p.dk_sh,
                        per_head ? ph_sb : p.dk_sb, 32))
       return cudaErrorInvalidValue;
     dim3 grid(p.Hq, p.B, (p.N + BT - 1) / BT);
@@ -517,11 +517,11 @@ cudaError_t launch_bwd_td(const BwdParams& p, cudaStream_t s) {
   // query-major: dQ
   {
     BwMaps m;
-    if (!make_map_bhsd(&m.x, p.q, D, p.M, p.Hq, p.B, p.q_ss, p.q_sh, p.q_sb, 128) ||
-        !make_map_bhsd(&m.y, p.dout, D, p.M, p.Hq, p.B, p.do_ss, p.do_sh, p.do_sb, 128) ||
-        !make_map_bhsd(&m.a, p.k, D, p.N, p.Hk, p.B, p.k_ss, p.k_sh, p.k_sb, 128) ||
-        !make_map_bhsd(&m.b, p.v, D, p.N, p.Hk, p.B, p.v_ss, p.v_sh, p.v_sb, 128) ||
-        !make_map_bhsd(&m.o0, p.dq, D, p.M, p.Hq, p.B, p.dq_ss, p.dq_sh, p.dq_sb, 32))
+    if (!make_map_bhsd(&m.x, p.q, p.D, p.M, p.Hq, p.B, p.q_ss, p.q_sh, p.q_sb, 128) ||
+        !make_map_bhsd(&m.y, p.dout, p.D, p.M, p.Hq, p.B, p.do_ss, p.do_sh, p.do_sb, 128) ||
+        !make_map_bhsd(&m.a, p.k, p.D, p.N, p.Hk, p.B, p.k_ss, p.k_sh, p.k_sb, 128) ||
+        !make_map_bhsd(&m.b, p.v, p.D, p.N, p.Hk, p.B, p.v_ss, p.v_sh, p.v_sb, 128) ||
+        !make_map_bhsd(&m.o0, p.dq, p.D, p.M, p.Hq, p.B, p.dq_ss, p.dq_sh, p.dq_sb, 32))
       return cudaErrorInvalidValue;
     m.o1 = m.o0;
     dim3 grid(p.Hq, p.B, (p.M + BT - 1) / BT);
@@ -542,7 +542,7 @@ size_t tc_bwd_workspace_bytes(int B, int Hq, int Hk, int M, int N, int D) {
 
 bool tc_bwd_supported(const BwdParams& p, int dtype) {
   (void)dtype;
-  if (p.D != 64 && p.D != 128) return false;
+  if (!tc_head_dim(p.D)) return false;
   if (p.drop.p > 0.f) return false;  // the dropout mask is regenerated by the CUDA-core kernels only
   if (!(p.sm_scale > 0.f)) return false;
   if (!device_is_sm100() || get_encode() == nullptr) return false;

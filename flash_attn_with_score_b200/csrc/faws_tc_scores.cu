@@ -235,7 +235,7 @@ cudaError_t launch_sc_d(const ScMaps& maps, const ScoresOnlyParams& p, cudaStrea
 
 bool tc_scores_only_supported(const ScoresOnlyParams& p, int dtype) {
   (void)dtype;
-  if (p.D != 64 && p.D != 128) return false;
+  if (!tc_head_dim(p.D)) return false;
   if (!device_is_sm100() || get_encode() == nullptr) return false;
   if (!ok16(p.q, p.q_sb, p.q_sh, p.q_ss) || !ok16(p.k, p.k_sb, p.k_sh, p.k_ss)) return false;
   // TMA store rows must start on 16-byte boundaries

@@ -48,6 +48,7 @@ extern "C" {
 
 /* kernel families ("backend" below) */
 #define FAWS_BACKEND_AUTO 0    /* tcgen05 kernels when the problem fits them   */
+                               /* (D 16 and 32 included: padded to 64)         */
 #define FAWS_BACKEND_GENERIC 1 /* CUDA-core kernels: any D in {16,32,64,128},  */
                                /* any alignment                                */
 #define FAWS_BACKEND_TCGEN05 2 /* TMA + tcgen05/TMEM kernels: D in {64,128},   */
