@@ -38,6 +38,7 @@
 #include "faws_internal.cuh"
 #include "faws_tc_host.cuh"
 #include "faws_tc_ptx.cuh"
+#include "faws_tc_store.cuh"
 
 namespace faws {
 namespace {
@@ -142,7 +143,8 @@ __device__ __forceinline__ void warp_column_sums(float (&v)[32], int lane) {
 // Score-tile hook compiled into a kernel instance (one per operator family).
 enum Hook : int {
   kHookNone = 0, kHookScores = 1, kHookRowSum = 2, kHookColPart = 3, kHookScratch = 4,
-  kHookScores16 = 5  // scores in the input dtype (what the reference kernel writes)
+  kHookScores16 = 5,  // scores in the input dtype (what the reference kernel writes)
+  kHookScoresAny = 6  // scores of either type in rows that TMA cannot address (odd lengths): plain stores
 };
 
 // Persistent launches: one CTA per SM walks a list of work items (an item is what one CTA of the
@@ -184,7 +186,8 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
   // block first): measured against interleaving the two kinds, cfg2 runs 2 % faster.
   // The geometry of the work item in hand.  Plain launches have one item per CTA, named by the block
   // index; persistent CTAs (never SPLIT, split-KV or fill launches) set it again for every item.
-  constexpr bool kStoreHook = HOOK == kHookScores || HOOK == kHookScores16 || HOOK == kHookScratch;
+  constexpr bool kStoreHook =
+      HOOK == kHookScores || HOOK == kHookScores16 || HOOK == kHookScoresAny || HOOK == kHookScratch;
   const bool persist = !SPLIT && !kStoreHook && wl.n_items > 0;  // (the launcher keeps the other instances plain)
   bool is_fill;
   int cb_rel, h, b, ksplit, kt0, hk, bh, ho, cb_abs, nt, rr_start;
@@ -275,6 +278,27 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
         }
         tma_store_commit();
         tma_store_wait<0>();
+      }
+      return;
+    }
+  }
+
+  if constexpr (HOOK == kHookScoresAny) {
+    if (is_fill) {  // a warp per row, rows dealt to the 12 warps
+      griddep_wait();
+      griddep_launch_dependents();
+      uint32_t word = p.masked_bits;
+      if (!p.scores_f32) {
+        const T mt = from_float<T>(__uint_as_float(p.masked_bits));
+        word = pack_bits<T>(mt, mt);
+      }
+      const int esize = p.scores_f32 ? 4 : 2;
+      for (int r = warp; r < CTA_ROWS; r += NTHREADS / 32) {
+        const int i = r_tile_of[0] + r, j0 = (r < BM ? nt_q[0] : nt_q[1]) * BN;
+        if (i >= p.m_end || j0 >= p.N) continue;
+        char* dst = static_cast<char*>(p.scores) + (((int64_t)bh * p.M + i) * p.N + j0) * esize;
+        if (p.scores_f32) fill_row_direct<4>(dst, p.N - j0, word, lane);
+        else fill_row_direct<2>(dst, p.N - j0, word, lane);
       }
       return;
     }
@@ -767,6 +791,67 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
           }
         }
       }
+      if constexpr (HOOK == kHookScoresAny) {
+        // Staged as for the TMA stores, then written row by row by the warp itself.  Costs about as many shared-memory
+        // and store instructions as the TMA form's staging; fp32 B1 Hq28 Hk4 S1531 causal: 117 us, 1 180 us on the
+        // CUDA-core kernel that took odd lengths before.
+        const int r0 = r_tile + lg * 32, rows = min(32, p.m_end - r0);
+        const int esize = p.scores_f32 ? 4 : 2;
+        char* dst = static_cast<char*>(p.scores) + (((int64_t)bh * p.M + r0) * p.N + n0) * esize;
+        const int64_t row_bytes = (int64_t)p.N * esize;
+        if (p.scores_f32) {
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            __syncwarp();  // the boxes of the round before have been read
+#pragma unroll
+            for (int c2 = 0; c2 < 2; ++c2) {
+              const int c = half * 2 + c2;
+#pragma unroll
+              for (int cc = 0; cc < 8; ++cc) {
+                float4 val;
+                val.x = FAWS_VIS(c * 32 + cc * 4 + 0) ? __uint_as_float(r[c * 32 + cc * 4 + 0]) * scale : masked_f;
+                val.y = FAWS_VIS(c * 32 + cc * 4 + 1) ? __uint_as_float(r[c * 32 + cc * 4 + 1]) * scale : masked_f;
+                val.z = FAWS_VIS(c * 32 + cc * 4 + 2) ? __uint_as_float(r[c * 32 + cc * 4 + 2]) * scale : masked_f;
+                val.w = FAWS_VIS(c * 32 + cc * 4 + 3) ? __uint_as_float(r[c * 32 + cc * 4 + 3]) * scale : masked_f;
+                *reinterpret_cast<float4*>(stage + c2 * 4096 + lane * 128 + ((cc ^ (lane & 7)) << 4)) = val;
+              }
+            }
+            __syncwarp();
+#pragma unroll
+            for (int c2 = 0; c2 < 2; ++c2) {
+              const int c = half * 2 + c2;
+              store_box_direct<4>(stage + c2 * 4096, dst + c * 128, row_bytes, rows, p.N - n0 - c * 32, lane, true);
+            }
+          }
+        } else {
+          const T masked_t = from_float<T>(masked_f);
+          const uint32_t masked2 = pack_bits<T>(masked_t, masked_t);
+          const bool pairs = p.N % 2 == 0 && (reinterpret_cast<uintptr_t>(p.scores) & 3) == 0;
+          __syncwarp();
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+#pragma unroll
+            for (int cc = 0; cc < 8; ++cc) {
+              uint32_t w[4];
+#pragma unroll
+              for (int e2 = 0; e2 < 4; ++e2) {
+                const int x = half * 64 + cc * 8 + e2 * 2;
+                w[e2] = pack2<T>(__uint_as_float(r[x]) * scale, __uint_as_float(r[x + 1]) * scale);
+                if (kMasked) {
+                  if (x >= nvis) w[e2] = masked2;
+                  else if (x + 1 >= nvis) w[e2] = (w[e2] & 0xffffu) | (masked2 & 0xffff0000u);
+                }
+              }
+              *reinterpret_cast<uint4*>(stage + half * 4096 + lane * 128 + ((cc ^ (lane & 7)) << 4)) =
+                  make_uint4(w[0], w[1], w[2], w[3]);
+            }
+          }
+          __syncwarp();
+#pragma unroll
+          for (int half = 0; half < 2; ++half)
+            store_box_direct<2>(stage + half * 4096, dst + half * 128, row_bytes, rows, p.N - n0 - half * 64, lane, pairs);
+        }
+      }
       if constexpr (store_scores || store_scratch) {
         // Two rounds of two 32-column chunks: both 4 KB staging buffers are rewritten per round,
         // one proxy fence per round, lanes 0 and 1 each issue (and later wait for) one TMA store.
@@ -863,44 +948,6 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
     m_run = FAWS_NEG_INF;
     l_run = 0.f;
     rs_raw = 0.f;
-
-    // Key tiles the causal loop never visits hold only the fill value.  They are written first,
-    // from one constant 32 x 32 tile, so that HBM is busy while the first tiles are computed
-    // (these stores carry 44 % of the bytes of a causal S = N problem).
-    if constexpr (store_scores) if (!p.fill_ctas && r_tile < p.m_end && my_nt * BN < p.N) {
-      const float4 fill = make_float4(masked_f, masked_f, masked_f, masked_f);
-#pragma unroll
-      for (int cc = 0; cc < 8; ++cc) *reinterpret_cast<float4*>(stage + lane * 128 + (cc << 4)) = fill;
-      fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0) {
-        const int r0 = r_tile + lg * 32 - p.m_begin;
-        for (int j0 = my_nt * BN; j0 < p.N; j0 += 32) {
-          // SPLIT: the two warpgroups share the rows, so they take alternate key tiles
-          if (!SPLIT || ((j0 / BN) & 1) == qt) tma_store_3d(&maps.st, stage, j0, r0, bh);
-        }
-        tma_store_commit();
-      }
-      __syncwarp();
-    }
-
-    if constexpr (store_scores16) if (!p.fill_ctas && r_tile < p.m_end && my_nt * BN < p.N) {
-      const T masked_t = from_float<T>(masked_f);
-      const uint32_t m2 = pack_bits<T>(masked_t, masked_t);
-      const uint4 fill = make_uint4(m2, m2, m2, m2);
-#pragma unroll
-      for (int cc = 0; cc < 8; ++cc) *reinterpret_cast<uint4*>(stage + lane * 128 + (cc << 4)) = fill;
-      fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0) {
-        const int r0 = r_tile + lg * 32 - p.m_begin;
-        for (int j0 = my_nt * BN; j0 < p.N; j0 += 64) {
-          if (!SPLIT || ((j0 / BN) & 1) == qt) tma_store_3d(&maps.st, stage, j0, r0, bh);
-        }
-        tma_store_commit();
-      }
-      __syncwarp();
-    }
 
     {
       int cnt = 0;
@@ -1525,7 +1572,8 @@ cudaError_t launch_fwd_s(const TcMaps& maps, const FwdParams& p, cudaStream_t s)
   const long long kv_bytes = 2LL * p.B * p.Hk * p.N * p.D * 2;
   pp.lpt_order = (p.causal && kv_bytes <= (48LL << 20) && 2 * ncb <= 65535) ? 1 : 0;
   // masked key tiles exist (causal, some row block ends before N): give them their own CTAs
-  pp.fill_ctas = ((HOOK == kHookScores || HOOK == kHookScores16) && p.causal && p.p_seq + p.m_begin + 128 < p.N) ? 1 : 0;
+  pp.fill_ctas = ((HOOK == kHookScores || HOOK == kHookScores16 || HOOK == kHookScoresAny) && p.causal &&
+                   p.p_seq + std::min(p.m_begin + BM, p.m_end) < p.N) ? 1 : 0;
   const int nslots = pp.fill_ctas ? 2 * ncb : ncb;
   // the causal round-robin walk (down from the CTA's last key tile) is the reverse order: take its cheaper index form
   if (pp.schedule == kRoundRobin && pp.causal) pp.schedule = kReverse;
@@ -1599,6 +1647,8 @@ cudaError_t launch_fwd_h(const TcMaps& maps, const FwdParams& p, cudaStream_t s)
 
 template <typename T, int D>
 cudaError_t launch_fwd_t(const TcMaps& maps, const FwdParams& p, cudaStream_t s) {
+  if (p.scores != nullptr && !tma_score_rows(p.scores, p.N, p.scores_f32 ? 4 : 2))
+    return launch_fwd_s<T, D, kHookScoresAny, false>(maps, p, s);
   if (p.scores != nullptr)
     return p.scores_f32 ? launch_fwd_h<T, D, kHookScores>(maps, p, s) : launch_fwd_h<T, D, kHookScores16>(maps, p, s);
   if (p.row_sum != nullptr) return launch_fwd_h<T, D, kHookRowSum>(maps, p, s);
@@ -1620,8 +1670,9 @@ bool tc_fwd_supported(const FwdParams& p, int dtype) {
   if (!ok16(p.q, p.q_sb, p.q_sh, p.q_ss) || !ok16(p.k, p.k_sb, p.k_sh, p.k_ss) ||
       !ok16(p.v, p.v_sb, p.v_sh, p.v_ss) || !ok16(p.o, p.o_sb, p.o_sh, p.o_ss))
     return false;
-  if (p.scores != nullptr) {  // TMA store rows must start on 16-byte boundaries
-    if (p.N % (p.scores_f32 ? 4 : 8) != 0 || reinterpret_cast<uintptr_t>(p.scores) % 16 != 0) return false;
+  if (p.scores != nullptr && !tma_score_rows(p.scores, p.N, p.scores_f32 ? 4 : 2)) {
+    if (p.drop.p > 0.f) return false;  // the plain-store hook has no dropout variant
+    if (reinterpret_cast<uintptr_t>(p.scores) % (p.scores_f32 ? 4 : 2) != 0) return false;
   }
   if (p.s_scratch != nullptr) {
     if (p.scores != nullptr) return false;
@@ -1643,7 +1694,7 @@ cudaError_t launch_tc_fwd(const FwdParams& p, int dtype, cudaStream_t s) {
   const int o_heads = p.Hq * (p.n_splits > 1 ? p.n_splits : 1);
   if (!make_map_bhsd(&maps.o, obase, p.D, q_rows, o_heads, p.B, p.o_ss, p.o_sh, p.o_sb, 32)) return cudaErrorInvalidValue;
   maps.st = maps.q;
-  if (p.scores != nullptr) {
+  if (p.scores != nullptr && tma_score_rows(p.scores, p.N, p.scores_f32 ? 4 : 2)) {
     const int esize = p.scores_f32 ? 4 : 2;
     char* base = static_cast<char*>(p.scores) + (int64_t)p.m_begin * p.N * esize;
     if (!make_map_store_f32(&maps.st, base, p.N, q_rows, p.N, (int64_t)p.M * p.N, p.B * p.Hq, esize))

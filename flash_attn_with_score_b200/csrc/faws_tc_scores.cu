@@ -16,6 +16,7 @@
 #include "faws_internal.cuh"
 #include "faws_tc_host.cuh"
 #include "faws_tc_ptx.cuh"
+#include "faws_tc_store.cuh"
 
 namespace faws {
 namespace {
@@ -53,6 +54,7 @@ struct ScMaps {
 struct ScParams {
   int M, N, Hq, G;
   float sm_scale;
+  char* scores;  // !TMA_OUT: rows that TMA cannot address (odd lengths) are written with plain stores
 };
 
 template <typename T> __device__ __forceinline__ uint32_t pack2(float a, float b);
@@ -65,7 +67,7 @@ template <> __device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float a, fl
   return *reinterpret_cast<uint32_t*>(&h);
 }
 
-template <typename T, int D, bool F32OUT>
+template <typename T, int D, bool F32OUT, bool TMA_OUT>
 __global__ void __launch_bounds__(NTHREADS, 1)
 tc_qk_scores_kernel(const __grid_constant__ ScMaps maps, const ScParams p, int* __restrict__ status) {
   using L = ScSmem<D>;
@@ -169,7 +171,7 @@ tc_qk_scores_kernel(const __grid_constant__ ScMaps maps, const ScParams p, int* 
           mbar_arrive(&bars->s_free[e]);
         }
         unsigned char* sb = stage + (nstaged & 1) * 4096;
-        if (lane == 0) tma_store_wait_read<1>();  // the store that last read this buffer has fetched it
+        if (TMA_OUT && lane == 0) tma_store_wait_read<1>();  // the store that last read this buffer has fetched it
         __syncwarp();
 #pragma unroll
         for (int cc = 0; cc < 8; ++cc) {
@@ -187,11 +189,20 @@ tc_qk_scores_kernel(const __grid_constant__ ScMaps maps, const ScParams p, int* 
           }
           *reinterpret_cast<uint4*>(sb + lane * 128 + ((cc ^ (lane & 7)) << 4)) = w;
         }
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) {
-          tma_store_3d(&maps.st, sb, n0 + c0, m0 + lg * 32, bh);
-          tma_store_commit();
+        if constexpr (TMA_OUT) {
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            tma_store_3d(&maps.st, sb, n0 + c0, m0 + lg * 32, bh);
+            tma_store_commit();
+          }
+        } else {
+          constexpr int kEsize = F32OUT ? 4 : 2;
+          __syncwarp();
+          const int r0 = m0 + lg * 32;
+          store_box_direct<kEsize>(sb, p.scores + (((int64_t)bh * p.M + r0) * p.N + n0 + c0) * kEsize, (int64_t)p.N * kEsize,
+                                   min(32, p.M - r0), p.N - n0 - c0, lane,
+                                   p.N % 2 == 0 && (reinterpret_cast<uintptr_t>(p.scores) & 3) == 0);
         }
         ++nstaged;
       }
@@ -213,22 +224,24 @@ tc_qk_scores_kernel(const __grid_constant__ ScMaps maps, const ScParams p, int* 
   }
 }
 
-template <typename T, int D, bool F32OUT>
+template <typename T, int D, bool F32OUT, bool TMA_OUT>
 cudaError_t launch_sc(const ScMaps& maps, const ScoresOnlyParams& p, cudaStream_t s) {
   using L = ScSmem<D>;
   static PerDeviceOnce attr_once;
-  if (cudaError_t e = set_max_smem_once(attr_once, tc_qk_scores_kernel<T, D, F32OUT>, L::alloc); e != cudaSuccess)
+  if (cudaError_t e = set_max_smem_once(attr_once, tc_qk_scores_kernel<T, D, F32OUT, TMA_OUT>, L::alloc); e != cudaSuccess)
     return e;
-  ScParams sp{p.M, p.N, p.Hq, p.Hq / p.Hk, p.sm_scale};
+  ScParams sp{p.M, p.N, p.Hq, p.Hq / p.Hk, p.sm_scale, static_cast<char*>(p.scores)};
   dim3 grid((p.M + BM - 1) / BM, p.Hq, p.B);
-  tc_qk_scores_kernel<T, D, F32OUT><<<grid, NTHREADS, L::alloc, s>>>(maps, sp, tc_status_word());
+  tc_qk_scores_kernel<T, D, F32OUT, TMA_OUT><<<grid, NTHREADS, L::alloc, s>>>(maps, sp, tc_status_word());
   count_launch();
   return cudaGetLastError();
 }
 
 template <typename T, int D>
 cudaError_t launch_sc_d(const ScMaps& maps, const ScoresOnlyParams& p, cudaStream_t s) {
-  return p.scores_f32 ? launch_sc<T, D, true>(maps, p, s) : launch_sc<T, D, false>(maps, p, s);
+  if (tma_score_rows(p.scores, p.N, p.scores_f32 ? 4 : 2))
+    return p.scores_f32 ? launch_sc<T, D, true, true>(maps, p, s) : launch_sc<T, D, false, true>(maps, p, s);
+  return p.scores_f32 ? launch_sc<T, D, true, false>(maps, p, s) : launch_sc<T, D, false, false>(maps, p, s);
 }
 
 }  // namespace
@@ -238,17 +251,16 @@ bool tc_scores_only_supported(const ScoresOnlyParams& p, int dtype) {
   if (!tc_head_dim(p.D)) return false;
   if (!device_is_sm100() || get_encode() == nullptr) return false;
   if (!ok16(p.q, p.q_sb, p.q_sh, p.q_ss) || !ok16(p.k, p.k_sb, p.k_sh, p.k_ss)) return false;
-  // TMA store rows must start on 16-byte boundaries
-  if (p.N % (p.scores_f32 ? 4 : 8) != 0 || reinterpret_cast<uintptr_t>(p.scores) % 16 != 0) return false;
-  return true;
+  return reinterpret_cast<uintptr_t>(p.scores) % (p.scores_f32 ? 4 : 2) == 0;
 }
 
 cudaError_t launch_tc_scores_only(const ScoresOnlyParams& p, int dtype, cudaStream_t s) {
-  ScMaps maps;
+  ScMaps maps{};
   const int esize = p.scores_f32 ? 4 : 2;
   if (!make_map_bhsd(&maps.q, p.q, p.D, p.M, p.Hq, p.B, p.q_ss, p.q_sh, p.q_sb, 128) ||
       !make_map_bhsd(&maps.k, p.k, p.D, p.N, p.Hk, p.B, p.k_ss, p.k_sh, p.k_sb, 128) ||
-      !make_map_store_f32(&maps.st, p.scores, p.N, p.M, p.N, (int64_t)p.M * p.N, p.B * p.Hq, esize))
+      (tma_score_rows(p.scores, p.N, esize) &&
+       !make_map_store_f32(&maps.st, p.scores, p.N, p.M, p.N, (int64_t)p.M * p.N, p.B * p.Hq, esize)))
     return cudaErrorInvalidValue;
   if (dtype == FAWS_FP16)
     return p.D == 128 ? launch_sc_d<__half, 128>(maps, p, s) : launch_sc_d<__half, 64>(maps, p, s);
