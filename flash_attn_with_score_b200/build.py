@@ -22,7 +22,6 @@ LIB = os.path.join(HERE, "libfaws.so")
 SOURCES = ["faws_abi.cu", "faws_generic.cu", "faws_tc.cu", "faws_tc_scores.cu", "faws_bwd.cu", "faws_tc_bwd.cu", "faws_noalloc.cu"]
 HEADERS = ["faws_internal.cuh", "faws_tc_ptx.cuh", "faws_tc_host.cuh", "faws_tc_store.cuh"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-SPLIT = ["-split-compile", "0"]  # the instances of one translation unit are compiled on all cores
 
 
 def _nvcc() -> str:
@@ -69,7 +68,7 @@ def _compile(src: str, force: bool, verbose: bool) -> tuple[str, int, str]:
     digest = _digest([path] + _deps(), " ".join(ARCH))
     if not force and os.path.exists(obj) and _read(obj + ".digest") == digest:
         return obj, 0, ""
-    cmd = [_nvcc(), "-c", "-Xcompiler", "-fPIC", "-O3", "-std=c++17", "-lineinfo"] + ARCH + SPLIT + [
+    cmd = [_nvcc(), "-c", "-Xcompiler", "-fPIC", "-O3", "-std=c++17", "-lineinfo"] + ARCH + [
         "-I", os.path.join(ROOT, "include"), "-I", CSRC, "-o", obj, path]
     if verbose:
         cmd[1:1] = ["-Xptxas", "-v"]
