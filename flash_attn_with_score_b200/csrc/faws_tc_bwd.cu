@@ -23,8 +23,8 @@
 // MMA-issuing lane, warps 4-7 / 8-11 consumers of half 0 / 1 (thread = owned row = TMEM lane).
 // Deterministic: every output element is written once, by one CTA, in a fixed order; with GQA the
 // key-major kernel writes per-query-head dK / dV and a second kernel adds the G heads in order.
-// Out-of-range rows need no predicates: TMA zero-fills the loads (a zero Q / dout / K / V row
-// contributes nothing to any accumulator) and clips the stores.  Every mbarrier wait is bounded.
+// Out-of-range query rows need no predicates: TMA zero-fills the loads (with L = delta = 0 their P is 1 and
+// their dS is 0, and the zero Q / dout row contributes nothing); stores are clipped.  Every mbarrier wait is bounded.
 #include <cuda.h>
 
 #include <type_traits>
@@ -297,11 +297,11 @@ tc_bwd_kernel(const __grid_constant__ BwMaps maps, const BwTcParams p, int* __re
       // causal: (query i, key j) is visible iff j <= i + p_seq.  Column x of the half is streamed row
       // str0 + x.  Key-major (own = j, streamed = i): visible iff x >= own - p_seq - str0.
       // Query-major (own = i, streamed = j): visible iff x <= own + p_seq - str0.
+      // Keys beyond N are masked too (query-major): their scores of zero against a very negative L would make
+      // P infinite, and infinity times the zero K row is not zero.
       int x_lo = 0, x_hi = HALF - 1;
-      if (p.causal) {
-        if (KM) x_lo = own - p.p_seq - str0;
-        else x_hi = own + p.p_seq - str0;
-      }
+      if (p.causal && KM) x_lo = own - p.p_seq - str0;
+      if (!KM) x_hi = min(p.N - 1, p.causal ? own + p.p_seq : p.N - 1) - str0;
       const float* vl = reinterpret_cast<const float*>(smem + L::vec_off + (u % NSTAGE) * 1024) + e * HALF;
       const float* vd = vl + 128;
       uint32_t pk[HALF / 2], dk[HALF / 2];

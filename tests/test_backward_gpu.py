@@ -91,6 +91,22 @@ def test_backward_with_dropout_matches_masked_oracle():
     _check((dq, dk, dv), ref, "dropout", False, tuple(x / (1.0 - p_drop) for x in sl))
 
 
+@pytest.mark.parametrize("D", [32, 64])
+@pytest.mark.parametrize("causal", [True, False], ids=["causal", "full"])
+def test_backward_with_very_negative_scores_and_a_ragged_last_key_tile(D, causal):
+    """Every score near -200: exp(0 - L) of the missing keys of the last tile is infinite and must not be used."""
+    g = torch.Generator().manual_seed(11)
+    M, N = 150, 130 if not causal else 150
+    c = (200.0 / D ** 0.5) ** 0.5
+    q = (c + 0.02 * torch.randn(1, 2, M, D, generator=g)).half()
+    k = (-c + 0.02 * torch.randn(1, 2, N, D, generator=g)).half()
+    v, do = (torch.randn(1, 2, n, D, generator=g).half() for n in (N, M))
+    ref = orc.attention_backward(q, k, v, do, causal, p_seq=N - M)
+    out, dq, dk, dv = _run(q, k, v, do, causal)
+    assert F.last_backend() == "tcgen05"
+    _check((dq, dk, dv), ref, "negative scores", False, orc.grad_slack(q, k, v, do, causal, p_seq=N - M))
+
+
 def test_backward_is_deterministic_and_frees_the_caller_from_L():
     q, k, v, do = _inputs((1, 4, 2, 320, 320, 64), torch.float16, seed=9)
     a = _run(q, k, v, do, True)
