@@ -38,6 +38,7 @@ DropoutParams make_drop(const faws_problem* p) {
     d.seed_lo = static_cast<uint32_t>(p->philox_seed);
     d.seed_hi = static_cast<uint32_t>(p->philox_seed >> 32);
     d.offset = static_cast<uint32_t>(p->philox_offset);
+    drop_threshold(&d);
   }
   return d;
 }
@@ -528,7 +529,7 @@ size_t faws_workspace_bytes(int32_t op, const faws_problem* p, int32_t split) {
       if (split < 1 || split > cdiv(p->N, kTcBlockN)) return 0;
       return split == 1 ? 0 : split_kv_bytes(p, split);
     case FAWS_OP_ATTENTION_BACKWARD:  // enough for either kernel family
-      return tc_bwd_workspace_bytes(p->B, p->Hq, p->Hk, p->M, p->N, p->D);
+      return tc_bwd_workspace_bytes(p->B, p->Hq, p->Hk, p->M, p->N, p->D, p->dropout_p > 0.f);
     case FAWS_OP_COL_SUM:
     case FAWS_OP_COL_SUM_SEQUENTIAL:
       return align256(partial_floats(p, 0, p->N) * 4) + align256(qsum_floats(p) * 4);

@@ -20,31 +20,46 @@ struct DropoutParams {
   float out_scale;    // multiplies out when p > 0
   uint32_t seed_lo, seed_hi;
   uint32_t offset;
+  uint32_t drop_lo;    // an entry is dropped iff (uint32)(x + drop_lo) <= drop_span, x its Philox word
+  uint32_t drop_span;  // (set by drop_threshold)
 };
 
+// The generator the reference kernels draw their masks from (flash.py:465) maps a Philox word x to [0, 1) as
+// u(x) = float(x < 0 ? ~x : x) * 2^-31 (sign-folded int32, rounded to fp32; triton's tl.rand) and keeps the entry iff
+// u > p.  u does not fall as the folded value grows, so the folded values that are dropped are 0 .. t - 1 with one t
+// per p, i.e. the words x in [-t, t - 1]: two integer instructions per entry instead of a conversion, which shares
+// its pipe with the exponentials, a multiplication and a comparison.
+constexpr float kPhiloxUnit = 4.6566127342e-10f;
+inline void drop_threshold(DropoutParams* d) {
+  uint32_t lo = 0, hi = 0x7fffffffu;  // folded value 0 gives u = 0, which is never > p; find the last dropped one
+  while (lo < hi) {
+    const uint32_t mid = lo + (hi - lo + 1) / 2;
+    const float u = static_cast<float>(static_cast<int32_t>(mid)) * kPhiloxUnit;
+    if (u > d->p) hi = mid - 1;
+    else lo = mid;
+  }
+  d->drop_lo = lo + 1;
+  d->drop_span = 2 * lo + 1;
+}
+
 #ifdef __CUDACC__
-// First output of Philox-4x32 with six rounds for counter (c, 0, 0, 0) and key (seed_lo, seed_hi),
-// mapped to [0, 1) the way triton's tl.rand does (sign-folded int32 times 2^-31 rounded to fp32):
-// the generator the reference kernels draw dropout masks from (flash.py:465).
-__device__ __forceinline__ float philox6_uniform(uint32_t c, uint32_t k0, uint32_t k1) {
+// First output of Philox-4x32 with six rounds for counter (c, 0, 0, 0) and key (k0, k1).
+__device__ __forceinline__ uint32_t philox6_word(uint32_t c, uint32_t k0, uint32_t k1) {
   uint32_t c0 = c, c1 = 0u, c2 = 0u, c3 = 0u;
 #pragma unroll
   for (int r = 0; r < 6; ++r) {
-    const uint32_t hb = __umulhi(0xCD9E8D57u, c2), lb = 0xCD9E8D57u * c2;
-    const uint32_t ha = __umulhi(0xD2511F53u, c0), la = 0xD2511F53u * c0;
-    c0 = hb ^ c1 ^ k0;
-    c2 = ha ^ c3 ^ k1;
-    c1 = lb;
-    c3 = la;
+    const uint64_t b = (uint64_t)0xCD9E8D57u * c2, a = (uint64_t)0xD2511F53u * c0;
+    c0 = (uint32_t)(b >> 32) ^ c1 ^ k0;
+    c2 = (uint32_t)(a >> 32) ^ c3 ^ k1;
+    c1 = (uint32_t)b;
+    c3 = (uint32_t)a;
     k0 += 0x9E3779B9u;
     k1 += 0xBB67AE85u;
   }
-  int x = static_cast<int>(c0);
-  x = x < 0 ? ~x : x;
-  return __int2float_rn(x) * 4.6566127342e-10f;
+  return c0;
 }
 __device__ __forceinline__ bool dropout_keep(const DropoutParams& d, uint32_t linear_index) {
-  return philox6_uniform(d.offset + linear_index, d.seed_lo, d.seed_hi) > d.p;
+  return philox6_word(d.offset + linear_index, d.seed_lo, d.seed_hi) + d.drop_lo > d.drop_span;
 }
 #endif
 
@@ -207,7 +222,7 @@ cudaError_t launch_tc_colsoftmax(const ColSoftmaxParams& p, int dtype, int group
 
 bool tc_bwd_supported(const BwdParams& p, int dtype);
 cudaError_t launch_tc_bwd(const BwdParams& p, int dtype, cudaStream_t s);  // p.delta = the workspace base
-size_t tc_bwd_workspace_bytes(int B, int Hq, int Hk, int M, int N, int D);
+size_t tc_bwd_workspace_bytes(int B, int Hq, int Hk, int M, int N, int D, bool dropout);
 
 int tc_read_status(int reset);  // synchronising read of the device status word
 cudaError_t launch_wait_give_up(cudaStream_t s);  // self-test: a bounded wait that runs out

@@ -91,6 +91,33 @@ def test_backward_with_dropout_matches_masked_oracle():
     _check((dq, dk, dv), ref, "dropout", False, tuple(x / (1.0 - p_drop) for x in sl))
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16], ids=["fp16", "bf16"])
+@pytest.mark.parametrize("shape,causal,p_drop,philox", [
+    ((2, 2, 2, 128, 128, 64), False, 0.1, (7, 0)),
+    ((1, 6, 2, 300, 300, 128), True, 0.3, ((3 << 32) | 5, 2 ** 31 - 70000)),  # linear index passes 2**31
+    ((1, 4, 1, 129, 257, 32), True, 0.5, (99, 4)),
+    ((2, 3, 3, 257, 130, 16), False, 0.9, (2 ** 63 - 1, 0)),
+    ((1, 4, 2, 1, 200, 64), True, 0.2, (5, 8)),
+    ((1, 4, 2, 260, 260, 32), True, 0.0, None),
+], ids=lambda x: "x".join(map(str, x)) if isinstance(x, tuple) else str(x))
+def test_backward_fine_modes(shape, causal, p_drop, philox, dtype):
+    """Dropout and small head dims on the tcgen05 kernels: dS in two 16-bit parts, so that nothing is further from
+    the oracle than on the CUDA-core kernels, which hold dS in fp32 (2 % for the order of the sums)."""
+    B, Hq, Hk, M, N, D = shape
+    bf16 = dtype == torch.bfloat16
+    q, k, v, do = _inputs(shape, dtype, seed=M + D)
+    keep = orc.dropout_keep_mask(*philox, B, Hq, M, N, p_drop) if p_drop else None
+    ref = orc.attention_backward(q, k, v, do, causal, p_seq=N - M, keep=keep, dropout_p=p_drop)
+    runs = {be: _run(q, k, v, do, causal, dropout_p=p_drop, philox=philox, backend=be)[1:] for be in ("generic", "auto")}
+    assert F.last_backend() == "tcgen05"
+    sl = tuple(x / (1.0 - p_drop) for x in orc.grad_slack(q, k, v, do, causal, p_seq=N - M, bf16=bf16))
+    _check(runs["auto"], ref, "fine", bf16, sl)
+    for name, x, y, r in zip(("dq", "dk", "dv"), runs["auto"], runs["generic"], ref):
+        ex, ey = ((t.double().cpu() - r.double()).norm() for t in (x, y))
+        assert ex <= 1.02 * ey + 1e-6 * r.double().norm(), (name, ex.item(), ey.item())
+    assert F.device_status() == 0
+
+
 @pytest.mark.parametrize("D", [32, 64])
 @pytest.mark.parametrize("causal", [True, False], ids=["causal", "full"])
 def test_backward_with_very_negative_scores_and_a_ragged_last_key_tile(D, causal):
