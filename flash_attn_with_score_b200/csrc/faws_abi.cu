@@ -216,6 +216,17 @@ SoftmaxWs carve_softmax_ws(const faws_problem* p, void* ws, int n_end, int split
   return w;
 }
 
+// Whether the buffered cross-token operator runs without its score buffer, as the second q.k^T of the two-pass
+// operator: whenever both passes fit the tcgen05 kernels, which contract the cross region faster than they could
+// write and read its scores.  fp16 D128 causal, B1 H32 S2048 split 768: 73 us against 100; B1 H32 S4096 split 2048:
+// 176 against 354; full B1 H8 S8192 split 4096: 333 against 440; B1 H32 S512 split 256: 18.3 against 20.1; split not a
+// multiple of 32 (a buffer that TMA could not write; B1 H32 S1024 split 400, full): 41 against 899.  The buffer stays
+// for the CUDA-core kernels, where the second q.k^T is the dearer one.
+bool buffered_recomputes(const faws_problem* p, int split) {
+  if (!tc_allowed(p) || p->v.ptr == nullptr || p->out.ptr == nullptr) return false;
+  return tc_fwd_supported(make_fwd(p), p->dtype) && tc_colsoftmax_supported(make_cs(p, nullptr, nullptr, split, split), p->dtype);
+}
+
 // Softmax-normalised column-type sums: forward pass (out, L[, score scratch]) then the
 // key-major pass and, unless per-q-head output was asked for, the group sum.
 int softmax_col_sums(const faws_problem* p, float* sum_out, int per_q_head, void* ws, size_t ws_bytes,
@@ -469,8 +480,14 @@ int faws_attention_cross_token_softmax_sum_buffered(const faws_problem* p, int32
                                                     void* workspace, size_t workspace_bytes,
                                                     void* stream) {
   if (p == nullptr || split <= 0 || split > p->N) return FAWS_EINVAL;
+  const int st = validate(p);
+  if (st != FAWS_OK) return st;
+  // a caller that forces the family gets it for the splits and options that its score buffer could serve
+  if (p->backend == FAWS_BACKEND_TCGEN05 && p->M > split && (split % 32 != 0 || p->dropout_p > 0.f))
+    return FAWS_EBACKEND;
+  const bool recompute = buffered_recomputes(p, split);
   return softmax_col_sums(p, sum_out, per_q_head, workspace, workspace_bytes, stream, split, split,
-                          split, kForward);
+                          recompute ? 0 : split, recompute ? kRoundRobin : kForward);
 }
 
 int faws_total_attention(const faws_problem* p, float* total, void* stream) {
@@ -543,7 +560,7 @@ size_t faws_workspace_bytes(int32_t op, const faws_problem* p, int32_t split) {
       return carve_softmax_ws(p, nullptr, split, 0).total;
     case FAWS_OP_CROSS_SOFTMAX_SUM_BUFFERED:
       if (split <= 0 || split > p->N) return 0;
-      return carve_softmax_ws(p, nullptr, split, split).total;
+      return carve_softmax_ws(p, nullptr, split, buffered_recomputes(p, split) ? 0 : split).total;
     default:
       return 0;
   }

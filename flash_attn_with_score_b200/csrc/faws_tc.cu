@@ -20,7 +20,6 @@
 //   row sum     per-thread running sum
 //   column sum  per-warp transpose-reduce with shuffles, 4 warps combined through smem,
 //               one partial row per 128-row query tile (summed later in fixed order)
-//   scratch     the cross region's scores (buffered cross-token variant) via TMA stores
 //
 // Every mbarrier wait is bounded (about 2 s); on give-up the CTA raises a flag in
 // *status, lets in-flight copies drain, frees its TMEM and returns.
@@ -65,7 +64,7 @@ constexpr float kRescaleThreshold = 8.0f;  // log2 units
 
 struct TcMaps {
   CUtensorMap q, k, v, o;  // o: 32-row store boxes of the output
-  CUtensorMap st;          // scores (or score-scratch) store map
+  CUtensorMap st;          // scores store map
 };
 
 // SPLIT = false: the CTA owns two query tiles (256 rows), one per softmax warpgroup.
@@ -142,9 +141,9 @@ __device__ __forceinline__ void warp_column_sums(float (&v)[32], int lane) {
 
 // Score-tile hook compiled into a kernel instance (one per operator family).
 enum Hook : int {
-  kHookNone = 0, kHookScores = 1, kHookRowSum = 2, kHookColPart = 3, kHookScratch = 4,
-  kHookScores16 = 5,  // scores in the input dtype (what the reference kernel writes)
-  kHookScoresAny = 6  // scores of either type in rows that TMA cannot address (odd lengths): plain stores
+  kHookNone = 0, kHookScores = 1, kHookRowSum = 2, kHookColPart = 3,
+  kHookScores16 = 4,  // scores in the input dtype (what the reference kernel writes)
+  kHookScoresAny = 5  // scores of either type in rows that TMA cannot address (odd lengths): plain stores
 };
 
 // Persistent launches: one CTA per SM walks a list of work items (an item is what one CTA of the
@@ -187,7 +186,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
   // The geometry of the work item in hand.  Plain launches have one item per CTA, named by the block
   // index; persistent CTAs (never SPLIT, split-KV or fill launches) set it again for every item.
   constexpr bool kStoreHook =
-      HOOK == kHookScores || HOOK == kHookScores16 || HOOK == kHookScoresAny || HOOK == kHookScratch;
+      HOOK == kHookScores || HOOK == kHookScores16 || HOOK == kHookScoresAny;
   const bool persist = !SPLIT && !kStoreHook && wl.n_items > 0;  // (the launcher keeps the other instances plain)
   bool is_fill;
   int cb_rel, h, b, ksplit, kt0, hk, bh, ho, cb_abs, nt, rr_start;
@@ -333,7 +332,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
     prefetch_tmap(&maps.k);
     prefetch_tmap(&maps.v);
     prefetch_tmap(&maps.o);
-    if constexpr (HOOK == kHookScores || HOOK == kHookScores16 || HOOK == kHookScratch) prefetch_tmap(&maps.st);
+    if constexpr (HOOK == kHookScores || HOOK == kHookScores16) prefetch_tmap(&maps.st);
   }
   if (threadIdx.x == 0) {
     mbar_init(&bars->q_full, 1);
@@ -618,7 +617,6 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
     float* colbuf = reinterpret_cast<float*>(smem + L::stage_off + qt * 32768);  // [2][4][128], col hook only
     constexpr bool store_scores = HOOK == kHookScores;
     constexpr bool store_scores16 = HOOK == kHookScores16;
-    constexpr bool store_scratch = HOOK == kHookScratch;
     const float masked_f = __uint_as_float(p.masked_bits);
     // per item
     int r_tile, i, my_nt, qb128;  // first row of the query tile, this thread's row, end of its key-tile range
@@ -852,47 +850,39 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
             store_box_direct<2>(stage + half * 4096, dst + half * 128, row_bytes, rows, p.N - n0 - half * 64, lane, pairs);
         }
       }
-      if constexpr (store_scores || store_scratch) {
+      if constexpr (store_scores) {
         // Two rounds of two 32-column chunks: both 4 KB staging buffers are rewritten per round,
         // one proxy fence per round, lanes 0 and 1 each issue (and later wait for) one TMA store.
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
-          const bool rows_in = store_scores || (r_tile + lg * 32 >= p.split);
-          const bool round_on = rows_in && (store_scores || n0 + half * 64 < p.split);
-          if (round_on) {
-            if (lane < 2) tma_store_wait_read<0>();
-            __syncwarp();
+          if (lane < 2) tma_store_wait_read<0>();
+          __syncwarp();
 #pragma unroll
-            for (int c2 = 0; c2 < 2; ++c2) {
-              const int c = half * 2 + c2;
-              unsigned char* sb = stage + c2 * 4096;
+          for (int c2 = 0; c2 < 2; ++c2) {
+            const int c = half * 2 + c2;
+            unsigned char* sb = stage + c2 * 4096;
 #pragma unroll
-              for (int cc = 0; cc < 8; ++cc) {
-                float4 val;
-                val.x = __uint_as_float(r[c * 32 + cc * 4 + 0]) * scale;
-                val.y = __uint_as_float(r[c * 32 + cc * 4 + 1]) * scale;
-                val.z = __uint_as_float(r[c * 32 + cc * 4 + 2]) * scale;
-                val.w = __uint_as_float(r[c * 32 + cc * 4 + 3]) * scale;
-                if (kMasked && store_scores) {
-                  if (!(c * 32 + cc * 4 + 0 < nvis)) val.x = masked_f;
-                  if (!(c * 32 + cc * 4 + 1 < nvis)) val.y = masked_f;
-                  if (!(c * 32 + cc * 4 + 2 < nvis)) val.z = masked_f;
-                  if (!(c * 32 + cc * 4 + 3 < nvis)) val.w = masked_f;
-                }
-                *reinterpret_cast<float4*>(sb + lane * 128 + ((cc ^ (lane & 7)) << 4)) = val;
+            for (int cc = 0; cc < 8; ++cc) {
+              float4 val;
+              val.x = __uint_as_float(r[c * 32 + cc * 4 + 0]) * scale;
+              val.y = __uint_as_float(r[c * 32 + cc * 4 + 1]) * scale;
+              val.z = __uint_as_float(r[c * 32 + cc * 4 + 2]) * scale;
+              val.w = __uint_as_float(r[c * 32 + cc * 4 + 3]) * scale;
+              if (kMasked) {
+                if (!(c * 32 + cc * 4 + 0 < nvis)) val.x = masked_f;
+                if (!(c * 32 + cc * 4 + 1 < nvis)) val.y = masked_f;
+                if (!(c * 32 + cc * 4 + 2 < nvis)) val.z = masked_f;
+                if (!(c * 32 + cc * 4 + 3 < nvis)) val.w = masked_f;
               }
+              *reinterpret_cast<float4*>(sb + lane * 128 + ((cc ^ (lane & 7)) << 4)) = val;
             }
-            fence_proxy_async_smem();
-            __syncwarp();
-            if (lane < 2) {
-              const int jb = n0 + (half * 2 + lane) * 32;
-              if (store_scores) {
-                tma_store_3d(&maps.st, stage + lane * 4096, jb, r_tile + lg * 32 - p.m_begin, bh);
-              } else if (jb < p.split) {
-                tma_store_3d(&maps.st, stage + lane * 4096, jb, r_tile + lg * 32 - p.split, bh);
-              }
-              tma_store_commit();
-            }
+          }
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane < 2) {
+            const int jb = n0 + (half * 2 + lane) * 32;
+            tma_store_3d(&maps.st, stage + lane * 4096, jb, r_tile + lg * 32 - p.m_begin, bh);
+            tma_store_commit();
           }
         }
       }
@@ -1635,7 +1625,7 @@ template <typename T, int D, int HOOK>
 cudaError_t launch_fwd_h(const TcMaps& maps, const FwdParams& p, cudaStream_t s) {
   // Score-materialising causal launches are bound by their stores, not by the chain of key
   // tiles: measured, the 256-row CTAs (half as many set-ups) are faster there.
-  if constexpr (HOOK != kHookScores16 && HOOK != kHookScratch) {
+  if constexpr (HOOK != kHookScores16) {
     // dropout: 256-row CTAs only (the mask generation, not the chain of key tiles, bounds it)
     if (p.drop.p > 0.f) return launch_fwd_s<T, D, HOOK, false, true>(maps, p, s);
   }
@@ -1653,7 +1643,6 @@ cudaError_t launch_fwd_t(const TcMaps& maps, const FwdParams& p, cudaStream_t s)
     return p.scores_f32 ? launch_fwd_h<T, D, kHookScores>(maps, p, s) : launch_fwd_h<T, D, kHookScores16>(maps, p, s);
   if (p.row_sum != nullptr) return launch_fwd_h<T, D, kHookRowSum>(maps, p, s);
   if (p.col_partial != nullptr) return launch_fwd_h<T, D, kHookColPart>(maps, p, s);
-  if (p.s_scratch != nullptr) return launch_fwd_h<T, D, kHookScratch>(maps, p, s);
   return launch_fwd_h<T, D, kHookNone>(maps, p, s);
 }
 
@@ -1662,8 +1651,9 @@ cudaError_t launch_fwd_t(const TcMaps& maps, const FwdParams& p, cudaStream_t s)
 bool tc_fwd_supported(const FwdParams& p, int dtype) {
   (void)dtype;
   if (!tc_head_dim(p.D)) return false;
-  if (p.drop.p > 0.f && (p.s_scratch != nullptr || (p.scores != nullptr && !p.scores_f32)))
-    return false;  // no dropout variant of the scratch and 16-bit-score hooks: CUDA-core kernels
+  if (p.s_scratch != nullptr) return false;  // the score buffer of the cross-token operator: CUDA-core kernels only
+  if (p.drop.p > 0.f && p.scores != nullptr && !p.scores_f32)
+    return false;  // no dropout variant of the 16-bit-score hook: CUDA-core kernels
   if (!(p.sm_scale > 0.f)) return false;  // the row max is taken on unscaled scores
   if (!device_is_sm100() || get_encode() == nullptr) return false;
   if (p.m_begin % BM != 0 || p.m_end <= p.m_begin) return false;
@@ -1673,10 +1663,6 @@ bool tc_fwd_supported(const FwdParams& p, int dtype) {
   if (p.scores != nullptr && !tma_score_rows(p.scores, p.N, p.scores_f32 ? 4 : 2)) {
     if (p.drop.p > 0.f) return false;  // the plain-store hook has no dropout variant
     if (reinterpret_cast<uintptr_t>(p.scores) % (p.scores_f32 ? 4 : 2) != 0) return false;
-  }
-  if (p.s_scratch != nullptr) {
-    if (p.scores != nullptr) return false;
-    if (p.split % 32 != 0 || reinterpret_cast<uintptr_t>(p.s_scratch) % 16 != 0) return false;
   }
   return true;
 }
@@ -1698,12 +1684,6 @@ cudaError_t launch_tc_fwd(const FwdParams& p, int dtype, cudaStream_t s) {
     const int esize = p.scores_f32 ? 4 : 2;
     char* base = static_cast<char*>(p.scores) + (int64_t)p.m_begin * p.N * esize;
     if (!make_map_store_f32(&maps.st, base, p.N, q_rows, p.N, (int64_t)p.M * p.N, p.B * p.Hq, esize))
-      return cudaErrorInvalidValue;
-  } else if (p.s_scratch != nullptr) {
-    const int rows = p.m_end - p.split;  // rows of the cross region inside the window
-    if (rows > 0 &&
-        !make_map_store_f32(&maps.st, p.s_scratch, p.split, rows, p.split, (int64_t)(p.M - p.split) * p.split,
-                            p.B * p.Hq))
       return cudaErrorInvalidValue;
   }
   if (dtype == FAWS_FP16)

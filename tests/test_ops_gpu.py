@@ -124,6 +124,26 @@ def test_all_entry_points(shape, causal, dtype, backend):
         _check_sum(xh, xs_ref, f"cross_softmax per head split={split}")
 
 
+@pytest.mark.parametrize("split", [1, 96, 129, 300])
+@pytest.mark.parametrize("shape,window", [((2, 4, 2, 300, 300, 64), None), ((1, 2, 2, 260, 333, 128), (128, 260)),
+                                          ((1, 4, 1, 77, 301, 32), None)], ids=["gqa", "window", "d32"])
+def test_buffered_cross_token_sums_recompute_the_region(shape, window, split):
+    """On the tcgen05 kernels the buffered operator is the two-pass one, without its score buffer: same bits, for
+    splits on both sides of the tile edges; the CUDA-core kernels still stream the buffer."""
+    q, k, v = (t.cuda() for t in _inputs(shape, torch.float16, seed=6))
+    for causal in (True, False):
+        a = F.attention_cross_token_softmax_sum_buffered(q, k, v, split, causal, q_rows=window)
+        assert F.last_backend() == "tcgen05"
+        b = F.attention_cross_token_softmax_sum(q, k, v, split, causal, q_rows=window)
+        c = F.attention_cross_token_softmax_sum_buffered(q, k, v, split, causal, q_rows=window, backend="generic")
+        rows = slice(*window) if window else slice(None)
+        assert torch.equal(a[0][:, :, rows], b[0][:, :, rows]) and torch.equal(a[1], b[1])
+        _check_sum(a[1], c[1].cpu(), f"split={split}")
+    if split % 32 and shape[3] > split and shape[5] >= 64:  # a forced family keeps refusing what its buffer could not hold
+        with pytest.raises(RuntimeError):
+            F.attention_cross_token_softmax_sum_buffered(q, k, v, split, True, backend="tcgen05")
+
+
 def test_determinism_and_buffers():
     q, k, v = (t.cuda() for t in _inputs((1, 4, 2, 320, 320, 64), torch.float16, seed=3))
     for fn, args in [(F.attention_with_col_sum, ()), (F.attention_with_softmax_col_sum, ()),
