@@ -261,27 +261,61 @@ int softmax_col_sums(const faws_problem* p, float* sum_out, int per_q_head, void
   return run_colsoftmax(p, c, sum_out, w.per_head, per_q_head ? 0 : 1, s);
 }
 
-// Decoding with grouped queries: when the G query heads of a kv head have so few rows that all of them
-// fit one 128-row tile, they are run as ONE head of G*M rows, so K and V are streamed once per kv head
-// instead of once per query head.  Pure re-indexing: row r = g*M + i of the packed head is row i of query
-// head hk*G + g, which for contiguous heads (stride_h == M * stride_s) is a plain row stride; out and L
-// index the same way.  Needs an unmasked problem (not causal, or a single query row, which sees every key).
-bool pack_gqa(const faws_problem* p, faws_problem* packed) {
+// Few query rows with grouped queries: the G query heads of a kv head are run as ONE head of G*M rows, so that
+// K and V are streamed once per 128 of those rows instead of once per query head and the rows of the 128-row tiles
+// are used.  Pure re-indexing: row r = g*M + i of the packed head is row i of query head hk*G + g, which for
+// contiguous heads (stride_h == M * stride_s) is a plain row stride; out and L index the same way.  The causal limit
+// of a packed row goes by its index within its head, `*pack_m` (0: no mask).  Taken when it visits fewer (query tile,
+// key tile) pairs than the heads one by one, whose causal tiles also skip the keys that none of their rows sees:
+// always for G*M <= 128, up to a few hundred rows against a long cache, not for self-attention.  bf16 D128 causal,
+// heads one by one and packed: B4 Hq32 Hk8 M16 N8192 72.9 and 31.9 us, B8 Hq28 Hk4 M40 N9000 150.5 and 68.3 us,
+// B1 Hq28 Hk4 M300 N30000 169 and 128 us, B2 Hq32 Hk8 M129 N8192 70.2 and 62.3 us.
+bool pack_gqa(const faws_problem* p, faws_problem* packed, int* pack_m) {
+  *pack_m = 0;
   const int G = p->Hq / p->Hk;
-  if (G <= 1 || (long long)G * p->M > kTcBlockM) return false;
-  if (p->causal && p->M != 1) return false;
+  if (G <= 1 || p->M > 4096) return false;
   if (p->causal && p->N < p->M) return false;
   if (p->dropout_p > 0.f || p->m_begin != 0 || p->m_end != p->M) return false;
   if (p->out.ptr == nullptr) return false;
   if (p->q.stride_h != (int64_t)p->M * p->q.stride_s || p->out.stride_h != (int64_t)p->M * p->out.stride_s) return false;
+  if ((long long)G * p->M > kTcBlockM) {
+    const int nkt = cdiv(p->N, kTcBlockN);
+    long long one_by_one = 0;
+    for (int r0 = 0; r0 < p->M; r0 += kTcBlockM) {
+      const int last = r0 + kTcBlockM < p->M ? r0 + kTcBlockM : p->M;
+      one_by_one += p->causal ? cdiv(p->N - p->M + last, kTcBlockN) : nkt;
+    }
+    if ((long long)cdiv(G * p->M, kTcBlockM) * nkt >= one_by_one * G) return false;
+  }
   *packed = *p;
   packed->Hq = p->Hk;
   packed->M = G * p->M;
   packed->m_end = G * p->M;
-  packed->causal = 0;
+  if (p->M == 1) packed->causal = 0;  // the one row of a head sees every key
+  else if (p->causal) *pack_m = p->M;
   packed->q.stride_h = p->q.stride_h * G;
   packed->out.stride_h = p->out.stride_h * G;
   return true;
+}
+
+// The forward parameters of a problem or, with pack_m > 0, of the packed form of one.
+FwdParams make_fwd_packed(const faws_problem* p, int pack_m) {
+  FwdParams f = make_fwd(p);
+  if (pack_m > 0) {
+    f.pack_m = pack_m;
+    f.p_seq = p->N - pack_m;
+  }
+  return f;
+}
+
+// Replaces *p by its packed form (kept in *packed) where that pays and the tcgen05 kernels take it.
+int use_packed(const faws_problem** p, faws_problem* packed) {
+  int pack_m = 0;
+  if (!tc_allowed(*p) || !pack_gqa(*p, packed, &pack_m)) return 0;
+  const FwdParams f = make_fwd_packed(packed, pack_m);
+  if (f.v == nullptr || !tc_fwd_supported(f, packed->dtype)) return 0;
+  *p = packed;
+  return pack_m;
 }
 
 // Number of key ranges for a problem that leaves most SMs idle: the plan of the reference's
@@ -327,11 +361,8 @@ int faws_attention(const faws_problem* p, void* stream) {
   int st = validate(p);
   if (st != FAWS_OK) return st;
   faws_problem packed;
-  if (tc_allowed(p) && pack_gqa(p, &packed)) {
-    FwdParams fp = make_fwd(&packed);
-    if (fp.v != nullptr && tc_fwd_supported(fp, packed.dtype)) p = &packed;
-  }
-  FwdParams f = make_fwd(p);
+  const int pack_m = use_packed(&p, &packed);
+  FwdParams f = make_fwd_packed(p, pack_m);
   int bm, bn;
   return run_fwd(p, f, static_cast<cudaStream_t>(stream), &bm, &bn);
 }
@@ -355,11 +386,8 @@ int32_t faws_split_kv_plan(const faws_problem* p) {
   if (p->dropout_p > 0.f || p->m_begin != 0 || p->m_end != p->M || !tc_allowed(p)) return 1;
   if (p->v.ptr == nullptr || p->out.ptr == nullptr) return 1;
   faws_problem packed;
-  if (pack_gqa(p, &packed)) {
-    FwdParams fp = make_fwd(&packed);
-    if (tc_fwd_supported(fp, packed.dtype)) p = &packed;
-  }
-  FwdParams f = make_fwd(p);
+  const int pack_m = use_packed(&p, &packed);
+  const FwdParams f = make_fwd_packed(p, pack_m);
   if (!tc_fwd_supported(f, p->dtype)) return 1;
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -379,11 +407,8 @@ int faws_attention_split_kv(const faws_problem* p, int32_t n_splits, void* works
     return FAWS_EWORKSPACE;
   if (p->out.ptr == nullptr || p->v.ptr == nullptr) return FAWS_EINVAL;
   faws_problem packed;  // same bytes of workspace either way: B*Hq*M is unchanged by the packing
-  if (tc_allowed(p) && pack_gqa(p, &packed)) {
-    FwdParams fp = make_fwd(&packed);
-    if (tc_fwd_supported(fp, packed.dtype)) p = &packed;
-  }
-  FwdParams f = make_fwd(p);
+  const int pack_m = use_packed(&p, &packed);
+  FwdParams f = make_fwd_packed(p, pack_m);
   if (!tc_allowed(p) || !tc_fwd_supported(f, p->dtype)) return FAWS_EBACKEND;
   float* L_part = static_cast<float*>(workspace);
   char* o_part = static_cast<char*>(workspace) + align256((size_t)p->B * p->Hq * n_splits * p->M * 4);

@@ -97,6 +97,8 @@ struct FwdParams {
   int n_splits;          // split-KV: key ranges per (batch, head); 0 or 1 = off.  o and L then address the
                          // partial buffers (B, Hq*n_splits, M, D) and (B, Hq, n_splits, M)
   int tiles_per_split;   // key tiles per range
+  int pack_m;            // > 0: the rows of a head are the pack_m query rows of each head of a group, one head after
+                         // the other (see pack_gqa); the causal limit goes by the row's index within its head
   int col_lin;           // column hook skips tiles that col_tile_linear() accepts (see below)
   int col_row_lo;        // max(col_row_begin, m_begin): first query row that contributes
   float* qsum;           // col_lin: (B,Hq,ceil(M/128),128) per-tile sums of the query rows, written by the

@@ -215,7 +215,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
       int hi = 0;
       if (r0 < p.m_end) {
         hi = p.N;
-        if (p.causal) hi = max(0, min(p.N, p.p_seq + min(r0 + BM, p.m_end)));
+        if (p.causal && p.pack_m == 0) hi = max(0, min(p.N, p.p_seq + min(r0 + BM, p.m_end)));
       }
       nt_q[t] = min(max((hi + BN - 1) / BN, kt0), kt0 + p.tiles_per_split);
     }
@@ -620,6 +620,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
     const float masked_f = __uint_as_float(p.masked_bits);
     // per item
     int r_tile, i, my_nt, qb128;  // first row of the query tile, this thread's row, end of its key-tile range
+    int vis_end;                  // causal: this thread's row sees the keys before it
     bool row_ok, part_on;
     uint32_t drop_row;  // Philox counter of (b, h, i, key 0) without the call's offset, 32-bit wrap-around
     float m_run, l_run, rs_raw;
@@ -641,7 +642,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
       int nvis = 128;  // visible columns form a prefix of the tile's row
       if (kMasked) {
         int lim = p.N;
-        if (p.causal) lim = min(lim, i + p.p_seq + 1);
+        if (p.causal) lim = min(lim, vis_end);
         nvis = max(0, min(128, lim - n0));
       }
 #define FAWS_VIS(x) (!kMasked || (x) < nvis)
@@ -931,6 +932,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
     r_tile = r_tile_of[qt];
     i = r_tile + row;
     my_nt = nt_q[qt];
+    vis_end = (p.pack_m > 0 ? i % p.pack_m : i) + p.p_seq + 1;
     row_ok = i >= p.m_begin && i < p.m_end;
     qb128 = r_tile / BM;
     part_on = HOOK == kHookColPart && qb128 >= p.qb_first && r_tile < p.m_end;
@@ -948,7 +950,9 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
         if (!mbar_wait(&bars->s_full[qt], s_cnt & 1, abort_flag)) { alive = false; break; }
         ++s_cnt;
         tc_fence_after();
-        const bool full_vis = (n0 + BN <= p.N) && (!p.causal || (n0 + BN - 1 <= r_tile + p.p_seq));
+        // (packed heads: the tile may hold the first row of a head)
+        const bool full_vis =
+            (n0 + BN <= p.N) && (!p.causal || (n0 + BN - 1 <= (p.pack_m > 0 ? 0 : r_tile) + p.p_seq));
         const bool ok = full_vis ? tile_body(std::false_type{}, cnt, n0) : tile_body(std::true_type{}, cnt, n0);
         if (!ok) { alive = false; break; }
         ++cnt;
@@ -1435,7 +1439,7 @@ namespace {
 bool persistent_allowed();
 
 struct WorkKey {
-  int gx, gy, gz, lpt, causal, p_seq, m_begin, m_end, N, rows, ctas;
+  int gx, gy, gz, lpt, causal, p_seq, m_begin, m_end, N, rows, ctas, pack_m;
   bool operator==(const WorkKey& o) const { return std::memcmp(this, &o, sizeof(WorkKey)) == 0; }
 };
 
@@ -1453,7 +1457,7 @@ bool make_work_list(const FwdParams& p, dim3 grid, int cta_rows, int ctas, WorkL
   thread_local WorkKey last_key{};
   thread_local WorkList last{};
   const WorkKey key{(int)grid.x, (int)grid.y, (int)grid.z, p.lpt_order, p.causal, p.p_seq, p.m_begin, p.m_end, p.N,
-                    cta_rows, ctas};
+                    cta_rows, ctas, p.pack_m};
   if (last.n_items > 0 && key == last_key) {
     *out = last;
     return true;
@@ -1474,7 +1478,7 @@ bool make_work_list(const FwdParams& p, dim3 grid, int cta_rows, int ctas, WorkL
       for (int t = 0; t * BM < cta_rows; ++t) {
         const int r = r0 + t * BM;
         int hi = 0;
-        if (r < p.m_end) hi = p.causal ? std::max(0, std::min(p.N, p.p_seq + std::min(r + BM, p.m_end))) : p.N;
+        if (r < p.m_end) hi = p.causal && p.pack_m == 0 ? std::max(0, std::min(p.N, p.p_seq + std::min(r + BM, p.m_end))) : p.N;
         tiles = std::max(tiles, (hi + BN - 1) / BN);
       }
       cost[slot] = 19 * tiles + 30;  // measured on cfg3: 1.90 us per key tile + 3.0 us per item (unit 0.1 us)

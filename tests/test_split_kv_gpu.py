@@ -56,6 +56,37 @@ def test_split_kv_matches_oracle_and_unsplit(shape, causal, dtype):
     assert F.device_status() == 0
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16], ids=["fp16", "bf16"])
+@pytest.mark.parametrize("interleaved", [False, True], ids=["bhsd", "bshd"])
+@pytest.mark.parametrize("shape", [
+    (2, 8, 2, 16, 300, 64),      # four heads in half a tile
+    (1, 7, 1, 40, 515, 128),     # 280 packed rows: heads across tile edges, a third tile of 24 rows
+    (2, 4, 1, 129, 1300, 64),    # 516 packed rows in 5 tiles instead of 8
+    (1, 8, 1, 16, 16, 32),       # self-attention, exactly one tile
+    (1, 4, 1, 33, 33, 128),      # self-attention, one row more than a tile: two tiles instead of four
+    (1, 4, 1, 100, 100, 64),     # self-attention: not packed
+    (1, 2, 1, 2, 257, 128),      # a last key tile of one key, hidden from the first row of each head
+], ids=lambda s: "x".join(map(str, s)))
+def test_few_causal_rows_with_grouped_queries(shape, interleaved, dtype):
+    """The heads of a group share a query tile and each row keeps its own causal limit (interleaved heads cannot be
+    packed and take the general route)."""
+    B, Hq, Hk, M, N, D = shape
+    q, k, v = _inputs(shape, dtype, seed=M)
+    ref_out, ref_scores = orc.naive_attention_with_scores(q, k, v, True, p_seq=N - M)
+    slack = orc.bf16_out_slack(ref_scores, v, ref_out) if dtype == torch.bfloat16 else None
+    Lref = orc.log_normalizer(ref_scores)
+    if interleaved:
+        q = q.transpose(1, 2).contiguous().transpose(1, 2)
+    qd, kd, vd = q.cuda(), k.cuda(), v.cuda()
+    for splits in {None, 1, min(3, (N + 127) // 128), (N + 127) // 128}:
+        out, L, _, _, _ = F.attention(qd, kd, vd, True, return_log_normalizer=True, kv_splits=splits)
+        assert F.last_backend() == "tcgen05"
+        ok, err = orc.check_out(out.cpu(), ref_out, slack)
+        assert ok, (splits, err)
+        assert (L.cpu() - Lref).abs().max() < 2e-3
+    assert F.device_status() == 0
+
+
 def test_split_plan_follows_the_occupancy_rule():
     lib = _lib.load()
     q, k, v = (t.cuda() for t in _inputs((1, 4, 2, 16, 16384, 128), torch.float16))
