@@ -1627,13 +1627,17 @@ bool use_split_kv(const FwdParams& p) {
 
 template <typename T, int D, int HOOK>
 cudaError_t launch_fwd_h(const TcMaps& maps, const FwdParams& p, cudaStream_t s) {
-  // Score-materialising causal launches are bound by their stores, not by the chain of key
-  // tiles: measured, the 256-row CTAs (half as many set-ups) are faster there.
-  if constexpr (HOOK != kHookScores16) {
+  // Score-materialising causal launches with more CTAs than SMs are bound by their stores, not by the chain of key
+  // tiles: measured, the 256-row CTAs (half as many set-ups) are faster there (fp16 D128 H32, 256 and 128 rows:
+  // S1024 36.8 and 39.9 us, S768 27.0 and 26.5, S640 19.2 and 19.1).  When the 128-row CTAs all run at once the chain
+  // is what counts again (D128 H16 S768 22.4 and 15.8 us, H8 S640 16.0 and 12.7; D64 H8 S512 15.9 and 10.6).
+  if constexpr (HOOK != kHookScores16 && HOOK != kHookScoresAny) {
     // dropout: 256-row CTAs only (the mask generation, not the chain of key tiles, bounds it)
     if (p.drop.p > 0.f) return launch_fwd_s<T, D, HOOK, false, true>(maps, p, s);
   }
-  const bool store_bound = (HOOK == kHookScores || HOOK == kHookScores16) && p.causal;
+  const long long ctas128 = (long long)((p.m_end - p.m_begin + 127) / 128) * p.Hq * p.B;
+  const bool store_bound = (HOOK == kHookScores || HOOK == kHookScores16 || HOOK == kHookScoresAny) && p.causal &&
+                           ctas128 > sm_count();
   static const bool forced = std::getenv("FAWS_SPLIT_KV") != nullptr;
   const bool split = use_split_kv(p) && (forced || !store_bound);
   return split ? launch_fwd_s<T, D, HOOK, true>(maps, p, s) : launch_fwd_s<T, D, HOOK, false>(maps, p, s);
@@ -1642,7 +1646,7 @@ cudaError_t launch_fwd_h(const TcMaps& maps, const FwdParams& p, cudaStream_t s)
 template <typename T, int D>
 cudaError_t launch_fwd_t(const TcMaps& maps, const FwdParams& p, cudaStream_t s) {
   if (p.scores != nullptr && !tma_score_rows(p.scores, p.N, p.scores_f32 ? 4 : 2))
-    return launch_fwd_s<T, D, kHookScoresAny, false>(maps, p, s);
+    return launch_fwd_h<T, D, kHookScoresAny>(maps, p, s);
   if (p.scores != nullptr)
     return p.scores_f32 ? launch_fwd_h<T, D, kHookScores>(maps, p, s) : launch_fwd_h<T, D, kHookScores16>(maps, p, s);
   if (p.row_sum != nullptr) return launch_fwd_h<T, D, kHookRowSum>(maps, p, s);

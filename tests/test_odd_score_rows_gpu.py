@@ -68,3 +68,17 @@ def test_window_of_odd_rows():
     assert bool((scores[:, :, :128] == 7.0).all()) and bool((scores[:, :, 271:] == 7.0).all())
     ok, viol, ok_mask = orc.check_scores(scores[:, :, 128:271].cpu(), ref[:, :, 128:271])
     assert ok and ok_mask, viol
+
+
+@pytest.mark.parametrize("N", [257, 260])
+def test_scores_of_many_heads(N):
+    """More 128-row CTAs than SMs: the launches of 256-row CTAs (the shapes above run 128-row ones)."""
+    g = torch.Generator().manual_seed(N)
+    q, k, v = (torch.randn(1, h, N, 64, generator=g).half() for h in (76, 38, 38))
+    ref_out, ref = orc.naive_attention_with_scores(q, k, v, True)
+    out, s = F.attention_with_scores(q.cuda(), k.cuda(), v.cuda(), True)
+    assert F.last_backend() == "tcgen05" and F.device_status() == 0
+    ok, err = orc.check_out(out.cpu(), ref_out)
+    assert ok, err
+    ok, viol, ok_mask = orc.check_scores(s.cpu(), ref)
+    assert ok and ok_mask, viol
