@@ -159,6 +159,14 @@ tc_bwd_kernel(const __grid_constant__ BwMaps maps, const BwTcParams p, int* __re
     nu = (hi + BT - 1) / BT;
   }
 
+  // Launch chain: pre-pass, query-major, key-major, group sum, each allowed to begin while the one before it drains.
+  // Only the key-major kernel's partials and the pre-pass's arrays pass between them: the query-major kernel waits
+  // for the pre-pass before it lets the key-major one begin, which therefore finds the arrays written and waits
+  // for the query-major kernel only before it exits (so that its own completion stands for all of the chain).
+  if (!KM) {
+    griddep_wait();
+    griddep_launch_dependents();
+  }
   if (threadIdx.x == 0) {
     mbar_init(&bars->x_full, 1);
     for (int s = 0; s < NSTAGE; ++s) {
@@ -484,6 +492,10 @@ tc_bwd_kernel(const __grid_constant__ BwMaps maps, const BwTcParams p, int* __re
   }
 
   // ------------------------------------------------------------ common exit
+  if (KM) {
+    griddep_launch_dependents();
+    griddep_wait();
+  }
   tc_fence_before();
   __syncthreads();
   if (*abort_flag) {
@@ -499,64 +511,118 @@ tc_bwd_kernel(const __grid_constant__ BwMaps maps, const BwTcParams p, int* __re
 
 // Pre-pass: delta_i = sum_d out_id * dout_id and -L_i * log2(e), both into arrays padded to whole
 // 128-row tiles (zeros in the padding), so that the kernels can fetch a tile's 128 values with one
-// aligned bulk copy.  One warp per (padded) row.
+// aligned bulk copy.  Bound by HBM: D / 8 lanes per row, 16 bytes of each operand a lane, four rows in flight
+// (bf16 B1 H28 S4096 D128: 15 us; 34 us with a warp and 4-byte loads to a row).
+constexpr int kPrepRows = 4;
 template <typename T>
-__global__ void bwd_prep_kernel(BwdParams p, float* negl2, float* delta, int Mpad) {
-  const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (w >= (int64_t)p.B * p.Hq * Mpad) return;
-  const int i = (int)(w % Mpad);
-  const int64_t bh = w / Mpad;
-  const int h = (int)(bh % p.Hq), b = (int)(bh / p.Hq);
-  float sum = 0.f, nl = 0.f;
-  if (i < p.M) {
-    const T* o = reinterpret_cast<const T*>(p.o) + b * p.o_sb + h * p.o_sh + (int64_t)i * p.o_ss;
-    const T* g = reinterpret_cast<const T*>(p.dout) + b * p.do_sb + h * p.do_sh + (int64_t)i * p.do_ss;
-    for (int d = lane * 2; d < p.D; d += 64) {
-      float2 a, c;
-      if constexpr (std::is_same<T, __half>::value) {
-        a = __half22float2(*reinterpret_cast<const __half2*>(o + d));
-        c = __half22float2(*reinterpret_cast<const __half2*>(g + d));
-      } else {
-        a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(o + d));
-        c = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(g + d));
-      }
+__global__ void __launch_bounds__(256) bwd_prep_kernel(BwdParams p, float* negl2, float* delta, int Mpad, int blocks_per_head) {
+  griddep_launch_dependents();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lpr = p.D >> 3, rows_at_once = 32 / lpr, sub = lane & (lpr - 1);
+  const int bh = blockIdx.x / blocks_per_head;
+  const int i0 = (blockIdx.x - bh * blocks_per_head) * (8 * kPrepRows * rows_at_once) + warp * kPrepRows * rows_at_once +
+                 lane / lpr;
+  const int h = bh % p.Hq, b = bh / p.Hq;
+  const T* o = reinterpret_cast<const T*>(p.o) + b * p.o_sb + h * p.o_sh + 8 * sub;
+  const T* g = reinterpret_cast<const T*>(p.dout) + b * p.do_sb + h * p.do_sh + 8 * sub;
+  uint4 ov[kPrepRows], gv[kPrepRows];
+#pragma unroll
+  for (int x = 0; x < kPrepRows; ++x) {
+    const int i = i0 + x * rows_at_once;
+    ov[x] = gv[x] = make_uint4(0u, 0u, 0u, 0u);
+    if (i < p.M) {
+      ov[x] = *reinterpret_cast<const uint4*>(o + (int64_t)i * p.o_ss);
+      gv[x] = *reinterpret_cast<const uint4*>(g + (int64_t)i * p.do_ss);
+    }
+  }
+#pragma unroll
+  for (int x = 0; x < kPrepRows; ++x) {
+    const int i = i0 + x * rows_at_once;
+    const uint32_t ow[4] = {ov[x].x, ov[x].y, ov[x].z, ov[x].w}, gw[4] = {gv[x].x, gv[x].y, gv[x].z, gv[x].w};
+    float sum = 0.f;
+#pragma unroll
+    for (int y = 0; y < 4; ++y) {
+      const float2 a = unpack2<T>(ow[y]), c = unpack2<T>(gw[y]);
       sum = fmaf(a.x, c.x, fmaf(a.y, c.y, sum));
     }
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, s);
-    const float Li = p.L[bh * p.M + i];
-    nl = (Li == __int_as_float(0xff800000)) ? 0.f : -Li * kLog2e;  // no visible key: every weight is masked anyway
-  }
-  if (lane == 0) {
-    delta[w] = sum;
-    negl2[w] = nl;
+    for (int s = lpr >> 1; s > 0; s >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, s);
+    if (sub == 0 && i < Mpad) {
+      float nl = 0.f;
+      if (i < p.M) {
+        const float Li = p.L[(int64_t)bh * p.M + i];
+        nl = (Li == __int_as_float(0xff800000)) ? 0.f : -Li * kLog2e;  // no visible key: every weight is masked anyway
+      }
+      delta[(int64_t)bh * Mpad + i] = sum;
+      negl2[(int64_t)bh * Mpad + i] = nl;
+    }
   }
 }
 
-// out[b,hk,j,:] = sum over the G query heads of the kv head, in head order, of part[b,hk*G+g,j,:]
+// out[b,hk,j,:] = sum over the G query heads of the kv head, in head order, of part[b,hk*G+g,j,:]; one thread per 8
+// elements, dK in the first half of the grid and dV in the second.  Bound by the reads (bf16 Hq28 Hk4 S4096 D128:
+// 15 us for both; 2 x 17 us with a launch each and 4 bytes a thread).
+struct GroupSumOut {
+  void* out;
+  int64_t sb, sh, ss;
+};
 template <typename T, typename P>
-__global__ void bwd_group_sum_kernel(const P* __restrict__ part, T* out, int64_t o_sb, int64_t o_sh, int64_t o_ss,
-                                     int B, int Hk, int G, int N, int D) {
-  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;  // one thread per 2 elements
-  const int half_d = D / 2;
-  if (idx >= (int64_t)B * Hk * N * half_d) return;
-  const int d2 = (int)(idx % half_d);
-  const int64_t r = idx / half_d;
+__global__ void __launch_bounds__(256) bwd_group_sum_kernel(const P* __restrict__ dk_part, const P* __restrict__ dv_part,
+                                                            GroupSumOut dk, GroupSumOut dv, int B, int Hk, int G, int N,
+                                                            int D) {
+  griddep_wait();
+  griddep_launch_dependents();
+  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int chunks = D >> 3;
+  if (idx >= (int64_t)B * Hk * N * chunks) return;
+  const bool second = blockIdx.y != 0;
+  const P* part = second ? dv_part : dk_part;
+  const GroupSumOut o = second ? dv : dk;
+  const int c = (int)(idx % chunks);
+  const int64_t r = idx / chunks;
   const int j = (int)(r % N);
   const int64_t bk = r / N;
   const int hk = (int)(bk % Hk), b = (int)(bk / Hk);
-  float s0 = 0.f, s1 = 0.f;
-  for (int g = 0; g < G; ++g) {
-    const P* src = part + ((((int64_t)b * Hk + hk) * G + g) * N + j) * D + d2 * 2;
-    float2 v;
-    if constexpr (std::is_same<P, float>::value) v = *reinterpret_cast<const float2*>(src);
-    else v = unpack2<T>(*reinterpret_cast<const uint32_t*>(src));
-    s0 += v.x;
-    s1 += v.y;
+  const P* src = part + (((bk * G) * N + j) * D + c * 8);
+  const int64_t step = (int64_t)N * D;
+  float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+  for (int g = 0; g < G; ++g, src += step) {
+    if constexpr (std::is_same<P, float>::value) {
+      const float4 a = *reinterpret_cast<const float4*>(src), e = *reinterpret_cast<const float4*>(src + 4);
+      s[0] += a.x; s[1] += a.y; s[2] += a.z; s[3] += a.w;
+      s[4] += e.x; s[5] += e.y; s[6] += e.z; s[7] += e.w;
+    } else {
+      const uint4 a = *reinterpret_cast<const uint4*>(src);
+      const uint32_t w[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+      for (int y = 0; y < 4; ++y) {
+        const float2 v = unpack2<T>(w[y]);
+        s[2 * y] += v.x;
+        s[2 * y + 1] += v.y;
+      }
+    }
   }
-  const uint32_t w = pack2<T>(s0, s1);
-  *reinterpret_cast<uint32_t*>(out + b * o_sb + hk * o_sh + (int64_t)j * o_ss + d2 * 2) = w;
+  T* dst = reinterpret_cast<T*>(o.out) + b * o.sb + hk * o.sh + (int64_t)j * o.ss + c * 8;
+  *reinterpret_cast<uint4*>(dst) =
+      make_uint4(pack2<T>(s[0], s[1]), pack2<T>(s[2], s[3]), pack2<T>(s[4], s[5]), pack2<T>(s[6], s[7]));
+}
+
+// A launch that may begin while the kernel before it drains (programmatic stream serialization).
+template <typename K, typename... A>
+cudaError_t launch_overlapped(K kernel, dim3 grid, int threads, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+  count_launch();
+  return e;
 }
 
 int mpad_of(int M) { return (M + BT - 1) / BT * BT; }
@@ -576,9 +642,11 @@ cudaError_t launch_bwd_td(const BwdParams& p, cudaStream_t s) {
   using Part = typename std::conditional<MODE == kPlain, T, float>::type;
   const size_t part_bytes = ((size_t)p.B * p.Hq * p.N * p.D * sizeof(Part) + 255) & ~size_t(255);
   {
-    const int64_t warps = (int64_t)p.B * p.Hq * Mpad;
-    bwd_prep_kernel<T><<<(unsigned)((warps * 32 + 255) / 256), 256, 0, s>>>(p, negl2, delta, Mpad);
+    const int rows = 8 * kPrepRows * (256 / p.D);  // of one block
+    const int blocks_per_head = (Mpad + rows - 1) / rows;
+    bwd_prep_kernel<T><<<(unsigned)(p.B * p.Hq * blocks_per_head), 256, 0, s>>>(p, negl2, delta, Mpad, blocks_per_head);
     count_launch();
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
   BwTcParams tp{};
   tp.Hq = p.Hq; tp.G = p.G; tp.M = p.M; tp.N = p.N; tp.p_seq = p.p_seq; tp.causal = p.causal; tp.Mpad = Mpad;
@@ -588,6 +656,21 @@ cudaError_t launch_bwd_td(const BwdParams& p, cudaStream_t s) {
   int* status_word = tc_status_word();
   const bool per_head = p.G > 1;
   const bool map_parts = per_head && MODE == kPlain;  // 16-bit partials go through the store maps
+  // query-major: dQ
+  {
+    BwMaps m;
+    if (!make_map_bhsd(&m.x, p.q, p.D, p.M, p.Hq, p.B, p.q_ss, p.q_sh, p.q_sb, 128) ||
+        !make_map_bhsd(&m.y, p.dout, p.D, p.M, p.Hq, p.B, p.do_ss, p.do_sh, p.do_sb, 128) ||
+        !make_map_bhsd(&m.a, p.k, p.D, p.N, p.Hk, p.B, p.k_ss, p.k_sh, p.k_sb, 128) ||
+        !make_map_bhsd(&m.b, p.v, p.D, p.N, p.Hk, p.B, p.v_ss, p.v_sh, p.v_sb, 128) ||
+        !make_map_bhsd(&m.o0, p.dq, p.D, p.M, p.Hq, p.B, p.dq_ss, p.dq_sh, p.dq_sb, 32))
+      return cudaErrorInvalidValue;
+    m.o1 = m.o0;
+    dim3 grid(p.Hq, p.B, (p.M + BT - 1) / BT);
+    if ((e = launch_overlapped(tc_bwd_kernel<T, D, false, MODE>, grid, NTHREADS, L::alloc, s, m, tp, status_word)) !=
+        cudaSuccess)
+      return e;
+  }
   // key-major: dV, dK (per query head)
   {
     BwMaps m;
@@ -609,35 +692,18 @@ cudaError_t launch_bwd_td(const BwdParams& p, cudaStream_t s) {
                        map_parts ? ph_sh : p.dk_sh, map_parts ? ph_sb : p.dk_sb, 32))
       return cudaErrorInvalidValue;
     dim3 grid(p.Hq, p.B, (p.N + BT - 1) / BT);
-    tc_bwd_kernel<T, D, true, MODE><<<grid, NTHREADS, L::alloc, s>>>(m, tp, status_word);
-    count_launch();
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if (per_head) {
-      const int64_t n = (int64_t)p.B * p.Hk * p.N * (p.D / 2);
-      const unsigned blocks = (unsigned)((n + 255) / 256);
-      bwd_group_sum_kernel<T, Part><<<blocks, 256, 0, s>>>(reinterpret_cast<const Part*>(part), reinterpret_cast<T*>(p.dk),
-                                                     p.dk_sb, p.dk_sh, p.dk_ss, p.B, p.Hk, p.G, p.N, p.D);
-      bwd_group_sum_kernel<T, Part><<<blocks, 256, 0, s>>>(reinterpret_cast<const Part*>(part + part_bytes),
-                                                     reinterpret_cast<T*>(p.dv), p.dv_sb, p.dv_sh, p.dv_ss, p.B, p.Hk,
-                                                     p.G, p.N, p.D);
-      count_launch(2);
-    }
+    if ((e = launch_overlapped(tc_bwd_kernel<T, D, true, MODE>, grid, NTHREADS, L::alloc, s, m, tp, status_word)) !=
+        cudaSuccess)
+      return e;
   }
-  // query-major: dQ
-  tp.part0 = tp.part1 = nullptr;
-  {
-    BwMaps m;
-    if (!make_map_bhsd(&m.x, p.q, p.D, p.M, p.Hq, p.B, p.q_ss, p.q_sh, p.q_sb, 128) ||
-        !make_map_bhsd(&m.y, p.dout, p.D, p.M, p.Hq, p.B, p.do_ss, p.do_sh, p.do_sb, 128) ||
-        !make_map_bhsd(&m.a, p.k, p.D, p.N, p.Hk, p.B, p.k_ss, p.k_sh, p.k_sb, 128) ||
-        !make_map_bhsd(&m.b, p.v, p.D, p.N, p.Hk, p.B, p.v_ss, p.v_sh, p.v_sb, 128) ||
-        !make_map_bhsd(&m.o0, p.dq, p.D, p.M, p.Hq, p.B, p.dq_ss, p.dq_sh, p.dq_sb, 32))
-      return cudaErrorInvalidValue;
-    m.o1 = m.o0;
-    dim3 grid(p.Hq, p.B, (p.M + BT - 1) / BT);
-    tc_bwd_kernel<T, D, false, MODE><<<grid, NTHREADS, L::alloc, s>>>(m, tp, status_word);
-    count_launch();
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  if (per_head) {
+    const int64_t n = (int64_t)p.B * p.Hk * p.N * (p.D / 8);
+    const dim3 grid((unsigned)((n + 255) / 256), 2, 1);
+    const GroupSumOut dk{p.dk, p.dk_sb, p.dk_sh, p.dk_ss}, dv{p.dv, p.dv_sb, p.dv_sh, p.dv_ss};
+    if ((e = launch_overlapped(bwd_group_sum_kernel<T, Part>, grid, 256, 0, s, reinterpret_cast<const Part*>(part),
+                               reinterpret_cast<const Part*>(part + part_bytes), dk, dv, p.B, p.Hk, p.G, p.N, p.D)) !=
+        cudaSuccess)
+      return e;
   }
   return cudaSuccess;
 }
