@@ -4,6 +4,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import struct
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libfaws.so")
@@ -49,6 +50,12 @@ class Problem(C.Structure):
         ("backend", C.c_int32), ("dropout_p", C.c_float), ("dropout_scale", C.c_float), ("reserved", C.c_int32),
         ("philox_seed", C.c_uint64), ("philox_offset", C.c_uint64),
     ]
+
+
+# The shape, window, tensor and family fields of a Problem in one go (sm_scale, dropout and philox are left zero): a
+# dozen attribute assignments through ctypes take as long as the launch itself.
+PACK = struct.Struct("<8i4x2i4x" + 4 * "Qqqq" + "Qi12x16x")
+assert PACK.size == C.sizeof(Problem)
 
 
 class Grads(C.Structure):

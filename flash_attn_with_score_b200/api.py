@@ -37,11 +37,13 @@ def maybe_contiguous(x):
 
 
 def _tensor(t):
-    return _lib.Tensor(t.data_ptr(), t.stride(0), t.stride(1), t.stride(2))
+    st = t.stride()
+    return _lib.Tensor(t.data_ptr(), st[0], st[1], st[2])
 
 
-def _stream(t):
-    return C.c_void_p(torch.cuda.current_stream(t.device).cuda_stream)
+# raw handle of a device's current stream, without building a Stream object for it where torch allows that
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (
+    lambda index: torch.cuda.current_stream(index).cuda_stream)
 
 
 def philox_cuda_seed_offset(increment, device=None):
@@ -63,15 +65,16 @@ class _Call:
     def __init__(self, q, k, v, causal, sm_scale, dropout_p, out=None, need_L=False, L=None,
                  q_rows=None, backend=None, msgs=None, philox=None, rescale=False):
         m = msgs or {}
-        Dq, Dk, Dv = q.shape[-1], k.shape[-1], v.shape[-1]
-        assert Dq == Dk == Dv, m.get("D", "feature size of q, k, v should be equal")
+        qs, ks, vs = q.shape, k.shape, v.shape
+        Dk = ks[-1]
+        assert qs[-1] == Dk == vs[-1], m.get("D", "feature size of q, k, v should be equal")
         assert Dk in {16, 32, 64, 128}, m.get("Dset", f"Unsupported head_dim: {Dk}")
-        B, H, M, D = q.shape
-        N = k.shape[2]
-        Hk, Hv = k.shape[1], v.shape[1]
-        assert Hk == Hv, m.get("Hkv", "num of heads in k and v should be equal")
+        B, H, M, D = qs
+        N = ks[2]
+        Hk = ks[1]
+        assert Hk == vs[1], m.get("Hkv", "num of heads in k and v should be equal")
         assert H % Hk == 0, m.get("G", "number of heads in q must be a multiple of that in k & v")
-        assert k.shape[0] == B and v.shape[0] == B and v.shape[2] == N
+        assert ks[0] == B and vs[0] == B and vs[2] == N
         if not q.is_cuda:
             raise RuntimeError("flash_attn_with_score_b200 runs on CUDA tensors only (no CPU fallback)")
         if q.dtype not in _DTYPES or k.dtype != q.dtype or v.dtype != q.dtype:
@@ -92,15 +95,15 @@ class _Call:
         assert 0 <= m_begin <= m_end <= M, f"q_rows must lie within [0, {M}]"
         if backend not in _lib.BACKENDS:
             raise ValueError(f"backend must be one of {sorted(k for k in _lib.BACKENDS if k)}")
-        p = _lib.Problem()
-        p.B, p.Hq, p.Hk, p.M, p.N, p.D = B, H, Hk, M, N, D
-        p.dtype = _DTYPES[q.dtype]
-        p.causal = 1 if causal else 0
+        buf = bytearray(_lib.PACK.size)
+        qt, kt, vt = self.q.stride(), self.k.stride(), self.v.stride()
+        ot = out.stride()
+        _lib.PACK.pack_into(buf, 0, B, H, Hk, M, N, D, _DTYPES[q.dtype], 1 if causal else 0, m_begin, m_end,
+                            self.q.data_ptr(), qt[0], qt[1], qt[2], self.k.data_ptr(), kt[0], kt[1], kt[2],
+                            self.v.data_ptr(), vt[0], vt[1], vt[2], out.data_ptr(), ot[0], ot[1], ot[2],
+                            L.data_ptr() if L is not None else 0, _lib.BACKENDS[backend])
+        p = _lib.Problem.from_buffer(buf)
         p.sm_scale = float(sm_scale)
-        p.m_begin, p.m_end = m_begin, m_end
-        p.q, p.k, p.v, p.out = _tensor(self.q), _tensor(self.k), _tensor(self.v), _tensor(self.out)
-        p.log_normalizer = L.data_ptr() if L is not None else None
-        p.backend = _lib.BACKENDS[backend]
         self.seed = self.offset = None
         if dropout_p and dropout_p > 0.0:
             assert dropout_p < 1.0, "dropout_p must be < 1"
@@ -125,9 +128,15 @@ class _Call:
         return ws, n
 
     def run(self, fn_name, *mid):
-        with torch.cuda.device(self.dev):
-            st = getattr(self.lib, fn_name)(C.byref(self.p), *mid, _stream(self.q))
-        _lib.check(st, fn_name)
+        index = self.dev.index
+        fn = getattr(self.lib, fn_name)
+        if index == torch.cuda.current_device():
+            st = fn(C.byref(self.p), *mid, _raw_stream(index))
+        else:
+            with torch.cuda.device(self.dev):
+                st = fn(C.byref(self.p), *mid, _raw_stream(index))
+        if st != 0:
+            _lib.check(st, fn_name)
 
 
 def _f32_bits(x: float) -> int:
@@ -164,10 +173,13 @@ class _AttentionFunction(torch.autograd.Function):
         ctx.causal, ctx.sm_scale, ctx.dropout_p, ctx.backend = causal, float(c.p.sm_scale), dropout_p, backend
         ctx.philox = (c.seed, c.offset) if c.seed is not None else None
         ctx.mark_non_differentiable(*[t for t in (c.L, tot) if t is not None])
+        ctx.set_materialize_grads(False)  # no zeros for the log-normaliser on every backward pass
         return c.out, c.L, tot, c.seed, c.offset
 
     @staticmethod
     def backward(ctx, do, *ignored):
+        if do is None:
+            return (None,) * 10
         q, k, v, o, L = ctx.saved_tensors
         do = maybe_contiguous(do)
         c = _Call(q, k, v, ctx.causal, ctx.sm_scale, ctx.dropout_p, out=o, L=L, backend=ctx.backend,
