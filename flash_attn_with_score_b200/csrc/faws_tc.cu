@@ -187,6 +187,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
   // index; persistent CTAs (never SPLIT, split-KV or fill launches) set it again for every item.
   constexpr bool kStoreHook =
       HOOK == kHookScores || HOOK == kHookScores16 || HOOK == kHookScoresAny;
+  const int pack_m = HOOK == kHookNone ? p.pack_m : 0;  // (only attention() packs; a test in the others costs them 1 %)
   const bool persist = !SPLIT && !kStoreHook && wl.n_items > 0;  // (the launcher keeps the other instances plain)
   bool is_fill;
   int cb_rel, h, b, ksplit, kt0, hk, bh, ho, cb_abs, nt, rr_start;
@@ -215,7 +216,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
       int hi = 0;
       if (r0 < p.m_end) {
         hi = p.N;
-        if (p.causal && p.pack_m == 0) hi = max(0, min(p.N, p.p_seq + min(r0 + BM, p.m_end)));
+        if (p.causal && pack_m == 0) hi = max(0, min(p.N, p.p_seq + min(r0 + BM, p.m_end)));
       }
       nt_q[t] = min(max((hi + BN - 1) / BN, kt0), kt0 + p.tiles_per_split);
     }
@@ -642,7 +643,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
       int nvis = 128;  // visible columns form a prefix of the tile's row
       if (kMasked) {
         int lim = p.N;
-        if (p.causal) lim = min(lim, vis_end);
+        if (p.causal) lim = min(lim, HOOK == kHookNone ? vis_end : i + p.p_seq + 1);
         nvis = max(0, min(128, lim - n0));
       }
 #define FAWS_VIS(x) (!kMasked || (x) < nvis)
@@ -932,7 +933,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
     r_tile = r_tile_of[qt];
     i = r_tile + row;
     my_nt = nt_q[qt];
-    vis_end = (p.pack_m > 0 ? i % p.pack_m : i) + p.p_seq + 1;
+    vis_end = (pack_m > 0 ? i % pack_m : i) + p.p_seq + 1;
     row_ok = i >= p.m_begin && i < p.m_end;
     qb128 = r_tile / BM;
     part_on = HOOK == kHookColPart && qb128 >= p.qb_first && r_tile < p.m_end;
@@ -952,7 +953,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
         tc_fence_after();
         // (packed heads: the tile may hold the first row of a head)
         const bool full_vis =
-            (n0 + BN <= p.N) && (!p.causal || (n0 + BN - 1 <= (p.pack_m > 0 ? 0 : r_tile) + p.p_seq));
+            (n0 + BN <= p.N) && (!p.causal || (n0 + BN - 1 <= (pack_m > 0 ? 0 : r_tile) + p.p_seq));
         const bool ok = full_vis ? tile_body(std::false_type{}, cnt, n0) : tile_body(std::true_type{}, cnt, n0);
         if (!ok) { alive = false; break; }
         ++cnt;
