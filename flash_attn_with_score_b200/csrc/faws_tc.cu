@@ -187,7 +187,10 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
   // index; persistent CTAs (never SPLIT, split-KV or fill launches) set it again for every item.
   constexpr bool kStoreHook =
       HOOK == kHookScores || HOOK == kHookScores16 || HOOK == kHookScoresAny;
-  const int pack_m = HOOK == kHookNone ? p.pack_m : 0;  // (only attention() packs; a test in the others costs them 1 %)
+  // Only attention() packs heads, and the test costs the TMA score hook 1 %; in the odd-row hook it makes ptxas keep the
+  // row's limit in a register instead of spilling 68 bytes (bf16 B1 Hq28 Hk4 S1531: 99 -> 94 us).
+  constexpr bool kRowLimit = HOOK == kHookNone || HOOK == kHookScoresAny;
+  const int pack_m = kRowLimit ? p.pack_m : 0;
   const bool persist = !SPLIT && !kStoreHook && wl.n_items > 0;  // (the launcher keeps the other instances plain)
   bool is_fill;
   int cb_rel, h, b, ksplit, kt0, hk, bh, ho, cb_abs, nt, rr_start;
@@ -643,7 +646,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
       int nvis = 128;  // visible columns form a prefix of the tile's row
       if (kMasked) {
         int lim = p.N;
-        if (p.causal) lim = min(lim, HOOK == kHookNone ? vis_end : i + p.p_seq + 1);
+        if (p.causal) lim = min(lim, kRowLimit ? vis_end : i + p.p_seq + 1);
         nvis = max(0, min(128, lim - n0));
       }
 #define FAWS_VIS(x) (!kMasked || (x) < nvis)
@@ -808,7 +811,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
       }
       if constexpr (HOOK == kHookScoresAny) {
         // Staged as for the TMA stores, then written row by row by the warp itself.  Costs about as many shared-memory
-        // and store instructions as the TMA form's staging; fp32 B1 Hq28 Hk4 S1531 causal: 117 us, 1 180 us on the
+        // and store instructions as the TMA form's staging; fp32 B1 Hq28 Hk4 S1531 causal: 94 us, 1 180 us on the
         // CUDA-core kernel that took odd lengths before.
         const int r0 = r_tile + lg * 32, rows = min(32, p.m_end - r0);
         const int esize = p.scores_f32 ? 4 : 2;
