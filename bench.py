@@ -69,11 +69,9 @@ def algorithmic(cfg, op="scores", split=None):
         out_bytes = B * Hk * S * 4
     elif op == "cross_qk":
         out_bytes = B * Hk * split * 4
-    elif op == "cross_softmax":
+    elif op in ("cross_softmax", "cross_softmax_buffered"):
         extra = (S - split) * split
         out_bytes = B * Hk * split * 4
-    elif op == "cross_softmax_buffered":
-        out_bytes = B * Hk * split * 4 + 2 * 4 * B * Hq * (S - split) * split
     flops = B * Hq * D * (4 * pairs + 2 * extra)
     io = 2 * B * Hq * S * D * 2 + 2 * B * Hk * S * D * 2
     return flops, io + out_bytes

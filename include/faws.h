@@ -231,10 +231,12 @@ int faws_attention_cross_token_softmax_sum(const faws_problem* p, int32_t split,
 
 /*
  * Replaces attention_cross_token_softmax_sum_buffered
- * (attention_cross_token_softmax_sum.py:639-732).  Pass 1 stores the scaled
- * raw scores of the cross region only (queries >= split, keys < split; the
- * reference stores the whole (B,H,M,N) tensor, :705) in the workspace; pass 2
- * reads them back instead of recomputing q.k^T.
+ * (attention_cross_token_softmax_sum.py:639-732).  Where the tcgen05 kernels
+ * fit, the same two passes as above: a second q.k^T over the cross region is
+ * faster there than writing and reading its scores.  On the CUDA-core kernels
+ * pass 1 stores the scaled raw scores of the cross region only (queries >=
+ * split, keys < split; the reference stores the whole (B,H,M,N) tensor, :705)
+ * in the workspace and pass 2 reads them back.
  */
 int faws_attention_cross_token_softmax_sum_buffered(const faws_problem* p, int32_t split,
                                                     float* sum_out, int32_t per_q_head,
@@ -266,7 +268,8 @@ typedef struct faws_grads {
 int faws_attention_backward(const faws_problem* p, const faws_grads* g, void* workspace,
                             size_t workspace_bytes, void* stream);
 
-/* Bytes of scratch `op` needs for `p` (0 if none).  Alignment: 256 bytes. */
+/* Bytes of scratch `op` needs for `p` (0 if none).  Alignment: 256 bytes.  `p` is the call's own: tensors, family and
+ * dropout decide the kernels and with them the scratch. */
 size_t faws_workspace_bytes(int32_t op, const faws_problem* p, int32_t split);
 
 /*
