@@ -24,11 +24,15 @@
 // Modes.  kPlain rounds dS to the 16-bit type for its MMAs.  kFine keeps it as the sum of two 16-bit values
 // (dS = hi + lo, one more MMA per accumulator and K-step; 16 significant bits in bf16, 22 in fp16) and adds the G
 // heads' dK / dV from fp32 partials: problems that the CUDA-core kernels, which hold dS in fp32, would otherwise take
-// (head dims 16 and 32) keep their precision this way.  kDrop is kFine with the dropout mask, drawn again from the
+// (head dims 16 and 32) keep their precision this way.  In fp16 the 22 bits hold between 2^-3 and 2^16 only, so dS is
+// moved there by a power of two per head, from the largest |dout|, |v| and |delta| that the pre-pass meets
+// (GradScale), and moved back in the epilogue: exact, and gradients of any size come out as from fp32 dS.
+// kDrop is kFine with the dropout mask, drawn again from the
 // counter-based generator in both kernels.  Fine modes walk the tile in chunks of 16 streamed rows, the K-step of
 // the accumulating MMAs; hi and lo of a chunk take the 16 columns that its dP' leaves.  fp16 B4 H16 S1024 D64 causal,
-// p = 0.1, forward and backward: 336 us, 3 717 us with the CUDA-core kernels; errors of the gradients against fp64 as
-// there (2.32e-4, 2.28e-4, 2.92e-4 for dq, dk, dv, fp16).
+// p = 0.1, forward and backward: 270 us (266 without the power of two), 3 717 us with the CUDA-core kernels; errors of the gradients against fp64 as
+// there (2.32e-4, 2.28e-4, 2.92e-4 for dq, dk, dv, fp16; dout of 1e-4, where the results are fp16 subnormals: 1.6e-3,
+// 6.6e-3 with an unmoved dS).
 // Deterministic: every output element is written once, by one CTA, in a fixed order; with GQA the
 // key-major kernel writes per-query-head dK / dV and a second kernel adds the G heads in order.
 // Out-of-range query rows need no predicates: TMA zero-fills the loads (with L = delta = 0 their P is 1 and
@@ -99,7 +103,14 @@ struct BwTcParams {
   int D;               // the head dim (the instance's D is 64 for 16 and 32)
   DropoutParams drop;
   float keep_scale;    // 1 / (1 - p)
+  const float2* g_stat;  // kScaledDs: (B,Hq,g_blocks) bounds of |dout_i|^2 and |delta_i| over a pre-pass block's rows,
+  const float* v_stat;   // (B,Hk,v_blocks) of |v_j|^2
+  int g_blocks, v_blocks;
 };
+
+// Modes that move dS by a power of two before it is split: fp16 ones (bf16 has the range of fp32).
+template <typename T, int MODE>
+constexpr bool kScaledDs = MODE != kPlain && std::is_same<T, __half>::value;
 
 template <typename T> __device__ __forceinline__ uint32_t pack2(float a, float b);
 template <> __device__ __forceinline__ uint32_t pack2<__half>(float a, float b) {
@@ -111,22 +122,39 @@ template <> __device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float a, fl
   return *reinterpret_cast<uint32_t*>(&h);
 }
 
-// the same, held at the largest finite value (hi + lo reaches twice as far as fp16 itself)
-template <typename T> __device__ __forceinline__ uint32_t pack2_finite(float a, float b) {
-  if constexpr (std::is_same<T, __half>::value) {
-    uint32_t w;
-    asm("cvt.rn.satfinite.f16x2.f32 %0, %1, %2;" : "=r"(w) : "f"(b), "f"(a));
-    return w;
-  } else {
-    return pack2<T>(a, b);
-  }
-}
 template <typename T> __device__ __forceinline__ float2 unpack2(uint32_t w);
 template <> __device__ __forceinline__ float2 unpack2<__half>(uint32_t w) {
   return __half22float2(*reinterpret_cast<__half2*>(&w));
 }
 template <> __device__ __forceinline__ float2 unpack2<__nv_bfloat16>(uint32_t w) {
   return __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&w));
+}
+
+// The power of two for a head's dS, and its inverse.  |dS_ij| = P |keep dP_ij / (1 - p) - delta_i| is at most
+// |dout_i| |v_j| / (1 - p) + |delta_i| (Cauchy-Schwarz, P <= 1); that bound goes to [2^13, 2^14), a quarter of fp16's
+// range.  A bound of zero, infinity or NaN leaves dS as it is: infinities of the inputs reach the gradients.
+struct GradScale {
+  float mul, inv;
+};
+// largest of the warp's values, none of them negative (their bits order as they do)
+__device__ __forceinline__ float warp_max(float x) {
+  return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(x)));
+}
+__device__ __forceinline__ GradScale grad_scale(const BwTcParams& p, int b, int h, int hk, int lane) {
+  const float2* gs = p.g_stat + ((int64_t)b * p.Hq + h) * p.g_blocks;
+  const float* vs = p.v_stat + ((int64_t)b * (p.Hq / p.G) + hk) * p.v_blocks;
+  float g2 = 0.f, dl = 0.f, v2 = 0.f;
+  for (int x = lane; x < p.g_blocks; x += 32) {
+    const float2 s = gs[x];
+    g2 = fmaxf(g2, s.x);
+    dl = fmaxf(dl, s.y);
+  }
+  for (int x = lane; x < p.v_blocks; x += 32) v2 = fmaxf(v2, vs[x]);
+  const float bound = fmaf(p.keep_scale * sqrtf(warp_max(g2)), sqrtf(warp_max(v2)), warp_max(dl));
+  int k = 0;
+  if (bound > 0.f && bound < __int_as_float(0x7f800000))
+    k = max(-100, min(100, 13 - ((__float_as_int(bound) >> 23) - 127)));
+  return {__int_as_float((127 + k) << 23), __int_as_float((127 - k) << 23)};
 }
 
 template <typename T, int D, bool KM, int MODE>
@@ -330,6 +358,14 @@ tc_bwd_kernel(const __grid_constant__ BwMaps maps, const BwTcParams p, int* __re
       my_nl = p.negl2[vec_row + own];  // own < Mpad always
       my_dl = p.delta[vec_row + own];
     }
+    [[maybe_unused]] GradScale gsc{1.f, 1.f};
+    if constexpr (kScaledDs<T, MODE>) {
+      gsc = grad_scale(p, b, h, hk, lane);
+      my_dl *= gsc.mul;
+    }
+    // what a kept entry's dP is multiplied by (keep_scale is 1 without dropout); query-major kernels put the power of
+    // two here and on delta, key-major ones, whose delta comes with the streamed rows, on P
+    const float kept = KM ? p.keep_scale : p.keep_scale * gsc.mul;
     bool alive = true;
     for (int u = 0; u < nu; ++u) {
       if (!mbar_wait(&bars->s_full[e], u & 1, abort_flag)) { alive = false; break; }
@@ -375,15 +411,20 @@ tc_bwd_kernel(const __grid_constant__ BwMaps maps, const BwTcParams p, int* __re
               const float nl = y ? nl2.y : nl2.x, dl = y ? dl2.y : dl2.x;
               const bool vis = (c + x + y >= x_lo) && (c + x + y <= x_hi);
               const float pe = vis ? fast_exp2(fmaf(__uint_as_float(sv[x + y]), c2, nl)) : 0.f;
-              float ks = 1.f;
-              if constexpr (MODE == kDrop) ks = dropout_keep(p.drop, lin + (uint32_t)(c + x + y) * lin_step) ? p.keep_scale : 0.f;
-              pr[y] = pe * ks;
-              ds[y] = pe * fmaf(__uint_as_float(dv[x + y]), ks, -dl);
+              float ks = kept;
+              if constexpr (MODE == kDrop) ks = dropout_keep(p.drop, lin + (uint32_t)(c + x + y) * lin_step) ? kept : 0.f;
+              const float t = fmaf(__uint_as_float(dv[x + y]), ks, -dl);
+              if (KM) {
+                pr[y] = pe * ks;
+                ds[y] = pe * gsc.mul * t;
+              } else {
+                ds[y] = pe * t;
+              }
             }
-            pk[x / 2] = pack2<T>(pr[0], pr[1]);
-            hi[x / 2] = pack2_finite<T>(ds[0], ds[1]);
+            if (KM) pk[x / 2] = pack2<T>(pr[0], pr[1]);
+            hi[x / 2] = pack2<T>(ds[0], ds[1]);
             const float2 h2 = unpack2<T>(hi[x / 2]);
-            lo[x / 2] = pack2_finite<T>(ds[0] - h2.x, ds[1] - h2.y);
+            lo[x / 2] = pack2<T>(ds[0] - h2.x, ds[1] - h2.y);
           }
           if (KM) tmem_st8(t_s + c / 2, pk);  // (columns that this and earlier chunks have been read from)
           tmem_st8(t_dp + c, hi);
@@ -441,7 +482,7 @@ tc_bwd_kernel(const __grid_constant__ BwMaps maps, const BwTcParams p, int* __re
       // key-major: warpgroup 0 stores dV (acc0), warpgroup 1 stores dK (acc1, times sm_scale);
       // query-major: dQ (acc0, times sm_scale), warpgroup w takes the 64-column sub-tiles w, w + 2, ...
       const uint32_t t_acc = t_lane + COL_ACC + (KM ? (uint32_t)(e * D) : 0u);
-      const float oscale = (KM && e == 0) ? 1.f : p.sm_scale;
+      const float oscale = (KM && e == 0) ? 1.f : p.sm_scale * gsc.inv;
       const int sub_first = KM ? 0 : e, sub_step = KM ? 1 : 2;
       float* part = MODE == kPlain ? nullptr : (e == 0 ? p.part0 : p.part1);
       for (int sub = sub_first; sub < D / 64; sub += sub_step) {
@@ -513,19 +554,75 @@ tc_bwd_kernel(const __grid_constant__ BwMaps maps, const BwTcParams p, int* __re
 // 128-row tiles (zeros in the padding), so that the kernels can fetch a tile's 128 values with one
 // aligned bulk copy.  Bound by HBM: D / 8 lanes per row, 16 bytes of each operand a lane, four rows in flight
 // (bf16 B1 H28 S4096 D128: 15 us; 34 us with a warp and 4-byte loads to a row).
+// STATS: each block also leaves bounds of its rows' |dout_i|^2 and |delta_i|, and further blocks one of |v_j|^2, for
+// grad_scale.  The squared norms are bounded by D / 8 times the largest of a row's D / 8 pieces: at most 1.5 bits (3 in
+// the product) above the norms themselves, which would take three or four shuffles a row.
 constexpr int kPrepRows = 4;
+struct BwStats {
+  float2* g;
+  float* v;
+  int g_blocks, v_blocks;  // per query head, per kv head
+};
 template <typename T>
-__global__ void __launch_bounds__(256) bwd_prep_kernel(BwdParams p, float* negl2, float* delta, int Mpad, int blocks_per_head) {
+__device__ __forceinline__ float norm2(const uint4& w4) {
+  const uint32_t w[4] = {w4.x, w4.y, w4.z, w4.w};
+  float sum = 0.f;
+#pragma unroll
+  for (int y = 0; y < 4; ++y) {
+    const float2 a = unpack2<T>(w[y]);
+    sum = fmaf(a.x, a.x, fmaf(a.y, a.y, sum));
+  }
+  return sum;
+}
+// the block's (8 warps') largest x and y, in thread 0
+__device__ __forceinline__ float2 block_max(float x, float y, float2 (&red)[8]) {
+  x = warp_max(x);
+  y = warp_max(y);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = make_float2(x, y);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int w = 1; w < 8; ++w) {
+      x = fmaxf(x, red[w].x);
+      y = fmaxf(y, red[w].y);
+    }
+  }
+  return make_float2(x, y);
+}
+template <typename T, bool STATS>
+__global__ void __launch_bounds__(256) bwd_prep_kernel(BwdParams p, float* negl2, float* delta, int Mpad, BwStats st) {
   griddep_launch_dependents();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int lpr = p.D >> 3, rows_at_once = 32 / lpr, sub = lane & (lpr - 1);
-  const int bh = blockIdx.x / blocks_per_head;
-  const int i0 = (blockIdx.x - bh * blocks_per_head) * (8 * kPrepRows * rows_at_once) + warp * kPrepRows * rows_at_once +
-                 lane / lpr;
+  const int block_rows = 8 * kPrepRows * rows_at_once;
+  const int row0 = warp * kPrepRows * rows_at_once + lane / lpr;  // within the block's rows
+  [[maybe_unused]] __shared__ float2 red[8];
+  if constexpr (STATS) {
+    const int vb = (int)blockIdx.x - p.B * p.Hq * st.g_blocks;
+    if (vb >= 0) {
+      const int bk = vb / st.v_blocks, j0 = (vb - bk * st.v_blocks) * block_rows + row0;
+      const T* v = reinterpret_cast<const T*>(p.v) + (bk / p.Hk) * p.v_sb + (bk % p.Hk) * p.v_sh + 8 * sub;
+      uint4 vv[kPrepRows];
+#pragma unroll
+      for (int x = 0; x < kPrepRows; ++x) {
+        const int j = j0 + x * rows_at_once;
+        vv[x] = j < p.N ? *reinterpret_cast<const uint4*>(v + (int64_t)j * p.v_ss) : make_uint4(0u, 0u, 0u, 0u);
+      }
+      float v2 = 0.f;
+#pragma unroll
+      for (int x = 0; x < kPrepRows; ++x) v2 = fmaxf(v2, norm2<T>(vv[x]));
+      v2 = block_max(v2, 0.f, red).x;
+      if (threadIdx.x == 0) st.v[vb] = v2 * (float)lpr;
+      return;
+    }
+  }
+  const int bh = blockIdx.x / st.g_blocks;
+  const int i0 = (blockIdx.x - bh * st.g_blocks) * block_rows + row0;
   const int h = bh % p.Hq, b = bh / p.Hq;
   const T* o = reinterpret_cast<const T*>(p.o) + b * p.o_sb + h * p.o_sh + 8 * sub;
   const T* g = reinterpret_cast<const T*>(p.dout) + b * p.do_sb + h * p.do_sh + 8 * sub;
   uint4 ov[kPrepRows], gv[kPrepRows];
+  [[maybe_unused]] float g2 = 0.f, dl = 0.f;
 #pragma unroll
   for (int x = 0; x < kPrepRows; ++x) {
     const int i = i0 + x * rows_at_once;
@@ -538,6 +635,7 @@ __global__ void __launch_bounds__(256) bwd_prep_kernel(BwdParams p, float* negl2
 #pragma unroll
   for (int x = 0; x < kPrepRows; ++x) {
     const int i = i0 + x * rows_at_once;
+    if constexpr (STATS) g2 = fmaxf(g2, norm2<T>(gv[x]));
     const uint32_t ow[4] = {ov[x].x, ov[x].y, ov[x].z, ov[x].w}, gw[4] = {gv[x].x, gv[x].y, gv[x].z, gv[x].w};
     float sum = 0.f;
 #pragma unroll
@@ -546,6 +644,7 @@ __global__ void __launch_bounds__(256) bwd_prep_kernel(BwdParams p, float* negl2
       sum = fmaf(a.x, c.x, fmaf(a.y, c.y, sum));
     }
     for (int s = lpr >> 1; s > 0; s >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, s);
+    if constexpr (STATS) dl = fmaxf(dl, fabsf(sum));
     if (sub == 0 && i < Mpad) {
       float nl = 0.f;
       if (i < p.M) {
@@ -555,6 +654,10 @@ __global__ void __launch_bounds__(256) bwd_prep_kernel(BwdParams p, float* negl2
       delta[(int64_t)bh * Mpad + i] = sum;
       negl2[(int64_t)bh * Mpad + i] = nl;
     }
+  }
+  if constexpr (STATS) {
+    const float2 m = block_max(g2, dl, red);
+    if (threadIdx.x == 0) st.g[blockIdx.x] = make_float2(m.x * (float)lpr, m.y);
   }
 }
 
@@ -627,6 +730,30 @@ cudaError_t launch_overlapped(K kernel, dim3 grid, int threads, size_t smem, cud
 
 int mpad_of(int M) { return (M + BT - 1) / BT * BT; }
 
+// Blocks of the pre-pass that `rows` rows of one head take.
+int prep_blocks(int rows, int D) {
+  const int block_rows = 8 * kPrepRows * (256 / D);
+  return (rows + block_rows - 1) / block_rows;
+}
+
+// Workspace: [-L*log2e | delta | pre-pass statistics (fine modes) | per-head dK | per-head dV]
+struct BwWs {
+  size_t delta, g_stat, v_stat, dk, dv, total;
+};
+BwWs bwd_ws(int B, int Hq, int Hk, int M, int N, int D, bool fine) {
+  auto up = [](size_t x) { return (x + 255) & ~size_t(255); };
+  BwWs w{};
+  const size_t vec_bytes = up((size_t)B * Hq * mpad_of(M) * 4);
+  const size_t part_bytes = Hq != Hk ? up((size_t)B * Hq * N * D * (fine ? 4 : 2)) : 0;
+  w.delta = vec_bytes;
+  w.g_stat = 2 * vec_bytes;
+  w.v_stat = w.g_stat + (fine ? up((size_t)B * Hq * prep_blocks(mpad_of(M), D) * sizeof(float2)) : 0);
+  w.dk = w.v_stat + (fine ? up((size_t)B * Hk * prep_blocks(N, D) * sizeof(float)) : 0);
+  w.dv = w.dk + part_bytes;
+  w.total = w.dv + part_bytes;
+  return w;
+}
+
 template <typename T, int D, int MODE>
 cudaError_t launch_bwd_td(const BwdParams& p, cudaStream_t s) {
   using L = BwSmem<D>;
@@ -635,16 +762,18 @@ cudaError_t launch_bwd_td(const BwdParams& p, cudaStream_t s) {
   if ((e = set_max_smem_once(once_km, tc_bwd_kernel<T, D, true, MODE>, L::alloc)) != cudaSuccess) return e;
   if ((e = set_max_smem_once(once_qm, tc_bwd_kernel<T, D, false, MODE>, L::alloc)) != cudaSuccess) return e;
   const int Mpad = mpad_of(p.M);
-  const size_t vec_bytes = ((size_t)p.B * p.Hq * Mpad * 4 + 255) & ~size_t(255);
-  float* negl2 = p.delta;  // workspace: [-L*log2e | delta | per-head dK | per-head dV]
-  float* delta = reinterpret_cast<float*>(reinterpret_cast<char*>(p.delta) + vec_bytes);
-  char* part = reinterpret_cast<char*>(p.delta) + 2 * vec_bytes;
+  const BwWs ws = bwd_ws(p.B, p.Hq, p.Hk, p.M, p.N, p.D, MODE != kPlain);
+  char* base = reinterpret_cast<char*>(p.delta);
+  float* negl2 = p.delta;
+  float* delta = reinterpret_cast<float*>(base + ws.delta);
+  char *dk_part = base + ws.dk, *dv_part = base + ws.dv;
   using Part = typename std::conditional<MODE == kPlain, T, float>::type;
-  const size_t part_bytes = ((size_t)p.B * p.Hq * p.N * p.D * sizeof(Part) + 255) & ~size_t(255);
+  const BwStats st{reinterpret_cast<float2*>(base + ws.g_stat), reinterpret_cast<float*>(base + ws.v_stat),
+                   prep_blocks(Mpad, p.D), prep_blocks(p.N, p.D)};
   {
-    const int rows = 8 * kPrepRows * (256 / p.D);  // of one block
-    const int blocks_per_head = (Mpad + rows - 1) / rows;
-    bwd_prep_kernel<T><<<(unsigned)(p.B * p.Hq * blocks_per_head), 256, 0, s>>>(p, negl2, delta, Mpad, blocks_per_head);
+    constexpr bool kStats = kScaledDs<T, MODE>;
+    const unsigned blocks = (unsigned)(p.B * p.Hq * st.g_blocks + (kStats ? p.B * p.Hk * st.v_blocks : 0));
+    bwd_prep_kernel<T, kStats><<<blocks, 256, 0, s>>>(p, negl2, delta, Mpad, st);
     count_launch();
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
@@ -653,6 +782,7 @@ cudaError_t launch_bwd_td(const BwdParams& p, cudaStream_t s) {
   tp.sm_scale = p.sm_scale; tp.negl2 = negl2; tp.delta = delta; tp.D = p.D;
   tp.drop = p.drop;
   tp.keep_scale = 1.f / (1.f - p.drop.p);
+  tp.g_stat = st.g; tp.v_stat = st.v; tp.g_blocks = st.g_blocks; tp.v_blocks = st.v_blocks;
   int* status_word = tc_status_word();
   const bool per_head = p.G > 1;
   const bool map_parts = per_head && MODE == kPlain;  // 16-bit partials go through the store maps
@@ -675,11 +805,11 @@ cudaError_t launch_bwd_td(const BwdParams& p, cudaStream_t s) {
   {
     BwMaps m;
     if (per_head && !map_parts) {
-      tp.part0 = reinterpret_cast<float*>(part + part_bytes);
-      tp.part1 = reinterpret_cast<float*>(part);
+      tp.part0 = reinterpret_cast<float*>(dv_part);
+      tp.part1 = reinterpret_cast<float*>(dk_part);
     }
-    void* dv_dst = map_parts ? static_cast<void*>(part + part_bytes) : p.dv;
-    void* dk_dst = map_parts ? static_cast<void*>(part) : p.dk;
+    void* dv_dst = map_parts ? static_cast<void*>(dv_part) : p.dv;
+    void* dk_dst = map_parts ? static_cast<void*>(dk_part) : p.dk;
     const int o_heads = per_head && !map_parts ? p.Hk : p.Hq;  // (those maps are not used with fp32 partials)
     const int64_t ph_ss = p.D, ph_sh = (int64_t)p.N * p.D, ph_sb = (int64_t)p.Hq * p.N * p.D;
     if (!make_map_bhsd(&m.x, p.k, p.D, p.N, p.Hk, p.B, p.k_ss, p.k_sh, p.k_sb, 128) ||
@@ -700,8 +830,8 @@ cudaError_t launch_bwd_td(const BwdParams& p, cudaStream_t s) {
     const int64_t n = (int64_t)p.B * p.Hk * p.N * (p.D / 8);
     const dim3 grid((unsigned)((n + 255) / 256), 2, 1);
     const GroupSumOut dk{p.dk, p.dk_sb, p.dk_sh, p.dk_ss}, dv{p.dv, p.dv_sb, p.dv_sh, p.dv_ss};
-    if ((e = launch_overlapped(bwd_group_sum_kernel<T, Part>, grid, 256, 0, s, reinterpret_cast<const Part*>(part),
-                               reinterpret_cast<const Part*>(part + part_bytes), dk, dv, p.B, p.Hk, p.G, p.N, p.D)) !=
+    if ((e = launch_overlapped(bwd_group_sum_kernel<T, Part>, grid, 256, 0, s, reinterpret_cast<const Part*>(dk_part),
+                               reinterpret_cast<const Part*>(dv_part), dk, dv, p.B, p.Hk, p.G, p.N, p.D)) !=
         cudaSuccess)
       return e;
   }
@@ -718,9 +848,7 @@ cudaError_t launch_bwd_t(const BwdParams& p, cudaStream_t s) {
 }  // namespace
 
 size_t tc_bwd_workspace_bytes(int B, int Hq, int Hk, int M, int N, int D, bool dropout) {
-  const size_t vec_bytes = ((size_t)B * Hq * mpad_of(M) * 4 + 255) & ~size_t(255);
-  const size_t part_bytes = ((size_t)B * Hq * N * D * (dropout || D < 64 ? 4 : 2) + 255) & ~size_t(255);
-  return 2 * vec_bytes + (Hq != Hk ? 2 * part_bytes : 0);
+  return bwd_ws(B, Hq, Hk, M, N, D, dropout || D < 64).total;
 }
 
 bool tc_bwd_supported(const BwdParams& p, int dtype) {

@@ -118,6 +118,39 @@ def test_backward_fine_modes(shape, causal, p_drop, philox, dtype):
     assert F.device_status() == 0
 
 
+@pytest.mark.parametrize("shape,p_drop", [((1, 2, 2, 1024, 1024, 64), 0.1), ((1, 4, 2, 1100, 1100, 32), 0.0),
+                                          ((2, 2, 1, 200, 1025, 128), 0.5), ((1, 2, 2, 1030, 1030, 16), 0.0)],
+                         ids=lambda x: "x".join(map(str, x)) if isinstance(x, tuple) else str(x))
+@pytest.mark.parametrize("size", [1e-5, 1e-4, 1e-3, 5e3])
+def test_backward_fine_modes_over_the_size_of_the_gradient(shape, p_drop, size):
+    """fp16, gradients of a mean loss and of a scaled one: as close to the oracle as the CUDA-core kernels' fp32 dS.  The
+    large ones come with small q and k and large v, so that dS passes fp16's range and the results do not."""
+    B, Hq, Hk, M, N, D = shape
+    q, k, v, do = _inputs(shape, torch.float16, seed=N + D)
+    do = (do.float() * size).half()
+    if size > 1:
+        q, k, v = q * 0.01, k * 0.01, v * 16
+    philox = (17, 8) if p_drop else None
+    keep = orc.dropout_keep_mask(*philox, B, Hq, M, N, p_drop) if p_drop else None
+    ref = orc.attention_backward(q, k, v, do, True, p_seq=N - M, keep=keep, dropout_p=p_drop)
+    runs = {be: _run(q, k, v, do, True, dropout_p=p_drop, philox=philox, backend=be)[1:] for be in ("generic", "auto")}
+    assert F.last_backend() == "tcgen05"
+    for name, x, y, r in zip(("dq", "dk", "dv"), runs["auto"], runs["generic"], ref):
+        assert torch.isfinite(y).all() and torch.isfinite(x).all(), name
+        ex, ey = ((t.double().cpu() - r.double()).norm() for t in (x, y))
+        assert ex <= 1.02 * ey + 1e-6 * r.double().norm(), (name, ex.item(), ey.item())
+    assert F.device_status() == 0
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_backward_fine_modes_keep_infinities_visible(bad):
+    q, k, v, do = _inputs((1, 2, 2, 200, 200, 64), torch.float16, seed=2)
+    do[0, 1, 77, 5] = bad
+    _, dq, dk, dv = _run(q, k, v, do, True, dropout_p=0.1, philox=(3, 0))
+    assert not torch.isfinite(dq[0, 1, 77]).any() and not torch.isfinite(dk[0, 1, :70]).all(dim=-1).any()
+    assert torch.isfinite(dq[0, 0]).all() and torch.isfinite(dk[0, 0]).all() and torch.isfinite(dv[0, 0]).all()
+
+
 @pytest.mark.parametrize("D", [32, 64])
 @pytest.mark.parametrize("causal", [True, False], ids=["causal", "full"])
 def test_backward_with_very_negative_scores_and_a_ragged_last_key_tile(D, causal):
