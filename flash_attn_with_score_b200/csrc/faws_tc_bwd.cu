@@ -27,16 +27,15 @@
 // (head dims 16 and 32) keep their precision this way.  In fp16 the 22 bits hold between 2^-3 and 2^16 only, so dS is
 // moved there by a power of two per head, from the largest |dout|, |v| and |delta| that the pre-pass meets
 // (GradScale), and moved back in the epilogue: exact, and gradients of any size come out as from fp32 dS.
-// kDrop is kFine with the dropout mask, drawn again from the
-// counter-based generator in both kernels.  Fine modes walk the tile in chunks of 16 streamed rows, the K-step of
-// the accumulating MMAs; hi and lo of a chunk take the 16 columns that its dP' leaves.  fp16 B4 H16 S1024 D64 causal,
-// p = 0.1, forward and backward: 270 us (266 without the power of two), 3 717 us with the CUDA-core kernels; errors of the gradients against fp64 as
-// there (2.32e-4, 2.28e-4, 2.92e-4 for dq, dk, dv, fp16; dout of 1e-4, where the results are fp16 subnormals: 1.6e-3,
-// 6.6e-3 with an unmoved dS).
+// kDrop is kFine with the dropout mask, drawn again from the counter-based generator in both kernels.  Fine modes
+// walk the tile in chunks of 16 streamed rows, the K-step of the accumulating MMAs; hi and lo of a chunk take the 16
+// columns that its dP' leaves.  fp16 B4 H16 S1024 D64 causal, p = 0.1, forward and backward: 270 us (266 without the
+// power of two), 3 717 us with the CUDA-core kernels; errors of the gradients against fp64 as there (2.32e-4, 2.28e-4,
+// 2.92e-4 for dq, dk, dv, fp16; dout of 1e-4, where the results are fp16 subnormals: 1.6e-3, 6.6e-3 with an unmoved dS).
 // Deterministic: every output element is written once, by one CTA, in a fixed order; with GQA the
 // key-major kernel writes per-query-head dK / dV and a second kernel adds the G heads in order.
-// Out-of-range query rows need no predicates: TMA zero-fills the loads (with L = delta = 0 their P is 1 and
-// their dS is 0, and the zero Q / dout row contributes nothing); stores are clipped.  Every mbarrier wait is bounded.
+// Out-of-range query rows need no predicates without dropout: TMA zero-fills the loads (with L = delta = 0 their P
+// is 1 and their dS is 0, and the zero Q / dout row contributes nothing); stores are clipped.  Every mbarrier wait is bounded.
 #include <cuda.h>
 
 #include <type_traits>
@@ -378,6 +377,9 @@ tc_bwd_kernel(const __grid_constant__ BwMaps maps, const BwTcParams p, int* __re
       // P infinite, and infinity times the zero K row is not zero.
       int x_lo = 0, x_hi = HALF - 1;
       if (p.causal && KM) x_lo = own - p.p_seq - str0;
+      // Query rows beyond M are masked under dropout (key-major): against their zero dout rows stand weights of
+      // 1 / (1 - p), which fp16 need not hold.
+      if (KM && MODE == kDrop) x_hi = p.M - 1 - str0;
       if (!KM) x_hi = min(p.N - 1, p.causal ? own + p.p_seq : p.N - 1) - str0;
       const float* vl = reinterpret_cast<const float*>(smem + L::vec_off + (u % NSTAGE) * 1024) + e * HALF;
       const float* vd = vl + 128;

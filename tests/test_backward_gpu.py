@@ -151,6 +151,17 @@ def test_backward_fine_modes_keep_infinities_visible(bad):
     assert torch.isfinite(dq[0, 0]).all() and torch.isfinite(dk[0, 0]).all() and torch.isfinite(dv[0, 0]).all()
 
 
+@pytest.mark.parametrize("M", [100, 129, 128])
+def test_backward_with_dropout_close_to_one_and_a_ragged_last_query_tile(M):
+    """1 / (1 - p) = 1e5 is beyond fp16: the missing rows of the last query tile must not enter dV with it."""
+    q, k, v, do = _inputs((1, 8, 8, M, 2048, 64), torch.float16, seed=M)
+    runs = [_run(q, k, v, do, False, dropout_p=0.99999, philox=(5, 0), backend=be) for be in ("generic", "auto")]
+    assert F.last_backend() == "tcgen05"
+    for x, y in zip(*runs):
+        assert torch.isfinite(x).all() and torch.isfinite(y).all()
+        assert (x.double() - y.double()).norm() <= 2e-3 * x.double().norm()
+
+
 @pytest.mark.parametrize("D", [32, 64])
 @pytest.mark.parametrize("causal", [True, False], ids=["causal", "full"])
 def test_backward_with_very_negative_scores_and_a_ragged_last_key_tile(D, causal):
