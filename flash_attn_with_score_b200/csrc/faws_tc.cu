@@ -161,7 +161,7 @@ struct WorkList {
   uint16_t ids[kMaxListedItems];
 };
 
-template <typename T, int D, int HOOK, bool SPLIT, bool DROP = false>
+template <typename T, int D, int HOOK, bool SPLIT, bool DROP = false, bool FEW = false>
 __global__ void __launch_bounds__(NTHREADS, 1)
 tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __grid_constant__ WorkList wl,
               int* __restrict__ status) {
@@ -187,10 +187,13 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
   // index; persistent CTAs (never SPLIT, split-KV or fill launches) set it again for every item.
   constexpr bool kStoreHook =
       HOOK == kHookScores || HOOK == kHookScores16 || HOOK == kHookScoresAny;
-  // Only attention() packs heads, and the test costs the TMA score hook 1 %; in the odd-row hook it makes ptxas keep the
-  // row's limit in a register instead of spilling 68 bytes (bf16 B1 Hq28 Hk4 S1531: 99 -> 94 us).
-  constexpr bool kRowLimit = HOOK == kHookNone || HOOK == kHookScoresAny;
-  const int pack_m = kRowLimit ? p.pack_m : 0;
+  // FEW: attention() with few query rows, whose heads may be packed (pack_m).  An instance of its own: the run-time test
+  // and the register of the row's limit cost unpacked launches 1 to 4 % (bf16 B1 Hq32 Hk8 D64 causal, M512 N512: 8.75 us
+  // without, 9.10 with; M512 N4096: 30.7 and 31.7).  The odd-row score hook, which packs nothing, is compiled with it all
+  // the same: ptxas 12.9 then happens to need no spills there, 68 bytes without (bf16 B1 Hq28 Hk4 S1531: 94 and 99 us;
+  // neither an opaque limit nor an opaque count of visible columns has the effect).
+  static_assert(!FEW || ((HOOK == kHookNone || HOOK == kHookScoresAny) && !DROP), "attention() without dropout");
+  const int pack_m = FEW ? p.pack_m : 0;
   const bool persist = !SPLIT && !kStoreHook && wl.n_items > 0;  // (the launcher keeps the other instances plain)
   bool is_fill;
   int cb_rel, h, b, ksplit, kt0, hk, bh, ho, cb_abs, nt, rr_start;
@@ -646,7 +649,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
       int nvis = 128;  // visible columns form a prefix of the tile's row
       if (kMasked) {
         int lim = p.N;
-        if (p.causal) lim = min(lim, kRowLimit ? vis_end : i + p.p_seq + 1);
+        if (p.causal) lim = min(lim, FEW ? vis_end : i + p.p_seq + 1);
         nvis = max(0, min(128, lim - n0));
       }
 #define FAWS_VIS(x) (!kMasked || (x) < nvis)
@@ -1573,11 +1576,11 @@ bool make_work_list(const FwdParams& p, dim3 grid, int cta_rows, int ctas, WorkL
   return true;
 }
 
-template <typename T, int D, int HOOK, bool SPLIT, bool DROP = false>
+template <typename T, int D, int HOOK, bool SPLIT, bool DROP = false, bool FEW = false>
 cudaError_t launch_fwd_s(const TcMaps& maps, const FwdParams& p, cudaStream_t s) {
   using L = Smem<D, SPLIT>;
   static PerDeviceOnce attr_once;
-  if (cudaError_t e = set_max_smem_once(attr_once, tc_fwd_kernel<T, D, HOOK, SPLIT, DROP>, L::alloc); e != cudaSuccess)
+  if (cudaError_t e = set_max_smem_once(attr_once, tc_fwd_kernel<T, D, HOOK, SPLIT, DROP, FEW>, L::alloc); e != cudaSuccess)
     return e;
   const int ncb = (p.m_end - p.m_begin + L::kRows - 1) / L::kRows;
   FwdParams pp = p;
@@ -1616,7 +1619,7 @@ cudaError_t launch_fwd_s(const TcMaps& maps, const FwdParams& p, cudaStream_t s)
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   int* status_word = tc_status_word();
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, tc_fwd_kernel<T, D, HOOK, SPLIT, DROP>, maps, pp, *wl, status_word);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, tc_fwd_kernel<T, D, HOOK, SPLIT, DROP, FEW>, maps, pp, *wl, status_word);
   count_launch();
   return e != cudaSuccess ? e : cudaGetLastError();
 }
@@ -1659,7 +1662,14 @@ cudaError_t launch_fwd_h(const TcMaps& maps, const FwdParams& p, cudaStream_t s)
                            ctas128 > sm_count();
   static const bool forced = std::getenv("FAWS_SPLIT_KV") != nullptr;
   const bool split = use_split_kv(p) && (forced || !store_bound);
-  return split ? launch_fwd_s<T, D, HOOK, true>(maps, p, s) : launch_fwd_s<T, D, HOOK, false>(maps, p, s);
+  if constexpr (HOOK == kHookNone) {
+    if (p.pack_m > 0)
+      return split ? launch_fwd_s<T, D, HOOK, true, false, true>(maps, p, s)
+                   : launch_fwd_s<T, D, HOOK, false, false, true>(maps, p, s);
+  }
+  constexpr bool kFew = HOOK == kHookScoresAny;
+  return split ? launch_fwd_s<T, D, HOOK, true, false, kFew>(maps, p, s)
+               : launch_fwd_s<T, D, HOOK, false, false, kFew>(maps, p, s);
 }
 
 template <typename T, int D>
