@@ -178,9 +178,9 @@ class _AttentionFunction(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, do, *ignored):
-        if do is None:
-            return (None,) * 10
         q, k, v, o, L = ctx.saved_tensors
+        if do is None:  # nothing downstream had a gradient for out
+            return (*map(torch.zeros_like, (q, k, v)), *(None,) * 7)
         do = maybe_contiguous(do)
         c = _Call(q, k, v, ctx.causal, ctx.sm_scale, ctx.dropout_p, out=o, L=L, backend=ctx.backend,
                   philox=ctx.philox, rescale=True)
