@@ -261,13 +261,73 @@ int softmax_col_sums(const faws_problem* p, float* sum_out, int per_q_head, void
   return run_colsoftmax(p, c, sum_out, w.per_head, per_q_head ? 0 : 1, s);
 }
 
+int device_sms() {
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+
+// Expected time (us) of a score-free launch of `ctas` 128-row CTAs whose nkt key tiles are cut into s ranges: whole
+// waves of one CTA per SM, each a fixed part and its key tiles; with s > 1 the combine: a fixed part, its chain over the
+// ranges and the partial results through memory.  Fitted to 3 900 launches (bf16, 2 to 118 CTAs, 4 to 235 key tiles, 1 to
+// 128 ranges; 9 % rms).
+double launch_us(long long ctas, int nkt, int s, int D, long long rows, int sms) {
+  const long long waves = (ctas * s + sms - 1) / sms;
+  double us = (double)waves * (4.0 + (D == 128 ? 1.0 : 0.8) * cdiv(nkt, s));
+  if (s > 1) us += 3.0 + 0.15 * s + 0.22e-6 * (double)rows * s * D * 4;
+  return us;
+}
+
+struct SplitPlan {
+  int splits;
+  double us;  // expected
+};
+
+// Number of key ranges for a problem that leaves SMs idle.  First the plan of the reference's
+// num_splits_herustic (split_kv.py:234-262; its tiles are 16 x 128, here 128 x 128), i.e. the
+// smallest count whose wave efficiency is within 85 % of the best, among counts that leave no range
+// empty.  That plan knows no fixed costs: it cuts a dozen key tiles of 112 CTAs into six ranges for the sake of the last
+// wave.  Where launch_us expects more than 1.25 times the best count's time (inside that its own error could decide) the
+// best count is taken: bf16 D128 causal, B4 Hq16 Hk4 M200 N1500 17 us unsplit, 44 in six ranges; B2 H12 M500 N512 9.9 us
+// unsplit, 25.4 cut in four.
+SplitPlan plan_splits(const faws_problem* p, int sms) {
+  const long long ctas = (long long)p->B * p->Hq * cdiv(p->M, kTcBlockM);
+  const long long rows = (long long)p->B * p->Hq * p->M;
+  const int nkt = cdiv(p->N, kTcBlockN);
+  const SplitPlan whole{1, launch_us(ctas, nkt, 1, p->D, rows, sms)};
+  if (ctas * 10 >= 8LL * sms) return whole;
+  int max_splits = sms < nkt ? sms : nkt;
+  if (max_splits > 128) max_splits = 128;
+  if ((long long)p->B * max_splits > 65535) max_splits = 65535 / p->B;
+  double best_eff = 0.0;
+  double eff[129];
+  SplitPlan best = whole;
+  for (int s = 1; s <= max_splits; ++s) {
+    const int per = cdiv(nkt, s);
+    eff[s] = -1.0;
+    if (s > 1 && per * s - nkt >= per) continue;  // the last range would be empty
+    const double waves = (double)(ctas * s) / sms;
+    const double full = waves > (double)(long long)waves ? (double)((long long)waves + 1) : waves;
+    eff[s] = waves / full;
+    if (eff[s] > best_eff) best_eff = eff[s];
+    const double us = launch_us(ctas, nkt, s, p->D, rows, sms);
+    if (us < best.us) best = SplitPlan{s, us};
+  }
+  for (int s = 1; s <= max_splits; ++s)
+    if (eff[s] >= 0.85 * best_eff) {
+      const SplitPlan wave{s, launch_us(ctas, nkt, s, p->D, rows, sms)};
+      return best.us < 0.8 * wave.us ? best : wave;
+    }
+  return whole;
+}
+
 // Few query rows with grouped queries: the G query heads of a kv head are run as ONE head of G*M rows, so that
 // K and V are streamed once per 128 of those rows instead of once per query head and the rows of the 128-row tiles
 // are used.  Pure re-indexing: row r = g*M + i of the packed head is row i of query head hk*G + g, which for
 // contiguous heads (stride_h == M * stride_s) is a plain row stride; out and L index the same way.  The causal limit
 // of a packed row goes by its index within its head, `*pack_m` (0: no mask).  Taken when it visits fewer (query tile,
-// key tile) pairs than the heads one by one, whose causal tiles also skip the keys that none of their rows sees:
-// always for G*M <= 128, up to a few hundred rows against a long cache, not for self-attention.  bf16 D128 causal,
+// key tile) pairs than the heads one by one, whose causal tiles also skip the keys that none of their rows sees, and
+// (use_packed) the launch is expected to be shorter: fewer CTAs need not finish earlier.  bf16 D128 causal,
 // heads one by one and packed: B4 Hq32 Hk8 M16 N8192 72.9 and 31.9 us, B8 Hq28 Hk4 M40 N9000 150.5 and 68.3 us,
 // B1 Hq28 Hk4 M300 N30000 169 and 128 us, B2 Hq32 Hk8 M129 N8192 70.2 and 62.3 us.
 bool pack_gqa(const faws_problem* p, faws_problem* packed, int* pack_m) {
@@ -314,35 +374,12 @@ int use_packed(const faws_problem** p, faws_problem* packed) {
   if (!tc_allowed(*p) || !pack_gqa(*p, packed, &pack_m)) return 0;
   const FwdParams f = make_fwd_packed(packed, pack_m);
   if (f.v == nullptr || !tc_fwd_supported(f, packed->dtype)) return 0;
+  if (pack_m > 0 || packed->M > kTcBlockM) {  // (one unmasked tile instead of G is the same launch with fewer CTAs)
+    const int sms = device_sms();
+    if (plan_splits(packed, sms).us >= plan_splits(*p, sms).us) return 0;
+  }
   *p = packed;
   return pack_m;
-}
-
-// Number of key ranges for a problem that leaves most SMs idle: the plan of the reference's
-// num_splits_herustic (split_kv.py:234-262; its tiles are 16 x 128, here 128 x 128), i.e. the
-// smallest count whose wave efficiency is within 85 % of the best, among counts that leave no range
-// empty.
-int plan_splits(const faws_problem* p, int sms) {
-  const long long ctas = (long long)p->B * p->Hq * cdiv(p->M, kTcBlockM);
-  if (ctas * 10 >= 8LL * sms) return 1;
-  const int nkt = cdiv(p->N, kTcBlockN);
-  int max_splits = sms < nkt ? sms : nkt;
-  if (max_splits > 128) max_splits = 128;
-  if ((long long)p->B * max_splits > 65535) max_splits = 65535 / p->B;
-  double best = 0.0;
-  double eff[129];
-  for (int s = 1; s <= max_splits; ++s) {
-    const int per = cdiv(nkt, s);
-    eff[s] = -1.0;
-    if (s > 1 && per * s - nkt >= per) continue;  // the last range would be empty
-    const double waves = (double)(ctas * s) / sms;
-    const double whole = waves > (double)(long long)waves ? (double)((long long)waves + 1) : waves;
-    eff[s] = waves / whole;
-    if (eff[s] > best) best = eff[s];
-  }
-  for (int s = 1; s <= max_splits; ++s)
-    if (eff[s] >= 0.85 * best) return s;
-  return 1;
 }
 
 size_t split_kv_bytes(const faws_problem* p, int n_splits) {
@@ -389,9 +426,7 @@ int32_t faws_split_kv_plan(const faws_problem* p) {
   const int pack_m = use_packed(&p, &packed);
   const FwdParams f = make_fwd_packed(p, pack_m);
   if (!tc_fwd_supported(f, p->dtype)) return 1;
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return plan_splits(p, sms);
+  return plan_splits(p, device_sms()).splits;
 }
 
 int faws_attention_split_kv(const faws_problem* p, int32_t n_splits, void* workspace, size_t workspace_bytes,

@@ -87,6 +87,31 @@ def test_few_causal_rows_with_grouped_queries(shape, interleaved, dtype):
     assert F.device_status() == 0
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16], ids=["fp16", "bf16"])
+@pytest.mark.parametrize("shape,causal", [
+    ((16, 28, 4, 40, 515, 64), True),    # 280 packed rows in three tiles, 192 CTAs instead of 448
+    ((16, 28, 4, 40, 515, 128), True),
+    ((12, 32, 4, 33, 260, 32), True),    # 264 packed rows: the third tile has eight
+    ((20, 16, 2, 70, 300, 64), False),   # no mask: 560 packed rows in five tiles instead of eight
+], ids=lambda x: "x".join(map(str, x)) if isinstance(x, tuple) else ("causal" if x else "full"))
+def test_packed_heads_over_several_tiles(shape, causal, dtype):
+    """Shapes whose packed launch is the shorter one; the same call with heads that cannot be packed agrees."""
+    B, Hq, Hk, M, N, D = shape
+    q, k, v = _inputs(shape, dtype, seed=M)
+    ref_out, ref_scores = orc.naive_attention_with_scores(q, k, v, causal, p_seq=N - M)
+    slack = orc.bf16_out_slack(ref_scores, v, ref_out) if dtype == torch.bfloat16 else None
+    Lref = orc.log_normalizer(ref_scores)
+    qd, kd, vd = q.cuda(), k.cuda(), v.cuda()
+    apart = torch.empty(B, Hq, M + 8, D, device="cuda", dtype=dtype)[:, :, :M].copy_(qd)
+    for x in (qd, apart):
+        out, L, _, _, _ = F.attention(x, kd, vd, causal, return_log_normalizer=True)
+        assert F.last_backend() == "tcgen05"
+        ok, err = orc.check_out(out.cpu(), ref_out, slack)
+        assert ok, err
+        assert (L.cpu() - Lref).abs().max() < 2e-3
+    assert F.device_status() == 0
+
+
 def test_split_plan_follows_the_occupancy_rule():
     lib = _lib.load()
     q, k, v = (t.cuda() for t in _inputs((1, 4, 2, 16, 16384, 128), torch.float16))
@@ -107,3 +132,7 @@ def test_split_plan_follows_the_occupancy_rule():
     big = torch.empty(4, 32, 1024, 128, device="cuda", dtype=torch.float16)
     assert plan(big, big, big) == 1               # 1024 CTAs: enough work already
     del out
+    # 96 to 118 CTAs of a few key tiles: the wave rule alone would cut them, for three times the time
+    for B, Hq, Hk, M, N, causal in ((4, 16, 4, 200, 1500, True), (2, 12, 12, 500, 512, True), (1, 28, 4, 513, 513, False)):
+        qq, kk = (torch.empty(B, h, s, 128, device="cuda", dtype=torch.float16) for h, s in ((Hq, M), (Hk, N)))
+        assert plan(qq, kk, kk, causal) == 1, (B, Hq, M, N)
