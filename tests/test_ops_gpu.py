@@ -327,3 +327,22 @@ def test_every_cta_mode_of_the_forward_kernel(env):
                           "-m", "gpu", "-k", "tcgen05_family or determinism or strided"],
                          env=env, capture_output=True, text=True, timeout=600, cwd=root)
     assert res.returncode == 0, res.stdout[-3000:] + res.stderr[-2000:]
+
+
+@pytest.mark.parametrize("G,S", [(1, 128), (7, 128), (16, 256), (3, 300), (5, 1100), (1, 2200)])
+@pytest.mark.parametrize("causal", [True, False], ids=["causal", "full"])
+def test_raw_column_sums_over_groups_and_query_tiles(G, S, causal):
+    """The reduce kernel deals (query head, query tile) pairs to four thread groups: fewer pairs than groups, remainders of
+    the eight loads in flight, tiles before and behind the linear ones, a ragged last tile.  Against fp64, fp32 sums:
+    1e-6 of the sum of absolute values is eight times what 35 k additions in another order are off by."""
+    g = torch.Generator(device="cuda").manual_seed(S + G)
+    q, k, v = (torch.randn(2, h, S, 64, device="cuda", generator=g).half() for h in (2 * G, 2, 2))
+    s = q.double() @ k.double().repeat_interleave(G, 1).transpose(-1, -2) / 8.0
+    if causal:
+        s = s.tril()
+    for fn, rows, cols in ((F.attention_with_col_sum, 0, S), (F.attention_cross_token_qk_sum, S // 3, S // 3)):
+        args = () if rows == 0 else (rows,)
+        _, got = fn(q, k, v, *args, causal)
+        part = s[:, :, rows:, :cols].reshape(2, 2, -1, cols)
+        assert bool(((got - part.sum(2)).abs() <= 1e-6 * part.abs().sum(2) + 1e-6).all()), fn.__name__
+    assert F.last_backend() == "tcgen05" and F.device_status() == 0
