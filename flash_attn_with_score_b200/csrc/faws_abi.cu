@@ -4,6 +4,7 @@
 #include <cstdio>
 
 #include "faws_internal.cuh"
+#include "faws_tc_store.cuh"
 
 namespace faws {
 
@@ -382,6 +383,24 @@ int use_packed(const faws_problem** p, faws_problem* packed) {
   return pack_m;
 }
 
+// Whether the CUDA-core kernel is expected to be the faster one for a score-only problem: a few 64 x 64 tiles, a CTA each
+// in whole waves, against 128-row CTAs that walk the keys.  Lines through 630 launches (16-bit inputs, 1 to 120 CTAs, N 1
+// to 2047; ns): the tcgen05 kernel's fixed part and its time per key by the way its rows are stored, the CUDA-core
+// kernel's by head dim.  Asked only for D < 64 and, at 64, rows that TMA cannot write; at D 128 the
+// tcgen05 kernel won every launch.  fp16 D16 H4 S333 4.0 us against 9.5,
+// D64 H4 S301 6.8 against 8.6, D32 H12 S512 14.0 against 6.4.
+bool scores_only_on_cuda_cores(const ScoresOnlyParams& p, int sms) {
+  const bool tma = tma_score_rows(p.scores, p.N, p.scores_f32 ? 4 : 2), pairs = !p.scores_f32 && p.N % 2 == 0;
+  if (p.D > 64 || (tma && p.D == 64)) return false;
+  const double fixed = tma ? (p.scores_f32 ? 4000.0 : 3750.0) : (pairs ? 3850.0 : 4300.0);
+  const double per_key = tma ? (p.scores_f32 ? 8.6 : 5.2) : (pairs ? 8.5 : 13.0);
+  const long long heads = (long long)p.B * p.Hq;
+  const long long ctas = heads * cdiv(p.M, 128), tiles = heads * cdiv(p.M, 64) * cdiv(p.N, 64);
+  const double tc = fixed + (double)((ctas + sms - 1) / sms) * per_key * p.N;
+  const double cuda_cores = 2950.0 + 60.0 * p.D + (double)((tiles + sms - 1) / sms - 1) * (100.0 + 50.0 * p.D);
+  return cuda_cores < tc;
+}
+
 size_t split_kv_bytes(const faws_problem* p, int n_splits) {
   return align256((size_t)p->B * p->Hq * n_splits * p->M * 4) +
          align256((size_t)p->B * p->Hq * n_splits * p->M * p->D * 2);
@@ -477,7 +496,9 @@ int faws_compute_attention_scores(const faws_problem* p, void* scores, int32_t s
   sp.B = p->B; sp.Hq = p->Hq; sp.Hk = p->Hk; sp.M = p->M; sp.N = p->N; sp.D = p->D;
   sp.sm_scale = p->sm_scale;
   bool use_tc = false;
-  if (tc_allowed(p)) use_tc = tc_scores_only_supported(sp, p->dtype);
+  if (tc_allowed(p))
+    use_tc = tc_scores_only_supported(sp, p->dtype) &&
+             (p->backend == FAWS_BACKEND_TCGEN05 || !scores_only_on_cuda_cores(sp, device_sms()));
   if (p->backend == FAWS_BACKEND_TCGEN05 && !use_tc) return FAWS_EBACKEND;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const cudaError_t e = use_tc ? launch_tc_scores_only(sp, p->dtype, s) : launch_generic_scores_only(sp, p->dtype, s);

@@ -58,6 +58,42 @@ def test_scores_only_in_odd_rows(M, N, kind):
     assert bool(((s.float().cpu() - ref).abs() <= (1e-3 + rel) * ref.abs() + 1e-4).all())
 
 
+@pytest.mark.parametrize("M,N", [(5, 127), (129, 258), (257, 131)])
+@pytest.mark.parametrize("D", [16, 32])
+@pytest.mark.parametrize("kind", ["fp32", "fp16", "bf16"])
+def test_scores_in_odd_rows_at_small_head_dims(M, N, D, kind):
+    dtype = torch.bfloat16 if kind == "bf16" else torch.float16
+    q, k, v = _inputs(M, N, D, dtype)
+    ref_out, ref = orc.naive_attention_with_scores(q, k, v, False)
+    out, s = F.attention_with_scores(q.cuda(), k.cuda(), v.cuda(), False,
+                                     scores_dtype=torch.float32 if kind == "fp32" else dtype)
+    assert F.last_backend() == "tcgen05" and F.device_status() == 0
+    slack = orc.bf16_out_slack(ref, v, ref_out) if kind == "bf16" else None
+    ok, err = orc.check_out(out.cpu(), ref_out, slack)
+    assert ok, err
+    rel = {"fp32": 0.0, "fp16": 2.0 ** -11, "bf16": 2.0 ** -8}[kind]
+    assert bool(((s.float().cpu() - ref).abs() <= (1e-3 + rel) * ref.abs() + 1e-4).all())
+
+
+@pytest.mark.parametrize("B,M,N", [(16, 200, 131), (1, 129, 131), (1, 300, 257), (16, 130, 200)])
+@pytest.mark.parametrize("D", [16, 32, 64])
+@pytest.mark.parametrize("kind", ["fp32", "fp16", "bf16"])
+def test_scores_only_on_either_side_of_the_family_rule(B, M, N, D, kind):
+    """Few tiles of a small head dim go to the CUDA cores, 64 heads to the tcgen05 kernel, odd rows or not."""
+    dtype = torch.bfloat16 if kind == "bf16" else torch.float16
+    q, k, _ = _inputs(M, N, D, dtype)
+    ref = orc.naive_attention_with_scores(q, k, k, False)[1]
+    s = F.compute_attention_scores(q.cuda().repeat(B, 1, 1, 1), k.cuda().repeat(B, 1, 1, 1),
+                                   scores_dtype=torch.float32 if kind == "fp32" else dtype)
+    if B == 16:
+        assert F.last_backend() == "tcgen05"
+    elif D == 16 or N == 257:
+        assert F.last_backend() == "generic"
+    rel = {"fp32": 0.0, "fp16": 2.0 ** -11, "bf16": 2.0 ** -8}[kind]
+    assert bool(((s.float().cpu() - ref).abs() <= (1e-3 + rel) * ref.abs() + 1e-4).all())
+    assert F.device_status() == 0
+
+
 def test_window_of_odd_rows():
     M, N = 300, 301
     q, k, v = _inputs(M, N, 64, torch.float16)
