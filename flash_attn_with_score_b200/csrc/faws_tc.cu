@@ -1652,14 +1652,16 @@ cudaError_t launch_fwd_h(const TcMaps& maps, const FwdParams& p, cudaStream_t s)
   // Score-materialising causal launches with more CTAs than SMs are bound by their stores, not by the chain of key
   // tiles: measured, the 256-row CTAs (half as many set-ups) are faster there (fp16 D128 H32, 256 and 128 rows:
   // S1024 36.8 and 39.9 us, S768 27.0 and 26.5, S640 19.2 and 19.1).  When the 128-row CTAs all run at once the chain
-  // is what counts again (D128 H16 S768 22.4 and 15.8 us, H8 S640 16.0 and 12.7; D64 H8 S512 15.9 and 10.6).
+  // is what counts again (D128 H16 S768 22.4 and 15.8 us, H8 S640 16.0 and 12.7; D64 H8 S512 15.9 and 10.6; H37 S512,
+  // 148 CTAs, 19.1 and 15.8), but for three key tiles, which two warpgroups share badly, when nearly every SM has one
+  // (D128 S384 H40 13.3 and 12.0, H44 13.2 and 13.2, H49 13.2 and 14.1).
   if constexpr (HOOK != kHookScores16 && HOOK != kHookScoresAny) {
     // dropout: 256-row CTAs only (the mask generation, not the chain of key tiles, bounds it)
     if (p.drop.p > 0.f) return launch_fwd_s<T, D, HOOK, false, true>(maps, p, s);
   }
   const long long ctas128 = (long long)((p.m_end - p.m_begin + 127) / 128) * p.Hq * p.B;
   const bool store_bound = (HOOK == kHookScores || HOOK == kHookScores16 || HOOK == kHookScoresAny) && p.causal &&
-                           ctas128 > sm_count();
+                           ctas128 > ((p.N + BN - 1) / BN == 3 ? sm_count() * 7 / 8 : sm_count());
   static const bool forced = std::getenv("FAWS_SPLIT_KV") != nullptr;
   const bool split = use_split_kv(p) && (forced || !store_bound);
   if constexpr (HOOK == kHookNone) {
