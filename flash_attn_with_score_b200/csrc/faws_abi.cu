@@ -566,7 +566,10 @@ int faws_attention_cross_token_softmax_sum_buffered(const faws_problem* p, int32
   // a caller that forces the family gets it for the splits and options that its score buffer could serve
   if (p->backend == FAWS_BACKEND_TCGEN05 && p->M > split && (split % 32 != 0 || p->dropout_p > 0.f))
     return FAWS_EBACKEND;
-  const bool recompute = buffered_recomputes(p, split);
+  // Scratch without room for the score buffer, sized for the same shape where the call recomputes (other tensors: their
+  // alignment decides), serves the two passes on the CUDA-core kernels as well.
+  const bool recompute = buffered_recomputes(p, split) ||
+                         (p->backend == FAWS_BACKEND_AUTO && workspace_bytes < carve_softmax_ws(p, nullptr, split, split).total);
   return softmax_col_sums(p, sum_out, per_q_head, workspace, workspace_bytes, stream, split, split,
                           recompute ? 0 : split, recompute ? kRoundRobin : kForward);
 }
@@ -587,8 +590,11 @@ int faws_attention_backward(const faws_problem* p, const faws_grads* g, void* wo
       g->dout.ptr == nullptr || g->dq.ptr == nullptr || g->dk.ptr == nullptr || g->dv.ptr == nullptr)
     return FAWS_EINVAL;
   if (p->m_begin != 0 || p->m_end != p->M) return FAWS_EINVAL;
+  // Scratch sized for the same shape with 16-bit partial gradients (before dropout was turned on) is enough for the
+  // CUDA-core kernels, which then run unless the family is forced.
+  const size_t least = tc_bwd_workspace_bytes(p->B, p->Hq, p->Hk, p->M, p->N, p->D, false);
   const size_t need = faws_workspace_bytes(FAWS_OP_ATTENTION_BACKWARD, p, 0);
-  if (workspace == nullptr || workspace_bytes < need || misaligned_ws(workspace)) return FAWS_EWORKSPACE;
+  if (workspace == nullptr || workspace_bytes < least || misaligned_ws(workspace)) return FAWS_EWORKSPACE;
   BwdParams b{};
   b.q = p->q.ptr; b.k = p->k.ptr; b.v = p->v.ptr; b.o = p->out.ptr;
   b.dout = g->dout.ptr; b.dq = g->dq.ptr; b.dk = g->dk.ptr; b.dv = g->dv.ptr;
@@ -609,6 +615,10 @@ int faws_attention_backward(const faws_problem* p, const faws_grads* g, void* wo
   bool use_tc = false;
   if (tc_allowed(p)) use_tc = tc_bwd_supported(b, p->dtype);
   if (p->backend == FAWS_BACKEND_TCGEN05 && !use_tc) return FAWS_EBACKEND;
+  if (use_tc && workspace_bytes < need) {
+    if (p->backend == FAWS_BACKEND_TCGEN05) return FAWS_EWORKSPACE;
+    use_tc = false;
+  }
   // the tcgen05 path has its own pre-pass (delta and L into tile-padded arrays in the workspace)
   if (!use_tc && launch_bwd_delta(b, p->dtype, s) != cudaSuccess) return FAWS_ECUDA;
   const cudaError_t e = use_tc ? launch_tc_bwd(b, p->dtype, s) : launch_generic_bwd(b, p->dtype, s);
@@ -627,7 +637,7 @@ size_t faws_workspace_bytes(int32_t op, const faws_problem* p, int32_t split) {
       if (split < 1 || split > cdiv(p->N, kTcBlockN)) return 0;
       return split == 1 ? 0 : split_kv_bytes(p, split);
     case FAWS_OP_ATTENTION_BACKWARD:  // enough for either kernel family
-      return tc_bwd_workspace_bytes(p->B, p->Hq, p->Hk, p->M, p->N, p->D, p->dropout_p > 0.f);
+      return tc_bwd_workspace_bytes(p->B, p->Hq, p->Hk, p->M, p->N, p->D, p->dropout_p > 0.f || p->D < 64);
     case FAWS_OP_COL_SUM:
     case FAWS_OP_COL_SUM_SEQUENTIAL:
       return align256(partial_floats(p, 0, p->N) * 4) + align256(qsum_floats(p) * 4);

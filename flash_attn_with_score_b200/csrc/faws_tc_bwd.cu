@@ -849,8 +849,8 @@ cudaError_t launch_bwd_t(const BwdParams& p, cudaStream_t s) {
 
 }  // namespace
 
-size_t tc_bwd_workspace_bytes(int B, int Hq, int Hk, int M, int N, int D, bool dropout) {
-  return bwd_ws(B, Hq, Hk, M, N, D, dropout || D < 64).total;
+size_t tc_bwd_workspace_bytes(int B, int Hq, int Hk, int M, int N, int D, bool fine) {
+  return bwd_ws(B, Hq, Hk, M, N, D, fine).total;
 }
 
 bool tc_bwd_supported(const BwdParams& p, int dtype) {

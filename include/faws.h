@@ -269,7 +269,9 @@ int faws_attention_backward(const faws_problem* p, const faws_grads* g, void* wo
                             size_t workspace_bytes, void* stream);
 
 /* Bytes of scratch `op` needs for `p` (0 if none).  Alignment: 256 bytes.  `p` is the call's own: tensors, family and
- * dropout decide the kernels and with them the scratch. */
+ * dropout decide the kernels and with them the scratch.  With FAWS_BACKEND_AUTO the backward pass and the buffered
+ * cross-token sums also take what was asked for the same shape with other tensors or without dropout, and run on the
+ * CUDA-core kernels where it is too small for the tcgen05 ones or for the score buffer. */
 size_t faws_workspace_bytes(int32_t op, const faws_problem* p, int32_t split);
 
 /*
