@@ -96,7 +96,7 @@ tc_qk_scores_kernel(const __grid_constant__ ScMaps maps, const ScParams p, int* 
     mbar_fence_init();
     prefetch_tmap(&maps.q);
     prefetch_tmap(&maps.k);
-    prefetch_tmap(&maps.st);
+    if constexpr (TMA_OUT) prefetch_tmap(&maps.st);
   }
   if (warp == 1) {
     tmem_alloc(&bars->tmem_base, TMEM_COLS);
@@ -207,7 +207,7 @@ tc_qk_scores_kernel(const __grid_constant__ ScMaps maps, const ScParams p, int* 
         ++nstaged;
       }
     }
-    if (lane == 0) tma_store_wait<0>();
+    if (TMA_OUT && lane == 0) tma_store_wait<0>();
   }
 
   // ------------------------------------------------------------ common exit
