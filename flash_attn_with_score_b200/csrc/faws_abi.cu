@@ -403,7 +403,7 @@ bool scores_only_on_cuda_cores(const ScoresOnlyParams& p, int sms) {
 
 size_t split_kv_bytes(const faws_problem* p, int n_splits) {
   return align256((size_t)p->B * p->Hq * n_splits * p->M * 4) +
-         align256((size_t)p->B * p->Hq * n_splits * p->M * p->D * 2);
+         align256((size_t)p->B * p->Hq * n_splits * p->M * p->D * 4);
 }
 
 }  // namespace
@@ -465,11 +465,9 @@ int faws_attention_split_kv(const faws_problem* p, int32_t n_splits, void* works
   FwdParams f = make_fwd_packed(p, pack_m);
   if (!tc_allowed(p) || !tc_fwd_supported(f, p->dtype)) return FAWS_EBACKEND;
   float* L_part = static_cast<float*>(workspace);
-  char* o_part = static_cast<char*>(workspace) + align256((size_t)p->B * p->Hq * n_splits * p->M * 4);
-  f.o = o_part;
-  f.o_ss = p->D;
-  f.o_sh = (int64_t)p->M * p->D;  // per (query head, key range)
-  f.o_sb = (int64_t)p->Hq * n_splits * p->M * p->D;
+  float* o_part = reinterpret_cast<float*>(static_cast<char*>(workspace) +
+                                           align256((size_t)p->B * p->Hq * n_splits * p->M * 4));
+  f.o = o_part;  // (B, Hq, n_splits, M, D)
   f.L = L_part;
   f.n_splits = n_splits;
   f.tiles_per_split = cdiv(nkt, n_splits);

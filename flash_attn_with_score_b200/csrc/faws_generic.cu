@@ -638,23 +638,23 @@ __global__ void reduce_ranks_kernel(const float* parts, int n_ranks, int64_t cou
 // One-row decoding, bf16 Hq32 Hk8 N9001 D128: B8 59.6 -> 57.1 us, B1 20.7 -> 14.4 us against a plain launch of
 // scalar loads.
 template <typename T, int V>
-__device__ __forceinline__ void combine_row(const T* __restrict__ o_part, const float* __restrict__ Ls, int64_t M, T* orow,
+__device__ __forceinline__ void combine_row(const float* __restrict__ o_part, const float* __restrict__ Ls, int64_t M, T* orow,
                                             int64_t s_step, int d, float mx, float inv, int S) {
   static_assert(V == 2 || V == 4, "dims of a lane");
   float acc[V];
 #pragma unroll
   for (int x = 0; x < V; ++x) acc[x] = 0.f;
   for (int s0 = 0; s0 < S; s0 += 4) {
-    uint32_t w[4][V / 2];
+    __align__(16) float w[4][V];
     float l[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       l[e] = FAWS_NEG_INF;
       if (s0 + e < S) {
         l[e] = Ls[(int64_t)(s0 + e) * M];
-        const uint32_t* src = reinterpret_cast<const uint32_t*>(o_part + (int64_t)(s0 + e) * s_step + d);
-#pragma unroll
-        for (int x = 0; x < V / 2; ++x) w[e][x] = src[x];
+        const float* src = o_part + (int64_t)(s0 + e) * s_step + d;
+        if constexpr (V == 4) *reinterpret_cast<float4*>(w[e]) = *reinterpret_cast<const float4*>(src);
+        else *reinterpret_cast<float2*>(w[e]) = *reinterpret_cast<const float2*>(src);
       }
     }
 #pragma unroll
@@ -662,11 +662,7 @@ __device__ __forceinline__ void combine_row(const T* __restrict__ o_part, const 
       if (l[e] == FAWS_NEG_INF) continue;
       const float f = exp2f((l[e] - mx) * kLog2e);
 #pragma unroll
-      for (int x = 0; x < V / 2; ++x) {
-        const T* t = reinterpret_cast<const T*>(&w[e][x]);
-        acc[2 * x] += f * to_f(t[0]);
-        acc[2 * x + 1] += f * to_f(t[1]);
-      }
+      for (int x = 0; x < V; ++x) acc[x] += f * w[e][x];
     }
   }
   __align__(8) T res[V];  // (rows of 16-byte alignment: the forward kernel's condition)
@@ -677,7 +673,7 @@ __device__ __forceinline__ void combine_row(const T* __restrict__ o_part, const 
 }
 
 template <typename T>
-__global__ void combine_splits_kernel(const T* __restrict__ o_part, const float* __restrict__ L_part, T* out,
+__global__ void combine_splits_kernel(const float* __restrict__ o_part, const float* __restrict__ L_part, T* out,
                                       int64_t o_sb, int64_t o_sh, int64_t o_ss, float* L, int B, int Hq, int M, int D,
                                       int S) {
   ptx::griddep_wait();
@@ -700,7 +696,7 @@ __global__ void combine_splits_kernel(const T* __restrict__ o_part, const float*
   }
   const float inv = den > 0.f ? 1.f / den : 0.f;
   T* orow = out + b * o_sb + h * o_sh + (int64_t)i * o_ss;
-  const T* part = o_part + (bh * S * M + i) * (int64_t)D;
+  const float* part = o_part + (bh * S * M + i) * (int64_t)D;
   const int64_t s_step = (int64_t)M * D;
   if (D == 128) combine_row<T, 4>(part, Ls, M, orow, s_step, lane * 4, mx, inv, S);
   else if (lane * 2 < D) combine_row<T, 2>(part, Ls, M, orow, s_step, lane * 2, mx, inv, S);
@@ -803,7 +799,7 @@ cudaError_t launch_group_sum(const float* in, float* out, int B, int Hk, int G, 
   return cudaGetLastError();
 }
 
-cudaError_t launch_combine_splits(const void* o_part, const float* L_part, void* out, int64_t o_sb, int64_t o_sh,
+cudaError_t launch_combine_splits(const float* o_part, const float* L_part, void* out, int64_t o_sb, int64_t o_sh,
                                   int64_t o_ss, float* L, int B, int Hq, int M, int D, int n_splits, int dtype,
                                   cudaStream_t s) {
   const int64_t rows = (int64_t)B * Hq * M;
@@ -818,11 +814,9 @@ cudaError_t launch_combine_splits(const void* o_part, const float* L_part, void*
   cfg.numAttrs = 1;
   cudaError_t e;
   if (dtype == FAWS_FP16)
-    e = cudaLaunchKernelEx(&cfg, combine_splits_kernel<__half>, static_cast<const __half*>(o_part), L_part,
-                           static_cast<__half*>(out), o_sb, o_sh, o_ss, L, B, Hq, M, D, n_splits);
+    e = cudaLaunchKernelEx(&cfg, combine_splits_kernel<__half>, o_part, L_part, static_cast<__half*>(out), o_sb, o_sh, o_ss, L, B, Hq, M, D, n_splits);
   else
-    e = cudaLaunchKernelEx(&cfg, combine_splits_kernel<__nv_bfloat16>, static_cast<const __nv_bfloat16*>(o_part), L_part,
-                           static_cast<__nv_bfloat16*>(out), o_sb, o_sh, o_ss, L, B, Hq, M, D, n_splits);
+    e = cudaLaunchKernelEx(&cfg, combine_splits_kernel<__nv_bfloat16>, o_part, L_part, static_cast<__nv_bfloat16*>(out), o_sb, o_sh, o_ss, L, B, Hq, M, D, n_splits);
   if (e != cudaSuccess) return e;
   count_launch();
   return cudaGetLastError();

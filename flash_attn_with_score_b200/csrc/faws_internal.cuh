@@ -95,7 +95,7 @@ struct FwdParams {
   int lpt_order;         // set by the tcgen05 launcher: heaviest causal row blocks of all heads first
   int fill_ctas;         // set by the tcgen05 launcher: masked score tiles are written by extra CTAs
   int n_splits;          // split-KV: key ranges per (batch, head); 0 or 1 = off.  o and L then address the
-                         // partial buffers (B, Hq*n_splits, M, D) and (B, Hq, n_splits, M)
+                         // fp32 partial buffers (B, Hq*n_splits, M, D) and (B, Hq, n_splits, M)
   int tiles_per_split;   // key tiles per range
   int pack_m;            // > 0: the rows of a head are the pack_m query rows of each head of a group, one head after
                          // the other (see pack_gqa); the causal limit goes by the row's index within its head
@@ -209,9 +209,8 @@ cudaError_t launch_group_sum(const float* in, float* out, int B, int Hk, int G, 
                              cudaStream_t s);
 cudaError_t launch_reduce_ranks(const float* parts, int n_ranks, int64_t count, float* out,
                                 cudaStream_t s);
-// out (B,Hq,M,D) and L (B,Hq,M) or null from the split-KV partials o_part (B,Hq,S,M,D) in the dtype of q
-// and L_part (B,Hq,S,M)
-cudaError_t launch_combine_splits(const void* o_part, const float* L_part, void* out, int64_t o_sb, int64_t o_sh,
+// out (B,Hq,M,D) and L (B,Hq,M) or null from the split-KV partials o_part (B,Hq,S,M,D) and L_part (B,Hq,S,M)
+cudaError_t launch_combine_splits(const float* o_part, const float* L_part, void* out, int64_t o_sb, int64_t o_sh,
                                   int64_t o_ss, float* L, int B, int Hq, int M, int D, int n_splits, int dtype,
                                   cudaStream_t s);
 

@@ -63,7 +63,7 @@ constexpr float kRescaleThreshold = 8.0f;  // log2 units
 #define FAWS_NEG_INF (__int_as_float(0xff800000))
 
 struct TcMaps {
-  CUtensorMap q, k, v, o;  // o: 32-row store boxes of the output
+  CUtensorMap q, k, v, o;  // o: 32-row store boxes of the output (split keys: of the fp32 partial results)
   CUtensorMap st;          // scores store map
 };
 
@@ -187,7 +187,8 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
   // index; persistent CTAs (never SPLIT, split-KV or fill launches) set it again for every item.
   constexpr bool kStoreHook =
       HOOK == kHookScores || HOOK == kHookScores16 || HOOK == kHookScoresAny;
-  // FEW: attention() with few query rows, whose heads may be packed (pack_m).  An instance of its own: the run-time test
+  // FEW: attention() with few query rows, whose heads may be packed (pack_m) and keys split over CTAs (n_splits, with
+  // fp32 partial results).  An instance of its own: the run-time test
   // and the register of the row's limit cost unpacked launches 1 to 4 % (bf16 B1 Hq32 Hk8 D64 causal, M512 N512: 8.75 us
   // without, 9.10 with; M512 N4096: 30.7 and 31.7).  The odd-row score hook, which packs nothing, is compiled with it all
   // the same: ptxas 12.9 then happens to need no spills there, 68 bytes without (bf16 B1 Hq28 Hk4 S1531: 94 and 99 us;
@@ -1043,6 +1044,30 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
             *reinterpret_cast<uint4*>(ost + (kHalfStage ? 0 : (c >> 1) * 4096) + lane * 128 + ((cc ^ (lane & 7)) << 4)) = w;
           }
         };
+        // Split keys: partial results stay fp32 (16-bit ones put a second rounding into out: its distance from fp64 was
+        // 1.22 times that of an unsplit call).  A warp of up to eight rows writes them from its registers; more go through
+        // the operands' shared memory, where a warp's whole block has room beside the merged state (alternating halves of
+        // the staging block: 1 us more on a launch).
+        [[maybe_unused]] const bool part_f32 = FEW && p.n_splits > 1;
+        [[maybe_unused]] const bool part_direct = part_f32 && p.m_end - (r_tile + lg * 32) <= 8;
+        [[maybe_unused]] unsigned char* pst = smem + (SPLIT ? L::kv_off + L::kTile : L::q_off) + (warp - 4) * (32 * D * 4);
+        [[maybe_unused]] auto put_part = [&](int c, const uint32_t (&ro)[32]) {
+          if (part_direct) {
+            if (row_ok && c * 32 < p.D) {
+              float* dst = reinterpret_cast<float*>(p.o) +
+                           (((int64_t)b * p.Hq * p.n_splits + ho) * p.M + i) * p.D + c * 32;
+#pragma unroll
+              for (int g = 0; g < 8; ++g)
+                if (c * 32 + g * 4 < p.D)
+                  *reinterpret_cast<uint4*>(dst + g * 4) = make_uint4(ro[g * 4], ro[g * 4 + 1], ro[g * 4 + 2], ro[g * 4 + 3]);
+            }
+            return;
+          }
+#pragma unroll
+          for (int g = 0; g < 8; ++g)
+            *reinterpret_cast<uint4*>(pst + c * 4096 + lane * 128 + ((g ^ (lane & 7)) << 4)) =
+                make_uint4(ro[g * 4], ro[g * 4 + 1], ro[g * 4 + 2], ro[g * 4 + 3]);
+        };
         // (all D / 32 loads of the row in flight together measured 2-3 % slower: the registers they hold)
 #pragma unroll 1
         for (int c = 0; c < D / 32; ++c) {
@@ -1069,6 +1094,12 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
 #pragma unroll
             for (int x = 0; x < 32; ++x) ro[x] = __float_as_uint(__uint_as_float(ro[x]) * inv);
           }
+          if constexpr (FEW && HOOK == kHookNone) {
+            if (part_f32) {
+              put_part(c, ro);
+              continue;
+            }
+          }
           put_chunk(c, ro);
           if (kHalfStage && (c & 1) == 1) {
             fence_proxy_async_smem();
@@ -1079,7 +1110,20 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
             }
           }
         }
-        if (!kHalfStage) {
+        if constexpr (FEW && HOOK == kHookNone) {
+          static_assert(SPLIT ? 4 * 32 * D * 4 <= (L::kSlots - 1) * L::kTile
+                              : 8 * 32 * D * 4 <= L::kQTiles * L::kTile + L::kSlots * L::kTile, "room for the partial results");
+          if (part_f32 && !part_direct) {
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              for (int c = 0; c * 32 < p.D; ++c)
+                tma_store_3d(&maps.o, pst + c * 4096, c * 32, r_tile + lg * 32, b * p.Hq * p.n_splits + ho);
+              tma_store_commit();
+            }
+          }
+        }
+        if (!kHalfStage && !(HOOK == kHookNone && part_f32)) {
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
@@ -1088,7 +1132,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
             tma_store_commit();
           }
         }
-      } else if (row_ok) {
+      } else if (row_ok && !(FEW && p.n_splits > 1)) {  // (the combine leaves out ranges with L = -inf)
         // no key is visible to this query tile: its rows are zero
         T* orow = reinterpret_cast<T*>(p.o) + b * p.o_sb + ho * p.o_sh + (int64_t)i * p.o_ss;
         const uint4 z = make_uint4(0u, 0u, 0u, 0u);
@@ -1665,7 +1709,7 @@ cudaError_t launch_fwd_h(const TcMaps& maps, const FwdParams& p, cudaStream_t s)
   static const bool forced = std::getenv("FAWS_SPLIT_KV") != nullptr;
   const bool split = use_split_kv(p) && (forced || !store_bound);
   if constexpr (HOOK == kHookNone) {
-    if (p.pack_m > 0)
+    if (p.pack_m > 0 || p.n_splits > 1)
       return split ? launch_fwd_s<T, D, HOOK, true, false, true>(maps, p, s)
                    : launch_fwd_s<T, D, HOOK, false, false, true>(maps, p, s);
   }
@@ -1714,11 +1758,14 @@ cudaError_t launch_tc_fwd(const FwdParams& p, int dtype, cudaStream_t s) {
       !make_map_bhsd(&maps.k, p.k, p.D, p.N, p.Hk, p.B, p.k_ss, p.k_sh, p.k_sb, 128) ||
       !make_map_bhsd(&maps.v, p.v, p.D, p.N, p.Hk, p.B, p.v_ss, p.v_sh, p.v_sb, 128))
     return cudaErrorInvalidValue;
-  const char* obase = static_cast<const char*>(p.o) + (int64_t)p.m_begin * p.o_ss * 2;
-  // split-KV: p.o is the (B, Hq * n_splits, M, D) buffer of partial results
-  const int o_heads = p.Hq * (p.n_splits > 1 ? p.n_splits : 1);
-  if (!make_map_bhsd(&maps.o, obase, p.D, q_rows, o_heads, p.B, p.o_ss, p.o_sh, p.o_sb, 32)) return cudaErrorInvalidValue;
-  maps.st = maps.q;
+  maps.o = maps.st = maps.q;
+  if (p.n_splits > 1) {  // p.o is the (B, Hq * n_splits, M, D) fp32 buffer of partial results (m_begin is 0)
+    if (!make_map_store_f32(&maps.o, p.o, p.D, p.M, p.D, (int64_t)p.M * p.D, p.B * p.Hq * p.n_splits))
+      return cudaErrorInvalidValue;
+  } else {
+    const char* obase = static_cast<const char*>(p.o) + (int64_t)p.m_begin * p.o_ss * 2;
+    if (!make_map_bhsd(&maps.o, obase, p.D, q_rows, p.Hq, p.B, p.o_ss, p.o_sh, p.o_sb, 32)) return cudaErrorInvalidValue;
+  }
   if (p.scores != nullptr && tma_score_rows(p.scores, p.N, p.scores_f32 ? 4 : 2)) {
     const int esize = p.scores_f32 ? 4 : 2;
     char* base = static_cast<char*>(p.scores) + (int64_t)p.m_begin * p.N * esize;

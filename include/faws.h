@@ -135,8 +135,9 @@ int faws_attention_with_scores(const faws_problem* p, void* scores, int32_t scor
  * CTA per (batch, head, 128 query rows) would leave most SMs idle: replaces the split path of
  * FlashAttention.forward (flash.py:68-70,97-134; kernels split_kv.py:14-227).  The keys are cut
  * into n_splits contiguous ranges of whole 128-key tiles, each range is attended to by its own
- * CTAs, which leave a normalised partial result in the dtype of q and its log-normaliser in the
- * workspace (the reference's multiple_o / multiple_l, flash.py:106-107), and a combine kernel
+ * CTAs, which leave a normalised fp32 partial result and its log-normaliser in the workspace (the
+ * reference's multiple_o / multiple_l, flash.py:106-107, the former in the dtype of q there: with
+ * fp32 a split call is as close to exact as an unsplit one), and a combine kernel
  * merges the ranges in a fixed order (deterministic).  faws_split_kv_plan returns the number of
  * ranges the library would choose for p (the rule of split_kv.py:234-262; 1 = do not split: enough
  * CTAs already, dropout, a query-row window, or a problem the tcgen05 kernels cannot take).
