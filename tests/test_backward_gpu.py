@@ -36,7 +36,8 @@ def _run(q, k, v, do, causal, **kw):
     qd, kd, vd = (t.cuda().requires_grad_(True) for t in (q, k, v))
     out = F.attention(qd, kd, vd, causal, **kw)
     assert out.requires_grad and out.grad_fn is not None
-    out.backward(do.cuda())
+    with torch.autograd.set_multithreading_enabled(False):  # last_backend() is this thread's: the backward pass's from here on
+        out.backward(do.cuda())
     return out.detach(), qd.grad, kd.grad, vd.grad
 
 

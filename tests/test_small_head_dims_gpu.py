@@ -45,7 +45,7 @@ def test_small_head_dims_match_the_oracle(M, N, D, dtype, interleaved):
     check(F.attention_cross_token_softmax_sum(qd, kd, vd, split, causal),
           orc.group_sum(orc.cross_token_softmax_sum(ref_scores, split), Hk), "cross_softmax")
     o, s = F.attention_with_scores(qd, kd, vd, causal)
-    check((o,), None, "scores") if N % 4 == 0 else None
+    check((o,), None, "scores")
     ok, viol, ok_mask = orc.check_scores(s.cpu(), ref_scores)
     assert ok and ok_mask, viol
     assert F.device_status() == 0
@@ -60,7 +60,8 @@ def test_small_head_dims_backward(M, N, D, interleaved):
     q, k, v, do = (_rows(B, h, s, D, torch.float16, g, interleaved) for h, s in ((Hq, M), (Hk, N), (Hk, N), (Hq, M)))
     ref = orc.attention_backward(q, k, v, do, True, p_seq=N - M)
     qd, kd, vd = (t.cuda().requires_grad_(True) for t in (q, k, v))
-    got = torch.autograd.grad(F.attention(qd, kd, vd, True), (qd, kd, vd), do.cuda())
+    with torch.autograd.set_multithreading_enabled(False):  # last_backend() is this thread's
+        got = torch.autograd.grad(F.attention(qd, kd, vd, True), (qd, kd, vd), do.cuda())
     assert F.last_backend() == "tcgen05"
     for name, x, r, sl in zip(("dq", "dk", "dv"), got, ref, orc.grad_slack(q, k, v, do, True, p_seq=N - M)):
         ok, viol, err = orc.check_grad(x.cpu(), r, False, sl)
