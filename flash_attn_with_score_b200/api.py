@@ -350,7 +350,8 @@ def attention_cross_token_softmax_sum(q, k, v, split, causal=False, sm_scale=Non
 
 def attention_cross_token_softmax_sum_buffered(q, k, v, split, causal=False, sm_scale=None, dropout_p=0.0,
                                                *, per_q_head=False, q_rows=None, backend=None, philox=None):
-    """Same sums as ``attention_cross_token_softmax_sum``; the first pass stores the cross
+    """Same sums as ``attention_cross_token_softmax_sum``, and the same two passes where the tcgen05 kernels run (a second
+    q.k^T is faster there than storing the region's scores); on the CUDA-core kernels the first pass stores the cross
     region's scores and the second reads them back (attention_cross_token_softmax_sum.py:639-732).
     ``dropout_p`` is accepted and ignored, as in the reference (:646,713-730)."""
     N = k.shape[2]

@@ -121,7 +121,7 @@ int run_colsoftmax(const faws_problem* p, ColSoftmaxParams& c, float* final_out,
                    int group_sum, cudaStream_t s) {
   bool use_tc = false;
   if (tc_allowed(p)) use_tc = tc_colsoftmax_supported(c, p->dtype);
-  if (p->backend == FAWS_BACKEND_TCGEN05 && !use_tc && c.s_scratch == nullptr) return FAWS_EBACKEND;
+  if (p->backend == FAWS_BACKEND_TCGEN05 && !use_tc) return FAWS_EBACKEND;
   cudaError_t e;
   if (c.s_scratch != nullptr) {  // buffered variant: stream the stored scores back
     // one CTA per (128 keys, query head): G times more CTAs in flight than walking the group inside
@@ -220,8 +220,9 @@ SoftmaxWs carve_softmax_ws(const faws_problem* p, void* ws, int n_end, int split
 // Whether the buffered cross-token operator runs without its score buffer, as the second q.k^T of the two-pass
 // operator: whenever both passes fit the tcgen05 kernels, which contract the cross region faster than they could
 // write and read its scores.  fp16 D128 causal, B1 H32 S2048 split 768: 73 us against 100; B1 H32 S4096 split 2048:
-// 176 against 354; full B1 H8 S8192 split 4096: 333 against 440; B1 H32 S512 split 256: 18.3 against 20.1; split not a
-// multiple of 32 (a buffer that TMA could not write; B1 H32 S1024 split 400, full): 41 against 899.  The buffer stays
+// 176 against 354; full B1 H8 S8192 split 4096: 333 against 440; B1 H32 S512 split 256: 18 against 20; split not a
+// multiple of 32 (a buffer that TMA could not write; B1 H32 S1024 split 400, full): 41 against 899.  Only regions of 64
+// query rows or fewer were up to 9 % faster with the buffer (B1 H32 S256 split 192: 12.5 us against 11.6).  It stays
 // for the CUDA-core kernels, where the second q.k^T is the dearer one.
 bool buffered_recomputes(const faws_problem* p, int split) {
   if (!tc_allowed(p) || p->v.ptr == nullptr || p->out.ptr == nullptr) return false;

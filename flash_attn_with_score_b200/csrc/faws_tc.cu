@@ -814,9 +814,9 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
         }
       }
       if constexpr (HOOK == kHookScoresAny) {
-        // Staged as for the TMA stores, then written row by row by the warp itself.  Costs about as many shared-memory
-        // and store instructions as the TMA form's staging; fp32 B1 Hq28 Hk4 S1531 causal: 94 us, 1 180 us on the
-        // CUDA-core kernel that took odd lengths before.
+        // Staged as for the TMA stores, then written row by row by the warp itself: 128 row loads and, in place of four
+        // TMA instructions, 128 row stores per tile and warp.  fp32 B1 Hq28 Hk4 S1531 causal: 94 us (62 us at S1536,
+        // where TMA stores), 1 180 us on the CUDA-core kernel that took odd lengths before.
         const int r0 = r_tile + lg * 32, rows = min(32, p.m_end - r0);
         const int esize = p.scores_f32 ? 4 : 2;
         char* dst = static_cast<char*>(p.scores) + (((int64_t)bh * p.M + r0) * p.N + n0) * esize;

@@ -29,9 +29,11 @@ inline EncodeTiledFn get_encode() {
 
 // Head dims the tcgen05 kernels take: instances for D = 128 and D = 64, the latter also for 32 and 16.  There the
 // 64-element boxes reach past the row's end: loads fill the missing columns with zeros (which add nothing to Q.K^T
-// and give zero columns of P.V), stores leave them out.  The padding costs tensor time that these shapes do not
-// lack: at D <= 64 a tile is bound by its exponentials.  Measured against the CUDA-core kernels that took these
-// dims before (fp16, B16 H8 S785 D32, softmax column sums): 1 640 us -> 117 us.
+// and give zero columns of P.V), stores leave them out.  The padding doubles or quadruples the tensor work, which is not
+// what bounds a tile there: its chain from one S to the next is (35 us of 117 are exponentials, fp16 B16 H8 S785 D32,
+// softmax column sums; the CUDA-core kernels that took these dims before needed 1 640 us).  The weights are 16-bit
+// on both families; exponentials here are ex2.approx.ftz, exp2f there (2^-22 and 2 ulp; results below 2^-126 are zero
+// here).
 inline bool tc_head_dim(int D) { return D == 16 || D == 32 || D == 64 || D == 128; }
 
 // (rows, 64 x 16-bit) boxes out of a (B, H, S, D) view

@@ -139,7 +139,8 @@ int faws_attention_with_scores(const faws_problem* p, void* scores, int32_t scor
  * reference's multiple_o / multiple_l, flash.py:106-107, the former in the dtype of q there: with
  * fp32 a split call is as close to exact as an unsplit one), and a combine kernel
  * merges the ranges in a fixed order (deterministic).  faws_split_kv_plan returns the number of
- * ranges the library would choose for p (the rule of split_kv.py:234-262; 1 = do not split: enough
+ * ranges the library would choose for p (the rule of split_kv.py:234-262, or the count with the
+ * shortest expected time where that rule's is much longer; 1 = do not split: enough
  * CTAs already, dropout, a query-row window, or a problem the tcgen05 kernels cannot take).
  * Workspace: faws_workspace_bytes(FAWS_OP_ATTENTION_SPLIT_KV, p, n_splits).  Dropout is refused
  * (FAWS_EUNSUPPORTED), as in the reference (flash.py:98).
@@ -233,8 +234,8 @@ int faws_attention_cross_token_softmax_sum(const faws_problem* p, int32_t split,
 /*
  * Replaces attention_cross_token_softmax_sum_buffered
  * (attention_cross_token_softmax_sum.py:639-732).  Where the tcgen05 kernels
- * fit, the same two passes as above: a second q.k^T over the cross region is
- * faster there than writing and reading its scores.  On the CUDA-core kernels
+ * fit, the same two passes as above: a second q.k^T over the cross region
+ * costs less there than writing and reading its scores.  On the CUDA-core kernels
  * pass 1 stores the scaled raw scores of the cross region only (queries >=
  * split, keys < split; the reference stores the whole (B,H,M,N) tensor, :705)
  * in the workspace and pass 2 reads them back.
