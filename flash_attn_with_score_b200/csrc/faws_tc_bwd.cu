@@ -13,14 +13,17 @@
 //   P' = exp(S'*scale - L), dS' = P' * (dP' - delta) in registers, written back to TMEM as 16-bit
 //   operands over S' and dP', then the accumulating MMAs (A operand from TMEM).
 //
-// The 128 streamed rows are processed as two halves of 64 with their own TMEM columns, each by
-// its own consumer warpgroup, so the tensor pipe works on one half while the other is in registers.
-// (Measured alternatives, all slower on the same box: four parts of 32 with four consumer
-// warpgroups, 1.5-1.7x; S' and dP' as full 128-column MMAs handed back in four chunks, 1.15-1.25x;
-// separate barriers for S' and dP' plus a hand-off per 32-column chunk, 1.1-1.2x.)
-// Warp roles (12 warps): warp 0 TMA producer (X, Y once, then a 2-stage ring of (A, B) pairs and,
-// key-major, the L / delta vectors of the streamed query tile), warp 1 TMEM allocation and the
-// MMA-issuing lane, warps 4-7 / 8-11 consumers of half 0 / 1 (thread = owned row = TMEM lane).
+// The tensor pipe is kept busy by the order of a step's MMAs, each group of 128 x 128 x D:
+//   key-major     dV += P_u^T.dout_u | S'_u+1 | dK += dS_u^T.Q_u | dP'_u+1     (S' and P share columns, dP' and dS too)
+//   query-major   S'_u+1 | dP'_u+1 | dQ += dS_u.K_u                            (two dP' buffers; S' is free once read)
+// so that P is computed while dK and dP' run, and dS while dV and the next S' do.  S' and dP' are whole 128-column MMAs:
+// with 64 columns an MMA reads 6 KB of shared memory per 32 cycles (51 cycles measured), with 128 8 KB per 64 (65
+// measured).  One thread issues them: the pipe's queue holds about six, and a whole warp that elects a lane for each
+// group spends another 100 cycles between groups (4 340 against 3 390 cycles a step, key-major D128).
+// The 128 streamed rows are shared out to two consumer warpgroups, 64 rows each.
+// Warp roles (12 warps): warp 0 TMA producer (X, Y once, then rings of A and B tiles), warp 1 TMEM allocation and
+// the MMA-issuing thread, warp 2 (key-major) the L / delta vectors of the streamed query tiles, warps 4-7 / 8-11
+// consumers of half 0 / 1 (thread = owned row = TMEM lane).
 // Modes.  kPlain rounds dS to the 16-bit type for its MMAs.  kFine keeps it as the sum of two 16-bit values
 // (dS = hi + lo, one more MMA per accumulator and K-step; 16 significant bits in bf16, 22 in fp16) and adds the G
 // heads' dK / dV from fp32 partials: problems that the CUDA-core kernels, which hold dS in fp32, would otherwise take
@@ -51,7 +54,6 @@ using namespace ptx;
 constexpr int BT = 128;        // tile edge (owned rows and streamed rows)
 constexpr int HALF = 64;       // streamed rows per consumer warpgroup
 constexpr int NTHREADS = 384;
-constexpr int NSTAGE = 2;
 constexpr int TMEM_COLS = 512;
 constexpr int REGS_LAUNCH = 168;
 constexpr int REGS_AUX = 88;
@@ -61,31 +63,37 @@ constexpr float kLog2e = 1.4426950408889634f;
 
 enum BwMode : int { kPlain = 0, kFine = 1, kDrop = 2 };
 
-// TMEM columns: S'_0, S'_1, dP'_0, dP'_1 (64 fp32 columns each), then the accumulators.
-constexpr uint32_t COL_S = 0, COL_DP = 128, COL_ACC = 256;
-
-template <int D>
+template <int D, bool KM>
 struct BwSmem {
   static constexpr int kTile = 128 * D * 2;
   static constexpr int kSub = 128 * 128;  // one 64-element-wide sub-tile: 128 rows x 128 B
+  // A tiles are held from S' to the last accumulating MMA of their step, B tiles for a shorter time
+  static constexpr int kStagesA = D == 128 ? 3 : 4, kStagesB = D == 128 ? 2 : 4;
+  // TMEM: S' buffers, dP' buffers (128 fp32 columns each), then the accumulators
+  static constexpr int kSBufs = KM && D == 64 ? 2 : 1, kDpBufs = KM ? 1 : 2;
+  static_assert((kSBufs + kDpBufs) * 128 + (KM ? 2 : 1) * D <= TMEM_COLS, "TMEM");
   static constexpr int x_off = 0;
   static constexpr int y_off = kTile;
-  static constexpr int ring_off = 2 * kTile;                    // NSTAGE x (A tile, B tile)
-  static constexpr int vec_off = ring_off + NSTAGE * 2 * kTile; // NSTAGE x (128 -L*log2e, 128 delta) floats
-  static constexpr int bar_off = vec_off + NSTAGE * 1024;
-  static constexpr int total = bar_off + 256;
-  static constexpr int alloc = total + 1024;
+  static constexpr int a_off = 2 * kTile;
+  static constexpr int b_off = a_off + kStagesA * kTile;
+  static constexpr int vec_off = b_off + kStagesB * kTile;  // 2 x (128 -L*log2e, 128 -delta) floats
+  static constexpr int bar_off = vec_off + (KM ? 2 * 1024 : 0);
+  static constexpr int total = bar_off + 384;
 };
 
 struct BwBars {
-  uint64_t x_full;
-  uint64_t r_full[NSTAGE], r_empty[NSTAGE];
-  uint64_t s_full[2];   // per half: S' and dP' written by the tensor pipe
-  uint64_t p_ready[2];  // per half: P' and dS' written by its 128 consumer threads
+  uint64_t x_full, y_full;
+  uint64_t a_full[4], a_empty[4], b_full[4], b_empty[4];
+  uint64_t s_full[2], dp_full[2];  // per buffer: written by the tensor pipe
+  uint64_t s_free;                 // query-major: S' is in the consumers' registers
+  uint64_t p_ready[2][2][2];       // key-major, per S' buffer, warpgroup, 32 of its streamed rows: P' written
+  uint64_t ds_ready[2][2];         // per dP' buffer, warpgroup: dS' written
+  uint64_t vec_full[2], vec_empty[2];
   uint64_t acc_done;
   uint32_t tmem_base;
   int abort_flag;
 };
+static_assert(sizeof(BwBars) <= 384, "room for the barriers");
 
 struct BwMaps {
   CUtensorMap x, y, a, b;  // loads, 128-row boxes
@@ -96,7 +104,7 @@ struct BwTcParams {
   int Hq, G, M, N, p_seq, causal, Mpad;
   float sm_scale;
   const float* negl2;  // (B,Hq,Mpad): -L_i * log2(e), 0 for padded rows and rows without a visible key
-  const float* delta;  // (B,Hq,Mpad): sum_d out_id * dout_id, 0 for padded rows
+  const float* neg_delta;  // (B,Hq,Mpad): -sum_d out_id * dout_id, 0 for padded rows
   float* part0;        // fine modes with grouped queries: fp32 (B,Hq,N,D) per-head dV and dK instead of the
   float* part1;        // store maps; null otherwise
   int D;               // the head dim (the instance's D is 64 for 16 and 32)
@@ -159,13 +167,18 @@ __device__ __forceinline__ GradScale grad_scale(const BwTcParams& p, int b, int 
 template <typename T, int D, bool KM, int MODE>
 __global__ void __launch_bounds__(NTHREADS, 1)
 tc_bwd_kernel(const __grid_constant__ BwMaps maps, const BwTcParams p, int* __restrict__ status) {
-  using L = BwSmem<D>;
-  extern __shared__ unsigned char smem_dyn[];
-  unsigned char* smem = reinterpret_cast<unsigned char*>(
-      (reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
+  using L = BwSmem<D, KM>;
+  constexpr int NA = L::kStagesA, NB = L::kStagesB;
+  constexpr int NSB = L::kSBufs, NDB = L::kDpBufs;
+  constexpr uint32_t COL_DP = NSB * 128, COL_ACC = (NSB + NDB) * 128;
+  extern __shared__ __align__(1024) unsigned char smem[];
   BwBars* bars = reinterpret_cast<BwBars*>(smem + L::bar_off);
   volatile int* abort_flag = &bars->abort_flag;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (smem_u32(smem) & 1023u) {  // 128-byte swizzle atoms are 1 KB; the full shared memory leaves no slack to align by
+    if (threadIdx.x == 0 && status != nullptr) atomicExch(status, 1);
+    return;
+  }
 
   // Heaviest work first in launch order: key-major, the first key tiles see the most queries when
   // causal; query-major, the last query tiles see the most keys.
@@ -196,14 +209,26 @@ tc_bwd_kernel(const __grid_constant__ BwMaps maps, const BwTcParams p, int* __re
   }
   if (threadIdx.x == 0) {
     mbar_init(&bars->x_full, 1);
-    for (int s = 0; s < NSTAGE; ++s) {
-      mbar_init(&bars->r_full[s], 1);
-      mbar_init(&bars->r_empty[s], 1);
+    mbar_init(&bars->y_full, 1);
+    for (int s = 0; s < NA; ++s) {
+      mbar_init(&bars->a_full[s], 1);
+      mbar_init(&bars->a_empty[s], 1);
     }
-    for (int e = 0; e < 2; ++e) {
-      mbar_init(&bars->s_full[e], 1);
-      mbar_init(&bars->p_ready[e], 128);
+    for (int s = 0; s < NB; ++s) {
+      mbar_init(&bars->b_full[s], 1);
+      mbar_init(&bars->b_empty[s], 1);
     }
+    for (int w = 0; w < 2; ++w) {
+      mbar_init(&bars->s_full[w], 1);
+      mbar_init(&bars->dp_full[w], 1);
+      mbar_init(&bars->vec_full[w], 1);
+      mbar_init(&bars->vec_empty[w], 8);
+      for (int e = 0; e < 2; ++e) {
+        for (int c = 0; c < 2; ++c) mbar_init(&bars->p_ready[w][e][c], 128);
+        mbar_init(&bars->ds_ready[w][e], 128);
+      }
+    }
+    mbar_init(&bars->s_free, 256);
     mbar_init(&bars->acc_done, 1);
     bars->abort_flag = 0;
     mbar_fence_init();
@@ -228,118 +253,134 @@ tc_bwd_kernel(const __grid_constant__ BwMaps maps, const BwTcParams p, int* __re
     reg_dealloc<REGS_AUX>();
     if (warp == 0 && lane == 0 && nu > 0) {
       // ---------------------------------------------------------- TMA producer
-      const int x_head = KM ? hk : h;
-      mbar_arrive_expect_tx(&bars->x_full, 2 * L::kTile);
-      for (int c = 0; c < D / 64; ++c) {
-        tma_load_4d(smem + L::x_off + c * L::kSub, &maps.x, &bars->x_full, c * 64, own0, x_head, b);
-        tma_load_4d(smem + L::y_off + c * L::kSub, &maps.y, &bars->x_full, c * 64, own0, x_head, b);
-      }
-      const int a_head = KM ? h : hk;
+      const int x_head = KM ? hk : h, a_head = KM ? h : hk;
+      auto load_tile = [&](int at, const CUtensorMap* m, uint64_t* bar, int row0, int head) {
+        mbar_arrive_expect_tx(bar, L::kTile);
+        for (int c = 0; c < D / 64; ++c) tma_load_4d(smem + at + c * L::kSub, m, bar, c * 64, row0, head, b);
+      };
+      load_tile(L::x_off, &maps.x, &bars->x_full, own0, x_head);
       for (int u = 0; u < nu; ++u) {
-        const int s = u % NSTAGE, use = u / NSTAGE;
-        if (use > 0 && !mbar_wait(&bars->r_empty[s], (use - 1) & 1, abort_flag)) break;
-        const int row0 = (u0 + u) * BT;
-        mbar_arrive_expect_tx(&bars->r_full[s], 2 * L::kTile + (KM ? 1024 : 0));
-        unsigned char* st = smem + L::ring_off + s * 2 * L::kTile;
-        for (int c = 0; c < D / 64; ++c) {
-          tma_load_4d(st + c * L::kSub, &maps.a, &bars->r_full[s], c * 64, row0, a_head, b);
-          tma_load_4d(st + L::kTile + c * L::kSub, &maps.b, &bars->r_full[s], c * 64, row0, a_head, b);
-        }
-        if (KM) {
-          bulk_load_1d(smem + L::vec_off + s * 1024, p.negl2 + vec_row + row0, 512, &bars->r_full[s]);
-          bulk_load_1d(smem + L::vec_off + s * 1024 + 512, p.delta + vec_row + row0, 512, &bars->r_full[s]);
-        }
+        const int row0 = (u0 + u) * BT, sa = u % NA, sb = u % NB;
+        if (u >= NA && !mbar_wait(&bars->a_empty[sa], (u / NA - 1) & 1, abort_flag)) break;
+        load_tile(L::a_off + sa * L::kTile, &maps.a, &bars->a_full[sa], row0, a_head);
+        if (u == 0) load_tile(L::y_off, &maps.y, &bars->y_full, own0, x_head);
+        if (u >= NB && !mbar_wait(&bars->b_empty[sb], (u / NB - 1) & 1, abort_flag)) break;
+        load_tile(L::b_off + sb * L::kTile, &maps.b, &bars->b_full[sb], row0, a_head);
       }
-    } else if (warp == 1 && nu > 0) {
-      // ---------------------------------------------------------- MMA issuer (whole warp loops, one lane issues)
+    } else if (KM && warp == 2 && lane == 0) {
+      // ---------------------------------------------------------- L and delta of the streamed query tiles
+      for (int u = 0; u < nu; ++u) {
+        const int s = u & 1;
+        if (u >= 2 && !mbar_wait(&bars->vec_empty[s], (u / 2 - 1) & 1, abort_flag)) break;
+        const int64_t at = vec_row + (u0 + u) * BT;
+        mbar_arrive_expect_tx(&bars->vec_full[s], 1024);
+        bulk_load_1d(smem + L::vec_off + s * 1024, p.negl2 + at, 512, &bars->vec_full[s]);
+        bulk_load_1d(smem + L::vec_off + s * 1024 + 512, p.neg_delta + at, 512, &bars->vec_full[s]);
+      }
+    } else if (warp == 1 && nu > 0 && elect_one()) {
+      // ---------------------------------------------------------- MMA issuer: one thread
       constexpr int kFmt = std::is_same<T, __half>::value ? 0 : 1;
-      constexpr uint32_t idesc1 = make_idesc_f16(128, HALF, kFmt, 0, 0);  // S', dP': 128 x 64, K = D
-      constexpr uint32_t idesc2 = make_idesc_f16(128, D, kFmt, 0, 1);     // accumulators: 128 x D, K = 64
+      constexpr uint32_t idesc1 = make_idesc_f16(128, BT, kFmt, 0, 0);  // S', dP': 128 x 128, K = D
+      constexpr uint32_t idesc2 = make_idesc_f16(128, D, kFmt, 0, 1);   // accumulators: 128 x D, K = streamed rows
       const uint64_t x_desc = make_desc_sw128(smem_u32(smem + L::x_off), 16, 1024);
       const uint64_t y_desc = make_desc_sw128(smem_u32(smem + L::y_off), 16, 1024);
-      const uint64_t ak_desc0 = make_desc_sw128(smem_u32(smem + L::ring_off), 16, 1024);          // A, B as K-major
-      const uint64_t am_desc0 = make_desc_sw128(smem_u32(smem + L::ring_off), L::kSub, 1024);     // A, B as MN-major
-      // S'_e = X . A_e^T and dP'_e = Y . B_e^T for the 64 streamed rows of half e in ring stage s
-      auto issue_mma1 = [&](int e, int s) {
-        const uint64_t a_rows = ak_desc0 + (uint64_t)((s * 2 * L::kTile + e * HALF * 128) >> 4);
-        const uint64_t b_rows = a_rows + (uint64_t)(L::kTile >> 4);
-        const uint32_t d_s = tmem_base + COL_S + (uint32_t)(e * HALF);
-        const uint32_t d_dp = tmem_base + COL_DP + (uint32_t)(e * HALF);
-        if (elect_one()) {
+      const uint64_t ak_desc = make_desc_sw128(smem_u32(smem + L::a_off), 16, 1024);       // streamed tiles as K-major
+      const uint64_t bk_desc = make_desc_sw128(smem_u32(smem + L::b_off), 16, 1024);
+      const uint64_t am_desc = make_desc_sw128(smem_u32(smem + L::a_off), L::kSub, 1024);  // and as MN-major operands
+      const uint64_t bm_desc = make_desc_sw128(smem_u32(smem + L::b_off), L::kSub, 1024);
+      // 128 x 128 product of a stationary and a streamed tile over the head dimension
+      auto issue_mma1 = [&](uint32_t d_col, uint64_t own_desc, uint64_t str_desc, uint64_t* full) {
 #pragma unroll
-          for (int kk = 0; kk < D / 16; ++kk) {
-            const uint64_t off = (uint64_t)(((kk >> 2) * L::kSub + (kk & 3) * 32) >> 4);
-            if (kk == 0) mma_ss(d_s, x_desc + off, a_rows + off, idesc1, 0u);
-            else mma_ss_acc(d_s, x_desc + off, a_rows + off, idesc1);
-          }
-#pragma unroll
-          for (int kk = 0; kk < D / 16; ++kk) {
-            const uint64_t off = (uint64_t)(((kk >> 2) * L::kSub + (kk & 3) * 32) >> 4);
-            if (kk == 0) mma_ss(d_dp, y_desc + off, b_rows + off, idesc1, 0u);
-            else mma_ss_acc(d_dp, y_desc + off, b_rows + off, idesc1);
-          }
-          mma_commit(&bars->s_full[e]);
+        for (int kk = 0; kk < D / 16; ++kk) {
+          const uint64_t off = (uint64_t)(((kk >> 2) * L::kSub + (kk & 3) * 32) >> 4);
+          if (kk == 0) mma_ss(tmem_base + d_col, own_desc + off, str_desc + off, idesc1, 0u);
+          else mma_ss_acc(tmem_base + d_col, own_desc + off, str_desc + off, idesc1);
         }
-        __syncwarp();
+        mma_commit(full);
       };
-      // accumulators (+)= the 16-bit operands of half e (in TMEM over S'_e / dP'_e) times the 64 streamed rows
-      auto issue_mma2 = [&](int e, int s, bool first) {
-        const uint64_t a_tile = am_desc0 + (uint64_t)((s * 2 * L::kTile) >> 4);
-        const uint64_t b_tile = a_tile + (uint64_t)(L::kTile >> 4);
-        const uint32_t t_p = tmem_base + COL_S + (uint32_t)(e * HALF);    // P'_e: 64 values = 32 columns
-        const uint32_t t_ds = tmem_base + COL_DP + (uint32_t)(e * HALF);  // dS'_e
-        const uint32_t acc0 = tmem_base + COL_ACC, acc1 = tmem_base + COL_ACC + (uint32_t)D;
-        if (elect_one()) {
-#pragma unroll
-          for (int k4 = 0; k4 < HALF / 16; ++k4) {
-            const uint64_t off = (uint64_t)(((e * 4 + k4) * 16 * 128) >> 4);  // 16 streamed rows per K-step
-            const uint32_t accumulate = (first && k4 == 0) ? 0u : 1u;
-            if constexpr (MODE != kPlain) {  // dS: hi in columns [16 k4, +8), lo in the 8 after them
-              const uint64_t s_tile = a_tile + off;
-              const uint32_t acc = KM ? acc1 : acc0;
-              if (KM) mma_ts(acc0, t_p + (uint32_t)(k4 * 8), b_tile + off, idesc2, accumulate);
-              mma_ts(acc, t_ds + (uint32_t)(k4 * 16), s_tile, idesc2, accumulate);
-              mma_ts(acc, t_ds + (uint32_t)(k4 * 16 + 8), s_tile, idesc2, 1u);
-            } else if (KM) {
-              mma_ts(acc0, t_p + (uint32_t)(k4 * 8), b_tile + off, idesc2, accumulate);   // dV += P^T . dout
-              mma_ts(acc1, t_ds + (uint32_t)(k4 * 8), a_tile + off, idesc2, accumulate);  // dK += dS^T . Q
-            } else {
-              mma_ts(acc0, t_ds + (uint32_t)(k4 * 8), a_tile + off, idesc2, accumulate);  // dQ += dS . K
-            }
-          }
-        }
-        __syncwarp();
-      };
-      auto commit = [&](uint64_t* bar) {
-        if (elect_one()) mma_commit(bar);
-        __syncwarp();
-      };
-      bool ok = mbar_wait(&bars->x_full, 0, abort_flag);
-      if (ok) ok = mbar_wait(&bars->r_full[0], 0, abort_flag);
-      if (ok) {
+      bool ok = true;
+      auto wait = [&](uint64_t* bar, int phase) {
+        if (ok) ok = mbar_wait(bar, phase & 1, abort_flag);
         tc_fence_after();
-        issue_mma1(0, 0);
-        issue_mma1(1, 0);
-      }
+      };
+      auto issue_s = [&](int u) {
+        wait(&bars->a_full[u % NA], u / NA);
+        if (!ok) return;
+        issue_mma1((uint32_t)((u % NSB) * 128), x_desc, ak_desc + (uint64_t)((u % NA) * (L::kTile >> 4)),
+                   &bars->s_full[u % NSB]);
+      };
+      auto issue_dp = [&](int u) {
+        wait(&bars->b_full[u % NB], u / NB);
+        if (!ok) return;
+        issue_mma1(COL_DP + (uint32_t)((u % NDB) * 128), y_desc, bk_desc + (uint64_t)((u % NB) * (L::kTile >> 4)),
+                   &bars->dp_full[u % NDB]);
+      };
+      // K-steps of 16 streamed rows of an accumulator: 32 rows of warpgroup e's 64 for dV, all 64 for dK / dQ.  The
+      // 16-bit operands of a warpgroup's rows lie over its own 64 columns of S' or dP'.
+      auto issue_dv = [&](int u, int e, int c) {
+        const uint64_t tile = bm_desc + (uint64_t)((u % NB) * (L::kTile >> 4));
+        const uint32_t t_p = tmem_base + (uint32_t)((u % NSB) * 128 + e * HALF);
+#pragma unroll
+        for (int k2 = 0; k2 < 2; ++k2) {
+          const int k4 = c * 2 + k2;
+          const uint64_t off = (uint64_t)(((e * 4 + k4) * 16 * 128) >> 4);
+          if (e == 0 && k4 == 0) mma_ts(tmem_base + COL_ACC, t_p, tile, idesc2, u == 0 ? 0u : 1u);
+          else mma_ts_acc(tmem_base + COL_ACC, t_p + (uint32_t)(k4 * 8), tile + off, idesc2);
+        }
+      };
+      auto issue_ds = [&](int u, int e, uint32_t acc_col) {
+        const uint64_t tile = am_desc + (uint64_t)((u % NA) * (L::kTile >> 4));
+        const uint32_t t_ds = tmem_base + COL_DP + (uint32_t)((u % NDB) * 128 + e * HALF);
+#pragma unroll
+        for (int k4 = 0; k4 < HALF / 16; ++k4) {
+          const uint64_t off = (uint64_t)(((e * 4 + k4) * 16 * 128) >> 4);
+          constexpr int kStep = MODE != kPlain ? 16 : 8;  // fine modes: hi in 8 columns, lo in the 8 after them
+          if (e == 0 && k4 == 0) mma_ts(tmem_base + acc_col, t_ds, tile, idesc2, u == 0 ? 0u : 1u);
+          else mma_ts_acc(tmem_base + acc_col, t_ds + (uint32_t)(k4 * kStep), tile + off, idesc2);
+          if (MODE != kPlain) mma_ts_acc(tmem_base + acc_col, t_ds + (uint32_t)(k4 * kStep + 8), tile + off, idesc2);
+        }
+      };
+      wait(&bars->x_full, 0);
+      issue_s(0);
+      wait(&bars->y_full, 0);
+      issue_dp(0);
+      if (!KM && ok) mma_commit(&bars->b_empty[0]);
       for (int u = 0; ok && u < nu; ++u) {
-        const int s = u % NSTAGE;
         const bool more = u + 1 < nu;
-        const int s1 = (u + 1) % NSTAGE;
-        if (!(ok = mbar_wait(&bars->p_ready[0], u & 1, abort_flag))) break;
-        tc_fence_after();
-        issue_mma2(0, s, u == 0);
-        if (more) {
-          if (!(ok = mbar_wait(&bars->r_full[s1], ((u + 1) / NSTAGE) & 1, abort_flag))) break;
-          tc_fence_after();
-          issue_mma1(0, s1);  // S'_0 of the next pair while half 1 of this one is still in registers
+        if constexpr (KM) {
+          if (NSB == 2 && more) issue_s(u + 1);
+#pragma unroll
+          for (int x = 0; x < 4; ++x) {
+            wait(&bars->p_ready[u % NSB][x & 1][x >> 1], u / NSB);
+            if (ok) issue_dv(u, x & 1, x >> 1);
+          }
+          if (!ok) break;
+          mma_commit(&bars->b_empty[u % NB]);
+          if (NSB == 1 && more) issue_s(u + 1);  // over P of this tile, which the MMAs before it have read
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            wait(&bars->ds_ready[u % NDB][e], u / NDB);
+            if (ok) issue_ds(u, e, COL_ACC + D);
+          }
+          if (!ok) break;
+          mma_commit(&bars->a_empty[u % NA]);
+          if (more) issue_dp(u + 1);
+        } else {
+          if (more) {
+            wait(&bars->s_free, u);
+            if (ok) issue_s(u + 1);
+            if (ok) issue_dp(u + 1);
+            if (ok) mma_commit(&bars->b_empty[(u + 1) % NB]);
+          }
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            wait(&bars->ds_ready[u % NDB][e], u / NDB);
+            if (ok) issue_ds(u, e, COL_ACC);
+          }
+          if (ok) mma_commit(&bars->a_empty[u % NA]);
         }
-        if (!(ok = mbar_wait(&bars->p_ready[1], u & 1, abort_flag))) break;
-        tc_fence_after();
-        issue_mma2(1, s, false);
-        commit(&bars->r_empty[s]);
-        if (more) issue_mma1(1, s1);
       }
-      if (ok) commit(&bars->acc_done);
+      if (ok) mma_commit(&bars->acc_done);
     }
   } else {
     reg_alloc<REGS_CONSUMER>();
@@ -349,128 +390,180 @@ tc_bwd_kernel(const __grid_constant__ BwMaps maps, const BwTcParams p, int* __re
     const int row = lg * 32 + lane;
     const int own = own0 + row;  // key j (key-major) or query i (query-major)
     const uint32_t t_lane = tmem_base + ((uint32_t)(lg * 32) << 16);
-    const uint32_t t_s = t_lane + COL_S + (uint32_t)(e * HALF);
-    const uint32_t t_dp = t_lane + COL_DP + (uint32_t)(e * HALF);
     const float c2 = p.sm_scale * kLog2e;
-    float my_nl = 0.f, my_dl = 0.f;  // query-major: this thread's query
+    const uint64_t c22 = pack_f32x2(c2, c2);
+    float my_nl = 0.f, my_nd = 0.f;  // query-major: this thread's query
     if (!KM) {
       my_nl = p.negl2[vec_row + own];  // own < Mpad always
-      my_dl = p.delta[vec_row + own];
+      my_nd = p.neg_delta[vec_row + own];
     }
     [[maybe_unused]] GradScale gsc{1.f, 1.f};
     if constexpr (kScaledDs<T, MODE>) {
       gsc = grad_scale(p, b, h, hk, lane);
-      my_dl *= gsc.mul;
+      my_nd *= gsc.mul;
     }
     // what a kept entry's dP is multiplied by (keep_scale is 1 without dropout); query-major kernels put the power of
     // two here and on delta, key-major ones, whose delta comes with the streamed rows, on P
     const float kept = KM ? p.keep_scale : p.keep_scale * gsc.mul;
-    bool alive = true;
-    for (int u = 0; u < nu; ++u) {
-      if (!mbar_wait(&bars->s_full[e], u & 1, abort_flag)) { alive = false; break; }
-      tc_fence_after();
+
+    // One streamed tile, kMasked where an entry of this warpgroup's 128 x 64 block may be hidden.
+    auto tile_body = [&](auto masked_tag, int u) -> bool {
+      constexpr bool kMasked = decltype(masked_tag)::value;
       const int str0 = (u0 + u) * BT + e * HALF;  // first streamed row of this half
       // causal: (query i, key j) is visible iff j <= i + p_seq.  Column x of the half is streamed row
       // str0 + x.  Key-major (own = j, streamed = i): visible iff x >= own - p_seq - str0.
       // Query-major (own = i, streamed = j): visible iff x <= own + p_seq - str0.
       // Keys beyond N are masked too (query-major): their scores of zero against a very negative L would make
       // P infinite, and infinity times the zero K row is not zero.
-      int x_lo = 0, x_hi = HALF - 1;
-      if (p.causal && KM) x_lo = own - p.p_seq - str0;
-      // Query rows beyond M are masked under dropout (key-major): against their zero dout rows stand weights of
-      // 1 / (1 - p), which fp16 need not hold.
-      if (KM && MODE == kDrop) x_hi = p.M - 1 - str0;
-      if (!KM) x_hi = min(p.N - 1, p.causal ? own + p.p_seq : p.N - 1) - str0;
-      const float* vl = reinterpret_cast<const float*>(smem + L::vec_off + (u % NSTAGE) * 1024) + e * HALF;
-      const float* vd = vl + 128;
-      if constexpr (MODE != kPlain) {
-        // Bound by the integer instructions of the mask when there is one (about 25 per entry and kernel); chunks of
-        // 16 keep the code and the live registers small.
-        uint32_t lin = 0;  // Philox counter of the half's first entry of this thread, 32-bit wrap-around
+      [[maybe_unused]] int x_lo = 0, x_hi = HALF - 1;
+      if constexpr (kMasked) {
+        if (p.causal && KM) x_lo = own - p.p_seq - str0;
+        // Query rows beyond M are masked under dropout (key-major): against their zero dout rows stand weights of
+        // 1 / (1 - p), which fp16 need not hold.
+        if (KM && MODE == kDrop) x_hi = p.M - 1 - str0;
+        if (!KM) x_hi = min(p.N - 1, p.causal ? own + p.p_seq : p.N - 1) - str0;
+      }
+      [[maybe_unused]] uint32_t keep[2] = {~0u, ~0u};  // bit x of the pair: entry x of this thread's 64 is kept
+      if constexpr (MODE == kDrop) {
+        // Philox counter of the half's first entry of this thread, 32-bit wrap-around.  About 25 integer instructions
+        // an entry bound the tile; a rolled loop of 16 keeps them in the instruction caches.
+        const uint32_t bh = (uint32_t)(b * p.Hq + h);
         const uint32_t lin_step = KM ? (uint32_t)p.N : 1u;
-        if constexpr (MODE == kDrop) {
-          const uint32_t bh = (uint32_t)(b * p.Hq + h);
-          lin = KM ? (bh * (uint32_t)p.M + (uint32_t)str0) * (uint32_t)p.N + (uint32_t)own
-                   : (bh * (uint32_t)p.M + (uint32_t)own) * (uint32_t)p.N + (uint32_t)str0;
-        }
+        uint32_t lin = KM ? (bh * (uint32_t)p.M + (uint32_t)str0) * (uint32_t)p.N + (uint32_t)own
+                          : (bh * (uint32_t)p.M + (uint32_t)own) * (uint32_t)p.N + (uint32_t)str0;
 #pragma unroll 1
-        for (int c = 0; c < HALF; c += 16) {
-          uint32_t sv[16], dv[16];
-          tmem_ld16(t_s + c, sv);
-          tmem_ld16(t_dp + c, dv);
-          tmem_wait_ld();
-          uint32_t pk[8], hi[8], lo[8];
+        for (int c = 0; c < 4; ++c) {
+          uint32_t bits = 0u;
 #pragma unroll
-          for (int x = 0; x < 16; x += 2) {
-            float pr[2], ds[2];
-            float2 nl2 = make_float2(my_nl, my_nl), dl2 = make_float2(my_dl, my_dl);
-            if (KM) {
-              nl2 = *reinterpret_cast<const float2*>(vl + c + x);
-              dl2 = *reinterpret_cast<const float2*>(vd + c + x);
-            }
-#pragma unroll
-            for (int y = 0; y < 2; ++y) {
-              const float nl = y ? nl2.y : nl2.x, dl = y ? dl2.y : dl2.x;
-              const bool vis = (c + x + y >= x_lo) && (c + x + y <= x_hi);
-              const float pe = vis ? fast_exp2(fmaf(__uint_as_float(sv[x + y]), c2, nl)) : 0.f;
-              float ks = kept;
-              if constexpr (MODE == kDrop) ks = dropout_keep(p.drop, lin + (uint32_t)(c + x + y) * lin_step) ? kept : 0.f;
-              const float t = fmaf(__uint_as_float(dv[x + y]), ks, -dl);
-              if (KM) {
-                pr[y] = pe * ks;
-                ds[y] = pe * gsc.mul * t;
-              } else {
-                ds[y] = pe * t;
-              }
-            }
-            if (KM) pk[x / 2] = pack2<T>(pr[0], pr[1]);
-            hi[x / 2] = pack2<T>(ds[0], ds[1]);
-            const float2 h2 = unpack2<T>(hi[x / 2]);
-            lo[x / 2] = pack2<T>(ds[0] - h2.x, ds[1] - h2.y);
-          }
-          if (KM) tmem_st8(t_s + c / 2, pk);  // (columns that this and earlier chunks have been read from)
-          tmem_st8(t_dp + c, hi);
-          tmem_st8(t_dp + c + 8, lo);
+          for (int x = 0; x < 16; ++x, lin += lin_step) bits |= dropout_keep(p.drop, lin) ? 1u << x : 0u;
+          if (c < 2) keep[0] = c == 0 ? bits : keep[0] | bits << 16;
+          else keep[1] = c == 2 ? bits : keep[1] | bits << 16;
         }
-      } else {
-      uint32_t sv[HALF], dv[HALF];
+      }
+      const uint32_t t_s = t_lane + (uint32_t)((u % NSB) * 128 + e * HALF);
+      const uint32_t t_dp = t_lane + COL_DP + (uint32_t)((u % NDB) * 128 + e * HALF);
+      const float* vl = reinterpret_cast<const float*>(smem + L::vec_off + (u & 1) * 1024) + e * HALF;
+      if (KM && !mbar_wait(&bars->vec_full[u & 1], (u >> 1) & 1, abort_flag)) return false;
+      if (!mbar_wait(&bars->s_full[u % NSB], (u / NSB) & 1, abort_flag)) return false;
+      tc_fence_after();
+      uint32_t sv[HALF];  // S', then P'
       tmem_ld32(t_s, reinterpret_cast<uint32_t(&)[32]>(sv[0]));
       tmem_ld32(t_s + 32, reinterpret_cast<uint32_t(&)[32]>(sv[32]));
-      tmem_ld32(t_dp, reinterpret_cast<uint32_t(&)[32]>(dv[0]));
-      tmem_ld32(t_dp + 32, reinterpret_cast<uint32_t(&)[32]>(dv[32]));
       tmem_wait_ld();
-      uint32_t pk[HALF / 2], dk[HALF / 2];
-#pragma unroll
-      for (int x = 0; x < HALF; x += 4) {
-        float nl[4], dl[4];
-        if (KM) {
-          const float4 a = *reinterpret_cast<const float4*>(vl + x);
-          const float4 d4 = *reinterpret_cast<const float4*>(vd + x);
-          nl[0] = a.x; nl[1] = a.y; nl[2] = a.z; nl[3] = a.w;
-          dl[0] = d4.x; dl[1] = d4.y; dl[2] = d4.z; dl[3] = d4.w;
-        } else {
-#pragma unroll
-          for (int y = 0; y < 4; ++y) { nl[y] = my_nl; dl[y] = my_dl; }
-        }
-        float pr[4], ds[4];
-#pragma unroll
-        for (int y = 0; y < 4; ++y) {
-          const bool vis = (x + y >= x_lo) && (x + y <= x_hi);
-          const float pe = fast_exp2(fmaf(__uint_as_float(sv[x + y]), c2, nl[y]));
-          pr[y] = vis ? pe : 0.f;
-          ds[y] = pr[y] * (__uint_as_float(dv[x + y]) - dl[y]);
-        }
-        pk[x / 2] = pack2<T>(pr[0], pr[1]);
-        pk[x / 2 + 1] = pack2<T>(pr[2], pr[3]);
-        dk[x / 2] = pack2<T>(ds[0], ds[1]);
-        dk[x / 2 + 1] = pack2<T>(ds[2], ds[3]);
+      if (!KM) {  // the next tile's S' may be written
+        tc_fence_before();
+        mbar_arrive(&bars->s_free);
       }
-      if (KM) tmem_st32(t_s, pk);  // P' is an operand only where dV is formed
-      tmem_st32(t_dp, dk);
+      // ---- P' = exp2(S' c2 - L log2e); key-major, where it is the operand of dV, handed over in chunks of 32 rows
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uint32_t pk[16];
+#pragma unroll
+        for (int x = c * 32; x < c * 32 + 32; x += 4) {
+          uint64_t n01 = pack_f32x2(my_nl, my_nl), n23 = n01;
+          if (KM) {
+            const float4 a = *reinterpret_cast<const float4*>(vl + x);
+            n01 = pack_f32x2(a.x, a.y);
+            n23 = pack_f32x2(a.z, a.w);
+          }
+          float t[4];
+          unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(sv[x]), __uint_as_float(sv[x + 1])), c22, n01), t[0], t[1]);
+          unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(sv[x + 2]), __uint_as_float(sv[x + 3])), c22, n23), t[2], t[3]);
+          float pr[4];
+#pragma unroll
+          for (int y = 0; y < 4; ++y) {
+            float pe = fast_exp2(t[y]);
+            if (kMasked && !(x + y >= x_lo && x + y <= x_hi)) pe = 0.f;
+            sv[x + y] = __float_as_uint(pe);
+            pr[y] = pe;
+            if constexpr (MODE == kDrop) pr[y] = (keep[c] >> (x + y - c * 32) & 1u) ? pe * kept : 0.f;
+          }
+          pk[(x - c * 32) / 2] = pack2<T>(pr[0], pr[1]);
+          pk[(x - c * 32) / 2 + 1] = pack2<T>(pr[2], pr[3]);
+        }
+        if (KM) {
+          tmem_st16(t_s + c * 16, pk);
+          tmem_wait_st();
+          tc_fence_before();
+          mbar_arrive(&bars->p_ready[u % NSB][e][c]);
+        }
+      }
+      // ---- dS' = P' (dP' - delta)
+      if (!mbar_wait(&bars->dp_full[u % NDB], (u / NDB) & 1, abort_flag)) return false;
+      tc_fence_after();
+      const float* vd = vl + 128;
+      auto neg_delta4 = [&](int x, float (&nd)[4]) {
+        if (KM) {
+          const float4 d4 = *reinterpret_cast<const float4*>(vd + x);
+          nd[0] = d4.x; nd[1] = d4.y; nd[2] = d4.z; nd[3] = d4.w;
+        } else {
+          nd[0] = nd[1] = nd[2] = nd[3] = my_nd;
+        }
+      };
+      if constexpr (MODE == kPlain) {
+        uint32_t dv[HALF], dk[HALF / 2];
+        tmem_ld32(t_dp, reinterpret_cast<uint32_t(&)[32]>(dv[0]));
+        tmem_ld32(t_dp + 32, reinterpret_cast<uint32_t(&)[32]>(dv[32]));
+        tmem_wait_ld();
+#pragma unroll
+        for (int x = 0; x < HALF; x += 4) {
+          float nd[4];
+          neg_delta4(x, nd);
+#pragma unroll
+          for (int y = 0; y < 4; y += 2) {
+            const uint64_t t = add_f32x2(pack_f32x2(__uint_as_float(dv[x + y]), __uint_as_float(dv[x + y + 1])),
+                                         pack_f32x2(nd[y], nd[y + 1]));
+            float d0, d1;
+            unpack_f32x2(mul_f32x2(t, pack_f32x2(__uint_as_float(sv[x + y]), __uint_as_float(sv[x + y + 1]))), d0, d1);
+            dk[(x + y) / 2] = pack2<T>(d0, d1);
+          }
+        }
+        tmem_st32(t_dp, dk);
+      } else {
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          uint32_t dv[32], out[32];  // out: per 16 streamed rows 8 columns of hi, 8 of lo
+          tmem_ld32(t_dp + c * 32, dv);
+          tmem_wait_ld();
+#pragma unroll
+          for (int x = 0; x < 32; x += 4) {
+            float nd[4], ds[4];
+            neg_delta4(c * 32 + x, nd);
+#pragma unroll
+            for (int y = 0; y < 4; ++y) {
+              const float ks = MODE == kDrop && !(keep[c] >> (x + y) & 1u) ? 0.f : kept;
+              const float t = fmaf(__uint_as_float(dv[x + y]), ks, nd[y]);
+              const float pe = __uint_as_float(sv[c * 32 + x + y]);
+              ds[y] = (KM ? pe * gsc.mul : pe) * t;
+            }
+#pragma unroll
+            for (int y = 0; y < 4; y += 2) {
+              const uint32_t hi = pack2<T>(ds[y], ds[y + 1]);
+              const float2 h2 = unpack2<T>(hi);
+              const int at = (x >> 4) * 16 + ((x & 15) + y) / 2;
+              out[at] = hi;
+              out[at + 8] = pack2<T>(ds[y] - h2.x, ds[y + 1] - h2.y);
+            }
+          }
+          tmem_st32(t_dp + c * 32, out);
+        }
       }
       tmem_wait_st();
       tc_fence_before();
-      mbar_arrive(&bars->p_ready[e]);
+      mbar_arrive(&bars->ds_ready[u % NDB][e]);
+      if (KM) {  // this warp has read the tile's L and delta
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars->vec_empty[u & 1]);
+      }
+      return true;
+    };
+    bool alive = true;
+    for (int u = 0; alive && u < nu; ++u) {
+      const int str0 = (u0 + u) * BT + e * HALF;
+      bool masked;
+      if (KM) masked = (p.causal && own0 + BT - 1 - p.p_seq > str0) || (MODE == kDrop && str0 + HALF > p.M);
+      else masked = str0 + HALF > (p.causal ? min(p.N, own0 + p.p_seq + 1) : p.N);
+      alive = masked ? tile_body(std::true_type{}, u) : tile_body(std::false_type{}, u);
     }
 
     // ---- epilogue: accumulators -> 16-bit -> swizzled smem -> TMA store (clips at the tensor's edge)
@@ -480,7 +573,7 @@ tc_bwd_kernel(const __grid_constant__ BwMaps maps, const BwTcParams p, int* __re
     }
     if (alive) {
       // Every MMA has completed, so the ring is free for staging: 32 rows x 64 columns (4 KB) per (warp, sub-tile).
-      unsigned char* ost = smem + L::ring_off + (warp - 4) * (32 * D * 2);
+      unsigned char* ost = smem + L::a_off + (warp - 4) * (32 * D * 2);
       // key-major: warpgroup 0 stores dV (acc0), warpgroup 1 stores dK (acc1, times sm_scale);
       // query-major: dQ (acc0, times sm_scale), warpgroup w takes the 64-column sub-tiles w, w + 2, ...
       const uint32_t t_acc = t_lane + COL_ACC + (KM ? (uint32_t)(e * D) : 0u);
@@ -539,6 +632,7 @@ tc_bwd_kernel(const __grid_constant__ BwMaps maps, const BwTcParams p, int* __re
     griddep_launch_dependents();
     griddep_wait();
   }
+  __syncwarp();
   tc_fence_before();
   __syncthreads();
   if (*abort_flag) {
@@ -592,7 +686,7 @@ __device__ __forceinline__ float2 block_max(float x, float y, float2 (&red)[8]) 
   return make_float2(x, y);
 }
 template <typename T, bool STATS>
-__global__ void __launch_bounds__(256) bwd_prep_kernel(BwdParams p, float* negl2, float* delta, int Mpad, BwStats st) {
+__global__ void __launch_bounds__(256) bwd_prep_kernel(BwdParams p, float* negl2, float* neg_delta, int Mpad, BwStats st) {
   griddep_launch_dependents();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int lpr = p.D >> 3, rows_at_once = 32 / lpr, sub = lane & (lpr - 1);
@@ -653,7 +747,7 @@ __global__ void __launch_bounds__(256) bwd_prep_kernel(BwdParams p, float* negl2
         const float Li = p.L[(int64_t)bh * p.M + i];
         nl = (Li == __int_as_float(0xff800000)) ? 0.f : -Li * kLog2e;  // no visible key: every weight is masked anyway
       }
-      delta[(int64_t)bh * Mpad + i] = sum;
+      neg_delta[(int64_t)bh * Mpad + i] = -sum;
       negl2[(int64_t)bh * Mpad + i] = nl;
     }
   }
@@ -758,16 +852,17 @@ BwWs bwd_ws(int B, int Hq, int Hk, int M, int N, int D, bool fine) {
 
 template <typename T, int D, int MODE>
 cudaError_t launch_bwd_td(const BwdParams& p, cudaStream_t s) {
-  using L = BwSmem<D>;
+  using Lk = BwSmem<D, true>;
+  using Lq = BwSmem<D, false>;
   static PerDeviceOnce once_km, once_qm;
   cudaError_t e;
-  if ((e = set_max_smem_once(once_km, tc_bwd_kernel<T, D, true, MODE>, L::alloc)) != cudaSuccess) return e;
-  if ((e = set_max_smem_once(once_qm, tc_bwd_kernel<T, D, false, MODE>, L::alloc)) != cudaSuccess) return e;
+  if ((e = set_max_smem_once(once_km, tc_bwd_kernel<T, D, true, MODE>, Lk::total)) != cudaSuccess) return e;
+  if ((e = set_max_smem_once(once_qm, tc_bwd_kernel<T, D, false, MODE>, Lq::total)) != cudaSuccess) return e;
   const int Mpad = mpad_of(p.M);
   const BwWs ws = bwd_ws(p.B, p.Hq, p.Hk, p.M, p.N, p.D, MODE != kPlain);
   char* base = reinterpret_cast<char*>(p.delta);
   float* negl2 = p.delta;
-  float* delta = reinterpret_cast<float*>(base + ws.delta);
+  float* neg_delta = reinterpret_cast<float*>(base + ws.delta);
   char *dk_part = base + ws.dk, *dv_part = base + ws.dv;
   using Part = typename std::conditional<MODE == kPlain, T, float>::type;
   const BwStats st{reinterpret_cast<float2*>(base + ws.g_stat), reinterpret_cast<float*>(base + ws.v_stat),
@@ -775,13 +870,13 @@ cudaError_t launch_bwd_td(const BwdParams& p, cudaStream_t s) {
   {
     constexpr bool kStats = kScaledDs<T, MODE>;
     const unsigned blocks = (unsigned)(p.B * p.Hq * st.g_blocks + (kStats ? p.B * p.Hk * st.v_blocks : 0));
-    bwd_prep_kernel<T, kStats><<<blocks, 256, 0, s>>>(p, negl2, delta, Mpad, st);
+    bwd_prep_kernel<T, kStats><<<blocks, 256, 0, s>>>(p, negl2, neg_delta, Mpad, st);
     count_launch();
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
   BwTcParams tp{};
   tp.Hq = p.Hq; tp.G = p.G; tp.M = p.M; tp.N = p.N; tp.p_seq = p.p_seq; tp.causal = p.causal; tp.Mpad = Mpad;
-  tp.sm_scale = p.sm_scale; tp.negl2 = negl2; tp.delta = delta; tp.D = p.D;
+  tp.sm_scale = p.sm_scale; tp.negl2 = negl2; tp.neg_delta = neg_delta; tp.D = p.D;
   tp.drop = p.drop;
   tp.keep_scale = 1.f / (1.f - p.drop.p);
   tp.g_stat = st.g; tp.v_stat = st.v; tp.g_blocks = st.g_blocks; tp.v_blocks = st.v_blocks;
@@ -799,7 +894,7 @@ cudaError_t launch_bwd_td(const BwdParams& p, cudaStream_t s) {
       return cudaErrorInvalidValue;
     m.o1 = m.o0;
     dim3 grid(p.Hq, p.B, (p.M + BT - 1) / BT);
-    if ((e = launch_overlapped(tc_bwd_kernel<T, D, false, MODE>, grid, NTHREADS, L::alloc, s, m, tp, status_word)) !=
+    if ((e = launch_overlapped(tc_bwd_kernel<T, D, false, MODE>, grid, NTHREADS, Lq::total, s, m, tp, status_word)) !=
         cudaSuccess)
       return e;
   }
@@ -824,7 +919,7 @@ cudaError_t launch_bwd_td(const BwdParams& p, cudaStream_t s) {
                        map_parts ? ph_sh : p.dk_sh, map_parts ? ph_sb : p.dk_sb, 32))
       return cudaErrorInvalidValue;
     dim3 grid(p.Hq, p.B, (p.N + BT - 1) / BT);
-    if ((e = launch_overlapped(tc_bwd_kernel<T, D, true, MODE>, grid, NTHREADS, L::alloc, s, m, tp, status_word)) !=
+    if ((e = launch_overlapped(tc_bwd_kernel<T, D, true, MODE>, grid, NTHREADS, Lk::total, s, m, tp, status_word)) !=
         cudaSuccess)
       return e;
   }
