@@ -595,7 +595,8 @@ int faws_attention_backward(const faws_problem* p, const faws_grads* g, void* wo
   // Scratch sized for the same shape with 16-bit partial gradients (before dropout was turned on) is enough for the
   // CUDA-core kernels, which then run unless the family is forced.
   const size_t least = tc_bwd_workspace_bytes(p->B, p->Hq, p->Hk, p->M, p->N, p->D, false);
-  const size_t need = faws_workspace_bytes(FAWS_OP_ATTENTION_BACKWARD, p, 0);
+  // Without room for the dropout mask the kernels draw it as they go.
+  const size_t need = tc_bwd_workspace_bytes(p->B, p->Hq, p->Hk, p->M, p->N, p->D, p->dropout_p > 0.f || p->D < 64);
   if (workspace == nullptr || workspace_bytes < least || misaligned_ws(workspace)) return FAWS_EWORKSPACE;
   BwdParams b{};
   b.q = p->q.ptr; b.k = p->k.ptr; b.v = p->v.ptr; b.o = p->out.ptr;
@@ -613,6 +614,8 @@ int faws_attention_backward(const faws_problem* p, const faws_grads* g, void* wo
   b.B = p->B; b.Hq = p->Hq; b.Hk = p->Hk; b.G = p->Hq / p->Hk; b.M = p->M; b.N = p->N; b.D = p->D;
   b.p_seq = p->N - p->M; b.causal = p->causal ? 1 : 0; b.sm_scale = p->sm_scale;
   b.drop = make_drop(p);
+  const size_t mask_bytes = p->dropout_p > 0.f ? tc_bwd_mask_bytes(p->B, p->Hq, p->M, p->N) : 0;
+  b.mask_scratch = mask_bytes > 0 && workspace_bytes >= need + mask_bytes;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   bool use_tc = false;
   if (tc_allowed(p)) use_tc = tc_bwd_supported(b, p->dtype);
@@ -639,7 +642,8 @@ size_t faws_workspace_bytes(int32_t op, const faws_problem* p, int32_t split) {
       if (split < 1 || split > cdiv(p->N, kTcBlockN)) return 0;
       return split == 1 ? 0 : split_kv_bytes(p, split);
     case FAWS_OP_ATTENTION_BACKWARD:  // enough for either kernel family
-      return tc_bwd_workspace_bytes(p->B, p->Hq, p->Hk, p->M, p->N, p->D, p->dropout_p > 0.f || p->D < 64);
+      return tc_bwd_workspace_bytes(p->B, p->Hq, p->Hk, p->M, p->N, p->D, p->dropout_p > 0.f || p->D < 64) +
+             (p->dropout_p > 0.f ? tc_bwd_mask_bytes(p->B, p->Hq, p->M, p->N) : 0);
     case FAWS_OP_COL_SUM:
     case FAWS_OP_COL_SUM_SEQUENTIAL:
       return align256(partial_floats(p, 0, p->N) * 4) + align256(qsum_floats(p) * 4);

@@ -30,11 +30,11 @@
 // (head dims 16 and 32) keep their precision this way.  In fp16 the 22 bits hold between 2^-3 and 2^16 only, so dS is
 // moved there by a power of two per head, from the largest |dout|, |v| and |delta| that the pre-pass meets
 // (GradScale), and moved back in the epilogue: exact, and gradients of any size come out as from fp32 dS.
-// kDrop is kFine with the dropout mask, drawn again from the counter-based generator in both kernels.  Fine modes
-// walk the tile in chunks of 16 streamed rows, the K-step of the accumulating MMAs; hi and lo of a chunk take the 16
-// columns that its dP' leaves.  fp16 B4 H16 S1024 D64 causal, p = 0.1, forward and backward: 270 us (266 without the
-// power of two), 3 717 us with the CUDA-core kernels; errors of the gradients against fp64 as there (2.32e-4, 2.28e-4,
-// 2.92e-4 for dq, dk, dv, fp16; dout of 1e-4, where the results are fp16 subnormals: 1.6e-3, 6.6e-3 with an unmoved dS).
+// kDrop is kFine with the dropout mask, which the pre-pass draws (draw_mask).  In fine modes hi and lo of 16 streamed
+// rows, the K-step of the accumulating MMAs, take the 16 columns that their dP' leaves.  fp16 B4 H16 S1024 D64 causal,
+// p = 0.1, forward and backward: 247 us, 3 717 us with the CUDA-core kernels; errors of the gradients against fp64 as
+// there (2.32e-4, 2.28e-4, 2.92e-4 for dq, dk, dv, fp16; dout of 1e-4, where the results are fp16 subnormals: 1.6e-3,
+// 6.6e-3 with an unmoved dS).
 // Deterministic: every output element is written once, by one CTA, in a fixed order; with GQA the
 // key-major kernel writes per-query-head dK / dV and a second kernel adds the G heads in order.
 // Out-of-range query rows need no predicates without dropout: TMA zero-fills the loads (with L = delta = 0 their P
@@ -113,7 +113,28 @@ struct BwTcParams {
   const float2* g_stat;  // kScaledDs: (B,Hq,g_blocks) bounds of |dout_i|^2 and |delta_i| over a pre-pass block's rows,
   const float* v_stat;   // (B,Hk,v_blocks) of |v_j|^2
   int g_blocks, v_blocks;
+  const uint32_t* mask;  // dropout: the mask as the pre-pass has drawn it (see draw_mask), or null
 };
+
+// The dropout mask in scratch, one bit per entry, 1 = kept: per (b, h, 128-row query tile, 128-key tile) 2 KB, four
+// words a row, bit x of word w of row r is entry (r, 32 w + x).  Both kernels need it, and a kernel with nothing else to
+// do draws it at twice the rate of the two consumer warps that a scheduler of the main kernels has: fp16 B4 H16 S1024 D64
+// causal, p = 0.1, forward and backward: 247 us, 282 with the mask drawn in both.  Beyond kMaskBytes of scratch (one bit
+// per entry grows with M * N) both kernels draw for themselves, as they do in scratch that has no room for it.
+constexpr size_t kMaskBytes = size_t(256) << 20;
+__device__ __forceinline__ int64_t mask_word(int bh, int qt, int kt, int nqt, int nkt) {
+  return (((int64_t)bh * nqt + qt) * nkt + kt) * 512;
+}
+// 32 x 32 bits across a warp: on entry bit k of lane l is A[l][k], on exit it is A[k][l].
+__device__ __forceinline__ uint32_t warp_transpose_bits(uint32_t x, int lane) {
+  uint32_t m = 0x0000ffffu;
+#pragma unroll
+  for (int j = 16; j >= 1; j >>= 1, m ^= m << j) {
+    const uint32_t y = __shfl_xor_sync(0xffffffffu, x, j);
+    x = (lane & j) ? (x & ~m) | ((y >> j) & m) : (x & m) | ((y & m) << j);
+  }
+  return x;
+}
 
 // Modes that move dS by a power of two before it is split: fp16 ones (bf16 has the range of fp32).
 template <typename T, int MODE>
@@ -406,6 +427,25 @@ tc_bwd_kernel(const __grid_constant__ BwMaps maps, const BwTcParams p, int* __re
     // two here and on delta, key-major ones, whose delta comes with the streamed rows, on P
     const float kept = KM ? p.keep_scale : p.keep_scale * gsc.mul;
 
+    // dropout: this thread's two words of the next tile's mask, fetched a tile ahead.  Query-major: entries [64 e, 64 e
+    // + 64) of its query row; key-major: the word of the warp's 32 keys in rows 64 e + lane and 64 e + 32 + lane.
+    [[maybe_unused]] uint32_t ahead[2] = {0u, 0u};
+    [[maybe_unused]] auto fetch_mask = [&](int u) {
+      const int bh = b * p.Hq + h, nqt = p.Mpad / BT, nkt = (p.N + BT - 1) / BT;
+      if (KM) {
+        const uint32_t* w = p.mask + mask_word(bh, u0 + u, own_tile, nqt, nkt) + (e * HALF + lane) * 4 + lg;
+        ahead[0] = __ldg(w);
+        ahead[1] = __ldg(w + 128);
+      } else {
+        const uint2 w = __ldg(reinterpret_cast<const uint2*>(p.mask + mask_word(bh, own_tile, u, nqt, nkt) + row * 4 + e * 2));
+        ahead[0] = w.x;
+        ahead[1] = w.y;
+      }
+    };
+    if constexpr (MODE == kDrop) {
+      if (p.mask != nullptr && nu > 0) fetch_mask(0);
+    }
+
     // One streamed tile, kMasked where an entry of this warpgroup's 128 x 64 block may be hidden.
     auto tile_body = [&](auto masked_tag, int u) -> bool {
       constexpr bool kMasked = decltype(masked_tag)::value;
@@ -424,7 +464,11 @@ tc_bwd_kernel(const __grid_constant__ BwMaps maps, const BwTcParams p, int* __re
         if (!KM) x_hi = min(p.N - 1, p.causal ? own + p.p_seq : p.N - 1) - str0;
       }
       [[maybe_unused]] uint32_t keep[2] = {~0u, ~0u};  // bit x of the pair: entry x of this thread's 64 is kept
-      if constexpr (MODE == kDrop) {
+      if (MODE == kDrop && p.mask != nullptr) {
+        keep[0] = KM ? warp_transpose_bits(ahead[0], lane) : ahead[0];
+        keep[1] = KM ? warp_transpose_bits(ahead[1], lane) : ahead[1];
+        if (u + 1 < nu) fetch_mask(u + 1);
+      } else if constexpr (MODE == kDrop) {
         // Philox counter of the half's first entry of this thread, 32-bit wrap-around.  About 25 integer instructions
         // an entry bound the tile; a rolled loop of 16 keeps them in the instruction caches.
         const uint32_t bh = (uint32_t)(b * p.Hq + h);
@@ -685,9 +729,29 @@ __device__ __forceinline__ float2 block_max(float x, float y, float2 (&red)[8]) 
   }
   return make_float2(x, y);
 }
-template <typename T, bool STATS>
-__global__ void __launch_bounds__(256) bwd_prep_kernel(BwdParams p, float* negl2, float* neg_delta, int Mpad, BwStats st) {
+// A word of the mask per thread, two blocks a tile; tiles without a visible entry are left out.
+__device__ __forceinline__ void draw_mask(const BwdParams& p, uint32_t* mask, int64_t block) {
+  const int nqt = (p.M + BT - 1) / BT, nkt = (p.N + BT - 1) / BT;
+  const int64_t tile = block >> 1;
+  const int kt = (int)(tile % nkt);
+  const int64_t rest = tile / nkt;
+  const int qt = (int)(rest % nqt), bh = (int)(rest / nqt);
+  if (p.causal && kt * BT > qt * BT + BT - 1 + p.p_seq) return;
+  const int at = (int)(block & 1) * 256 + threadIdx.x;
+  uint32_t lin = ((uint32_t)bh * (uint32_t)p.M + (uint32_t)(qt * BT + (at >> 2))) * (uint32_t)p.N + (uint32_t)(kt * BT + (at & 3) * 32);
+  uint32_t bits = 0u;
+#pragma unroll 8
+  for (int x = 0; x < 32; ++x) bits |= dropout_keep(p.drop, lin + (uint32_t)x) ? 1u << x : 0u;
+  mask[tile * 512 + at] = bits;
+}
+template <typename T, bool STATS, bool DRAW>
+__global__ void __launch_bounds__(256) bwd_prep_kernel(BwdParams p, float* negl2, float* neg_delta, int Mpad, BwStats st,
+                                                       uint32_t* mask, unsigned mask_block0) {
   griddep_launch_dependents();
+  if (DRAW && blockIdx.x >= mask_block0) {
+    draw_mask(p, mask, blockIdx.x - mask_block0);
+    return;
+  }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int lpr = p.D >> 3, rows_at_once = 32 / lpr, sub = lane & (lpr - 1);
   const int block_rows = 8 * kPrepRows * rows_at_once;
@@ -832,10 +896,13 @@ int prep_blocks(int rows, int D) {
   return (rows + block_rows - 1) / block_rows;
 }
 
-// Workspace: [-L*log2e | delta | pre-pass statistics (fine modes) | per-head dK | per-head dV]
+// Workspace: [-L*log2e | delta | pre-pass statistics (fine modes) | per-head dK | per-head dV | dropout mask]
 struct BwWs {
-  size_t delta, g_stat, v_stat, dk, dv, total;
+  size_t delta, g_stat, v_stat, dk, dv, mask, total;
 };
+size_t mask_bytes(int B, int Hq, int M, int N) {
+  return (size_t)B * Hq * (mpad_of(M) / BT) * ((N + BT - 1) / BT) * 2048;
+}
 BwWs bwd_ws(int B, int Hq, int Hk, int M, int N, int D, bool fine) {
   auto up = [](size_t x) { return (x + 255) & ~size_t(255); };
   BwWs w{};
@@ -846,7 +913,8 @@ BwWs bwd_ws(int B, int Hq, int Hk, int M, int N, int D, bool fine) {
   w.v_stat = w.g_stat + (fine ? up((size_t)B * Hq * prep_blocks(mpad_of(M), D) * sizeof(float2)) : 0);
   w.dk = w.v_stat + (fine ? up((size_t)B * Hk * prep_blocks(N, D) * sizeof(float)) : 0);
   w.dv = w.dk + part_bytes;
-  w.total = w.dv + part_bytes;
+  w.mask = w.dv + part_bytes;
+  w.total = w.mask;  // without the mask
   return w;
 }
 
@@ -864,13 +932,16 @@ cudaError_t launch_bwd_td(const BwdParams& p, cudaStream_t s) {
   float* negl2 = p.delta;
   float* neg_delta = reinterpret_cast<float*>(base + ws.delta);
   char *dk_part = base + ws.dk, *dv_part = base + ws.dv;
+  uint32_t* mask = MODE == kDrop && p.mask_scratch ? reinterpret_cast<uint32_t*>(base + ws.mask) : nullptr;
   using Part = typename std::conditional<MODE == kPlain, T, float>::type;
   const BwStats st{reinterpret_cast<float2*>(base + ws.g_stat), reinterpret_cast<float*>(base + ws.v_stat),
                    prep_blocks(Mpad, p.D), prep_blocks(p.N, p.D)};
   {
     constexpr bool kStats = kScaledDs<T, MODE>;
-    const unsigned blocks = (unsigned)(p.B * p.Hq * st.g_blocks + (kStats ? p.B * p.Hk * st.v_blocks : 0));
-    bwd_prep_kernel<T, kStats><<<blocks, 256, 0, s>>>(p, negl2, neg_delta, Mpad, st);
+    const unsigned rows_blocks = (unsigned)(p.B * p.Hq * st.g_blocks + (kStats ? p.B * p.Hk * st.v_blocks : 0));
+    const unsigned mask_blocks = mask != nullptr ? (unsigned)(mask_bytes(p.B, p.Hq, p.M, p.N) / 1024) : 0u;
+    bwd_prep_kernel<T, kStats, MODE == kDrop><<<rows_blocks + mask_blocks, 256, 0, s>>>(p, negl2, neg_delta, Mpad, st, mask,
+                                                                                      rows_blocks);
     count_launch();
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
@@ -879,6 +950,7 @@ cudaError_t launch_bwd_td(const BwdParams& p, cudaStream_t s) {
   tp.sm_scale = p.sm_scale; tp.negl2 = negl2; tp.neg_delta = neg_delta; tp.D = p.D;
   tp.drop = p.drop;
   tp.keep_scale = 1.f / (1.f - p.drop.p);
+  tp.mask = mask;
   tp.g_stat = st.g; tp.v_stat = st.v; tp.g_blocks = st.g_blocks; tp.v_blocks = st.v_blocks;
   int* status_word = tc_status_word();
   const bool per_head = p.G > 1;
@@ -946,6 +1018,11 @@ cudaError_t launch_bwd_t(const BwdParams& p, cudaStream_t s) {
 
 size_t tc_bwd_workspace_bytes(int B, int Hq, int Hk, int M, int N, int D, bool fine) {
   return bwd_ws(B, Hq, Hk, M, N, D, fine).total;
+}
+
+size_t tc_bwd_mask_bytes(int B, int Hq, int M, int N) {
+  const size_t bytes = mask_bytes(B, Hq, M, N);
+  return bytes <= kMaskBytes ? bytes : 0;
 }
 
 bool tc_bwd_supported(const BwdParams& p, int dtype) {
