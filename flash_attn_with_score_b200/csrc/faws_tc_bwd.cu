@@ -86,8 +86,8 @@ struct BwBars {
   uint64_t a_full[4], a_empty[4], b_full[4], b_empty[4];
   uint64_t s_full[2], dp_full[2];  // per buffer: written by the tensor pipe
   uint64_t s_free;                 // query-major: S' is in the consumers' registers
-  uint64_t p_ready[2][2][2];       // key-major, per S' buffer, warpgroup, 32 of its streamed rows: P' written
-  uint64_t ds_ready[2][2];         // per dP' buffer, warpgroup: dS' written
+  uint64_t p_ready[2][2];          // key-major, per S' buffer: P' of the first, last 32 rows of each warpgroup written
+  uint64_t ds_ready[2];            // per dP' buffer: dS' written
   uint64_t vec_full[2], vec_empty[2];
   uint64_t acc_done;
   uint32_t tmem_base;
@@ -244,10 +244,8 @@ tc_bwd_kernel(const __grid_constant__ BwMaps maps, const BwTcParams p, int* __re
       mbar_init(&bars->dp_full[w], 1);
       mbar_init(&bars->vec_full[w], 1);
       mbar_init(&bars->vec_empty[w], 8);
-      for (int e = 0; e < 2; ++e) {
-        for (int c = 0; c < 2; ++c) mbar_init(&bars->p_ready[w][e][c], 128);
-        mbar_init(&bars->ds_ready[w][e], 128);
-      }
+      for (int c = 0; c < 2; ++c) mbar_init(&bars->p_ready[w][c], 256);
+      mbar_init(&bars->ds_ready[w], 256);
     }
     mbar_init(&bars->s_free, 256);
     mbar_init(&bars->acc_done, 1);
@@ -371,18 +369,18 @@ tc_bwd_kernel(const __grid_constant__ BwMaps maps, const BwTcParams p, int* __re
         if constexpr (KM) {
           if (NSB == 2 && more) issue_s(u + 1);
 #pragma unroll
-          for (int x = 0; x < 4; ++x) {
-            wait(&bars->p_ready[u % NSB][x & 1][x >> 1], u / NSB);
-            if (ok) issue_dv(u, x & 1, x >> 1);
+          for (int c = 0; c < 2; ++c) {
+            wait(&bars->p_ready[u % NSB][c], u / NSB);
+            if (!ok) break;
+            issue_dv(u, 0, c);
+            issue_dv(u, 1, c);
           }
           if (!ok) break;
           mma_commit(&bars->b_empty[u % NB]);
           if (NSB == 1 && more) issue_s(u + 1);  // over P of this tile, which the MMAs before it have read
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            wait(&bars->ds_ready[u % NDB][e], u / NDB);
-            if (ok) issue_ds(u, e, COL_ACC + D);
-          }
+          wait(&bars->ds_ready[u % NDB], u / NDB);
+          if (ok) issue_ds(u, 0, COL_ACC + D);
+          if (ok) issue_ds(u, 1, COL_ACC + D);
           if (!ok) break;
           mma_commit(&bars->a_empty[u % NA]);
           if (more) issue_dp(u + 1);
@@ -393,11 +391,9 @@ tc_bwd_kernel(const __grid_constant__ BwMaps maps, const BwTcParams p, int* __re
             if (ok) issue_dp(u + 1);
             if (ok) mma_commit(&bars->b_empty[(u + 1) % NB]);
           }
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            wait(&bars->ds_ready[u % NDB][e], u / NDB);
-            if (ok) issue_ds(u, e, COL_ACC);
-          }
+          wait(&bars->ds_ready[u % NDB], u / NDB);
+          if (ok) issue_ds(u, 0, COL_ACC);
+          if (ok) issue_ds(u, 1, COL_ACC);
           if (ok) mma_commit(&bars->a_empty[u % NA]);
         }
       }
@@ -529,7 +525,7 @@ tc_bwd_kernel(const __grid_constant__ BwMaps maps, const BwTcParams p, int* __re
           tmem_st16(t_s + c * 16, pk);
           tmem_wait_st();
           tc_fence_before();
-          mbar_arrive(&bars->p_ready[u % NSB][e][c]);
+          mbar_arrive(&bars->p_ready[u % NSB][c]);
         }
       }
       // ---- dS' = P' (dP' - delta)
@@ -594,7 +590,7 @@ tc_bwd_kernel(const __grid_constant__ BwMaps maps, const BwTcParams p, int* __re
       }
       tmem_wait_st();
       tc_fence_before();
-      mbar_arrive(&bars->ds_ready[u % NDB][e]);
+      mbar_arrive(&bars->ds_ready[u % NDB]);
       if (KM) {  // this warp has read the tile's L and delta
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars->vec_empty[u & 1]);
