@@ -1381,6 +1381,9 @@ tc_colsoftmax_kernel(const __grid_constant__ CsMaps maps, const ColSoftmaxParams
       return v;
     };
 
+    // A warp without a key of the sum hands its scores back unread (fp16 B16 H8 S785 D32, where that is an eighth of all
+    // warps and another sixteenth of the query columns: 114 -> 107 us with the forward pass).
+    const bool no_keys = nk0 + lg * 32 >= p.n_end;
     bool alive = true;
     int mine = 0;  // tiles this warpgroup has processed
     const bool padded = p.negl_pad != nullptr;  // the producer fetches -L*log2e; else the warpgroup loads L itself
@@ -1401,20 +1404,27 @@ tc_colsoftmax_kernel(const __grid_constant__ CsMaps maps, const ColSoftmaxParams
       }
       if (!mbar_wait(&bars->s_full[wg], mine & 1, abort_flag)) { alive = false; break; }
       tc_fence_after();
+      if (no_keys) {
+        tc_fence_before();
+        mbar_arrive(&bars->s_free[wg]);
+        continue;
+      }
       const int g = u / ntq, qt = qt0 + (u - g * ntq);
       const int i0 = qt * BM;
+      // half tiles of queries that do not contribute (their -L is -inf) are left out
+      const int c_begin = i0 + CS_CHUNK <= i_lo ? CS_CHUNK : 0, c_end = i0 + CS_CHUNK >= p.m_end && c_begin == 0 ? CS_CHUNK : BM;
       // causal: query column x is visible to key j iff i0 + x + p_seq >= j
       const int xlo = p.causal ? (j - p.p_seq - i0) : 0;
       const bool full = !p.causal || (nk0 + BN - 1 - p.p_seq - i0 <= 0);
       float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
 #pragma unroll 1
-      for (int c0 = 0; c0 < BM; c0 += CS_CHUNK) {
+      for (int c0 = c_begin; c0 < c_end; c0 += CS_CHUNK) {
         uint32_t r[CS_CHUNK];
 #pragma unroll
         for (int c = 0; c < CS_CHUNK; c += 32)
           tmem_ld32(t_buf + c0 + c, reinterpret_cast<uint32_t(&)[32]>(r[c]));
         tmem_wait_ld();
-        if (c0 + CS_CHUNK == BM) {  // the buffer can take the next S^T of this warpgroup
+        if (c0 + CS_CHUNK == c_end) {  // the buffer can take the next S^T of this warpgroup
           tc_fence_before();
           mbar_arrive(&bars->s_free[wg]);
         }
