@@ -1382,7 +1382,7 @@ tc_colsoftmax_kernel(const __grid_constant__ CsMaps maps, const ColSoftmaxParams
     };
 
     // A warp without a key of the sum hands its scores back unread (fp16 B16 H8 S785 D32, where that is an eighth of all
-    // warps and another sixteenth of the query columns: 114 -> 107 us with the forward pass).
+    // warps and another sixteenth of the query columns: 114 -> 108 us with the forward pass).
     const bool no_keys = nk0 + lg * 32 >= p.n_end;
     bool alive = true;
     int mine = 0;  // tiles this warpgroup has processed
