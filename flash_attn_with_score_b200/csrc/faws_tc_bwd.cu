@@ -516,7 +516,8 @@ tc_bwd_kernel(const __grid_constant__ BwMaps maps, const BwTcParams p, int* __re
             if (kMasked && !(x + y >= x_lo && x + y <= x_hi)) pe = 0.f;
             sv[x + y] = __float_as_uint(pe);
             pr[y] = pe;
-            if constexpr (MODE == kDrop) pr[y] = (keep[c] >> (x + y - c * 32) & 1u) ? pe * kept : 0.f;
+            // a product, not a select: a weight that is not finite stays visible where it is dropped
+            if constexpr (MODE == kDrop) pr[y] = pe * ((keep[c] >> (x + y - c * 32) & 1u) ? kept : 0.f);
           }
           pk[(x - c * 32) / 2] = pack2<T>(pr[0], pr[1]);
           pk[(x - c * 32) / 2 + 1] = pack2<T>(pr[2], pr[3]);
