@@ -638,7 +638,7 @@ __global__ void reduce_ranks_kernel(const float* parts, int n_ranks, int64_t cou
 // One-row decoding, bf16 Hq32 Hk8 N9001 D128: B8 59.6 -> 57.1 us, B1 20.7 -> 14.4 us against a plain launch of
 // scalar loads.
 template <typename T, int V>
-__device__ __forceinline__ void combine_row(const float* __restrict__ o_part, const float* __restrict__ Ls, int64_t M, T* orow,
+__device__ __forceinline__ void combine_row(const float* o_part, const float* Ls, int64_t M, T* orow,
                                             int64_t s_step, int d, float mx, float inv, int S) {
   static_assert(V == 2 || V == 4, "dims of a lane");
   float acc[V];
@@ -673,7 +673,7 @@ __device__ __forceinline__ void combine_row(const float* __restrict__ o_part, co
 }
 
 template <typename T>
-__global__ void combine_splits_kernel(const float* __restrict__ o_part, const float* __restrict__ L_part, T* out,
+__global__ void combine_splits_kernel(const float* o_part, const float* L_part, T* out,
                                       int64_t o_sb, int64_t o_sh, int64_t o_ss, float* L, int B, int Hq, int M, int D,
                                       int S) {
   ptx::griddep_wait();

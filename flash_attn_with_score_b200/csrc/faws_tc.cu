@@ -1899,7 +1899,7 @@ bool tc_colsoftmax_supported(const ColSoftmaxParams& p, int dtype) {
 namespace {
 // -L_i*log2e into the tile-padded array the key-major kernel copies from; -inf for rows that do not
 // contribute (outside [i_lo, m_end), padding, or without a visible key).
-__global__ void negl_prep_kernel(const float* __restrict__ L, float* __restrict__ out, int M, int m_pad, int i_lo,
+__global__ void negl_prep_kernel(const float* L, float* out, int M, int m_pad, int i_lo,
                                  int m_end, long long total) {
   griddep_wait();  // L comes from the forward pass before this launch
   griddep_launch_dependents();

@@ -430,10 +430,10 @@ tc_bwd_kernel(const __grid_constant__ BwMaps maps, const BwTcParams p, int* __re
       const int bh = b * p.Hq + h, nqt = p.Mpad / BT, nkt = (p.N + BT - 1) / BT;
       if (KM) {
         const uint32_t* w = p.mask + mask_word(bh, u0 + u, own_tile, nqt, nkt) + (e * HALF + lane) * 4 + lg;
-        ahead[0] = __ldg(w);
-        ahead[1] = __ldg(w + 128);
+        ahead[0] = w[0];
+        ahead[1] = w[128];
       } else {
-        const uint2 w = __ldg(reinterpret_cast<const uint2*>(p.mask + mask_word(bh, own_tile, u, nqt, nkt) + row * 4 + e * 2));
+        const uint2 w = *reinterpret_cast<const uint2*>(p.mask + mask_word(bh, own_tile, u, nqt, nkt) + row * 4 + e * 2);
         ahead[0] = w.x;
         ahead[1] = w.y;
       }
@@ -826,7 +826,7 @@ struct GroupSumOut {
   int64_t sb, sh, ss;
 };
 template <typename T, typename P>
-__global__ void __launch_bounds__(256) bwd_group_sum_kernel(const P* __restrict__ dk_part, const P* __restrict__ dv_part,
+__global__ void __launch_bounds__(256) bwd_group_sum_kernel(const P* dk_part, const P* dv_part,
                                                             GroupSumOut dk, GroupSumOut dv, int B, int Hk, int G, int N,
                                                             int D) {
   griddep_wait();

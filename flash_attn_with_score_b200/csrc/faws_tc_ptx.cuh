@@ -160,6 +160,9 @@ __device__ __forceinline__ void named_bar_sync(uint32_t id, uint32_t nthreads) {
 // A kernel launched with the programmatic-stream-serialization attribute may start while the
 // previous kernel of the stream drains; it must not touch global memory before griddep_wait().
 // griddep_launch_dependents() lets such a successor start once every CTA of this grid has issued it.
+// What the previous kernel may still be writing is read with plain loads, never through the non-coherent path (__ldg, or
+// const pointers marked __restrict__, which the compiler may load that way): neither the compiler nor the cache holds
+// such loads to the order of the wait.
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void griddep_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
