@@ -20,7 +20,7 @@ CSRC = os.path.join(HERE, "csrc")
 OBJDIR = os.path.join(ROOT, "build", "libfaws")
 LIB = os.path.join(HERE, "libfaws.so")
 SOURCES = ["faws_abi.cu", "faws_generic.cu", "faws_tc.cu", "faws_tc_scores.cu", "faws_bwd.cu", "faws_tc_bwd.cu", "faws_noalloc.cu"]
-HEADERS = ["faws_internal.cuh", "faws_tc_ptx.cuh", "faws_tc_host.cuh", "faws_tc_store.cuh"]
+HEADERS = ["faws_internal.cuh", "faws_tc_ptx.cuh", "faws_tc_host.cuh", "faws_tc_store.cuh", "faws_launch_plan.h"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

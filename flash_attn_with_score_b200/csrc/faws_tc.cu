@@ -35,6 +35,7 @@
 #include <type_traits>
 
 #include "faws_internal.cuh"
+#include "faws_launch_plan.h"
 #include "faws_tc_host.cuh"
 #include "faws_tc_ptx.cuh"
 #include "faws_tc_store.cuh"
@@ -144,21 +145,6 @@ enum Hook : int {
   kHookNone = 0, kHookScores = 1, kHookRowSum = 2, kHookColPart = 3,
   kHookScores16 = 4,  // scores in the input dtype (what the reference kernel writes)
   kHookScoresAny = 5  // scores of either type in rows that TMA cannot address (odd lengths): plain stores
-};
-
-// Persistent launches: one CTA per SM walks a list of work items (an item is what one CTA of the
-// plain launch does: a row block of one head), in the order of the plain launch's grid.  The
-// lists are made on the host (longest item first onto the least loaded CTA) and travel as a
-// kernel parameter, so that no device-side counter is shared between launches; launches with
-// more items than the lists hold deal the items to the CTAs in rounds of alternating direction.
-constexpr int kMaxListedItems = 2048;
-constexpr int kMaxListCtas = 192;
-struct WorkList {
-  int n_items;  // 0: plain launch, every CTA does the item its block index names
-  int listed;   // 1: CTA c does ids[start[c]] .. ids[start[c + 1] - 1]
-  int gx, gy, gz;  // the grid of the plain launch; an item is a linear block index of it (x fastest)
-  uint16_t start[kMaxListCtas + 1];
-  uint16_t ids[kMaxListedItems];
 };
 
 template <typename T, int D, int HOOK, bool SPLIT, bool DROP = false, bool FEW = false>
@@ -1510,125 +1496,11 @@ int* tc_status_word() {
 
 namespace {
 
-// Work lists of a persistent launch.  An item costs its key tiles plus a fixed part; the items, heaviest
-// first, go one by one to the CTA with the least work so far (what the hardware does with the CTAs of a
-// plain launch, here decided ahead).  Made once per problem geometry and kept for the next call.
 bool persistent_allowed();
-
-struct WorkKey {
-  int gx, gy, gz, lpt, causal, p_seq, m_begin, m_end, N, rows, ctas, pack_m;
-  bool operator==(const WorkKey& o) const { return std::memcmp(this, &o, sizeof(WorkKey)) == 0; }
-};
 
 const WorkList& plain_work_list() {
   static const WorkList wl{};  // n_items = 0
   return wl;
-}
-
-// false: the launch should stay a plain one
-bool make_work_list(const FwdParams& p, dim3 grid, int cta_rows, int ctas, WorkList* out) {
-  const int n_items = (int)(grid.x * grid.y * grid.z);
-  if (ctas > kMaxListCtas || n_items <= ctas || n_items > 65535) return false;
-  const bool listed = n_items <= kMaxListedItems;
-  if (!listed && p.causal) return false;  // unequal items in no useful order: leave them to the hardware
-  thread_local WorkKey last_key{};
-  thread_local WorkList last{};
-  const WorkKey key{(int)grid.x, (int)grid.y, (int)grid.z, p.lpt_order, p.causal, p.p_seq, p.m_begin, p.m_end, p.N,
-                    cta_rows, ctas, p.pack_m};
-  if (last.n_items > 0 && key == last_key) {
-    *out = last;
-    return true;
-  }
-  WorkList& wl = last;
-  wl = WorkList{};
-  wl.n_items = n_items;
-  wl.listed = listed ? 1 : 0;
-  wl.gx = (int)grid.x;
-  wl.gy = (int)grid.y;
-  wl.gz = (int)grid.z;
-  if (listed) {
-    const int ncb = (int)(p.lpt_order ? grid.z : grid.x);
-    std::vector<int> cost(ncb);
-    for (int slot = 0; slot < ncb; ++slot) {
-      const int r0 = p.m_begin + (ncb - 1 - slot) * cta_rows;
-      int tiles = 0;
-      for (int t = 0; t * BM < cta_rows; ++t) {
-        const int r = r0 + t * BM;
-        int hi = 0;
-        if (r < p.m_end) hi = p.causal && p.pack_m == 0 ? std::max(0, std::min(p.N, p.p_seq + std::min(r + BM, p.m_end))) : p.N;
-        tiles = std::max(tiles, (hi + BN - 1) / BN);
-      }
-      cost[slot] = 19 * tiles + 30;  // measured on cfg3: 1.90 us per key tile + 3.0 us per item (unit 0.1 us)
-    }
-    auto cost_of = [&](int item) {
-      const int ix = item % wl.gx, iz = item / (wl.gx * wl.gy);
-      return cost[p.lpt_order ? iz : ix];
-    };
-    std::vector<int> order(n_items);
-    for (int i = 0; i < n_items; ++i) order[i] = i;
-    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cost_of(a) > cost_of(b); });
-    // Heaviest item first onto the CTA with the least work so far (what the hardware does with the CTAs
-    // of a plain grid), then exchanges of single items between any two CTAs that bring their loads closer
-    // together, fuller CTAs first against the emptiest.  Exchanges keep the number of items per CTA, so
-    // the result does not lean on the fixed cost per item, which differs between the hooks (3 us plain,
-    // 6 us with the column hook, measured on cfg3; packing to a capacity instead put up to 30 small items
-    // on one CTA and was 30 % slower under the column hook).  cfg3: 48..56 key tiles per CTA -> 50..52.
-    std::vector<std::vector<uint16_t>> mine(ctas);
-    std::vector<long long> load(ctas, 0);
-    {
-      using Load = std::pair<long long, int>;  // (work so far, CTA)
-      std::priority_queue<Load, std::vector<Load>, std::greater<Load>> heap;
-      for (int c = 0; c < ctas; ++c) heap.push({0, c});
-      for (int item : order) {
-        Load l = heap.top();
-        heap.pop();
-        mine[l.second].push_back((uint16_t)item);
-        load[l.second] = l.first + cost_of(item);
-        heap.push({load[l.second], l.second});
-      }
-    }
-    for (int round = 0; round < 32; ++round) {
-      bool improved = false;
-      std::vector<int> by_load(ctas);
-      for (int c = 0; c < ctas; ++c) by_load[c] = c;
-      std::stable_sort(by_load.begin(), by_load.end(), [&](int x, int y) { return load[x] > load[y]; });
-      for (int ai = 0; ai < ctas; ++ai) {
-        const int A = by_load[ai];
-        for (int bi = ctas - 1; bi >= 0; --bi) {
-          const int B = by_load[bi];
-          const long long gap = load[A] - load[B];
-          if (gap <= 0) break;  // (the order is the one before this round's exchanges: good enough)
-          long long best_gain = 0, best_d = 0;
-          int bia = -1, bib = -1;
-          for (size_t ia = 0; ia < mine[A].size(); ++ia)
-            for (size_t ib = 0; ib < mine[B].size(); ++ib) {
-              const long long d = cost_of(mine[A][ia]) - cost_of(mine[B][ib]);
-              if (d <= 0 || d >= gap) continue;
-              const long long after = gap - 2 * d;
-              const long long gain = gap - (after < 0 ? -after : after);  // how much closer the two get
-              if (gain > best_gain) { best_gain = gain; best_d = d; bia = (int)ia; bib = (int)ib; }
-            }
-          if (bia < 0) continue;
-          std::swap(mine[A][bia], mine[B][bib]);
-          load[A] -= best_d;
-          load[B] += best_d;
-          improved = true;
-        }
-      }
-      if (!improved) break;
-    }
-    for (int c = 0; c < ctas; ++c)  // heaviest item first within a CTA
-      std::stable_sort(mine[c].begin(), mine[c].end(), [&](uint16_t x, uint16_t y) { return cost_of(x) > cost_of(y); });
-    int at = 0;
-    for (int c = 0; c < ctas; ++c) {
-      wl.start[c] = (uint16_t)at;
-      for (uint16_t id : mine[c]) wl.ids[at++] = id;
-    }
-    for (int c = ctas; c <= kMaxListCtas; ++c) wl.start[c] = (uint16_t)at;
-  }
-  last_key = key;
-  *out = wl;
-  return true;
 }
 
 template <typename T, int D, int HOOK, bool SPLIT, bool DROP = false, bool FEW = false>
@@ -1655,8 +1527,9 @@ cudaError_t launch_fwd_s(const TcMaps& maps, const FwdParams& p, cudaStream_t s)
   WorkList wl_persist;
   const WorkList* wl = &plain_work_list();
   if constexpr (!SPLIT && (HOOK == kHookNone || HOOK == kHookRowSum || HOOK == kHookColPart)) {
-    if (pp.n_splits == 1 && !pp.fill_ctas && persistent_allowed() &&
-        make_work_list(pp, grid, L::kRows, sm_count(), &wl_persist)) {
+    const WorkShape shape{(int)grid.x, (int)grid.y, (int)grid.z, pp.lpt_order, pp.causal, pp.p_seq, pp.m_begin, pp.m_end,
+                          pp.N, L::kRows, sm_count(), pp.pack_m};
+    if (pp.n_splits == 1 && !pp.fill_ctas && persistent_allowed() && make_work_list(shape, &wl_persist)) {
       wl = &wl_persist;
       grid = dim3(sm_count(), 1, 1);
     }
