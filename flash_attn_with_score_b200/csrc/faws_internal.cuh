@@ -226,7 +226,7 @@ bool tc_bwd_supported(const BwdParams& p, int dtype);
 cudaError_t launch_tc_bwd(const BwdParams& p, int dtype, cudaStream_t s);  // p.delta = the workspace base
 // fine: with dropout or a head dim below 64 (fp32 partials, statistics of the pre-pass)
 size_t tc_bwd_workspace_bytes(int B, int Hq, int Hk, int M, int N, int D, bool fine);
-size_t tc_bwd_mask_bytes(int B, int Hq, int M, int N);  // the dropout mask, behind that; 0 where it is not kept
+size_t tc_bwd_mask_bytes(int B, int Hq, int M, int N);  // of the dropout mask of the heads that take a turn; 0 where none is kept
 
 int tc_read_status(int reset);  // synchronising read of the device status word
 cudaError_t launch_wait_give_up(cudaStream_t s);  // self-test: a bounded wait that runs out

@@ -41,6 +41,7 @@
 // is 1 and their dS is 0, and the zero Q / dout row contributes nothing); stores are clipped.  Every mbarrier wait is bounded.
 #include <cuda.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "faws_internal.cuh"
@@ -114,14 +115,19 @@ struct BwTcParams {
   const float* v_stat;   // (B,Hk,v_blocks) of |v_j|^2
   int g_blocks, v_blocks;
   const uint32_t* mask;  // dropout: the mask as the pre-pass has drawn it (see draw_mask), or null
+  int bh0;               // dropout: the launch's first (batch, head)
 };
 
 // The dropout mask in scratch, one bit per entry, 1 = kept: per (b, h, 128-row query tile, 128-key tile) 2 KB, four
 // words a row, bit x of word w of row r is entry (r, 32 w + x).  Both kernels need it, and a kernel with nothing else to
 // do draws it at twice the rate of the two consumer warps that a scheduler of the main kernels has: fp16 B4 H16 S1024 D64
-// causal, p = 0.1, forward and backward: 247 us, 282 with the mask drawn in both.  Beyond kMaskBytes of scratch (one bit
-// per entry grows with M * N) both kernels draw for themselves, as they do in scratch that has no room for it.
-constexpr size_t kMaskBytes = size_t(256) << 20;
+// causal, p = 0.1, forward and backward: 247 us, 282 with the mask drawn in both.  One bit per entry grows with M * N:
+// beyond kMaskBytes the heads take turns, pre-pass and both kernels for as many at a time as fit, or as keep the SMs
+// busy (kMaskCtas) if those are more: backward passes of fp16 B2 H32 S8192 D64 causal 8.96 -> 6.5 ms against drawing in
+// both, bf16 B8 Hq32 Hk8 S4096 D128 causal 10.2 -> 8.3 (two shares each).  Heads whose mask is above kMaskBytesMost draw in both kernels, as calls with
+// scratch that has no room for a mask do.
+constexpr size_t kMaskBytes = size_t(256) << 20, kMaskBytesMost = size_t(1) << 30;
+constexpr int kMaskCtas = 1024;  // seven waves
 __device__ __forceinline__ int64_t mask_word(int bh, int qt, int kt, int nqt, int nkt) {
   return (((int64_t)bh * nqt + qt) * nkt + kt) * 512;
 }
@@ -205,7 +211,12 @@ tc_bwd_kernel(const __grid_constant__ BwMaps maps, const BwTcParams p, int* __re
   // causal; query-major, the last query tiles see the most keys.
   const int own_tiles = (int)gridDim.z;
   const int own_tile = KM ? (int)blockIdx.z : (p.causal ? own_tiles - 1 - (int)blockIdx.z : (int)blockIdx.z);
-  const int h = blockIdx.x, b = blockIdx.y;
+  int h = blockIdx.x, b = blockIdx.y;
+  if constexpr (MODE == kDrop) {  // the heads of a launch are consecutive, of several batches maybe
+    const int bh = p.bh0 + b * (int)gridDim.x + h;
+    b = bh / p.Hq;
+    h = bh - b * p.Hq;
+  }
   const int hk = h / p.G;
   const int own0 = own_tile * BT;  // first owned row: key n0 (key-major) or query i0 (query-major)
 
@@ -427,7 +438,7 @@ tc_bwd_kernel(const __grid_constant__ BwMaps maps, const BwTcParams p, int* __re
     // + 64) of its query row; key-major: the word of the warp's 32 keys in rows 64 e + lane and 64 e + 32 + lane.
     [[maybe_unused]] uint32_t ahead[2] = {0u, 0u};
     [[maybe_unused]] auto fetch_mask = [&](int u) {
-      const int bh = b * p.Hq + h, nqt = p.Mpad / BT, nkt = (p.N + BT - 1) / BT;
+      const int bh = b * p.Hq + h - p.bh0, nqt = p.Mpad / BT, nkt = (p.N + BT - 1) / BT;
       if (KM) {
         const uint32_t* w = p.mask + mask_word(bh, u0 + u, own_tile, nqt, nkt) + (e * HALF + lane) * 4 + lg;
         ahead[0] = w[0];
@@ -726,13 +737,13 @@ __device__ __forceinline__ float2 block_max(float x, float y, float2 (&red)[8]) 
   }
   return make_float2(x, y);
 }
-// A word of the mask per thread, two blocks a tile; tiles without a visible entry are left out.
-__device__ __forceinline__ void draw_mask(const BwdParams& p, uint32_t* mask, int64_t block) {
+// A word of the mask per thread, two blocks a tile; tiles without a visible entry are left out.  The mask's first head is bh0.
+__device__ __forceinline__ void draw_mask(const BwdParams& p, uint32_t* mask, int bh0, int64_t block) {
   const int nqt = (p.M + BT - 1) / BT, nkt = (p.N + BT - 1) / BT;
   const int64_t tile = block >> 1;
   const int kt = (int)(tile % nkt);
   const int64_t rest = tile / nkt;
-  const int qt = (int)(rest % nqt), bh = (int)(rest / nqt);
+  const int qt = (int)(rest % nqt), bh = bh0 + (int)(rest / nqt);
   if (p.causal && kt * BT > qt * BT + BT - 1 + p.p_seq) return;
   const int at = (int)(block & 1) * 256 + threadIdx.x;
   uint32_t lin = ((uint32_t)bh * (uint32_t)p.M + (uint32_t)(qt * BT + (at >> 2))) * (uint32_t)p.N + (uint32_t)(kt * BT + (at & 3) * 32);
@@ -743,10 +754,10 @@ __device__ __forceinline__ void draw_mask(const BwdParams& p, uint32_t* mask, in
 }
 template <typename T, bool STATS, bool DRAW>
 __global__ void __launch_bounds__(256) bwd_prep_kernel(BwdParams p, float* negl2, float* neg_delta, int Mpad, BwStats st,
-                                                       uint32_t* mask, unsigned mask_block0) {
+                                                       uint32_t* mask, int bh0, unsigned mask_block0) {
   griddep_launch_dependents();
   if (DRAW && blockIdx.x >= mask_block0) {
-    draw_mask(p, mask, blockIdx.x - mask_block0);
+    draw_mask(p, mask, bh0, blockIdx.x - mask_block0);
     return;
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -897,8 +908,15 @@ int prep_blocks(int rows, int D) {
 struct BwWs {
   size_t delta, g_stat, v_stat, dk, dv, mask, total;
 };
-size_t mask_bytes(int B, int Hq, int M, int N) {
-  return (size_t)B * Hq * (mpad_of(M) / BT) * ((N + BT - 1) / BT) * 2048;
+size_t head_mask_bytes(int M, int N) { return (size_t)(mpad_of(M) / BT) * ((N + BT - 1) / BT) * 2048; }
+// (batch, head) pairs whose mask is held at a time; 0: none is.  Shares of as equal size as they come.
+int mask_heads(int B, int Hq, int M, int N) {
+  const size_t per = head_mask_bytes(M, N);
+  const size_t heads = (size_t)B * Hq, ctas = std::min(mpad_of(M) / BT, (N + BT - 1) / BT);  // a head's, of the smaller launch
+  const size_t fit = std::min(std::max(kMaskBytes / per, (kMaskCtas + ctas - 1) / ctas), kMaskBytesMost / per);
+  if (fit == 0) return 0;
+  const size_t shares = (heads + fit - 1) / fit;
+  return (int)((heads + shares - 1) / shares);
 }
 BwWs bwd_ws(int B, int Hq, int Hk, int M, int N, int D, bool fine) {
   auto up = [](size_t x) { return (x + 255) & ~size_t(255); };
@@ -930,18 +948,23 @@ cudaError_t launch_bwd_td(const BwdParams& p, cudaStream_t s) {
   float* neg_delta = reinterpret_cast<float*>(base + ws.delta);
   char *dk_part = base + ws.dk, *dv_part = base + ws.dv;
   uint32_t* mask = MODE == kDrop && p.mask_scratch ? reinterpret_cast<uint32_t*>(base + ws.mask) : nullptr;
+  const int heads = p.B * p.Hq, share = mask != nullptr ? mask_heads(p.B, p.Hq, p.M, p.N) : heads;
   using Part = typename std::conditional<MODE == kPlain, T, float>::type;
   const BwStats st{reinterpret_cast<float2*>(base + ws.g_stat), reinterpret_cast<float*>(base + ws.v_stat),
                    prep_blocks(Mpad, p.D), prep_blocks(p.N, p.D)};
-  {
+  // One round, or (dropout) one per share of the heads, whose pre-pass waits for the kernels that read the last mask: it is
+  // launched plainly.  The rows' arrays of all heads come with the first.
+  auto prepare = [&](int bh0) -> cudaError_t {
     constexpr bool kStats = kScaledDs<T, MODE>;
-    const unsigned rows_blocks = (unsigned)(p.B * p.Hq * st.g_blocks + (kStats ? p.B * p.Hk * st.v_blocks : 0));
-    const unsigned mask_blocks = mask != nullptr ? (unsigned)(mask_bytes(p.B, p.Hq, p.M, p.N) / 1024) : 0u;
-    bwd_prep_kernel<T, kStats, MODE == kDrop><<<rows_blocks + mask_blocks, 256, 0, s>>>(p, negl2, neg_delta, Mpad, st, mask,
+    const int n = std::min(share, heads - bh0);
+    const unsigned rows_blocks = bh0 > 0 ? 0u : (unsigned)(p.B * p.Hq * st.g_blocks + (kStats ? p.B * p.Hk * st.v_blocks : 0));
+    const unsigned mask_blocks = mask != nullptr ? (unsigned)(n * (head_mask_bytes(p.M, p.N) / 1024)) : 0u;
+    bwd_prep_kernel<T, kStats, MODE == kDrop><<<rows_blocks + mask_blocks, 256, 0, s>>>(p, negl2, neg_delta, Mpad, st, mask, bh0,
                                                                                       rows_blocks);
     count_launch();
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  }
+    return cudaGetLastError();
+  };
+  if ((e = prepare(0)) != cudaSuccess) return e;
   BwTcParams tp{};
   tp.Hq = p.Hq; tp.G = p.G; tp.M = p.M; tp.N = p.N; tp.p_seq = p.p_seq; tp.causal = p.causal; tp.Mpad = Mpad;
   tp.sm_scale = p.sm_scale; tp.negl2 = negl2; tp.neg_delta = neg_delta; tp.D = p.D;
@@ -952,9 +975,14 @@ cudaError_t launch_bwd_td(const BwdParams& p, cudaStream_t s) {
   int* status_word = tc_status_word();
   const bool per_head = p.G > 1;
   const bool map_parts = per_head && MODE == kPlain;  // 16-bit partials go through the store maps
-  // query-major: dQ
-  {
-    BwMaps m;
+  BwTcParams tk = tp;  // the key-major launches': with the fp32 partials
+  if (per_head && !map_parts) {
+    tk.part0 = reinterpret_cast<float*>(dv_part);
+    tk.part1 = reinterpret_cast<float*>(dk_part);
+  }
+  BwMaps qm, km;
+  {  // query-major: dQ
+    BwMaps& m = qm;
     if (!make_map_bhsd(&m.x, p.q, p.D, p.M, p.Hq, p.B, p.q_ss, p.q_sh, p.q_sb, 128) ||
         !make_map_bhsd(&m.y, p.dout, p.D, p.M, p.Hq, p.B, p.do_ss, p.do_sh, p.do_sb, 128) ||
         !make_map_bhsd(&m.a, p.k, p.D, p.N, p.Hk, p.B, p.k_ss, p.k_sh, p.k_sb, 128) ||
@@ -962,18 +990,9 @@ cudaError_t launch_bwd_td(const BwdParams& p, cudaStream_t s) {
         !make_map_bhsd(&m.o0, p.dq, p.D, p.M, p.Hq, p.B, p.dq_ss, p.dq_sh, p.dq_sb, 32))
       return cudaErrorInvalidValue;
     m.o1 = m.o0;
-    dim3 grid(p.Hq, p.B, (p.M + BT - 1) / BT);
-    if ((e = launch_overlapped(tc_bwd_kernel<T, D, false, MODE>, grid, NTHREADS, Lq::total, s, m, tp, status_word)) !=
-        cudaSuccess)
-      return e;
   }
-  // key-major: dV, dK (per query head)
-  {
-    BwMaps m;
-    if (per_head && !map_parts) {
-      tp.part0 = reinterpret_cast<float*>(dv_part);
-      tp.part1 = reinterpret_cast<float*>(dk_part);
-    }
+  {  // key-major: dV, dK (per query head)
+    BwMaps& m = km;
     void* dv_dst = map_parts ? static_cast<void*>(dv_part) : p.dv;
     void* dk_dst = map_parts ? static_cast<void*>(dk_part) : p.dk;
     const int o_heads = per_head && !map_parts ? p.Hk : p.Hq;  // (those maps are not used with fp32 partials)
@@ -987,9 +1006,17 @@ cudaError_t launch_bwd_td(const BwdParams& p, cudaStream_t s) {
         !make_map_bhsd(&m.o1, dk_dst, p.D, p.N, o_heads, p.B, map_parts ? ph_ss : p.dk_ss,
                        map_parts ? ph_sh : p.dk_sh, map_parts ? ph_sb : p.dk_sb, 32))
       return cudaErrorInvalidValue;
-    dim3 grid(p.Hq, p.B, (p.N + BT - 1) / BT);
-    if ((e = launch_overlapped(tc_bwd_kernel<T, D, true, MODE>, grid, NTHREADS, Lk::total, s, m, tp, status_word)) !=
-        cudaSuccess)
+  }
+  for (int bh0 = 0; bh0 < heads; bh0 += share) {
+    if (bh0 > 0 && (e = prepare(bh0)) != cudaSuccess) return e;
+    tp.bh0 = tk.bh0 = bh0;
+    const bool all = share == heads;
+    const unsigned gx = all ? p.Hq : std::min(share, heads - bh0), gy = all ? p.B : 1;
+    if ((e = launch_overlapped(tc_bwd_kernel<T, D, false, MODE>, dim3(gx, gy, (p.M + BT - 1) / BT), NTHREADS, Lq::total, s,
+                               qm, tp, status_word)) != cudaSuccess)
+      return e;
+    if ((e = launch_overlapped(tc_bwd_kernel<T, D, true, MODE>, dim3(gx, gy, (p.N + BT - 1) / BT), NTHREADS, Lk::total, s,
+                               km, tk, status_word)) != cudaSuccess)
       return e;
   }
   if (per_head) {
@@ -1018,8 +1045,7 @@ size_t tc_bwd_workspace_bytes(int B, int Hq, int Hk, int M, int N, int D, bool f
 }
 
 size_t tc_bwd_mask_bytes(int B, int Hq, int M, int N) {
-  const size_t bytes = mask_bytes(B, Hq, M, N);
-  return bytes <= kMaskBytes ? bytes : 0;
+  return mask_heads(B, Hq, M, N) * head_mask_bytes(M, N);
 }
 
 bool tc_bwd_supported(const BwdParams& p, int dtype) {
