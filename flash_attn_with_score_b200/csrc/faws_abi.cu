@@ -643,7 +643,7 @@ size_t faws_workspace_bytes(int32_t op, const faws_problem* p, int32_t split) {
       return split == 1 ? 0 : split_kv_bytes(p, split);
     case FAWS_OP_ATTENTION_BACKWARD:  // enough for either kernel family
       return tc_bwd_workspace_bytes(p->B, p->Hq, p->Hk, p->M, p->N, p->D, p->dropout_p > 0.f || p->D < 64) +
-             (p->dropout_p > 0.f ? tc_bwd_mask_bytes(p->B, p->Hq, p->M, p->N) : 0);
+             (p->dropout_p > 0.f && tc_allowed(p) ? tc_bwd_mask_bytes(p->B, p->Hq, p->M, p->N) : 0);
     case FAWS_OP_COL_SUM:
     case FAWS_OP_COL_SUM_SEQUENTIAL:
       return align256(partial_floats(p, 0, p->N) * 4) + align256(qsum_floats(p) * 4);

@@ -274,7 +274,7 @@ int faws_attention_backward(const faws_problem* p, const faws_grads* g, void* wo
  * dropout decide the kernels and with them the scratch.  With FAWS_BACKEND_AUTO the backward pass and the buffered
  * cross-token sums also take what was asked for the same shape with other tensors or without dropout, and run on the
  * CUDA-core kernels where it is too small for the tcgen05 ones or for the score buffer.
- * With dropout the backward pass's scratch ends with the mask of as many heads as take a turn (one bit per query and
+ * With dropout the scratch of the tcgen05 backward pass ends with the mask of as many heads as take a turn (one bit per query and
  * key in tiles of 128 x 128): up to 256 MB, or up to 1 GB for heads of more than some 16384 tokens.  Those bytes may be
  * left out: the tcgen05 kernels then draw the mask as they go, with the same results, but slower (B2 Hq32 S8192 D64
  * causal, backward pass: 9.0 ms, 6.5 with the mask). */

@@ -72,6 +72,22 @@ def test_validation_without_gpu(lib):
     assert lib.faws_reduce_ranks(None, 2, 4, None, None) == -1
 
 
+def test_backward_scratch_holds_a_mask_for_the_family_that_reads_one(lib):
+    from flash_attn_with_score_b200 import _lib
+    p = _lib.Problem()
+    p.B, p.Hq, p.Hk, p.M, p.N, p.D, p.m_end, p.sm_scale = 2, 4, 2, 300, 200, 64, 300, 0.125
+    for t, h, n in ((p.q, 4, 300), (p.k, 2, 200), (p.v, 2, 200), (p.out, 4, 300)):  # fake addresses, never dereferenced
+        t.ptr, t.stride_b, t.stride_h, t.stride_s = 1 << 21, h * n * 64, n * 64, 64
+    size = {}
+    for dropout in (0.0, 0.25):
+        for backend in (_lib.BACKEND_AUTO, _lib.BACKEND_GENERIC, _lib.BACKEND_TCGEN05):
+            p.dropout_p, p.backend = dropout, backend
+            size[dropout, backend] = lib.faws_workspace_bytes(_lib.OP_ATTENTION_BACKWARD, C.byref(p), 0)
+    mask = 2 * 4 * 3 * 2 * 2048  # a bit per entry of 3 x 2 tiles a head
+    assert size[0.25, _lib.BACKEND_AUTO] == size[0.25, _lib.BACKEND_TCGEN05] == size[0.25, _lib.BACKEND_GENERIC] + mask
+    assert size[0.0, _lib.BACKEND_AUTO] == size[0.0, _lib.BACKEND_GENERIC] < size[0.25, _lib.BACKEND_GENERIC]
+
+
 def test_python_asserts_mirror_reference():
     import flash_attn_with_score_b200 as F
     q = torch.zeros(1, 4, 8, 64, dtype=torch.float16)
