@@ -89,7 +89,7 @@ struct Smem {
 
 struct Bars {
   uint64_t q_full;
-  uint64_t q_empty;       // persistent CTAs: the item's last Q.K^T has completed, the next item's Q tiles may land
+  uint64_t q_empty;       // persistent CTAs: the last Q.K^T of an item with key tiles has completed, the next Q tiles may land
   uint64_t kv_full[MAX_KV_SLOTS], kv_empty[MAX_KV_SLOTS];
   uint64_t s_full[2];     // per query tile: S_t written by the tensor pipe
   uint64_t p_half[2];     // per query tile: the first 64 columns of P_t are in TMEM
@@ -380,18 +380,21 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
       // Persistent CTAs: the ring runs on across items, so the next item's first K and V tiles arrive
       // while the current item's last tiles are computed; its Q tiles follow as soon as the current
       // item's last Q.K^T has completed.
+      // Items without key tiles (causal, rows that see no key) take no part in q_full and q_empty: the MMA warp goes
+      // through them without waiting for anybody, and two phases of q_empty that complete before this thread looks
+      // would read as none.
       int ring_base = 0;
+      int q_loads = nt > 0 ? 1 : 0;  // items whose Q tiles were loaded
       bool ok = true;
       for (int k = 0; ok; ++k) {
-        if (k > 0) {
-          if (!(ok = mbar_wait(&bars->q_empty, (k - 1) & 1, abort_flag))) break;
-          if (nt > 0) {
-            mbar_arrive_expect_tx(&bars->q_full, L::kQTiles * L::kTile);
-            for (int t = 0; t < L::kQTiles; ++t)
-              for (int c = 0; c < D / 64; ++c)
-                tma_load_4d(smem + L::q_off + t * L::kTile + c * L::kSub, &maps.q, &bars->q_full, c * 64,
-                            r_tile_of[t] - p.m_begin, h, b);
-          }
+        if (k > 0 && nt > 0) {
+          if (q_loads > 0 && !(ok = mbar_wait(&bars->q_empty, (q_loads - 1) & 1, abort_flag))) break;
+          ++q_loads;
+          mbar_arrive_expect_tx(&bars->q_full, L::kQTiles * L::kTile);
+          for (int t = 0; t < L::kQTiles; ++t)
+            for (int c = 0; c < D / 64; ++c)
+              tma_load_4d(smem + L::q_off + t * L::kTile + c * L::kSub, &maps.q, &bars->q_full, c * 64,
+                          r_tile_of[t] - p.m_begin, h, b);
         }
         for (int idx = (k == 0 ? n_early : 0); idx < 2 * nt; ++idx) {
           const int g = ring_base + idx;
@@ -438,9 +441,12 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
         }
       }
       __syncwarp();
-      if (lane == 0) mbar_arrive(&bars->q_empty);  // this warp no longer reads the item's Q tiles
-      // (its arrival for the next item must not be counted in this item's phase)
-      if (!persist || !mbar_wait(&bars->q_empty, k & 1, abort_flag) || !goto_item(k + 1)) break;
+      if (nt > 0) {
+        if (lane == 0) mbar_arrive(&bars->q_empty);  // this warp no longer reads the item's Q tiles
+        // (its arrival for the next item must not be counted in this item's phase)
+        if (persist && !mbar_wait(&bars->q_empty, (q_cnt - 1) & 1, abort_flag)) break;
+      }
+      if (!goto_item(k + 1)) break;
       }
     } else if (warp == 1) {
       // ---------------------------------------------------------- MMA issuer
@@ -589,10 +595,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
       }  // !SPLIT
       if (ok) commit(&bars->o_done);
       ring_base += 2 * nt;
-      } else {  // an item without key tiles: nothing was loaded, nothing to issue
-        if (elect_one()) mbar_arrive(&bars->q_empty);
-        __syncwarp();
-      }
+      }  // (an item without key tiles: nothing was loaded, nothing to issue)
       if (!ok || !goto_item(k + 1)) break;
       }
     }
