@@ -95,7 +95,7 @@ struct Bars {
   uint64_t p_half[2];     // per query tile: the first 64 columns of P_t are in TMEM
   uint64_t p_ready[2];    // per query tile: P_t written by its 128 softmax threads
   uint64_t col_ready[2];  // per query tile: column-sum partial rows of its 4 warps are in smem
-  uint64_t o_done;        // every MMA of the CTA has completed
+  uint64_t o_done[2];     // per warpgroup: every MMA of an item in which it has key tiles has completed
   uint64_t merge_ready;   // SPLIT: warpgroup 1 has published its (m, l, row sum)
   uint32_t tmem_base;
   int abort_flag;
@@ -341,7 +341,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
       mbar_init(&bars->p_ready[t], 128);
       mbar_init(&bars->col_ready[t], 128);
     }
-    mbar_init(&bars->o_done, 1);
+    for (int t = 0; t < 2; ++t) mbar_init(&bars->o_done[t], 1);
     mbar_init(&bars->merge_ready, 128);
     bars->abort_flag = 0;
     mbar_fence_init();
@@ -593,7 +593,10 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
         }
       }
       }  // !SPLIT
-      if (ok) commit(&bars->o_done);
+      // A warpgroup without key tiles in an item does not wait for it: with one barrier for both, the item after its last
+      // one could complete that barrier's next phase before the warpgroup looks, and two phases read as none.
+      for (int t = 0; t < 2; ++t)
+        if (ok && nt_q[t] > kt0) commit(&bars->o_done[t]);
       ring_base += 2 * nt;
       }  // (an item without key tiles: nothing was loaded, nothing to issue)
       if (!ok || !goto_item(k + 1)) break;
@@ -625,7 +628,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
     bool alive = true;
     int hook_cnt = 0;  // column hook executions (selects its smem buffer and barrier phase)
     int s_cnt = 0;     // key tiles processed (phase of s_full)
-    int o_cnt = 0;     // items with key tiles (phase of o_done)
+    int o_cnt = 0;     // items in which this warpgroup has key tiles (phase of its o_done)
 
     // One key tile.  The row's 128 scores are read from TMEM once and stay in registers: first
     // for the max and exp2 passes (the chain the tensor pipe waits on), then, after P has been
@@ -974,10 +977,10 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
 
     // ---- epilogue: O / l -> out, log-normaliser, row sums, masked fill of unvisited tiles
     if (alive && my_nt > kt0) {
-      if (!mbar_wait(&bars->o_done, o_cnt & 1, abort_flag)) alive = false;
+      if (!mbar_wait(&bars->o_done[qt], o_cnt & 1, abort_flag)) alive = false;
+      ++o_cnt;
       tc_fence_after();
     }
-    if (nt > 0) ++o_cnt;
     // SPLIT: warpgroup 1 publishes its running state; warpgroup 0 merges the two partial results.
     float* merge = reinterpret_cast<float*>(smem + L::kv_off);  // ring is free after o_done
     bool write_out = alive && r_tile < p.m_end;
