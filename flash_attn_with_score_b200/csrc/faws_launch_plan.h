@@ -34,31 +34,86 @@ struct WorkShape {
   bool operator==(const WorkShape& o) const { return std::memcmp(this, &o, sizeof(WorkShape)) == 0; }
 };
 
-// Fewer than two items per CTA: the heaviest items one to a CTA, then the rest back from the last CTA, so that the lightest
-// of the first round get the heaviest that are left.  Along the grid's row-block axis the items come heaviest first, and
-// every head has the same, so that nothing is sorted or weighed.  Over S 128 to 8192 and all head counts with 149 to 295 items the
-// heaviest CTA is never heavier than in the list that greedy dealing and exchanges make (below), which takes 65 to 160 us of host time,
-// three times the kernel where every call has another length: sixteen lengths around causal S2048 H28 D128, a call among
-// others 122 us with that list; the 128-row launch without one 55.
-inline void deal_pairs(const WorkShape& sh, WorkList* wl) {
-  const int n = wl->n_items, ncb = sh.lpt ? sh.gz : sh.gx, per_block = n / ncb;
-  auto ranked = [&](int k) -> uint16_t {  // k-th item, heaviest first
-    if (sh.lpt) return (uint16_t)k;       // row blocks are the slowest axis: launch order
-    return (uint16_t)(k / per_block + k % per_block * sh.gx);
-  };
-  int at = 0;
-  for (int c = 0; c < sh.ctas; ++c) {
-    wl->start[c] = (uint16_t)at;
-    wl->ids[at++] = ranked(c);
-    if (2 * sh.ctas - 1 - c < n) wl->ids[at++] = ranked(2 * sh.ctas - 1 - c);
+// Cost of the work items of each row block, by the block's place on the grid's row-block axis, which is heaviest first.
+inline std::vector<int> block_costs(const WorkShape& sh) {
+  const int ncb = sh.lpt ? sh.gz : sh.gx;
+  std::vector<int> cost(ncb);
+  for (int slot = 0; slot < ncb; ++slot) {
+    const int r0 = sh.m_begin + (ncb - 1 - slot) * sh.rows;
+    int tiles = 0;
+    for (int t = 0; t * kPlanTile < sh.rows; ++t) {
+      const int r = r0 + t * kPlanTile;
+      int hi = 0;
+      if (r < sh.m_end)
+        hi = sh.causal && sh.pack_m == 0 ? std::max(0, std::min(sh.N, sh.p_seq + std::min(r + kPlanTile, sh.m_end))) : sh.N;
+      tiles = std::max(tiles, (hi + kPlanTile - 1) / kPlanTile);
+    }
+    cost[slot] = 19 * tiles + 30;  // measured on cfg3: 1.90 us per key tile + 3.0 us per item (unit 0.1 us)
   }
-  for (int c = sh.ctas; c <= kMaxListCtas; ++c) wl->start[c] = (uint16_t)at;
+  return cost;
+}
+
+// Fewer than two items per CTA: heaviest item first, those of equal cost in launch order (neighbours share K and V: full S512
+// H144 20.4 us, 20.9 row block by row block), each to the CTA with the least work so far (the first of them), and no exchanges after
+// that (below), which would not make the heaviest CTA lighter.  A few microseconds at most, for kernels of 20 to 70;
+// with a sort of the items, a heap of the CTAs and exchanges it was 65 to 160: sixteen lengths around causal S2048 H28
+// D128, a call among others 122 us, the 128-row launch without a list 55.  The CTAs wait in bins of equal load, so that a step
+// takes the lowest bit of the first bin.  (Pairing the items off from both ends is simpler still and makes no CTA heavier, but
+// causal B5 H12 S1024 D128 took 32.1 us for 31.8, with row sums 34.9 for 34.1.)
+inline void deal_short(const WorkShape& sh, const std::vector<int>& cost, WorkList* wl) {
+  const int n = wl->n_items, ncb = (int)cost.size(), per_block = n / ncb;
+  uint16_t order[2 * kMaxListCtas], of[2 * kMaxListCtas];  // the items, heaviest first; their CTAs
+  for (int slot = 0, k = 0; slot < ncb;) {
+    int end = slot + 1;
+    while (end < ncb && cost[end] == cost[slot]) ++end;
+    if (sh.lpt) {  // row blocks are the slowest axis of the grid: launch order
+      for (const int to = end * per_block; k < to; ++k) order[k] = (uint16_t)k;
+    } else {
+      for (int rest = 0; rest < per_block; ++rest)
+        for (int x = slot; x < end; ++x) order[k++] = (uint16_t)(x + rest * sh.gx);
+    }
+    slot = end;
+  }
+  struct Bin {
+    int load;
+    uint64_t ctas[kMaxListCtas / 64];
+  };
+  std::vector<Bin> bins;  // lightest last
+  auto put = [&](int load, int cta) {
+    size_t at = bins.size();
+    while (at > 0 && bins[at - 1].load < load) --at;
+    if (at == 0 || bins[at - 1].load != load) bins.insert(bins.begin() + at, Bin{load, {}});
+    else --at;
+    bins[at].ctas[cta >> 6] |= uint64_t(1) << (cta & 63);
+  };
+  for (int k = 0; k < n; ++k) {
+    int cta = k, load = 0;
+    if (k >= sh.ctas) {
+      Bin& lightest = bins.back();
+      int w = 0;
+      while (lightest.ctas[w] == 0) ++w;
+      cta = w * 64 + __builtin_ctzll(lightest.ctas[w]);
+      load = lightest.load;
+      lightest.ctas[w] &= lightest.ctas[w] - 1;
+      bool empty = true;
+      for (uint64_t word : lightest.ctas) empty = empty && word == 0;
+      if (empty) bins.pop_back();
+    }
+    of[k] = (uint16_t)cta;
+    put(load + cost[k / per_block], cta);
+  }
+  uint16_t count[kMaxListCtas] = {};
+  for (int k = 0; k < n; ++k) ++count[of[k]];
+  wl->start[0] = 0;
+  for (int c = 0; c < kMaxListCtas; ++c) wl->start[c + 1] = (uint16_t)(wl->start[c] + count[c]);
+  uint16_t at[kMaxListCtas];
+  std::memcpy(at, wl->start, sizeof(at));
+  for (int k = 0; k < n; ++k) wl->ids[at[of[k]]++] = order[k];  // (a CTA's items come heaviest first)
 }
 
 // Work lists of a persistent launch.  An item costs its key tiles plus a fixed part; the items, heaviest
 // first, go one by one to the CTA with the least work so far (what the hardware does with the CTAs of a
 // plain launch, here decided ahead).  Made once per problem geometry and kept for the next call.
-// (Fewer than two items per CTA are dealt in pairs.)
 // false: the launch should stay a plain one
 inline bool make_work_list(const WorkShape& sh, WorkList* out) {
   const int n_items = sh.gx * sh.gy * sh.gz, ctas = sh.ctas;
@@ -67,7 +122,7 @@ inline bool make_work_list(const WorkShape& sh, WorkList* out) {
   if (!listed && sh.causal) return false;  // unequal items in no useful order: leave them to the hardware
   if (n_items < 2 * ctas) {
     *out = WorkList{n_items, 1, sh.gx, sh.gy, sh.gz, {}, {}};
-    deal_pairs(sh, out);
+    deal_short(sh, block_costs(sh), out);
     return true;
   }
   thread_local WorkShape last_shape{};
@@ -84,20 +139,7 @@ inline bool make_work_list(const WorkShape& sh, WorkList* out) {
   wl.gy = sh.gy;
   wl.gz = sh.gz;
   if (listed) {
-    const int ncb = sh.lpt ? sh.gz : sh.gx;
-    std::vector<int> cost(ncb);
-    for (int slot = 0; slot < ncb; ++slot) {
-      const int r0 = sh.m_begin + (ncb - 1 - slot) * sh.rows;
-      int tiles = 0;
-      for (int t = 0; t * kPlanTile < sh.rows; ++t) {
-        const int r = r0 + t * kPlanTile;
-        int hi = 0;
-        if (r < sh.m_end)
-          hi = sh.causal && sh.pack_m == 0 ? std::max(0, std::min(sh.N, sh.p_seq + std::min(r + kPlanTile, sh.m_end))) : sh.N;
-        tiles = std::max(tiles, (hi + kPlanTile - 1) / kPlanTile);
-      }
-      cost[slot] = 19 * tiles + 30;  // measured on cfg3: 1.90 us per key tile + 3.0 us per item (unit 0.1 us)
-    }
+    const std::vector<int> cost = block_costs(sh);
     auto cost_of = [&](int item) {
       const int ix = item % wl.gx, iz = item / (wl.gx * wl.gy);
       return cost[sh.lpt ? iz : ix];
@@ -168,5 +210,4 @@ inline bool make_work_list(const WorkShape& sh, WorkList* out) {
   *out = wl;
   return true;
 }
-
 }  // namespace faws
