@@ -1,5 +1,5 @@
-// Host side of the forward launches: the work lists of persistent launches.  Plain C++, compiled into the library and,
-// alone, into its test.
+// Host side of the forward launches: the row count of a CTA and the work lists of persistent launches.  Plain C++, compiled
+// into the library and, alone, into its tests.
 #pragma once
 #include <algorithm>
 #include <cstdint>
@@ -209,5 +209,74 @@ inline bool make_work_list(const WorkShape& sh, WorkList* out) {
   last_shape = sh;
   *out = wl;
   return true;
+}
+
+
+// The row count of a CTA, for launches of fewer than two 256-row CTAs per SM (above, 256 rows always).  128-row CTAs, whose two
+// warpgroups split the key tiles, shorten the chain of dependent key tiles of launches with few CTAs; they fetch each K / V
+// tile twice as often and are launched plainly, where 256-row ones walk balanced lists.
+struct RowChoice {
+  long long heads;  // of all batches
+  int m_begin, m_end, N, p_seq, causal, sms;
+  int blocks(int rows) const { return (m_end - m_begin + rows - 1) / rows; }
+};
+enum RowChoiceKind { kPlainOut, kWithRowSums, kWithColSums };
+
+// us: of a CTA, of a key tile, of a launch; how much the CTAs of unequal length of a launch of two waves and more add to it; of a
+// CTA without a visible key; of a key tile of a last row block that is not whole (column sums: such a block reduces every
+// tile itself)
+struct LaunchFit {
+  double fix, per, base, uneven, empty, ragged;
+};
+// Fitted to 1 576 launches of either row count, for the choice between the two more than for the times (fp16 and bf16,
+// multi-head and grouped, head dims 32 to 128, M 129 to 4096 rows against 129 to 4096 keys, M < N, M = N and M > N, 75 to
+// 295 256-row CTAs, causal and not).
+inline const LaunchFit& launch_fit(bool d128, RowChoiceKind kind, int rows) {
+  static constexpr LaunchFit kFits[3][2][2] = {  // [kind][D = 128][128 rows]
+      {{{4.51, 1.59, 1.01, 1.00, 4.02, 0.0}, {4.51, 0.81, 0.27, 1.09, 1.66, 0.0}},
+       {{4.66, 1.81, 2.08, 1.00, 0.01, 0.0}, {4.88, 0.98, 0.76, 1.12, 2.06, 0.0}}},
+      {{{5.20, 1.70, 1.17, 1.05, 0.00, 0.0}, {4.89, 0.86, 0.58, 1.07, 1.93, 0.0}},
+       {{5.58, 1.86, 2.01, 1.07, 0.00, 0.0}, {5.41, 1.04, 0.85, 1.08, 2.59, 0.0}}},
+      {{{6.62, 1.77, 6.52, 1.36, 0.00, 1.21}, {7.30, 0.98, 4.18, 1.31, 1.49, 0.91}},
+       {{7.96, 2.04, 6.75, 1.33, 0.00, 1.14}, {8.52, 1.14, 5.20, 1.24, 1.48, 0.89}}}};
+  return kFits[kind][d128 ? 1 : 0][rows == 128 ? 1 : 0];
+}
+
+// A lower bound of the launch's makespan, one CTA per SM at a time (the longest CTA, the mean load, and what the j SMs + 1
+// longest CTAs force onto one SM), lengthened where it takes several waves of unequal CTAs.  The row blocks of a head get
+// heavier towards its end (causal) or are alike, and every head has the same ones.
+inline double expected_us(const RowChoice& c, bool d128, RowChoiceKind kind, int rows) {
+  const LaunchFit& f = launch_fit(d128, kind, rows);
+  const int ncb = c.blocks(rows);
+  const long long n = ncb * c.heads;
+  auto job = [&](int cb) -> double {
+    const int end = std::min(c.m_begin + (cb + 1) * rows, c.m_end);
+    const int hi = c.causal ? std::max(0, std::min(c.N, c.p_seq + end)) : c.N;
+    const int tiles = (hi + kPlanTile - 1) / kPlanTile;
+    const bool ragged = cb == ncb - 1 && (c.m_end - c.m_begin) % kPlanTile != 0;
+    return tiles == 0 ? f.empty : f.fix + (f.per + (ragged ? f.ragged : 0.0)) * tiles;
+  };
+  auto ranked = [&](long long i) -> double { return i < n ? job(ncb - 1 - (int)(i / c.heads)) : 0.0; };
+  double total = 0.0;
+  for (int cb = 0; cb < ncb; ++cb) total += job(cb);
+  const double longest = job(ncb - 1);
+  double us = std::max(longest, total * (double)c.heads / c.sms);
+  for (int j = 1; j <= 3 && (long long)j * c.sms < n; ++j) {
+    double sum = 0.0;
+    for (int x = 0; x <= j; ++x) sum += ranked((long long)j * c.sms - x);
+    us = std::max(us, sum);
+  }
+  if (n <= c.sms || longest <= 0.0) return f.base + us;
+  return f.base + us * (1.0 + (f.uneven - 1.0) * (1.0 - job(0) / longest) * std::min(1.0, (double)(n - c.sms) / c.sms));
+}
+
+// 256 rows have to be expected 3 % faster, 4 % where there are column sums.  Of 4 605 such launches with each row count 2 943 take
+// 256, 14 of which run more than 2 % slower than with 128 (5.5 % at most); the mean launch is 0.2 % behind the better
+// of the two.  128 rows everywhere are 8 to 11 % slower in the mean, up to 1.5 times: causal D128 S2048 H32 48.4 and 39.4 us, full S512 H144 34.7 and
+// 23.1, S1024 H64 48.0 and 36.5; the other way causal S2048 H8 19.2 and 33.4, full S2048 H24 57.4 and 63.3, causal M2048 N700
+// H20 with column sums, where most row blocks see no key, 18.7 and 26.9.
+inline bool prefer_256_rows(const RowChoice& c, bool d128, RowChoiceKind kind) {
+  const double small = expected_us(c, d128, kind, 128), large = expected_us(c, d128, kind, 256);
+  return small > (kind == kWithColSums ? 1.04 : 1.03) * large;
 }
 }  // namespace faws

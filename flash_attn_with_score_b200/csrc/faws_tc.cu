@@ -1567,57 +1567,7 @@ bool persistent_allowed() {
   return on;
 }
 
-// Lower bound of a launch's makespan in CTAs of `rows` query rows, one per SM at a time, each `fix` + `per` us a key tile:
-// the longest CTA, the mean load, and what the j SMs + 1 longest CTAs force onto one SM.  The row blocks of a head get
-// heavier towards its end (causal) or are alike, and every head has the same ones.
-double makespan_us(const FwdParams& p, int rows, double fix, double per, bool* waves) {
-  const int ncb = (p.m_end - p.m_begin + rows - 1) / rows, sms = sm_count();
-  const long long heads = (long long)p.B * p.Hq, n = ncb * heads;
-  auto job = [&](int cb) -> double {
-    const int end = std::min(p.m_begin + (cb + 1) * rows, p.m_end);
-    const int hi = p.causal ? std::max(0, std::min(p.N, p.p_seq + end)) : p.N;
-    return fix + per * ((hi + BN - 1) / BN);
-  };
-  auto ranked = [&](long long i) -> double { return i < n ? job(ncb - 1 - (int)(i / heads)) : 0.0; };
-  double total = 0.0;
-  for (int cb = 0; cb < ncb; ++cb) total += job(cb);
-  double us = std::max(job(ncb - 1), total * (double)heads / sms);
-  for (int j = 1; j <= 3 && (long long)j * sms < n; ++j) {
-    double sum = 0.0;
-    for (int x = 0; x <= j; ++x) sum += ranked((long long)j * sms - x);
-    us = std::max(us, sum);
-  }
-  *waves = n > sms;
-  return us;
-}
-
-// 128-row CTAs, whose two warpgroups split the key tiles, shorten the chain of dependent key tiles of launches with few
-// CTAs; they fetch each K / V tile twice as often and are launched plainly, where 256-row ones walk balanced lists.
-// Which is faster: above two 256-row CTAs per SM the latter; below, by a bound of the makespan and constants fitted to 139
-// launches of each (fp16, 60 to 288 256-row CTAs, S 512 to 4096, causal and not; 4 to 6 % rms).  256-row CTAs have to be expected
-// 8 % faster, so that the fit's own error costs no launch more than a few percent.  The line at two CTAs per SM that stood
-// here alone was up to 1.5 times slower:
-// causal D128 S2048 H32 48.4 and 39.4 us, full S512 H144 34.7 and 23.1, S1024 H64 48.0 and 36.5; the other way causal
-// S2048 H8 19.2 and 33.4, full S2048 H24 57.4 and 63.3.
 // FAWS_SPLIT_KV=0/1 in the environment overrides the choice (tests, ablations).
-struct LaunchFit {
-  double fix, per, base, uneven;  // us a CTA, a key tile, a launch; factor for causal launches of several waves
-};
-template <int D, int HOOK>
-double expected_us(const FwdParams& p, bool split) {
-  constexpr bool d128 = D == 128;
-  constexpr LaunchFit kNone[2] = {d128 ? LaunchFit{4.03, 1.62, 3.4, 1.09} : LaunchFit{3.41, 1.46, 2.9, 1.10},
-                                  d128 ? LaunchFit{4.71, 0.87, 0.8, 1.12} : LaunchFit{3.98, 0.75, 0.8, 1.14}};
-  constexpr LaunchFit kRow[2] = {d128 ? LaunchFit{4.59, 1.66, 3.4, 1.15} : LaunchFit{4.04, 1.55, 2.7, 1.17},
-                                 d128 ? LaunchFit{5.05, 0.91, 0.8, 1.15} : LaunchFit{4.15, 0.77, 1.1, 1.19}};
-  constexpr LaunchFit kCol[2] = {d128 ? LaunchFit{7.86, 1.79, 7.2, 1.16} : LaunchFit{5.52, 1.60, 8.1, 1.21},
-                                 d128 ? LaunchFit{7.01, 0.97, 6.3, 1.28} : LaunchFit{5.54, 0.84, 6.6, 1.34}};
-  const LaunchFit f = (HOOK == kHookColPart ? kCol : HOOK == kHookRowSum ? kRow : kNone)[split ? 1 : 0];
-  bool waves = false;
-  const double us = makespan_us(p, split ? 128 : 256, f.fix, f.per, &waves);
-  return f.base + us * (p.causal && waves ? f.uneven : 1.0);
-}
-
 template <int D, int HOOK>
 bool use_split_kv(const FwdParams& p) {
   static const int forced = [] {
@@ -1625,12 +1575,11 @@ bool use_split_kv(const FwdParams& p) {
     return e == nullptr ? -1 : (e[0] == '1' ? 1 : 0);
   }();
   if (forced >= 0) return forced == 1;
-  const int sms = sm_count();
-  const long long ctas256 = (long long)((p.m_end - p.m_begin + 255) / 256) * p.Hq * p.B;
-  if (ctas256 >= 2LL * sms) return false;
+  const RowChoice c{(long long)p.B * p.Hq, p.m_begin, p.m_end, p.N, p.p_seq, p.causal, sm_count()};
+  if (c.blocks(256) * c.heads >= 2LL * c.sms) return false;
   constexpr bool kStores = HOOK == kHookScores || HOOK == kHookScores16 || HOOK == kHookScoresAny;
-  if (kStores || p.n_splits > 1 || p.pack_m > 0) return true;  // (the fit knows none of these)
-  return expected_us<D, HOOK>(p, true) <= 1.08 * expected_us<D, HOOK>(p, false);
+  if (kStores || p.n_splits > 1 || p.pack_m > 0) return true;  // (the expected times know none of these)
+  return !prefer_256_rows(c, D == 128, HOOK == kHookColPart ? kWithColSums : HOOK == kHookRowSum ? kWithRowSums : kPlainOut);
 }
 
 template <typename T, int D, int HOOK>
