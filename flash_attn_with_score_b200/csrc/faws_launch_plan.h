@@ -270,11 +270,11 @@ inline double expected_us(const RowChoice& c, bool d128, RowChoiceKind kind, int
   return f.base + us * (1.0 + (f.uneven - 1.0) * (1.0 - job(0) / longest) * std::min(1.0, (double)(n - c.sms) / c.sms));
 }
 
-// 256 rows have to be expected 3 % faster, 4 % where there are column sums.  Of 4 605 such launches with each row count 2 943 take
-// 256, 14 of which run more than 2 % slower than with 128 (5.5 % at most); the mean launch is 0.2 % behind the better
-// of the two.  128 rows everywhere are 8 to 11 % slower in the mean, up to 1.5 times: causal D128 S2048 H32 48.4 and 39.4 us, full S512 H144 34.7 and
-// 23.1, S1024 H64 48.0 and 36.5; the other way causal S2048 H8 19.2 and 33.4, full S2048 H24 57.4 and 63.3, causal M2048 N700
-// H20 with column sums, where most row blocks see no key, 18.7 and 26.9.
+// 256 rows have to be expected 3 % faster, 4 % where there are column sums.  Of 4 605 such launches with each row count
+// 2 943 take 256, 14 of which run more than 2 % slower than with 128 (5.5 % at most); the mean launch is 0.2 % behind the
+// better of the two.  128 rows everywhere are 8 to 11 % slower in the mean, up to 1.5 times: causal D128 S2048 H32 48.4 and
+// 39.4 us, full S512 H144 34.7 and 23.1, S1024 H64 48.0 and 36.5; the other way causal S2048 H8 19.2 and 33.4, full S2048
+// H24 57.4 and 63.3, causal M2048 N700 H20 with column sums, where most row blocks see no key, 18.7 and 26.9.
 inline bool prefer_256_rows(const RowChoice& c, bool d128, RowChoiceKind kind) {
   const double small = expected_us(c, d128, kind, 128), large = expected_us(c, d128, kind, 256);
   return small > (kind == kWithColSums ? 1.04 : 1.03) * large;

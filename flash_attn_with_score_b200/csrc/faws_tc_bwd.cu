@@ -19,7 +19,7 @@
 // so that P is computed while dK and dP' run, and dS while dV and the next S' do.  S' and dP' are whole 128-column MMAs:
 // with 64 columns an MMA reads 6 KB of shared memory per 32 cycles (51 cycles measured), with 128 8 KB per 64 (65
 // measured).  One thread issues them: the pipe's queue holds about six, and a whole warp that elects a lane for each
-// group spends another 100 cycles between groups (4 340 against 3 390 cycles a step, key-major D128).
+// group spends another 100 cycles between groups (4 340 against 3 390 cycles a step, key-major D128, all else alike).
 // The 128 streamed rows are shared out to two consumer warpgroups, 64 rows each.
 // Warp roles (12 warps): warp 0 TMA producer (X, Y once, then rings of A and B tiles), warp 1 TMEM allocation and
 // the MMA-issuing thread, warp 2 (key-major) the L / delta vectors of the streamed query tiles, warps 4-7 / 8-11
@@ -32,7 +32,7 @@
 // (GradScale), and moved back in the epilogue: exact, and gradients of any size come out as from fp32 dS.
 // kDrop is kFine with the dropout mask, which the pre-pass draws (draw_mask).  In fine modes hi and lo of 16 streamed
 // rows, the K-step of the accumulating MMAs, take the 16 columns that their dP' leaves.  fp16 B4 H16 S1024 D64 causal,
-// p = 0.1, forward and backward: 247 us, 3 717 us with the CUDA-core kernels; errors of the gradients against fp64 as
+// p = 0.1, forward and backward: 240 us, 3 717 us with the CUDA-core kernels; errors of the gradients against fp64 as
 // there (2.32e-4, 2.28e-4, 2.92e-4 for dq, dk, dv, fp16; dout of 1e-4, where the results are fp16 subnormals: 1.6e-3,
 // 6.6e-3 with an unmoved dS).
 // Deterministic: every output element is written once, by one CTA, in a fixed order; with GQA the
@@ -124,8 +124,8 @@ struct BwTcParams {
 // causal, p = 0.1, forward and backward: 247 us, 282 with the mask drawn in both.  One bit per entry grows with M * N:
 // beyond kMaskBytes the heads take turns, pre-pass and both kernels for as many at a time as fit, or as keep the SMs
 // busy (kMaskCtas) if those are more: backward passes of fp16 B2 H32 S8192 D64 causal 8.96 -> 6.5 ms against drawing in
-// both, bf16 B8 Hq32 Hk8 S4096 D128 causal 10.2 -> 8.3 (two shares each).  Heads whose mask is above kMaskBytesMost draw in both kernels, as calls with
-// scratch that has no room for a mask do.
+// both, bf16 B8 Hq32 Hk8 S4096 D128 causal 10.2 -> 8.3 (two shares each).  Heads whose mask is above kMaskBytesMost draw
+// in both kernels, as calls with scratch that has no room for a mask do.
 constexpr size_t kMaskBytes = size_t(256) << 20, kMaskBytesMost = size_t(1) << 30;
 constexpr int kMaskCtas = 1024;  // seven waves
 __device__ __forceinline__ int64_t mask_word(int bh, int qt, int kt, int nqt, int nkt) {
