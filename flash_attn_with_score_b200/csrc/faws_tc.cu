@@ -28,10 +28,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <algorithm>
-#include <cstring>
 #include <mutex>
-#include <queue>
-#include <vector>
 #include <type_traits>
 
 #include "faws_internal.cuh"
