@@ -21,11 +21,13 @@ OP_SOFTMAX_COL_SUM, OP_CROSS_QK_SUM, OP_CROSS_SOFTMAX_SUM, OP_CROSS_SOFTMAX_SUM_
 OP_TOTAL_ATTENTION = 9
 OP_ATTENTION_BACKWARD = 10
 OP_ATTENTION_SPLIT_KV = 11
+OP_ATTENTION_BACKWARD_MASKED = 12
 
 # every symbol include/faws.h declares
 EXPORTS = [
     "faws_attention", "faws_attention_with_scores", "faws_compute_attention_scores", "faws_split_kv_plan",
     "faws_attention_split_kv", "faws_attention_with_row_sum",
+    "faws_dropout_mask_bytes", "faws_attention_keep_mask", "faws_attention_backward_masked",
     "faws_attention_with_col_sum", "faws_attention_with_col_sum_noalloc",
     "faws_attention_with_col_sum_sequential",
     "faws_attention_with_softmax_col_sum", "faws_attention_cross_token_qk_sum",
@@ -79,6 +81,9 @@ def load():
     vp, i32, u32, sz = C.c_void_p, C.c_int32, C.c_uint32, C.c_size_t
     protos = {
         "faws_attention": (i32, [PP, vp]),
+        "faws_dropout_mask_bytes": (sz, [PP]),
+        "faws_attention_keep_mask": (i32, [PP, vp, sz, vp]),
+        "faws_attention_backward_masked": (i32, [PP, C.POINTER(Grads), vp, sz, vp, sz, vp]),
         "faws_attention_with_scores": (i32, [PP, vp, i32, u32, vp]),
         "faws_compute_attention_scores": (i32, [PP, vp, i32, vp]),
         "faws_split_kv_plan": (i32, [PP]),

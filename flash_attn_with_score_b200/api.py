@@ -104,7 +104,7 @@ class _Call:
                             L.data_ptr() if L is not None else 0, _lib.BACKENDS[backend])
         p = _lib.Problem.from_buffer(buf)
         p.sm_scale = float(sm_scale)
-        self.seed = self.offset = None
+        self.seed = self.offset = self.mask = None
         if dropout_p and dropout_p > 0.0:
             assert dropout_p < 1.0, "dropout_p must be < 1"
             seed, offset = philox if philox is not None else philox_cuda_seed_offset(B * H * M * N, q.device)
@@ -144,14 +144,19 @@ def _f32_bits(x: float) -> int:
 
 
 def _attention_forward(q, k, v, causal, sm_scale, dropout_p, need_L, want_total, q_rows, backend, philox,
-                       kv_splits=None):
+                       kv_splits=None, keep_mask=False):
     c = _Call(q, k, v, causal, sm_scale, dropout_p, need_L=need_L, q_rows=q_rows, backend=backend,
               philox=philox, rescale=True)
+    # dropout in training: the mask is drawn once, for both passes, where the library would rather keep it
+    mask_bytes = int(c.lib.faws_dropout_mask_bytes(C.byref(c.p))) if keep_mask and c.seed is not None else 0
     # few query rows (decoding): split the keys over more CTAs, as flash.py:68-70,97-134 does
     n_splits = int(c.lib.faws_split_kv_plan(C.byref(c.p))) if kv_splits is None else int(kv_splits)
     if n_splits > 1:
         ws, n = c.workspace(_lib.OP_ATTENTION_SPLIT_KV, n_splits)
         c.run("faws_attention_split_kv", n_splits, C.c_void_p(ws.data_ptr()), n)
+    elif mask_bytes:
+        c.mask = torch.empty(mask_bytes, device=c.dev, dtype=torch.uint8)
+        c.run("faws_attention_keep_mask", C.c_void_p(c.mask.data_ptr()), mask_bytes)
     else:
         c.run("faws_attention")
     tot = None
@@ -168,8 +173,8 @@ class _AttentionFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, causal, sm_scale, dropout_p, want_total, backend, philox, kv_splits):
         c, tot = _attention_forward(q, k, v, causal, sm_scale, dropout_p, True, want_total, None, backend, philox,
-                                    kv_splits)
-        ctx.save_for_backward(c.q, c.k, c.v, c.out, c.L)
+                                    kv_splits, keep_mask=True)
+        ctx.save_for_backward(c.q, c.k, c.v, c.out, c.L, c.mask)
         ctx.causal, ctx.sm_scale, ctx.dropout_p, ctx.backend = causal, float(c.p.sm_scale), dropout_p, backend
         ctx.philox = (c.seed, c.offset) if c.seed is not None else None
         ctx.mark_non_differentiable(*[t for t in (c.L, tot) if t is not None])
@@ -178,7 +183,7 @@ class _AttentionFunction(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, do, *ignored):
-        q, k, v, o, L = ctx.saved_tensors
+        q, k, v, o, L, mask = ctx.saved_tensors
         if do is None:  # nothing downstream had a gradient for out
             return (*map(torch.zeros_like, (q, k, v)), *(None,) * 7)
         do = maybe_contiguous(do)
@@ -186,8 +191,13 @@ class _AttentionFunction(torch.autograd.Function):
                   philox=ctx.philox, rescale=True)
         dq, dk, dv = torch.empty_like(c.q), torch.empty_like(c.k), torch.empty_like(c.v)
         g = _lib.Grads(_tensor(do), _tensor(dq), _tensor(dk), _tensor(dv))
-        ws, n = c.workspace(_lib.OP_ATTENTION_BACKWARD)
-        c.run("faws_attention_backward", C.byref(g), C.c_void_p(ws.data_ptr()), n)
+        if mask is not None:
+            ws, n = c.workspace(_lib.OP_ATTENTION_BACKWARD_MASKED)
+            c.run("faws_attention_backward_masked", C.byref(g), C.c_void_p(mask.data_ptr()), mask.numel(),
+                  C.c_void_p(ws.data_ptr()), n)
+        else:
+            ws, n = c.workspace(_lib.OP_ATTENTION_BACKWARD)
+            c.run("faws_attention_backward", C.byref(g), C.c_void_p(ws.data_ptr()), n)
         return dq, dk, dv, None, None, None, None, None, None, None
 
 

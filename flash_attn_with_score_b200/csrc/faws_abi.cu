@@ -405,6 +405,17 @@ bool scores_only_on_cuda_cores(const ScoresOnlyParams& p, int sms) {
   return cuda_cores < tc;
 }
 
+// Bytes of the dropout mask that a forward pass leaves for its backward pass, 0 where it leaves none.  Drawing it takes both
+// passes 1.4 us a million entries; keeping it costs memory from one to the other, and a launch.  Kept where it is no larger
+// than the queries, which are kept as well (up to 16 D keys), and at least 1 MB.
+size_t kept_mask_bytes(const faws_problem* p) {
+  if (!(p->dropout_p > 0.f) || p->m_begin != 0 || p->m_end != p->M || p->v.ptr == nullptr || p->out.ptr == nullptr) return 0;
+  const size_t bytes = (size_t)p->B * p->Hq * cdiv(p->M, 128) * cdiv(p->N, 128) * 2048;
+  if (bytes < (size_t(1) << 20) || bytes > (size_t)p->B * p->Hq * p->M * p->D * 2) return 0;
+  if (!tc_allowed(p) || !tc_fwd_supported(make_fwd(p), p->dtype)) return 0;
+  return bytes;
+}
+
 size_t split_kv_bytes(const faws_problem* p, int n_splits) {
   return align256((size_t)p->B * p->Hq * n_splits * p->M * 4) +
          align256((size_t)p->B * p->Hq * n_splits * p->M * p->D * 4);
@@ -425,6 +436,22 @@ int faws_attention(const faws_problem* p, void* stream) {
   FwdParams f = make_fwd_packed(p, pack_m);
   int bm, bn;
   return run_fwd(p, f, static_cast<cudaStream_t>(stream), &bm, &bn);
+}
+
+size_t faws_dropout_mask_bytes(const faws_problem* p) { return validate(p) == FAWS_OK ? kept_mask_bytes(p) : 0; }
+
+int faws_attention_keep_mask(const faws_problem* p, void* mask, size_t mask_bytes, void* stream) {
+  const int st = validate(p);
+  if (st != FAWS_OK) return st;
+  const size_t need = kept_mask_bytes(p);
+  if (need == 0) return FAWS_EUNSUPPORTED;
+  if (mask == nullptr || mask_bytes < need || misaligned_ws(mask)) return FAWS_EWORKSPACE;
+  FwdParams f = make_fwd(p);
+  f.drop_mask = static_cast<uint32_t*>(mask);
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (launch_dropout_mask(f, static_cast<uint32_t*>(mask), s) != cudaSuccess) return FAWS_ECUDA;
+  int bm, bn;
+  return run_fwd(p, f, s, &bm, &bn);
 }
 
 int faws_attention_with_scores(const faws_problem* p, void* scores, int32_t scores_dtype,
@@ -584,8 +611,8 @@ int faws_total_attention(const faws_problem* p, float* total, void* stream) {
   return run_colsoftmax(p, c, total, nullptr, 0, static_cast<cudaStream_t>(stream));
 }
 
-int faws_attention_backward(const faws_problem* p, const faws_grads* g, void* workspace,
-                            size_t workspace_bytes, void* stream) {
+static int backward(const faws_problem* p, const faws_grads* g, const void* mask, void* workspace, size_t workspace_bytes,
+                    void* stream) {
   int st = validate(p);
   if (st != FAWS_OK) return st;
   if (g == nullptr || p->v.ptr == nullptr || p->out.ptr == nullptr || p->log_normalizer == nullptr ||
@@ -614,6 +641,7 @@ int faws_attention_backward(const faws_problem* p, const faws_grads* g, void* wo
   b.B = p->B; b.Hq = p->Hq; b.Hk = p->Hk; b.G = p->Hq / p->Hk; b.M = p->M; b.N = p->N; b.D = p->D;
   b.p_seq = p->N - p->M; b.causal = p->causal ? 1 : 0; b.sm_scale = p->sm_scale;
   b.drop = make_drop(p);
+  b.mask = static_cast<const uint32_t*>(mask);
   const size_t mask_bytes = p->dropout_p > 0.f ? tc_bwd_mask_bytes(p->B, p->Hq, p->M, p->N) : 0;
   b.mask_scratch = mask_bytes > 0 && workspace_bytes >= need + mask_bytes;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -635,6 +663,21 @@ int faws_attention_backward(const faws_problem* p, const faws_grads* g, void* wo
   return FAWS_OK;
 }
 
+int faws_attention_backward(const faws_problem* p, const faws_grads* g, void* workspace,
+                            size_t workspace_bytes, void* stream) {
+  return backward(p, g, nullptr, workspace, workspace_bytes, stream);
+}
+
+int faws_attention_backward_masked(const faws_problem* p, const faws_grads* g, const void* mask, size_t mask_bytes,
+                                   void* workspace, size_t workspace_bytes, void* stream) {
+  const int st = validate(p);
+  if (st != FAWS_OK) return st;
+  const size_t need = kept_mask_bytes(p);
+  if (need == 0) return FAWS_EUNSUPPORTED;
+  if (mask == nullptr || mask_bytes < need || misaligned_ws(mask)) return FAWS_EWORKSPACE;
+  return backward(p, g, mask, workspace, workspace_bytes, stream);
+}
+
 size_t faws_workspace_bytes(int32_t op, const faws_problem* p, int32_t split) {
   if (validate(p) != FAWS_OK) return 0;
   switch (op) {
@@ -644,6 +687,8 @@ size_t faws_workspace_bytes(int32_t op, const faws_problem* p, int32_t split) {
     case FAWS_OP_ATTENTION_BACKWARD:  // enough for either kernel family
       return tc_bwd_workspace_bytes(p->B, p->Hq, p->Hk, p->M, p->N, p->D, p->dropout_p > 0.f || p->D < 64) +
              (p->dropout_p > 0.f && tc_allowed(p) ? tc_bwd_mask_bytes(p->B, p->Hq, p->M, p->N) : 0);
+    case FAWS_OP_ATTENTION_BACKWARD_MASKED:
+      return tc_bwd_workspace_bytes(p->B, p->Hq, p->Hk, p->M, p->N, p->D, true);
     case FAWS_OP_COL_SUM:
     case FAWS_OP_COL_SUM_SEQUENTIAL:
       return align256(partial_floats(p, 0, p->N) * 4) + align256(qsum_floats(p) * 4);

@@ -103,6 +103,7 @@ struct FwdParams {
   int col_row_lo;        // max(col_row_begin, m_begin): first query row that contributes
   float* qsum;           // col_lin: (B,Hq,ceil(M/128),128) per-tile sums of the query rows, written by the
   DropoutParams drop;
+  const uint32_t* drop_mask;  // tcgen05 attention(): the mask, drawn by launch_dropout_mask; null: drawn in the kernel
 };
 
 // Raw column sums are linear in q: for a 128 x 128 (query tile, key tile) pair in which every
@@ -182,6 +183,7 @@ struct BwdParams {
   float sm_scale;
   DropoutParams drop;  // out_scale unused: the kept weights are rescaled by 1/(1-p) (flash.py:655,713,724)
   int mask_scratch;    // dropout, tcgen05: the workspace has room for the mask behind the rest
+  const uint32_t* mask;  // dropout, tcgen05: the mask that the forward pass read, or null
 };
 
 // Score-only operator (compute_attention_scores, attention_scores.py:154-223): scores = q.k^T * sm_scale.
@@ -221,6 +223,13 @@ cudaError_t launch_tc_fwd(const FwdParams& p, int dtype, cudaStream_t s);
 bool tc_colsoftmax_supported(const ColSoftmaxParams& p, int dtype);
 bool tc_colsoftmax_group_in_kernel(const ColSoftmaxParams& p);
 cudaError_t launch_tc_colsoftmax(const ColSoftmaxParams& p, int dtype, int group_sum, cudaStream_t s);
+
+// The dropout mask, one bit per entry, 1 = kept: per (b, h, 128-row query tile, 128-key tile) 2 KB, four words a row, bit x
+// of word w of row r is entry (r, 32 w + x).  First word of a tile:
+__host__ __device__ inline int64_t mask_word(int bh, int qt, int kt, int nqt, int nkt) {
+  return (((int64_t)bh * nqt + qt) * nkt + kt) * 512;
+}
+cudaError_t launch_dropout_mask(const FwdParams& p, uint32_t* mask, cudaStream_t s);  // of all heads
 
 bool tc_bwd_supported(const BwdParams& p, int dtype);
 cudaError_t launch_tc_bwd(const BwdParams& p, int dtype, cudaStream_t s);  // p.delta = the workspace base

@@ -144,7 +144,10 @@ enum Hook : int {
   kHookScoresAny = 5  // scores of either type in rows that TMA cannot address (odd lengths): plain stores
 };
 
-template <typename T, int D, int HOOK, bool SPLIT, bool DROP = false, bool FEW = false>
+// Dropout: the weights' mask drawn in the kernel, or read from memory (attention() whose backward pass will want it too).
+enum Drop : int { kNoDrop = 0, kDrawMask = 1, kReadMask = 2 };
+
+template <typename T, int D, int HOOK, bool SPLIT, int DROP = kNoDrop, bool FEW = false>
 __global__ void __launch_bounds__(NTHREADS, 1)
 tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __grid_constant__ WorkList wl,
               int* __restrict__ status) {
@@ -176,7 +179,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
   // without, 9.10 with; M512 N4096: 30.7 and 31.7).  The odd-row score hook, which packs nothing, is compiled with it all
   // the same: ptxas 12.9 then happens to need no spills there, 68 bytes without (bf16 B1 Hq28 Hk4 S1531: 94 and 99 us;
   // neither an opaque limit nor an opaque count of visible columns has the effect).
-  static_assert(!FEW || ((HOOK == kHookNone || HOOK == kHookScoresAny) && !DROP), "attention() without dropout");
+  static_assert(!FEW || ((HOOK == kHookNone || HOOK == kHookScoresAny) && DROP == kNoDrop), "attention() without dropout");
   const int pack_m = FEW ? p.pack_m : 0;
   const bool persist = !SPLIT && !kStoreHook && wl.n_items > 0;  // (the launcher keeps the other instances plain)
   bool is_fill;
@@ -630,6 +633,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
     // One key tile.  The row's 128 scores are read from TMEM once and stay in registers: first
     // for the max and exp2 passes (the chain the tensor pipe waits on), then, after P has been
     // handed back, for the score-tile hook.  kMasked = false is the fully visible tile.
+    [[maybe_unused]] uint4 kept;  // kReadMask: the row's 128 bits of the key tile in hand
     auto tile_body = [&](auto masked_tag, int cnt, int n0) -> bool {
       constexpr bool kMasked = decltype(masked_tag)::value;
       uint32_t r[128];
@@ -714,7 +718,13 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
           }
           lp0 = add_f32x2(lp0, add_f32x2(pack_f32x2(e[0], e[1]), pack_f32x2(e[4], e[5])));
           lp1 = add_f32x2(lp1, add_f32x2(pack_f32x2(e[2], e[3]), pack_f32x2(e[6], e[7])));
-          if constexpr (DROP) {
+          if constexpr (DROP == kReadMask) {
+            const uint32_t word = c == 0 ? kept.x : c == 1 ? kept.y : c == 2 ? kept.z : kept.w;
+#pragma unroll
+            for (int y = 0; y < 8; ++y)
+              if (!(word >> (g * 8 + y) & 1u)) e[y] = 0.f;
+          }
+          if constexpr (DROP == kDrawMask) {
             // dropout acts on the weights that multiply V only; the row sums above are taken
             // before it (flash.py:459-466)
             const uint32_t base = drop_row + (uint32_t)(n0 + c * 32 + g * 8);
@@ -735,7 +745,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
           mbar_arrive(&bars->p_half[qt]);
         }
       };
-      if constexpr (DROP && HOOK == kHookNone) {
+      if constexpr (DROP == kDrawMask && HOOK == kHookNone) {
         // Under dropout 128 columns unrolled are more instructions than the caches hold (fetches were the first stall
         // of the softmax warps); the scores of a chunk are read again, its P goes over columns already consumed.
         // fp16 B4 H16 S1024 D64 causal: 116 -> 80 us.
@@ -959,6 +969,8 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
         const int tk = tile_of(it);
         if (SPLIT ? ((it & 1) != qt) : (tk >= my_nt)) continue;
         const int n0 = tk * BN;
+        if constexpr (DROP == kReadMask)
+          kept = *reinterpret_cast<const uint4*>(p.drop_mask + mask_word(bh, r_tile / BM, tk, (p.M + BM - 1) / BM, (p.N + BN - 1) / BN) + row * 4);
         if (!mbar_wait(&bars->s_full[qt], s_cnt & 1, abort_flag)) { alive = false; break; }
         ++s_cnt;
         tc_fence_after();
@@ -1004,7 +1016,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
     }
     if (write_out) {
       float inv = l_all > 0.f ? 1.f / l_all : 0.f;
-      if constexpr (DROP) inv *= p.drop.out_scale;
+      if constexpr (DROP != kNoDrop) inv *= p.drop.out_scale;
       if (my_nt > kt0) {
         // Each warp stages its 32 x D output block (128B-swizzled) and stores it with TMA: in its own
         // staging block where the hook leaves that free, so that a persistent CTA's next Q tiles can land
@@ -1506,7 +1518,7 @@ const WorkList& plain_work_list() {
   return wl;
 }
 
-template <typename T, int D, int HOOK, bool SPLIT, bool DROP = false, bool FEW = false>
+template <typename T, int D, int HOOK, bool SPLIT, int DROP = kNoDrop, bool FEW = false>
 cudaError_t launch_fwd_s(const TcMaps& maps, const FwdParams& p, cudaStream_t s) {
   using L = Smem<D, SPLIT>;
   static PerDeviceOnce attr_once;
@@ -1589,7 +1601,10 @@ cudaError_t launch_fwd_h(const TcMaps& maps, const FwdParams& p, cudaStream_t s)
   // (D128 S384 H40 13.3 and 12.0, H44 13.2 and 13.2, H49 13.2 and 14.1).
   if constexpr (HOOK != kHookScores16 && HOOK != kHookScoresAny) {
     // dropout: 256-row CTAs only (the mask generation, not the chain of key tiles, bounds it)
-    if (p.drop.p > 0.f) return launch_fwd_s<T, D, HOOK, false, true>(maps, p, s);
+    if constexpr (HOOK == kHookNone) {
+      if (p.drop_mask != nullptr) return launch_fwd_s<T, D, HOOK, false, kReadMask>(maps, p, s);
+    }
+    if (p.drop.p > 0.f) return launch_fwd_s<T, D, HOOK, false, kDrawMask>(maps, p, s);
   }
   const long long ctas128 = (long long)((p.m_end - p.m_begin + 127) / 128) * p.Hq * p.B;
   const bool store_bound = (HOOK == kHookScores || HOOK == kHookScores16 || HOOK == kHookScoresAny) && p.causal &&
@@ -1598,12 +1613,12 @@ cudaError_t launch_fwd_h(const TcMaps& maps, const FwdParams& p, cudaStream_t s)
   const bool split = use_split_kv<D, HOOK>(p) && (forced || !store_bound);
   if constexpr (HOOK == kHookNone) {
     if (p.pack_m > 0 || p.n_splits > 1)
-      return split ? launch_fwd_s<T, D, HOOK, true, false, true>(maps, p, s)
-                   : launch_fwd_s<T, D, HOOK, false, false, true>(maps, p, s);
+      return split ? launch_fwd_s<T, D, HOOK, true, kNoDrop, true>(maps, p, s)
+                   : launch_fwd_s<T, D, HOOK, false, kNoDrop, true>(maps, p, s);
   }
   constexpr bool kFew = HOOK == kHookScoresAny;
-  return split ? launch_fwd_s<T, D, HOOK, true, false, kFew>(maps, p, s)
-               : launch_fwd_s<T, D, HOOK, false, false, kFew>(maps, p, s);
+  return split ? launch_fwd_s<T, D, HOOK, true, kNoDrop, kFew>(maps, p, s)
+               : launch_fwd_s<T, D, HOOK, false, kNoDrop, kFew>(maps, p, s);
 }
 
 template <typename T, int D>

@@ -32,7 +32,7 @@
 // (GradScale), and moved back in the epilogue: exact, and gradients of any size come out as from fp32 dS.
 // kDrop is kFine with the dropout mask, which the pre-pass draws (draw_mask).  In fine modes hi and lo of 16 streamed
 // rows, the K-step of the accumulating MMAs, take the 16 columns that their dP' leaves.  fp16 B4 H16 S1024 D64 causal,
-// p = 0.1, forward and backward: 240 us, 3 717 us with the CUDA-core kernels; errors of the gradients against fp64 as
+// p = 0.1, forward and backward: 194 us, 3 717 us with the CUDA-core kernels; errors of the gradients against fp64 as
 // there (2.32e-4, 2.28e-4, 2.92e-4 for dq, dk, dv, fp16; dout of 1e-4, where the results are fp16 subnormals: 1.6e-3,
 // 6.6e-3 with an unmoved dS).
 // Deterministic: every output element is written once, by one CTA, in a fixed order; with GQA the
@@ -118,8 +118,7 @@ struct BwTcParams {
   int bh0;               // dropout: the launch's first (batch, head)
 };
 
-// The dropout mask in scratch, one bit per entry, 1 = kept: per (b, h, 128-row query tile, 128-key tile) 2 KB, four
-// words a row, bit x of word w of row r is entry (r, 32 w + x).  Both kernels need it, and a kernel with nothing else to
+// The dropout mask (mask_word) in scratch, where the forward pass kept none.  Both kernels need it, and a kernel with nothing else to
 // do draws it at twice the rate of the two consumer warps that a scheduler of the main kernels has: fp16 B4 H16 S1024 D64
 // causal, p = 0.1, forward and backward: 247 us, 282 with the mask drawn in both.  One bit per entry grows with M * N:
 // beyond kMaskBytes the heads take turns, pre-pass and both kernels for as many at a time as fit, or as keep the SMs
@@ -128,9 +127,6 @@ struct BwTcParams {
 // in both kernels, as calls with scratch that has no room for a mask do.
 constexpr size_t kMaskBytes = size_t(256) << 20, kMaskBytesMost = size_t(1) << 30;
 constexpr int kMaskCtas = 1024;  // seven waves
-__device__ __forceinline__ int64_t mask_word(int bh, int qt, int kt, int nqt, int nkt) {
-  return (((int64_t)bh * nqt + qt) * nkt + kt) * 512;
-}
 // 32 x 32 bits across a warp: on entry bit k of lane l is A[l][k], on exit it is A[k][l].
 __device__ __forceinline__ uint32_t warp_transpose_bits(uint32_t x, int lane) {
   uint32_t m = 0x0000ffffu;
@@ -752,6 +748,14 @@ __device__ __forceinline__ void draw_mask(const BwdParams& p, uint32_t* mask, in
   for (int x = 0; x < 32; ++x) bits |= dropout_keep(p.drop, lin + (uint32_t)x) ? 1u << x : 0u;
   mask[tile * 512 + at] = bits;
 }
+// The mask alone, before a forward pass that reads it and leaves it to the backward pass.  Drawn once, in a kernel that does
+// nothing else, it takes what the backward pass's pre-pass took for it, and the forward pass less than half of what it takes to
+// draw: fp16 B4 H16 S1024 D64 causal, p = 0.1, forward and backward 241 -> 194 us (forward 90 -> 57 + 41, pre-pass 63 -> 6).
+__global__ void __launch_bounds__(256) dropout_mask_kernel(BwdParams p, uint32_t* mask) {
+  griddep_launch_dependents();
+  griddep_wait();  // the mask's memory may have been another one's
+  draw_mask(p, mask, 0, blockIdx.x);
+}
 template <typename T, bool STATS, bool DRAW>
 __global__ void __launch_bounds__(256) bwd_prep_kernel(BwdParams p, float* negl2, float* neg_delta, int Mpad, BwStats st,
                                                        uint32_t* mask, int bh0, unsigned mask_block0) {
@@ -947,7 +951,7 @@ cudaError_t launch_bwd_td(const BwdParams& p, cudaStream_t s) {
   float* negl2 = p.delta;
   float* neg_delta = reinterpret_cast<float*>(base + ws.delta);
   char *dk_part = base + ws.dk, *dv_part = base + ws.dv;
-  uint32_t* mask = MODE == kDrop && p.mask_scratch ? reinterpret_cast<uint32_t*>(base + ws.mask) : nullptr;
+  uint32_t* mask = MODE == kDrop && p.mask_scratch && p.mask == nullptr ? reinterpret_cast<uint32_t*>(base + ws.mask) : nullptr;
   const int heads = p.B * p.Hq, share = mask != nullptr ? mask_heads(p.B, p.Hq, p.M, p.N) : heads;
   using Part = typename std::conditional<MODE == kPlain, T, float>::type;
   const BwStats st{reinterpret_cast<float2*>(base + ws.g_stat), reinterpret_cast<float*>(base + ws.v_stat),
@@ -970,7 +974,7 @@ cudaError_t launch_bwd_td(const BwdParams& p, cudaStream_t s) {
   tp.sm_scale = p.sm_scale; tp.negl2 = negl2; tp.neg_delta = neg_delta; tp.D = p.D;
   tp.drop = p.drop;
   tp.keep_scale = 1.f / (1.f - p.drop.p);
-  tp.mask = mask;
+  tp.mask = p.mask != nullptr ? p.mask : mask;
   tp.g_stat = st.g; tp.v_stat = st.v; tp.g_blocks = st.g_blocks; tp.v_blocks = st.v_blocks;
   int* status_word = tc_status_word();
   const bool per_head = p.G > 1;
@@ -1046,6 +1050,15 @@ size_t tc_bwd_workspace_bytes(int B, int Hq, int Hk, int M, int N, int D, bool f
 
 size_t tc_bwd_mask_bytes(int B, int Hq, int M, int N) {
   return mask_heads(B, Hq, M, N) * head_mask_bytes(M, N);
+}
+
+cudaError_t launch_dropout_mask(const FwdParams& p, uint32_t* mask, cudaStream_t s) {
+  BwdParams b{};
+  b.B = p.B; b.Hq = p.Hq; b.M = p.M; b.N = p.N; b.p_seq = p.p_seq; b.causal = p.causal;
+  b.drop = p.drop;
+  const unsigned blocks = (unsigned)((size_t)p.B * p.Hq * (head_mask_bytes(p.M, p.N) / 1024));
+  const cudaError_t e = launch_overlapped(dropout_mask_kernel, dim3(blocks), 256, 0, s, b, mask);
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 bool tc_bwd_supported(const BwdParams& p, int dtype) {

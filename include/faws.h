@@ -67,6 +67,7 @@ extern "C" {
 #define FAWS_OP_TOTAL_ATTENTION 9
 #define FAWS_OP_ATTENTION_BACKWARD 10
 #define FAWS_OP_ATTENTION_SPLIT_KV 11
+#define FAWS_OP_ATTENTION_BACKWARD_MASKED 12
 
 /* A (B,H,S,D) view; strides in elements; the D axis has stride 1. */
 typedef struct faws_tensor {
@@ -117,6 +118,16 @@ typedef struct faws_problem {
 
 /* Replaces attention() forward (flash.py:264-295, kernel flash.py:335-498). */
 int faws_attention(const faws_problem* p, void* stream);
+
+/*
+ * The same with dropout, for a caller that will run the backward pass: the mask is drawn into `mask`, a bit per entry, read
+ * by the forward pass and handed to faws_attention_backward_masked, which need not draw it again.  faws_dropout_mask_bytes
+ * says how large it is, or 0 where the plain calls are to be made: no dropout, a query-row window, problems that the
+ * tcgen05 kernels do not take, a mask below 1 MB or larger than the queries.  `mask` starts on a 256-byte boundary.
+ * The results are those of the plain calls bit for bit.
+ */
+size_t faws_dropout_mask_bytes(const faws_problem* p);
+int faws_attention_keep_mask(const faws_problem* p, void* mask, size_t mask_bytes, void* stream);
 
 /*
  * Replaces attention_with_scores (attention_with_scores.py:214-333).
@@ -269,6 +280,11 @@ typedef struct faws_grads {
 } faws_grads;
 int faws_attention_backward(const faws_problem* p, const faws_grads* g, void* workspace,
                             size_t workspace_bytes, void* stream);
+
+/* With the mask that faws_attention_keep_mask left for the same problem.  Workspace:
+ * faws_workspace_bytes(FAWS_OP_ATTENTION_BACKWARD_MASKED, p, 0). */
+int faws_attention_backward_masked(const faws_problem* p, const faws_grads* g, const void* mask, size_t mask_bytes,
+                                   void* workspace, size_t workspace_bytes, void* stream);
 
 /* Bytes of scratch `op` needs for `p` (0 if none).  Alignment: 256 bytes.  `p` is the call's own: tensors, family and
  * dropout decide the kernels and with them the scratch.  With FAWS_BACKEND_AUTO the backward pass and the buffered
