@@ -645,6 +645,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
     // One key tile.  The row's 128 scores are read from TMEM once and stay in registers: first
     // for the max and exp2 passes (the chain the tensor pipe waits on), then, after P has been
     // handed back, for the score-tile hook.  kMasked = false is the fully visible tile.
+    [[maybe_unused]] float carry[3] = {0.f, 0.f, 0.f};  // odd score rows: the last three columns of the tile before
     [[maybe_unused]] uint4 kept;  // kReadMask: the row's 128 bits of the key tile in hand
     auto tile_body = [&](auto masked_tag, int cnt, int n0) -> bool {
       constexpr bool kMasked = decltype(masked_tag)::value;
@@ -825,14 +826,68 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
         }
       }
       if constexpr (HOOK == kHookScoresAny) {
-        // Staged as for the TMA stores, then written row by row by the warp itself: 128 row loads and, in place of four
-        // TMA instructions, 128 row stores per tile and warp.  fp32 B1 Hq28 Hk4 S1531 causal: 94 us (62 us at S1536,
-        // where TMA stores), 1 180 us on the CUDA-core kernel that took odd lengths before.
+        // Staged as for the TMA stores, then written row by row by the warp itself.  fp32 B1 Hq28 Hk4 S1531 causal: 87 us (59
+        // us at S1536, where TMA stores), 1 180 us on the CUDA-core kernel that took odd lengths before.
         const int r0 = r_tile + lg * 32, rows = min(32, p.m_end - r0);
         const int esize = p.scores_f32 ? 4 : 2;
         char* dst = static_cast<char*>(p.scores) + (((int64_t)bh * p.M + r0) * p.N + n0) * esize;
         const int64_t row_bytes = (int64_t)p.N * esize;
-        if (p.scores_f32) {
+        if (!SPLIT && p.scores_f32 && n0 + BN <= p.N) {
+          // Whole tiles, which come in ascending order: the row moves in registers by the s columns that its start lies
+          // behind a 16-byte boundary, so that what is staged are quads as they lie in memory, stored 16 bytes a lane, the
+          // first of them with the last s columns of the tile before.  What lies before a row's first quad and behind its
+          // last one the thread of the row writes itself.  A quarter of the row stores of the word-wise form
+          // below: bf16 Hq28 Hk4 S1531 D128 causal 94.3 -> 87.1 us, fp16 H32 S2045 D64 169 -> 153 (full 216 -> 175); with both
+          // ends of every tile written by its threads, 32 rows an instruction, 89.9.  Not with 128-row CTAs, whose
+          // warpgroups take alternate tiles and so have both ends of each to write (87 -> 95).
+          float* srow = static_cast<float*>(p.scores) + ((int64_t)bh * p.M + i) * p.N + n0;
+          const int s = (int)((reinterpret_cast<uintptr_t>(srow) >> 2) & 3);
+          const bool by1 = (s & 1) != 0, by2 = (s & 2) != 0;
+          auto val = [&](int x) { return FAWS_VIS(x) ? __uint_as_float(r[x]) * scale : masked_f; };
+          if (s != 0 && row_ok && n0 == 0) {
+            srow[0] = val(0);
+            if (s <= 2) srow[1] = val(1);
+            if (s == 1) srow[2] = val(2);
+          }
+          if (s != 0 && row_ok && (n0 + BN >= my_nt * BN || n0 + 2 * BN > p.N)) {
+            if (s == 3) srow[125] = val(125);
+            if (s >= 2) srow[126] = val(126);
+            srow[127] = val(127);
+          }
+          const int sub = lane >> 4, q = lane & 15;  // a round of 64 columns: two rows of 16 quads at a time
+          // (a quad goes to the boundary that its columns' address lies behind)
+          const uintptr_t to = reinterpret_cast<uintptr_t>(static_cast<float*>(p.scores) +
+                                                           ((int64_t)bh * p.M + r0 + sub * 16) * p.N + n0 + q * 4);
+          const unsigned char* from = stage + (q >> 3) * 4096 + sub * 2048;
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            float b0 = by1 ? carry[0] : carry[1], b1 = by1 ? carry[1] : carry[2], prev = carry[2];
+            __syncwarp();  // the boxes of the round before have been read
+#pragma unroll
+            for (int x = 0; x < 64; x += 4) {
+              float o[4];
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const float cur = val(half * 64 + x + e), t = by1 ? prev : cur;
+                o[e] = by2 ? b0 : t;
+                b0 = b1;
+                b1 = t;
+                prev = cur;
+                if (x + e >= 61) carry[x + e - 61] = cur;
+              }
+              *reinterpret_cast<float4*>(stage + (x >> 5) * 4096 + lane * 128 + ((((x >> 2) & 7) ^ (lane & 7)) << 4)) =
+                  make_float4(o[0], o[1], o[2], o[3]);
+            }
+            __syncwarp();
+            const bool first = half == 0 && n0 == 0 && q == 0;
+            uintptr_t at = to + half * 256;
+#pragma unroll 8
+            for (int rr = 0; rr < 16; ++rr, at += row_bytes) {
+              const float4 v = *reinterpret_cast<const float4*>(from + rr * 128 + (((q & 7) ^ (rr & 7)) << 4));
+              if (rr + sub * 16 < rows && !(first && (at & 15) != 0)) *reinterpret_cast<float4*>(at & ~uintptr_t(15)) = v;
+            }
+          }
+        } else if (p.scores_f32) {
 #pragma unroll
           for (int half = 0; half < 2; ++half) {
             __syncwarp();  // the boxes of the round before have been read
