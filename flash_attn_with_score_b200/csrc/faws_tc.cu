@@ -333,7 +333,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
     if (kStoreHook && nt > 0) {
       for (int t = 0; t < L::kQTiles; ++t)
         for (int c = 0; c < D / 64; ++c) tma_prefetch_4d(&maps.q, c * 64, r_tile_of[t] - p.m_begin, h, b);
-      for (int idx = 0; idx < min(nt, 4); ++idx)
+      for (int idx = 0; idx < min(nt, 2); ++idx)
         for (int c = 0; c < D / 64; ++c) {
           tma_prefetch_4d(&maps.k, c * 64, tile_of(idx) * BN, hk, b);
           tma_prefetch_4d(&maps.v, c * 64, tile_of(idx) * BN, hk, b);
@@ -647,6 +647,9 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
     // handed back, for the score-tile hook.  kMasked = false is the fully visible tile.
     [[maybe_unused]] float carry[3] = {0.f, 0.f, 0.f};  // odd score rows: the last three columns of the tile before
     [[maybe_unused]] uint4 kept;  // kReadMask: the row's 128 bits of the key tile in hand
+    auto fully_visible = [&](int n0) {
+      return n0 + BN <= p.N && (!p.causal || n0 + BN - 1 <= (pack_m > 0 ? 0 : r_tile) + p.p_seq);
+    };
     auto tile_body = [&](auto masked_tag, int cnt, int n0) -> bool {
       constexpr bool kMasked = decltype(masked_tag)::value;
       uint32_t r[128];
@@ -832,8 +835,8 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
         const int esize = p.scores_f32 ? 4 : 2;
         char* dst = static_cast<char*>(p.scores) + (((int64_t)bh * p.M + r0) * p.N + n0) * esize;
         const int64_t row_bytes = (int64_t)p.N * esize;
-        if (!SPLIT && p.scores_f32 && n0 + BN <= p.N) {
-          // Whole tiles, which come in ascending order: the row moves in registers by the s columns that its start lies
+        if (!SPLIT && !kMasked && p.scores_f32) {
+          // Visible tiles, which come in ascending order: the row moves in registers by the s columns that its start lies
           // behind a 16-byte boundary, so that what is staged are quads as they lie in memory, stored 16 bytes a lane, the
           // first of them with the last s columns of the tile before.  What lies before a row's first quad and behind its
           // last one the thread of the row writes itself.  A quarter of the row stores of the word-wise form
@@ -843,13 +846,13 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
           float* srow = static_cast<float*>(p.scores) + ((int64_t)bh * p.M + i) * p.N + n0;
           const int s = (int)((reinterpret_cast<uintptr_t>(srow) >> 2) & 3);
           const bool by1 = (s & 1) != 0, by2 = (s & 2) != 0;
-          auto val = [&](int x) { return FAWS_VIS(x) ? __uint_as_float(r[x]) * scale : masked_f; };
+          auto val = [&](int x) { return __uint_as_float(r[x]) * scale; };
           if (s != 0 && row_ok && n0 == 0) {
             srow[0] = val(0);
             if (s <= 2) srow[1] = val(1);
             if (s == 1) srow[2] = val(2);
           }
-          if (s != 0 && row_ok && (n0 + BN >= my_nt * BN || n0 + 2 * BN > p.N)) {
+          if (s != 0 && row_ok && !fully_visible(n0 + BN)) {
             if (s == 3) srow[125] = val(125);
             if (s >= 2) srow[126] = val(126);
             srow[127] = val(127);
@@ -1042,9 +1045,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
         ++s_cnt;
         tc_fence_after();
         // (packed heads: the tile may hold the first row of a head)
-        const bool full_vis =
-            (n0 + BN <= p.N) && (!p.causal || (n0 + BN - 1 <= (pack_m > 0 ? 0 : r_tile) + p.p_seq));
-        const bool ok = full_vis ? tile_body(std::false_type{}, cnt, n0) : tile_body(std::true_type{}, cnt, n0);
+        const bool ok = fully_visible(n0) ? tile_body(std::false_type{}, cnt, n0) : tile_body(std::true_type{}, cnt, n0);
         if (!ok) { alive = false; break; }
         ++cnt;
       }
@@ -1674,10 +1675,17 @@ cudaError_t launch_fwd_h(const TcMaps& maps, const FwdParams& p, cudaStream_t s)
     if (p.drop.p > 0.f) return launch_fwd_s<T, D, HOOK, false, kDrawMask>(maps, p, s);
   }
   const long long ctas128 = (long long)((p.m_end - p.m_begin + 127) / 128) * p.Hq * p.B;
+  const bool odd_f32 = HOOK == kHookScoresAny && p.scores_f32;
   const bool store_bound = (HOOK == kHookScores || HOOK == kHookScores16 || HOOK == kHookScoresAny) && p.causal &&
-                           ctas128 > ((p.N + BN - 1) / BN == 3 ? sm_count() * 7 / 8 : sm_count());
+                           (odd_f32 ? 3 * ctas128 > 5LL * sm_count()
+                                    : ctas128 > ((p.N + BN - 1) / BN == 3 ? sm_count() * 7 / 8 : sm_count()));
+  // fp32 scores in odd rows, no mask: 256-row CTAs take some 1.65 times as long as 128-row ones and write 16 bytes a lane,
+  // so whole waves decide.
+  const long long ctas256 = (long long)((p.m_end - p.m_begin + 255) / 256) * p.Hq * p.B;
+  const bool fewer_waves = odd_f32 && !p.causal &&
+                           5 * ((ctas256 + sm_count() - 1) / sm_count()) <= 3 * ((ctas128 + sm_count() - 1) / sm_count());
   static const bool forced = std::getenv("FAWS_SPLIT_KV") != nullptr;
-  const bool split = use_split_kv<D, HOOK>(p) && (forced || !store_bound);
+  const bool split = use_split_kv<D, HOOK>(p) && (forced || !(store_bound || fewer_waves));
   if constexpr (HOOK == kHookNone) {
     if (p.pack_m > 0 || p.n_splits > 1)
       return split ? launch_fwd_s<T, D, HOOK, true, kNoDrop, true>(maps, p, s)
