@@ -104,7 +104,7 @@ class _Call:
                             L.data_ptr() if L is not None else 0, _lib.BACKENDS[backend])
         p = _lib.Problem.from_buffer(buf)
         p.sm_scale = float(sm_scale)
-        self.seed = self.offset = self.mask = None
+        self.seed = self.offset = None
         if dropout_p and dropout_p > 0.0:
             assert dropout_p < 1.0, "dropout_p must be < 1"
             seed, offset = philox if philox is not None else philox_cuda_seed_offset(B * H * M * N, q.device)
@@ -174,7 +174,7 @@ class _AttentionFunction(torch.autograd.Function):
     def forward(ctx, q, k, v, causal, sm_scale, dropout_p, want_total, backend, philox, kv_splits):
         c, tot = _attention_forward(q, k, v, causal, sm_scale, dropout_p, True, want_total, None, backend, philox,
                                     kv_splits, keep_mask=True)
-        ctx.save_for_backward(c.q, c.k, c.v, c.out, c.L, c.mask)
+        ctx.save_for_backward(c.q, c.k, c.v, c.out, c.L, getattr(c, "mask", None))
         ctx.causal, ctx.sm_scale, ctx.dropout_p, ctx.backend = causal, float(c.p.sm_scale), dropout_p, backend
         ctx.philox = (c.seed, c.offset) if c.seed is not None else None
         ctx.mark_non_differentiable(*[t for t in (c.L, tot) if t is not None])
