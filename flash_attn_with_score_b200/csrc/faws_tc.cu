@@ -652,10 +652,14 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
     };
     auto tile_body = [&](auto masked_tag, int cnt, int n0) -> bool {
       constexpr bool kMasked = decltype(masked_tag)::value;
-      uint32_t r[128];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) tmem_ld32(t_s + c * 32, reinterpret_cast<uint32_t(&)[32]>(r[c * 32]));
-      tmem_wait_ld();
+      // Masked tiles, one or two to a query tile, take their columns 32 at a time in rolled loops and read S again for the
+      // exponentials: a quarter of the code, with which visible tiles share the instruction caches.  fp16 B16 H8 S785 D32 with
+      // softmax column sums 108.6 -> 107.2 us, B4 H16 S1024 D64 with dropout (both passes) 192.5 -> 190.9, bf16 Hq28 Hk4 S4096
+      // D128 row sums 130.1 -> 129.0.  Not where scores are stored, which would come before the exponentials then (fp16 H8
+      // S512 D64 10.6 -> 11.6), nor under column sums, whose shuffles would.
+      constexpr bool kRolled = kMasked && (HOOK == kHookNone || HOOK == kHookRowSum);
+      constexpr bool kReread = kRolled || (DROP == kDrawMask && HOOK == kHookNone);
+      uint32_t r[kRolled ? 1 : 128];
       int nvis = 128;  // visible columns form a prefix of the tile's row
       if (kMasked) {
         int lim = p.N;
@@ -666,15 +670,49 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
 
       // ---- row max (4 independent chains)
       float a0 = FAWS_NEG_INF, a1 = FAWS_NEG_INF, a2 = FAWS_NEG_INF, a3 = FAWS_NEG_INF;
+      if constexpr (kRolled) {
+        [[maybe_unused]] float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+#pragma unroll 1
+        for (int c = 0; c < 4; ++c) {
+          uint32_t sv[32];
+          tmem_ld32(t_s + c * 32, sv);
+          tmem_wait_ld();
+          const int nv = nvis - c * 32;
 #pragma unroll
+          for (int x = 0; x < 32; x += 8) {
+            float y[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) y[e] = x + e < nv ? __uint_as_float(sv[x + e]) : FAWS_NEG_INF;
+            a0 = fmax3(a0, y[0], y[1]);
+            a1 = fmax3(a1, y[2], y[3]);
+            a2 = fmax3(a2, y[4], y[5]);
+            a3 = fmax3(a3, y[6], y[7]);
+            if constexpr (HOOK == kHookRowSum) {
+#pragma unroll
+              for (int e = 0; e < 8; e += 4) {
+                s0 += x + e < nv ? __uint_as_float(sv[x + e]) : 0.f;
+                s1 += x + e + 1 < nv ? __uint_as_float(sv[x + e + 1]) : 0.f;
+                s2 += x + e + 2 < nv ? __uint_as_float(sv[x + e + 2]) : 0.f;
+                s3 += x + e + 3 < nv ? __uint_as_float(sv[x + e + 3]) : 0.f;
+              }
+            }
+          }
+        }
+        if constexpr (HOOK == kHookRowSum) rs_raw += (s0 + s1) + (s2 + s3);
+      } else {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) tmem_ld32(t_s + c * 32, reinterpret_cast<uint32_t(&)[32]>(r[c * 32]));
+        tmem_wait_ld();
 #define FAWS_SV(x) (FAWS_VIS(x) ? __uint_as_float(r[x]) : FAWS_NEG_INF)
-      for (int x = 0; x < 128; x += 8) {  // three-input max: 64 instructions for 128 values
-        a0 = fmax3(a0, FAWS_SV(x), FAWS_SV(x + 1));
-        a1 = fmax3(a1, FAWS_SV(x + 2), FAWS_SV(x + 3));
-        a2 = fmax3(a2, FAWS_SV(x + 4), FAWS_SV(x + 5));
-        a3 = fmax3(a3, FAWS_SV(x + 6), FAWS_SV(x + 7));
-      }
+#pragma unroll
+        for (int x = 0; x < 128; x += 8) {  // three-input max: 64 instructions for 128 values
+          a0 = fmax3(a0, FAWS_SV(x), FAWS_SV(x + 1));
+          a1 = fmax3(a1, FAWS_SV(x + 2), FAWS_SV(x + 3));
+          a2 = fmax3(a2, FAWS_SV(x + 4), FAWS_SV(x + 5));
+          a3 = fmax3(a3, FAWS_SV(x + 6), FAWS_SV(x + 7));
+        }
 #undef FAWS_SV
+      }
       const float mx = fmaxf(fmaxf(a0, a1), fmaxf(a2, a3)) * scale_log2;  // sm_scale > 0
 
       // ---- running max, lazy rescale of O.  s_full for this tile was committed after this
@@ -761,7 +799,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
           mbar_arrive(&bars->p_half[qt]);
         }
       };
-      if constexpr (DROP == kDrawMask && HOOK == kHookNone) {
+      if constexpr (kReread) {
         // Under dropout 128 columns unrolled are more instructions than the caches hold (fetches were the first stall
         // of the softmax warps); the scores of a chunk are read again, its P goes over columns already consumed.
         // fp16 B4 H16 S1024 D64 causal: 116 -> 80 us.
@@ -784,7 +822,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
       mbar_arrive(&bars->p_ready[qt]);
 
       // ---- score-tile hooks: off the chain above, they overlap this tile's P.V MMA
-      if constexpr (HOOK == kHookRowSum) {
+      if constexpr (HOOK == kHookRowSum && !kRolled) {
         float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;  // (packed 2 x fp32 adds measured 3 % slower here)
 #pragma unroll
         for (int x = 0; x < 128; x += 4) {
@@ -829,7 +867,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
         }
       }
       if constexpr (HOOK == kHookScoresAny) {
-        // Staged as for the TMA stores, then written row by row by the warp itself.  fp32 B1 Hq28 Hk4 S1531 causal: 87 us (59
+        // Staged as for the TMA stores, then written row by row by the warp itself.  fp32 B1 Hq28 Hk4 S1531 causal: 78 us (59
         // us at S1536, where TMA stores), 1 180 us on the CUDA-core kernel that took odd lengths before.
         const int r0 = r_tile + lg * 32, rows = min(32, p.m_end - r0);
         const int esize = p.scores_f32 ? 4 : 2;
@@ -1675,12 +1713,15 @@ cudaError_t launch_fwd_h(const TcMaps& maps, const FwdParams& p, cudaStream_t s)
     if (p.drop.p > 0.f) return launch_fwd_s<T, D, HOOK, false, kDrawMask>(maps, p, s);
   }
   const long long ctas128 = (long long)((p.m_end - p.m_begin + 127) / 128) * p.Hq * p.B;
+  // fp32 scores in odd rows: the line lies at 1.7 CTAs of 128 rows per SM (D128, 256 and 128 rows: H20 S1021, 160 of them,
+  // 49.7 and 32.3 us; H16 S1531, 192, 70.3 and 50.6; H20 S1531, 240, 69.0 and 63.3; H32 S1021, 256, 51.2 and 49.5; H28
+  // S1531, 336, 78.2 and 86.8).
   const bool odd_f32 = HOOK == kHookScoresAny && p.scores_f32;
   const bool store_bound = (HOOK == kHookScores || HOOK == kHookScores16 || HOOK == kHookScoresAny) && p.causal &&
                            (odd_f32 ? 3 * ctas128 > 5LL * sm_count()
                                     : ctas128 > ((p.N + BN - 1) / BN == 3 ? sm_count() * 7 / 8 : sm_count()));
-  // fp32 scores in odd rows, no mask: 256-row CTAs take some 1.65 times as long as 128-row ones and write 16 bytes a lane,
-  // so whole waves decide.
+  // Without a mask 256-row CTAs take some 1.65 times as long as 128-row ones, so whole waves decide (D128 full, 256 and 128
+  // rows: H24 S1531, 144 and 288 CTAs, 76.1 and 97.6 us; H28, 168 and 336, 147 and 129).
   const long long ctas256 = (long long)((p.m_end - p.m_begin + 255) / 256) * p.Hq * p.B;
   const bool fewer_waves = odd_f32 && !p.causal &&
                            5 * ((ctas256 + sm_count() - 1) / sm_count()) <= 3 * ((ctas128 + sm_count() - 1) / sm_count());
