@@ -115,6 +115,25 @@ def load():
     return lib
 
 
+OP_SCORES_ONLY = 100  # of plain_call alone: compute_attention_scores has no workspace and no operator id
+_plain = None
+
+
+def plain_call(*args):
+    """Runs ``(op, q, k, v, causal, sm_scale, split, per_q_head)`` natively, outputs and launch, or returns None where a
+    tensor or the moment is out of the ordinary (csrc/faws_torch.cpp): the caller then goes the long way."""
+    global _plain
+    if _plain is None:
+        load()
+        try:
+            from . import _plain as module
+        except ImportError as e:
+            raise ImportError("flash_attn_with_score_b200/_plain.so is missing or was built for another torch: run "
+                              "`python -m flash_attn_with_score_b200.build`") from e
+        _plain = module.call
+    return _plain(*args)
+
+
 def check(status: int, what: str):
     if status != 0:
         msg = load().faws_strerror(status).decode()

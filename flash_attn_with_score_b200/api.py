@@ -28,6 +28,7 @@ import torch
 
 from . import _lib
 
+_NEG_INF = float("-inf")
 _DTYPES = {torch.float16: _lib.FP16, torch.bfloat16: _lib.BF16}
 
 
@@ -218,6 +219,11 @@ def attention(q, k, v, causal=False, sm_scale=None, dropout_p=0.0,
         out, L, tot, seed, offset = _AttentionFunction.apply(q, k, v, causal, sm_scale, dropout_p,
                                                              return_total_attention, backend, philox, kv_splits)
     else:
+        if (not dropout_p and q_rows is None and backend is None and kv_splits is None
+                and not (return_log_normalizer or return_total_attention or return_seed_offset)):
+            got = _lib.plain_call(_lib.OP_ATTENTION, q, k, v, causal, sm_scale, 0, False)
+            if got is not None:
+                return got
         need_L = return_log_normalizer or return_total_attention
         c, tot = _attention_forward(q, k, v, causal, sm_scale, dropout_p, need_L, return_total_attention,
                                     q_rows, backend, philox, kv_splits)
@@ -234,6 +240,11 @@ def attention_with_scores(q, k, v, causal=False, sm_scale=None, dropout_p=0.0,
     """``(out, scores)`` with q.k^T computed once (attention_with_scores.py:214-333).
 
     scores: (B,Hq,M,N), ``scores_dtype`` (fp32 or q.dtype), hidden entries = ``masked_value``."""
+    if (not dropout_p and q_rows is None and backend is None and out is None and scores is None
+            and scores_dtype is torch.float32 and masked_value == _NEG_INF):
+        got = _lib.plain_call(_lib.OP_SCORES, q, k, v, causal, sm_scale, 0, False)
+        if got is not None:
+            return got
     c = _Call(q, k, v, causal, sm_scale, dropout_p, out=out, q_rows=q_rows, backend=backend,
               philox=philox, rescale=True)
     if scores_dtype not in (torch.float32, q.dtype):
@@ -251,6 +262,10 @@ def compute_attention_scores(q, k, causal=False, sm_scale=None, *, scores_dtype=
     """``q @ k^T * sm_scale`` as a (B,Hq,M,N) tensor in q.dtype, no softmax, no V: the reference's
     ``compute_attention_scores`` (attention_scores.py:154-223).  ``causal`` is accepted and ignored,
     exactly as there (:166,:171): no mask is applied.  ``scores_dtype=torch.float32`` keeps fp32."""
+    if backend is None and (scores_dtype is None or scores_dtype is q.dtype):
+        got = _lib.plain_call(_lib.OP_SCORES_ONLY, q, k, k, False, sm_scale, 0, False)
+        if got is not None:
+            return got
     Dq, Dk = q.shape[-1], k.shape[-1]
     assert Dq == Dk, "Q and K must have the same head_dim"
     assert Dk in {16, 32, 64, 128}, f"head_dim must be one of 16, 32, 64, 128, got {Dk}"
@@ -269,6 +284,10 @@ def attention_with_row_sum(q, k, v, causal=False, sm_scale=None, dropout_p=0.0, 
                            philox=None):
     """``(out, row_sum)``; row_sum (B,Hq,M) fp32 = sum over visible keys of the scaled
     score (attention_with_row_sum.py:204-326)."""
+    if not dropout_p and q_rows is None and backend is None:
+        got = _lib.plain_call(_lib.OP_ROW_SUM, q, k, v, causal, sm_scale, 0, False)
+        if got is not None:
+            return got
     c = _Call(q, k, v, causal, sm_scale, dropout_p, q_rows=q_rows, backend=backend, philox=philox)
     rs = torch.empty((c.B, c.H, c.M), device=c.dev, dtype=torch.float32)
     c.run("faws_attention_with_row_sum", C.c_void_p(rs.data_ptr()))
@@ -277,6 +296,11 @@ def attention_with_row_sum(q, k, v, causal=False, sm_scale=None, dropout_p=0.0, 
 
 def _col_like(fn_name, op, q, k, v, causal, sm_scale, dropout_p, per_q_head, q_rows, backend,
               split=None, out=None, sum_out=None, msgs=None, philox=None):
+    if (not dropout_p and q_rows is None and backend is None and out is None and sum_out is None
+            and (split is None or type(split) is int)):
+        got = _lib.plain_call(op, q, k, v, causal, sm_scale, split or 0, per_q_head)
+        if got is not None:
+            return got
     c = _Call(q, k, v, causal, sm_scale, dropout_p, out=out, q_rows=q_rows, backend=backend, msgs=msgs,
               philox=philox)
     length = c.N if split is None else split

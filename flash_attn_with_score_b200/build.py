@@ -1,4 +1,5 @@
-"""Builds libfaws.so (the C-ABI library of include/faws.h) in-tree with nvcc for sm_100a.
+"""Builds libfaws.so (the C-ABI library of include/faws.h) in-tree with nvcc for sm_100a, and _plain.so, the native form of
+the operators' plain calls from Python, with g++ against the installed torch.
 
     python -m flash_attn_with_score_b200.build [--force] [--verbose]
 
@@ -10,15 +11,19 @@ from __future__ import annotations
 
 import concurrent.futures
 import hashlib
+import importlib.util
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 OBJDIR = os.path.join(ROOT, "build", "libfaws")
 LIB = os.path.join(HERE, "libfaws.so")
+PLAIN = os.path.join(HERE, "_plain.so")
+PLAIN_SOURCE = os.path.join(CSRC, "faws_torch.cpp")
 SOURCES = ["faws_abi.cu", "faws_generic.cu", "faws_tc.cu", "faws_tc_scores.cu", "faws_bwd.cu", "faws_tc_bwd.cu", "faws_noalloc.cu"]
 HEADERS = ["faws_internal.cuh", "faws_tc_ptx.cuh", "faws_tc_host.cuh", "faws_tc_store.cuh", "faws_launch_plan.h"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -58,8 +63,34 @@ def _lib_digest() -> str:
     return _digest([os.path.join(CSRC, f) for f in SOURCES] + _deps(), " ".join(ARCH))
 
 
+def _torch_dir() -> str:
+    return importlib.util.find_spec("torch").submodule_search_locations[0]
+
+
+def _plain_digest() -> str:
+    """Of what _plain.so is made from, the torch and Python that it is bound to among them."""
+    return _digest([PLAIN_SOURCE, os.path.join(ROOT, "include", "faws.h"), os.path.join(_torch_dir(), "version.py")], sys.version)
+
+
 def needs_build() -> bool:
-    return not os.path.exists(LIB) or _read(os.path.join(OBJDIR, "libfaws.digest")) != _lib_digest()
+    return (not os.path.exists(LIB) or _read(os.path.join(OBJDIR, "libfaws.digest")) != _lib_digest()
+            or not os.path.exists(PLAIN) or _read(os.path.join(OBJDIR, "plain.digest")) != _plain_digest())
+
+
+def _build_plain(verbose: bool) -> None:
+    torch, digest = _torch_dir(), _plain_digest()
+    cuda = os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")
+    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-o", PLAIN, PLAIN_SOURCE, "-I", os.path.join(ROOT, "include"),
+           "-I", os.path.join(torch, "include"), "-I", os.path.join(torch, "include", "torch", "csrc", "api", "include"),
+           "-I", sysconfig.get_paths()["include"], "-I", cuda, "-L", HERE, "-l:libfaws.so", "-L", os.path.join(torch, "lib"),
+           "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python", "-Wl,-rpath,$ORIGIN"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if verbose or res.returncode != 0:
+        sys.stderr.write(res.stdout + res.stderr)
+    if res.returncode != 0:
+        raise RuntimeError("g++ failed building _plain.so")
+    with open(os.path.join(OBJDIR, "plain.digest"), "w") as f:
+        f.write(digest)
 
 
 def _compile(src: str, force: bool, verbose: bool) -> tuple[str, int, str]:
@@ -102,6 +133,8 @@ def build(force: bool = False, verbose: bool = False) -> str:
     if lib_digest == _lib_digest():  # nothing changed while compiling
         with open(os.path.join(OBJDIR, "libfaws.digest"), "w") as f:
             f.write(lib_digest)
+    if force or not os.path.exists(PLAIN) or _read(os.path.join(OBJDIR, "plain.digest")) != _plain_digest():
+        _build_plain(verbose)
     return LIB
 
 
