@@ -466,7 +466,10 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
       // lane issues the tcgen05 instructions.
       constexpr int kFmt = std::is_same<T, __half>::value ? 0 : 1;
       constexpr uint32_t idesc_qk = make_idesc_f16(128, BN, kFmt, 0, 0);
-      constexpr uint32_t idesc_pv = make_idesc_f16(128, D, kFmt, 0, 1);
+      // Head dims 16 and 32 in the D = 64 instances: K-steps and output columns of nothing but padding are left out (fp16 B16 H8
+      // S785 D32 57.0 -> 55.0 us, with softmax column sums 107.2 -> 104.8; head dim 64 as before).
+      const int k_steps = D == 64 ? (p.D + 15) / 16 : D / 16;
+      const uint32_t idesc_pv = D == 64 && p.D <= 32 ? make_idesc_f16(128, 32, kFmt, 0, 1) : make_idesc_f16(128, D, kFmt, 0, 1);
       // Operand descriptors are built once; inside the loops only compile-time offsets (in
       // 16-byte units) are added to their address field, so the issuing thread spends a few
       // instructions per MMA.
@@ -491,7 +494,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
           for (int kk = 0; kk < D / 16; ++kk) {
             const uint64_t off = (uint64_t)(((kk >> 2) * L::kSub + (kk & 3) * 32) >> 4);
             if (kk == 0) mma_ss(d_tmem, qd + off, kd + off, idesc_qk, 0u);
-            else mma_ss_acc(d_tmem, qd + off, kd + off, idesc_qk);
+            else if (kk < k_steps) mma_ss_acc(d_tmem, qd + off, kd + off, idesc_qk);
           }
           mma_commit(&bars->s_full[t]);
         }
@@ -1176,8 +1179,9 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
                 make_uint4(ro[g * 4], ro[g * 4 + 1], ro[g * 4 + 2], ro[g * 4 + 3]);
         };
         // (all D / 32 loads of the row in flight together measured 2-3 % slower: the registers they hold)
+        const int o_chunks = D == 64 && p.D <= 32 && !kHalfStage ? 1 : D / 32;  // (the store leaves the other columns out)
 #pragma unroll 1
-        for (int c = 0; c < D / 32; ++c) {
+        for (int c = 0; c < o_chunks; ++c) {
           uint32_t ro[32];
           tmem_ld32(t_o + c * 32, ro);
           if (kHalfStage && (c & 1) == 0 && (c > 0 || k > 0)) {  // the store before this one has read the half block
@@ -1434,6 +1438,7 @@ tc_colsoftmax_kernel(const __grid_constant__ CsMaps maps, const ColSoftmaxParams
       // pass, 199 this way; where the power cap sets the pace (B4 Hq32 Hk8 S16384 full) 26.3 and 26.4 ms.
       constexpr int kFmt = std::is_same<T, __half>::value ? 0 : 1;
       constexpr uint32_t idesc = make_idesc_f16(128, BM, kFmt, 0, 0);
+      const int k_steps = D == 64 ? (p.D + 15) / 16 : D / 16;  // (head dims 16 and 32: no K-steps of padding)
       const uint64_t k_desc = make_desc_sw128(smem_u32(smem + L::k_off), 16, 1024);
       const uint64_t q_desc0 = make_desc_sw128(smem_u32(smem + L::q_off), 16, 1024);
       bool ok = mbar_wait(&bars->k_full, 0, abort_flag);
@@ -1453,7 +1458,7 @@ tc_colsoftmax_kernel(const __grid_constant__ CsMaps maps, const ColSoftmaxParams
           for (int kk = 0; kk < D / 16; ++kk) {
             const uint64_t off = (uint64_t)(((kk >> 2) * L::kSub + (kk & 3) * 32) >> 4);
             if (kk == 0) mma_ss(d_tmem, kd + off, qd + off, idesc, 0u);
-            else mma_ss_acc(d_tmem, kd + off, qd + off, idesc);
+            else if (kk < k_steps) mma_ss_acc(d_tmem, kd + off, qd + off, idesc);
           }
           if (kt == CS_KT - 1) mma_commit(&bars->q_empty[s]);
           mma_commit(&bars->s_full[buf0 + kt]);
