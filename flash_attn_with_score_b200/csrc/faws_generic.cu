@@ -520,13 +520,12 @@ __device__ __forceinline__ float sum_dealt_pairs(const float* base, int64_t head
     return x;
   };
   float s = 0.f;
-  for (; left >= 8; left -= 8) {
+  for (; left > 0; left -= 8) {  // (the last few together as well: one after the other each would wait for its load)
     float v[8];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) v[e] = next();
+    for (int e = 0; e < 8; ++e) v[e] = e < left ? next() : 0.f;
     s += ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
   }
-  for (; left > 0; --left) s += next();
   return s;
 }
 
@@ -558,6 +557,7 @@ __global__ void __launch_bounds__(128 * kLinGroups, 3) reduce_colsum_lin_kernel(
       kr[x] = *reinterpret_cast<const uint4*>(kbase + (int64_t)jr * p.k_ss);
   }
 
+  ptx::griddep_wait();  // the sums and partial rows come from the forward pass, which this launch may overlap; k does not
   // linear query tiles [lin_lo, lin_hi) and, among [seen_lo, seen_hi), the others, which left partial rows:
   // col_tile_linear and the forward kernel's visits, as ranges
   int lin_lo = (p.row_lo + 127) / 128, lin_hi = p.m_end / 128;
@@ -779,9 +779,18 @@ cudaError_t launch_scratch_colsum(const ColSoftmaxParams& p, int group_sum, cuda
 cudaError_t launch_reduce_partials(const ReducePartialParams& p, int dtype, cudaStream_t s) {
   if (p.n_end <= 0) return cudaSuccess;
   if (p.lin) {
-    dim3 grid((p.n_end + 127) / 128, p.per_q_head ? p.Hq : p.Hk, p.B);
-    if (dtype == FAWS_FP16) reduce_colsum_lin_kernel<__half><<<grid, 128 * kLinGroups, 0, s>>>(p);
-    else reduce_colsum_lin_kernel<__nv_bfloat16><<<grid, 128 * kLinGroups, 0, s>>>(p);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((p.n_end + 127) / 128, p.per_q_head ? p.Hq : p.Hk, p.B);
+    cfg.blockDim = dim3(128 * kLinGroups, 1, 1);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = p.overlap;
+    const cudaError_t e = dtype == FAWS_FP16 ? cudaLaunchKernelEx(&cfg, reduce_colsum_lin_kernel<__half>, p)
+                                             : cudaLaunchKernelEx(&cfg, reduce_colsum_lin_kernel<__nv_bfloat16>, p);
+    if (e != cudaSuccess) return e;
   } else {
     dim3 grid((p.n_end + 255) / 256, p.per_q_head ? p.Hq : p.Hk, p.B);
     reduce_partials_kernel<<<grid, 256, 0, s>>>(p);

@@ -157,6 +157,7 @@ struct ReducePartialParams {
   const void* k;
   int64_t k_sb, k_sh, k_ss;
   float sm_scale;
+  int overlap;           // the launch may begin while the forward pass drains
 };
 
 // Backward pass of attention(): inputs q, k, v, out, dout, L; outputs dq (B,Hq,M,D), dk, dv (B,Hk,N,D).
