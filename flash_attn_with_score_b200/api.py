@@ -193,6 +193,8 @@ class _AttentionFunction(torch.autograd.Function):
         dq, dk, dv = torch.empty_like(c.q), torch.empty_like(c.k), torch.empty_like(c.v)
         g = _lib.Grads(_tensor(do), _tensor(dq), _tensor(dk), _tensor(dv))
         if mask is not None:
+            if not mask.is_contiguous() or mask.data_ptr() % 256 != 0:  # (what a saved-tensor hook made of it)
+                mask = mask.clone(memory_format=torch.contiguous_format)
             ws, n = c.workspace(_lib.OP_ATTENTION_BACKWARD_MASKED)
             c.run("faws_attention_backward_masked", C.byref(g), C.c_void_p(mask.data_ptr()), mask.numel(),
                   C.c_void_p(ws.data_ptr()), n)

@@ -412,9 +412,10 @@ bool scores_only_on_cuda_cores(const ScoresOnlyParams& p, int sms) {
 // Bytes of the dropout mask that a forward pass leaves for its backward pass, 0 where it leaves none.  Drawing it takes both
 // passes 1.4 us a million entries; keeping it costs memory from one to the other, and a launch.  Kept where it is no larger
 // than the queries, which are kept as well (up to 16 D keys), and at least 1 MB.
+size_t mask_bytes_of(const faws_problem* p) { return (size_t)p->B * p->Hq * cdiv(p->M, 128) * cdiv(p->N, 128) * 2048; }
 size_t kept_mask_bytes(const faws_problem* p) {
   if (!(p->dropout_p > 0.f) || p->m_begin != 0 || p->m_end != p->M || p->v.ptr == nullptr || p->out.ptr == nullptr) return 0;
-  const size_t bytes = (size_t)p->B * p->Hq * cdiv(p->M, 128) * cdiv(p->N, 128) * 2048;
+  const size_t bytes = mask_bytes_of(p);
   if (bytes < (size_t(1) << 20) || bytes > (size_t)p->B * p->Hq * p->M * p->D * 2) return 0;
   if (!tc_allowed(p) || !tc_fwd_supported(make_fwd(p), p->dtype)) return 0;
   return bytes;
@@ -676,9 +677,9 @@ int faws_attention_backward_masked(const faws_problem* p, const faws_grads* g, c
                                    void* workspace, size_t workspace_bytes, void* stream) {
   const int st = validate(p);
   if (st != FAWS_OK) return st;
-  const size_t need = kept_mask_bytes(p);
-  if (need == 0) return FAWS_EUNSUPPORTED;
-  if (mask == nullptr || mask_bytes < need || misaligned_ws(mask)) return FAWS_EWORKSPACE;
+  if (!(p->dropout_p > 0.f)) return FAWS_EINVAL;
+  // (tensors that have moved since to where only the CUDA-core kernels can read them: those draw the mask themselves)
+  if (mask == nullptr || mask_bytes < mask_bytes_of(p) || misaligned_ws(mask)) return FAWS_EWORKSPACE;
   return backward(p, g, mask, workspace, workspace_bytes, stream);
 }
 

@@ -46,6 +46,27 @@ def test_kept_mask(monkeypatch, B, Hq, Hk, M, N, D, causal, dtype):
     assert F.device_status() == 0
 
 
+def test_saved_tensors_that_come_back_elsewhere():
+    """Hooks that give the tensors back at addresses that TMA cannot read: the CUDA-core kernels, which draw the mask."""
+    g = torch.Generator(device="cuda").manual_seed(1)
+    q, k, v, do = [torch.randn(1, 64, 300, 128, device="cuda", generator=g).half() for _ in range(4)]
+    for t in (q, k, v):
+        t.requires_grad_(True)
+
+    def elsewhere(t):
+        return torch.empty(t.numel() + 1, device="cuda", dtype=t.dtype)[1:].view(t.shape).copy_(t)
+    grads = []
+    for unpack in (lambda t: t, elsewhere):
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: t, unpack):
+            out = F.attention(q, k, v, True, dropout_p=0.3, philox=(11, 8))
+        assert out.grad_fn.saved_tensors[5] is not None
+        with torch.autograd.set_multithreading_enabled(False):  # last_backend() is this thread's
+            grads.append(torch.autograd.grad(out, (q, k, v), do))
+        assert F.last_backend() == ("tcgen05" if len(grads) == 1 else "generic")
+    for x, y in zip(*grads):  # 16-bit weights and results on both families
+        assert (x.double() - y.double()).norm() <= 2e-3 * y.double().norm()
+
+
 def test_what_keeps_no_mask():
     """Larger than the queries, smaller than 1 MB, no gradient wanted, rows that TMA cannot read: the plain calls."""
     for M, N, D, H, off in ((512, 1100, 64, 16, 0), (256, 256, 64, 8, 0), (1024, 1024, 64, 16, 1)):
