@@ -659,8 +659,10 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
       // exponentials: a quarter of the code, with which visible tiles share the instruction caches.  fp16 B16 H8 S785 D32 with
       // softmax column sums 108.6 -> 107.2 us, B4 H16 S1024 D64 with dropout (both passes) 192.5 -> 190.9, bf16 Hq28 Hk4 S4096
       // D128 row sums 130.1 -> 129.0.  Not where scores are stored, which would come before the exponentials then (fp16 H8
-      // S512 D64 10.6 -> 11.6), nor under column sums, whose shuffles would.
-      constexpr bool kRolled = kMasked && (HOOK == kHookNone || HOOK == kHookRowSum);
+      // S512 D64 10.6 -> 11.6), nor under column sums, whose shuffles would; nor with 128-row CTAs, few of whose tiles are not
+      // masked and whose chain it lengthens (fp16 B10 H16
+      // M34 N617 D128 causal 20.6 us, 20.0 without).
+      constexpr bool kRolled = kMasked && !SPLIT && (HOOK == kHookNone || HOOK == kHookRowSum);
       constexpr bool kReread = kRolled || (DROP == kDrawMask && HOOK == kHookNone);
       uint32_t r[kRolled ? 1 : 128];
       int nvis = 128;  // visible columns form a prefix of the tile's row
