@@ -1,5 +1,5 @@
 """Builds libfaws.so (the C-ABI library of include/faws.h) in-tree with nvcc for sm_100a, and _plain.so, the native form of
-the operators' plain calls from Python, with g++ against the installed torch.
+the operators' plain calls from Python, against the installed torch.
 
     python -m flash_attn_with_score_b200.build [--force] [--verbose]
 
@@ -67,6 +67,17 @@ def _torch_dir() -> str:
     return importlib.util.find_spec("torch").submodule_search_locations[0]
 
 
+def _plain_command() -> list[str]:
+    """nvcc as the driver of g++: it knows where CUDA's headers are, by whatever name or wrapper it was called."""
+    torch = _torch_dir()
+    return [_nvcc(), "-O2", "-std=c++17", "-shared", "-Xcompiler", "-fPIC", "--cudart", "none",
+            "-Wno-deprecated-gpu-targets", PLAIN_SOURCE,
+            "-I", os.path.join(ROOT, "include"), "-I", os.path.join(torch, "include"),
+            "-I", os.path.join(torch, "include", "torch", "csrc", "api", "include"), "-I", sysconfig.get_paths()["include"],
+            "-L", HERE, "-Xlinker", "-l:libfaws.so", "-L", os.path.join(torch, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu",
+            "-ltorch_python", "-Xlinker", "-rpath,$ORIGIN"]
+
+
 def _plain_digest() -> str:
     """Of what _plain.so is made from, the torch and Python that it is bound to among them."""
     return _digest([PLAIN_SOURCE, os.path.join(ROOT, "include", "faws.h"), os.path.join(_torch_dir(), "version.py")], sys.version)
@@ -78,17 +89,12 @@ def needs_build() -> bool:
 
 
 def _build_plain(verbose: bool) -> None:
-    torch, digest = _torch_dir(), _plain_digest()
-    cuda = os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")
-    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-o", PLAIN, PLAIN_SOURCE, "-I", os.path.join(ROOT, "include"),
-           "-I", os.path.join(torch, "include"), "-I", os.path.join(torch, "include", "torch", "csrc", "api", "include"),
-           "-I", sysconfig.get_paths()["include"], "-I", cuda, "-L", HERE, "-l:libfaws.so", "-L", os.path.join(torch, "lib"),
-           "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python", "-Wl,-rpath,$ORIGIN"]
-    res = subprocess.run(cmd, capture_output=True, text=True)
+    digest = _plain_digest()
+    res = subprocess.run(_plain_command() + ["-o", PLAIN], capture_output=True, text=True)
     if verbose or res.returncode != 0:
         sys.stderr.write(res.stdout + res.stderr)
     if res.returncode != 0:
-        raise RuntimeError("g++ failed building _plain.so")
+        raise RuntimeError("nvcc failed building _plain.so")
     with open(os.path.join(OBJDIR, "plain.digest"), "w") as f:
         f.write(digest)
 
