@@ -80,7 +80,8 @@ def _plain_command() -> list[str]:
 
 def _plain_digest() -> str:
     """Of what _plain.so is made from, the torch and Python that it is bound to among them."""
-    return _digest([PLAIN_SOURCE, os.path.join(ROOT, "include", "faws.h"), os.path.join(_torch_dir(), "version.py")], sys.version)
+    return _digest([PLAIN_SOURCE, os.path.join(ROOT, "include", "faws.h"), os.path.join(_torch_dir(), "version.py")],
+                   " ".join(_plain_command()) + sys.version)
 
 
 def needs_build() -> bool:

@@ -1,4 +1,4 @@
-"""The build of _plain.so."""
+"""The build of _plain.so: CUDA's headers, and what makes it out of date."""
 import shutil
 
 from flash_attn_with_score_b200 import build
@@ -17,3 +17,9 @@ def test_plain_is_built_with_an_nvcc_of_any_name(tmp_path, monkeypatch):
         monkeypatch.setattr(build, name, str(path))
     build._build_plain(False)
     assert (tmp_path / "_plain.so").exists() and (tmp_path / "plain.digest").read_text() == build._plain_digest()
+
+
+def test_another_compiler_call_makes_plain_out_of_date(monkeypatch):
+    before = build._plain_digest()
+    monkeypatch.setenv("NVCC", shutil.which("true"))
+    assert build._plain_digest() != before
