@@ -116,22 +116,21 @@ def load():
 
 
 OP_SCORES_ONLY = 100  # of plain_call alone: compute_attention_scores has no workspace and no operator id
-_plain = None
+_plain = None  # the native call once it is imported, False where it cannot be
 
 
 def plain_call(*args):
     """Runs ``(op, q, k, v, causal, sm_scale, split, per_q_head)`` natively, outputs and launch, or returns None where a
-    tensor or the moment is out of the ordinary (csrc/faws_torch.cpp): the caller then goes the long way."""
+    tensor or the moment is out of the ordinary (csrc/faws_torch.cpp), or _plain.so is missing or was built for another
+    torch or Python: the caller then goes the long way."""
     global _plain
     if _plain is None:
-        load()
         try:
             from . import _plain as module
-        except ImportError as e:
-            raise ImportError("flash_attn_with_score_b200/_plain.so is missing or was built for another torch: run "
-                              "`python -m flash_attn_with_score_b200.build`") from e
-        _plain = module.call
-    return _plain(*args)
+            _plain = module.call
+        except ImportError:
+            _plain = False
+    return _plain(*args) if _plain else None
 
 
 def check(status: int, what: str):

@@ -13,6 +13,7 @@ import concurrent.futures
 import hashlib
 import importlib.util
 import os
+import runpy
 import subprocess
 import sys
 import sysconfig
@@ -70,9 +71,10 @@ def _torch_dir() -> str:
 def _plain_command() -> list[str]:
     """nvcc as the driver of g++: it knows where CUDA's headers are, by whatever name or wrapper it was called."""
     torch = _torch_dir()
+    version = runpy.run_path(os.path.join(torch, "version.py"))["__version__"]
     return [_nvcc(), "-O2", "-std=c++17", "-shared", "-Xcompiler", "-fPIC", "--cudart", "none",
             "-Wno-deprecated-gpu-targets", PLAIN_SOURCE,
-            "-I", os.path.join(ROOT, "include"), "-I", os.path.join(torch, "include"),
+            f'-DFAWS_TORCH_VERSION="{version}"', "-I", os.path.join(ROOT, "include"), "-I", os.path.join(torch, "include"),
             "-I", os.path.join(torch, "include", "torch", "csrc", "api", "include"), "-I", sysconfig.get_paths()["include"],
             "-L", HERE, "-Xlinker", "-l:libfaws.so", "-L", os.path.join(torch, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu",
             "-ltorch_python", "-Xlinker", "-rpath,$ORIGIN"]
@@ -80,8 +82,7 @@ def _plain_command() -> list[str]:
 
 def _plain_digest() -> str:
     """Of what _plain.so is made from, the torch and Python that it is bound to among them."""
-    return _digest([PLAIN_SOURCE, os.path.join(ROOT, "include", "faws.h"), os.path.join(_torch_dir(), "version.py")],
-                   " ".join(_plain_command()) + sys.version)
+    return _digest([PLAIN_SOURCE, os.path.join(ROOT, "include", "faws.h")], " ".join(_plain_command()) + sys.version)
 
 
 def needs_build() -> bool:

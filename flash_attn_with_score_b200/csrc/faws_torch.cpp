@@ -12,6 +12,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <cmath>
+#include <cstring>
 
 #include "faws.h"
 
@@ -179,4 +180,23 @@ PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_plain", nullptr, -1, kMethods, n
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__plain() { return PyModule_Create(&kModule); }
+// Tensors are read by the layout of the torch that this was compiled against, so no other one may load it, and no other
+// Python.
+PyMODINIT_FUNC PyInit__plain() {
+#define FAWS_STR2(x) #x
+#define FAWS_STR(x) FAWS_STR2(x)
+  static const char python[] = FAWS_STR(PY_MAJOR_VERSION) "." FAWS_STR(PY_MINOR_VERSION) ".";
+  if (std::strncmp(Py_GetVersion(), python, sizeof(python) - 1) != 0) {
+    PyErr_Format(PyExc_ImportError, "_plain.so was built for Python %s, this is %s", python, Py_GetVersion());
+    return nullptr;
+  }
+  PyObject* torch = PyImport_ImportModule("torch");
+  if (torch == nullptr) return nullptr;
+  PyObject* version = PyObject_GetAttrString(torch, "__version__");
+  Py_DECREF(torch);
+  if (version == nullptr) return nullptr;
+  const bool same = PyUnicode_Check(version) && PyUnicode_CompareWithASCIIString(version, FAWS_TORCH_VERSION) == 0;
+  if (!same) PyErr_Format(PyExc_ImportError, "_plain.so was built for torch " FAWS_TORCH_VERSION ", this is %S", version);
+  Py_DECREF(version);
+  return same ? PyModule_Create(&kModule) : nullptr;
+}
