@@ -327,18 +327,6 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
     prefetch_tmap(&maps.v);
     prefetch_tmap(&maps.o);
     if constexpr (HOOK == kHookScores || HOOK == kHookScores16) prefetch_tmap(&maps.st);
-    // The first tiles on their way into L2 while the kernel before this one still drains: behind a launch that writes
-    // scores, whose stores keep DRAM busy, the first loads take 3 us (0.8 us otherwise).  fp16 H32 S1024 D128 causal, calls
-    // back to back: 36.3 -> 35.1 us; nothing (0 to 1 % slower) where no scores are written.
-    if (kStoreHook && nt > 0) {
-      for (int t = 0; t < L::kQTiles; ++t)
-        for (int c = 0; c < D / 64; ++c) tma_prefetch_4d(&maps.q, c * 64, r_tile_of[t] - p.m_begin, h, b);
-      for (int idx = 0; idx < min(nt, 2); ++idx)
-        for (int c = 0; c < D / 64; ++c) {
-          tma_prefetch_4d(&maps.k, c * 64, tile_of(idx) * BN, hk, b);
-          tma_prefetch_4d(&maps.v, c * 64, tile_of(idx) * BN, hk, b);
-        }
-    }
   }
   if (threadIdx.x == 0) {
     mbar_init(&bars->q_full, 1);
