@@ -520,12 +520,13 @@ __device__ __forceinline__ float sum_dealt_pairs(const float* base, int64_t head
     return x;
   };
   float s = 0.f;
-  for (; left > 0; left -= 8) {  // (the last few together as well: one after the other each would wait for its load)
+  for (; left >= 8; left -= 8) {
     float v[8];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) v[e] = e < left ? next() : 0.f;
+    for (int e = 0; e < 8; ++e) v[e] = next();
     s += ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
   }
+  for (; left > 0; --left) s += next();
   return s;
 }
 
