@@ -140,7 +140,6 @@ struct ColSoftmaxParams {
   float* negl_pad;       // scratch (B,Hq,m_pad) or null: the tcgen05 launcher fills it with -L_i*log2e (-inf for
                          // rows that do not contribute) and the kernel fetches it tile by tile with bulk copies
   int m_pad;             // M rounded up to the query-tile height
-  int keys_slowest;      // set by the tcgen05 launcher: the CTAs of a head's last keys come behind those of all heads' first ones
 };
 
 struct ReducePartialParams {

@@ -1339,12 +1339,11 @@ tc_colsoftmax_kernel(const __grid_constant__ CsMaps maps, const ColSoftmaxParams
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // Causal: key tiles are the slowest grid dimension, so the key tiles that see the most queries
-  // (the first ones) of all heads are dispatched first.  Otherwise key tiles are fastest, but where the last CTA of a head
-  // has few keys (p.keys_slowest): those come last.
-  const int n0 = (p.keys_slowest ? blockIdx.z : blockIdx.x) * (CS_KT * BN);  // first key of the CTA's CS_KT key tiles
-  const int ho = p.keys_slowest ? blockIdx.x : blockIdx.y;
-  const int b = p.keys_slowest ? blockIdx.y : blockIdx.z;
-  const int n_heads_out = p.keys_slowest ? gridDim.x : gridDim.y;
+  // (the first ones) of all heads are dispatched first.  Otherwise key tiles are fastest.
+  const int n0 = (p.causal ? blockIdx.z : blockIdx.x) * (CS_KT * BN);  // first key of the CTA's CS_KT key tiles
+  const int ho = p.causal ? blockIdx.x : blockIdx.y;
+  const int b = p.causal ? blockIdx.y : blockIdx.z;
+  const int n_heads_out = p.causal ? gridDim.x : gridDim.y;
   const int h0 = ho * heads_per_cta;  // first query head of this CTA
   const int hk = h0 / p.G;
 
@@ -1895,10 +1894,14 @@ cudaError_t launch_cs_t(const CsMaps& maps, const ColSoftmaxParams& call, int he
   const int nkt = (p.n_end + CS_KT * BN - 1) / (CS_KT * BN);  // CTAs along the keys: CS_KT key tiles each
   // A head's last CTA of one key tile at most, which takes half as long: last (fp16 B16 H8 S785 D32, 17 of 256 keys, with the
   // forward pass 104.8 -> 103.4 us, B4 H32 S300 D128 39.9 -> 36.4); as long as the queries stay in L2, so that the CTAs of a
-  // head need not run together.
+  // head need not run together.  The order is that of a causal launch, and a causal launch whose queries all see every key
+  // is a full one: the kernel need not tell them apart (a field for the order cost it registers, and causal launches 0.5 %).
   const int last = p.n_end - (nkt - 1) * CS_KT * BN;
-  p.keys_slowest = p.causal || (last <= BN && nkt > 1 && nkt <= 65535 && 2LL * p.B * p.Hq * p.m_end * p.D <= (48LL << 20));
-  dim3 grid = p.keys_slowest ? dim3(p.Hq / heads_per_cta, p.B, nkt) : dim3(nkt, p.Hq / heads_per_cta, p.B);
+  if (!p.causal && last <= BN && nkt > 1 && nkt <= 65535 && 2LL * p.B * p.Hq * p.m_end * p.D <= (48LL << 20)) {
+    p.causal = 1;
+    p.p_seq = nkt * CS_KT * BN;
+  }
+  dim3 grid = p.causal ? dim3(p.Hq / heads_per_cta, p.B, nkt) : dim3(nkt, p.Hq / heads_per_cta, p.B);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(CS_THREADS, 1, 1);
