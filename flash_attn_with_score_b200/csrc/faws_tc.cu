@@ -455,9 +455,11 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
       constexpr int kFmt = std::is_same<T, __half>::value ? 0 : 1;
       constexpr uint32_t idesc_qk = make_idesc_f16(128, BN, kFmt, 0, 0);
       // Head dims 16 and 32 in the D = 64 instances: K-steps and output columns of nothing but padding are left out (fp16 B16 H8
-      // S785 D32 57.0 -> 55.0 us, with softmax column sums 107.2 -> 104.8; head dim 64 as before).
-      const int k_steps = D == 64 ? (p.D + 15) / 16 : D / 16;
-      const uint32_t idesc_pv = D == 64 && p.D <= 32 ? make_idesc_f16(128, 32, kFmt, 0, 1) : make_idesc_f16(128, D, kFmt, 0, 1);
+      // S785 D32 57.0 -> 55.0 us, with softmax column sums 107.2 -> 104.8; head dim 64 as before), but not in the FEW instances, where
+      // it gains nothing (bf16 B2 H16 M1 N16517 D32 37.2 us, 37.0 without; D64 39.65 and 39.35).
+      constexpr bool kPadded = D == 64 && !FEW;
+      const int k_steps = kPadded ? (p.D + 15) / 16 : D / 16;
+      const uint32_t idesc_pv = kPadded && p.D <= 32 ? make_idesc_f16(128, 32, kFmt, 0, 1) : make_idesc_f16(128, D, kFmt, 0, 1);
       // Operand descriptors are built once; inside the loops only compile-time offsets (in
       // 16-byte units) are added to their address field, so the issuing thread spends a few
       // instructions per MMA.
@@ -1169,7 +1171,8 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
                 make_uint4(ro[g * 4], ro[g * 4 + 1], ro[g * 4 + 2], ro[g * 4 + 3]);
         };
         // (all D / 32 loads of the row in flight together measured 2-3 % slower: the registers they hold)
-        const int o_chunks = D == 64 && p.D <= 32 && !kHalfStage ? 1 : D / 32;  // (the store leaves the other columns out)
+        // (head dims 16 and 32: the store leaves the other columns out)
+        const int o_chunks = D == 64 && !FEW && p.D <= 32 && !kHalfStage ? 1 : D / 32;
 #pragma unroll 1
         for (int c = 0; c < o_chunks; ++c) {
           uint32_t ro[32];
