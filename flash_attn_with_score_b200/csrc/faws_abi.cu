@@ -421,6 +421,19 @@ size_t kept_mask_bytes(const faws_problem* p) {
   return bytes;
 }
 
+// Whether the forward kernel draws the mask that it leaves, or a kernel of its own before it.  The forward kernel's draw rides
+// on its softmax warps and costs 3 % over a pass that keeps nothing; the other kernel draws with the whole chip, which is what
+// counts where the forward CTAs (256 rows) do not fill it.  So the first where causal ones, heaviest first, are some 1.25 per
+// SM, and full ones leave at most a seventh of their waves' row tiles empty.  fp16 D64, drawn apart and in the kernel, forward
+// alone and with the backward pass (us): full B16 H16 S900 472 and 407, 1013 and 956; causal 306 and 276, 684 and 661; full B4 H16 S1000, 256 CTAs, 125 and
+// 126, 273 and 276; B5 H8, 160 CTAs, 93 and 126, 202 and 237; causal B3 H16 S1024, 192, 65 and 64, 141 and 143; B2 H20 S1000,
+// 160, 58 and 64, 125 and 133; B1 H16, 64, 39 and 63, 77 and 103.  D128 alike.
+bool forward_draws_mask(const faws_problem* p) {
+  const long long heads = (long long)p->B * p->Hq, sms = device_sms();
+  const long long tiles = heads * cdiv(p->M, 128), ctas = heads * cdiv(p->M, 256);
+  return p->causal ? 2 * tiles >= 5 * sms : 6 * 2 * sms * ((ctas + sms - 1) / sms) <= 7 * tiles;
+}
+
 size_t split_kv_bytes(const faws_problem* p, int n_splits) {
   return align256((size_t)p->B * p->Hq * n_splits * p->M * 4) +
          align256((size_t)p->B * p->Hq * n_splits * p->M * p->D * 4);
@@ -454,7 +467,8 @@ int faws_attention_keep_mask(const faws_problem* p, void* mask, size_t mask_byte
   FwdParams f = make_fwd(p);
   f.drop_mask = static_cast<uint32_t*>(mask);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (launch_dropout_mask(f, static_cast<uint32_t*>(mask), s) != cudaSuccess) return FAWS_ECUDA;
+  f.mask_drawn = !forward_draws_mask(p);
+  if (f.mask_drawn && launch_dropout_mask(f, f.drop_mask, s) != cudaSuccess) return FAWS_ECUDA;
   int bm, bn;
   return run_fwd(p, f, s, &bm, &bn);
 }

@@ -103,7 +103,8 @@ struct FwdParams {
   int col_row_lo;        // max(col_row_begin, m_begin): first query row that contributes
   float* qsum;           // col_lin: (B,Hq,ceil(M/128),128) per-tile sums of the query rows, written by the
   DropoutParams drop;
-  const uint32_t* drop_mask;  // tcgen05 attention(): the mask, drawn by launch_dropout_mask; null: drawn in the kernel
+  uint32_t* drop_mask;   // tcgen05 attention(): the mask in memory (mask_word), or null
+  int mask_drawn;        // launch_dropout_mask has drawn it; 0: the forward kernel draws it and leaves it there
 };
 
 // Raw column sums are linear in q: for a 128 x 128 (query tile, key tile) pair in which every

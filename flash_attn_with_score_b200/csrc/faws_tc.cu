@@ -144,8 +144,9 @@ enum Hook : int {
   kHookScoresAny = 5  // scores of either type in rows that TMA cannot address (odd lengths): plain stores
 };
 
-// Dropout: the weights' mask drawn in the kernel, or read from memory (attention() whose backward pass will want it too).
-enum Drop : int { kNoDrop = 0, kDrawMask = 1, kReadMask = 2 };
+// Dropout: the weights' mask drawn in the kernel, or, in attention() whose backward pass will want it too, read from memory
+// or drawn and left there.
+enum Drop : int { kNoDrop = 0, kDrawMask = 1, kReadMask = 2, kKeepMask = 3 };
 
 template <typename T, int D, int HOOK, bool SPLIT, int DROP = kNoDrop, bool FEW = false>
 __global__ void __launch_bounds__(NTHREADS, 1)
@@ -639,7 +640,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
     // for the max and exp2 passes (the chain the tensor pipe waits on), then, after P has been
     // handed back, for the score-tile hook.  kMasked = false is the fully visible tile.
     [[maybe_unused]] float carry[3] = {0.f, 0.f, 0.f};  // odd score rows: the last three columns of the tile before
-    [[maybe_unused]] uint4 kept;  // kReadMask: the row's 128 bits of the key tile in hand
+    [[maybe_unused]] uint4 kept = make_uint4(0u, 0u, 0u, 0u);  // kReadMask, kKeepMask: the row's 128 bits of the key tile in hand
     auto fully_visible = [&](int n0) {
       return n0 + BN <= p.N && (!p.causal || n0 + BN - 1 <= (pack_m > 0 ? 0 : r_tile) + p.p_seq);
     };
@@ -653,7 +654,8 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
       // masked and whose chain it lengthens (fp16 B10 H16
       // M34 N617 D128 causal 20.6 us, 20.0 without).
       constexpr bool kRolled = kMasked && !SPLIT && (HOOK == kHookNone || HOOK == kHookRowSum);
-      constexpr bool kReread = kRolled || (DROP == kDrawMask && HOOK == kHookNone);
+      constexpr bool kDraw = DROP == kDrawMask || DROP == kKeepMask;
+      constexpr bool kReread = kRolled || (kDraw && HOOK == kHookNone);
       uint32_t r[kRolled ? 1 : 128];
       int nvis = 128;  // visible columns form a prefix of the tile's row
       if (kMasked) {
@@ -744,6 +746,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
       const int nvis_warp = kMasked ? __reduce_max_sync(0xffffffffu, nvis) : 128;
       auto p_chunk = [&](int c, const uint32_t (&sv)[32]) {  // 32 key columns
         uint32_t pk[16];
+        [[maybe_unused]] uint32_t bits = 0u;  // kKeepMask (zero where the warp's rows see nothing: such weights are zero)
         const bool block_hidden = kMasked && c * 32 >= nvis_warp;
         if (block_hidden) {
 #pragma unroll
@@ -773,13 +776,15 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
             for (int y = 0; y < 8; ++y)
               if (!(word >> (g * 8 + y) & 1u)) e[y] = 0.f;
           }
-          if constexpr (DROP == kDrawMask) {
+          if constexpr (kDraw) {
             // dropout acts on the weights that multiply V only; the row sums above are taken
             // before it (flash.py:459-466)
             const uint32_t base = drop_row + (uint32_t)(n0 + c * 32 + g * 8);
 #pragma unroll
-            for (int y = 0; y < 8; ++y)
+            for (int y = 0; y < 8; ++y) {
               if (!dropout_keep(p.drop, base + (uint32_t)y)) e[y] = 0.f;
+              else if (DROP == kKeepMask) bits |= 1u << (g * 8 + y);
+            }
           }
           pk[g * 4 + 0] = pack2<T>(e[0], e[1]);
           pk[g * 4 + 1] = pack2<T>(e[2], e[3]);
@@ -787,6 +792,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
           pk[g * 4 + 3] = pack2<T>(e[6], e[7]);
         }
         }
+        if constexpr (DROP == kKeepMask) kept = make_uint4(kept.y, kept.z, kept.w, bits);
         tmem_st16(t_s + c * 16, pk);
         if (c == 1) {  // first 64 key columns of P are complete: let their P.V K-steps start
           tmem_wait_st();
@@ -1072,14 +1078,17 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
         const int tk = tile_of(it);
         if (SPLIT ? ((it & 1) != qt) : (tk >= my_nt)) continue;
         const int n0 = tk * BN;
-        if constexpr (DROP == kReadMask)
-          kept = *reinterpret_cast<const uint4*>(p.drop_mask + mask_word(bh, r_tile / BM, tk, (p.M + BM - 1) / BM, (p.N + BN - 1) / BN) + row * 4);
+        [[maybe_unused]] uint4* mask_row = nullptr;
+        if constexpr (DROP == kReadMask || DROP == kKeepMask)
+          mask_row = reinterpret_cast<uint4*>(p.drop_mask + mask_word(bh, r_tile / BM, tk, (p.M + BM - 1) / BM, (p.N + BN - 1) / BN)) + row;
+        if constexpr (DROP == kReadMask) kept = *mask_row;
         if (!mbar_wait(&bars->s_full[qt], s_cnt & 1, abort_flag)) { alive = false; break; }
         ++s_cnt;
         tc_fence_after();
         // (packed heads: the tile may hold the first row of a head)
         const bool ok = fully_visible(n0) ? tile_body(std::false_type{}, cnt, n0) : tile_body(std::true_type{}, cnt, n0);
         if (!ok) { alive = false; break; }
+        if constexpr (DROP == kKeepMask) *mask_row = kept;
         ++cnt;
       }
     }
@@ -1704,9 +1713,11 @@ cudaError_t launch_fwd_h(const TcMaps& maps, const FwdParams& p, cudaStream_t s)
   // 148 CTAs, 19.1 and 15.8), but for three key tiles, which two warpgroups share badly, when nearly every SM has one
   // (D128 S384 H40 13.3 and 12.0, H44 13.2 and 13.2, H49 13.2 and 14.1).
   if constexpr (HOOK != kHookScores16 && HOOK != kHookScoresAny) {
-    // dropout: 256-row CTAs only (the mask generation, not the chain of key tiles, bounds it)
+    // dropout: 256-row CTAs only (the mask generation, not the chain of key tiles, bounds what draws it)
     if constexpr (HOOK == kHookNone) {
-      if (p.drop_mask != nullptr) return launch_fwd_s<T, D, HOOK, false, kReadMask>(maps, p, s);
+      if (p.drop_mask != nullptr)
+        return p.mask_drawn ? launch_fwd_s<T, D, HOOK, false, kReadMask>(maps, p, s)
+                            : launch_fwd_s<T, D, HOOK, false, kKeepMask>(maps, p, s);
     }
     if (p.drop.p > 0.f) return launch_fwd_s<T, D, HOOK, false, kDrawMask>(maps, p, s);
   }

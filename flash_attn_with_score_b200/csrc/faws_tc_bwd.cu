@@ -753,9 +753,9 @@ __device__ __forceinline__ void draw_mask(const BwdParams& p, uint32_t* mask, in
   for (int x = 0; x < 32; ++x) bits |= dropout_keep(p.drop, lin + (uint32_t)x) ? 1u << x : 0u;
   mask[tile * 512 + at] = bits;
 }
-// The mask alone, before a forward pass that reads it and leaves it to the backward pass.  Drawn once, in a kernel that does
-// nothing else, it takes what the backward pass's pre-pass took for it, and the forward pass less than half of what it takes to
-// draw: fp16 B4 H16 S1024 D64 causal, p = 0.1, forward and backward 241 -> 194 us (forward 90 -> 57 + 41, pre-pass 63 -> 6).
+// The mask alone, before a forward pass that reads it and leaves it to the backward pass, where the forward pass's own CTAs
+// would not fill the chip with the draw: fp16 B1 H16 S1000 D64 causal, p = 0.1, forward and backward 77 us, 103 with the mask
+// drawn in the forward kernel and kept, 117 drawn in both passes.
 __global__ void __launch_bounds__(256) dropout_mask_kernel(BwdParams p, uint32_t* mask) {
   griddep_launch_dependents();
   griddep_wait();  // the mask's memory may have been another one's

@@ -46,6 +46,27 @@ def test_kept_mask(monkeypatch, B, Hq, Hk, M, N, D, causal, dtype):
     assert F.device_status() == 0
 
 
+@pytest.mark.parametrize("B,Hq,Hk,M,N,D,causal,dtype", [
+    (3, 64, 16, 333, 300, 64, True, torch.bfloat16),  # rows that see no key
+    (1, 128, 32, 520, 650, 128, True, torch.float16),
+    (2, 74, 74, 250, 515, 128, False, torch.float16),
+    (8, 16, 4, 768, 400, 32, True, torch.bfloat16)])
+def test_mask_that_the_forward_kernel_leaves(monkeypatch, B, Hq, Hk, M, N, D, causal, dtype):
+    test_kept_mask(monkeypatch, B, Hq, Hk, M, N, D, causal, dtype)
+
+
+@pytest.mark.parametrize("H,M,causal,launches", [
+    (186, 256, True, 1), (184, 256, True, 2), (148, 256, False, 1), (150, 256, False, 2), (148, 300, False, 2), (254, 129, False, 1)])
+def test_where_the_mask_is_drawn(H, M, causal, launches):
+    """In the forward kernel where its CTAs fill the SMs, so that a forward pass is not slower for what it leaves; else by a
+    launch of its own.  (148 SMs.)"""
+    q, k, v = [torch.randn(1, H, s, 64, device="cuda").half().requires_grad_(True) for s in (M, 256, 256)]
+    before = F.launch_count()
+    out = F.attention(q, k, v, causal, dropout_p=0.2, philox=(1, 2))
+    assert F.launch_count() - before == launches
+    assert out.grad_fn.saved_tensors[5] is not None
+
+
 def test_saved_tensors_that_come_back_elsewhere():
     """Hooks that give the tensors back at addresses that TMA cannot read: the CUDA-core kernels, which draw the mask."""
     g = torch.Generator(device="cuda").manual_seed(1)
