@@ -122,9 +122,9 @@ int faws_attention(const faws_problem* p, void* stream);
 /*
  * The same with dropout, for a caller that will run the backward pass: the mask is left in `mask`, a bit per entry, and handed
  * to faws_attention_backward_masked, which need not draw it again (bits of entries that no query sees may be zero).
- * faws_dropout_mask_bytes
- * says how large it is, or 0 where the plain calls are to be made: no dropout, a query-row window, problems that the
- * tcgen05 kernels do not take, a mask below 1 MB or larger than the queries.  `mask` starts on a 256-byte boundary.
+ * faws_dropout_mask_bytes says how large it is, or 0 where the plain calls are to be made: no dropout, a query-row window,
+ * problems that the tcgen05 kernels do not take, a mask below 1 MB, more than 16 D keys (a mask larger than the queries,
+ * both in whole 128-row tiles).  `mask` starts on a 256-byte boundary.
  * The results are those of the plain calls bit for bit.
  */
 size_t faws_dropout_mask_bytes(const faws_problem* p);

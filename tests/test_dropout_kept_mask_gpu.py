@@ -11,6 +11,9 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("B,Hq,Hk,M,N,D,causal,dtype", [
     (4, 8, 8, 512, 512, 32, True, torch.float16),         # 1 MB, as much as the queries: the smallest and the longest kept
+    (1, 16, 16, 1000, 1023, 64, True, torch.float16),     # the last key tile of a kept mask, lengths between whole tiles
+    (1, 32, 8, 400, 500, 32, False, torch.bfloat16),
+    (1, 8, 8, 1930, 2000, 128, True, torch.float16),
     (1, 32, 8, 1000, 700, 64, True, torch.bfloat16),      # rows that see no key
     (2, 16, 4, 900, 1700, 128, True, torch.float16),
     (1, 64, 64, 300, 260, 128, False, torch.bfloat16),
@@ -89,8 +92,8 @@ def test_saved_tensors_that_come_back_elsewhere():
 
 
 def test_what_keeps_no_mask():
-    """Larger than the queries, smaller than 1 MB, no gradient wanted, rows that TMA cannot read: the plain calls."""
-    for M, N, D, H, off in ((512, 1100, 64, 16, 0), (256, 256, 64, 8, 0), (1024, 1024, 64, 16, 1)):
+    """More than 16 D keys, smaller than 1 MB, no gradient wanted, rows that TMA cannot read: the plain calls."""
+    for M, N, D, H, off in ((512, 1100, 64, 16, 0), (1000, 1025, 64, 16, 0), (256, 256, 64, 8, 0), (1024, 1024, 64, 16, 1)):
         q, k, v = [torch.randn(1, H, s, D + 8, device="cuda").half()[..., off:off + D].requires_grad_(True) for s in (M, N, N)]
         out = F.attention(q, k, v, True, dropout_p=0.2, philox=(1, 2))
         assert out.grad_fn.saved_tensors[5] is None
