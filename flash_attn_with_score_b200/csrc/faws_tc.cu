@@ -177,10 +177,8 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
   // FEW: attention() with few query rows, whose heads may be packed (pack_m) and keys split over CTAs (n_splits, with
   // fp32 partial results).  An instance of its own: the run-time test
   // and the register of the row's limit cost unpacked launches 1 to 4 % (bf16 B1 Hq32 Hk8 D64 causal, M512 N512: 8.75 us
-  // without, 9.10 with; M512 N4096: 30.7 and 31.7).  The odd-row score hook, which packs nothing, is compiled with it all
-  // the same: ptxas 12.9 then happens to need no spills there, 68 bytes without (bf16 B1 Hq28 Hk4 S1531: 94 and 99 us;
-  // neither an opaque limit nor an opaque count of visible columns has the effect).
-  static_assert(!FEW || ((HOOK == kHookNone || HOOK == kHookScoresAny) && DROP == kNoDrop), "attention() without dropout");
+  // without, 9.10 with; M512 N4096: 30.7 and 31.7).
+  static_assert(!FEW || (HOOK == kHookNone && DROP == kNoDrop), "attention() without dropout");
   const int pack_m = FEW ? p.pack_m : 0;
   const bool persist = !SPLIT && !kStoreHook && wl.n_items > 0;  // (the launcher keeps the other instances plain)
   bool is_fill;
@@ -1207,7 +1205,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
 #pragma unroll
             for (int x = 0; x < 32; ++x) ro[x] = __float_as_uint(__uint_as_float(ro[x]) * inv);
           }
-          if constexpr (FEW && HOOK == kHookNone) {
+          if constexpr (FEW) {
             if (part_f32) {
               put_part(c, ro);
               continue;
@@ -1223,7 +1221,7 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
             }
           }
         }
-        if constexpr (FEW && HOOK == kHookNone) {
+        if constexpr (FEW) {
           static_assert(SPLIT ? 4 * 32 * D * 4 <= (L::kSlots - 1) * L::kTile
                               : 8 * 32 * D * 4 <= L::kQTiles * L::kTile + L::kSlots * L::kTile, "room for the partial results");
           if (part_f32 && !part_direct) {
@@ -1741,9 +1739,7 @@ cudaError_t launch_fwd_h(const TcMaps& maps, const FwdParams& p, cudaStream_t s)
       return split ? launch_fwd_s<T, D, HOOK, true, kNoDrop, true>(maps, p, s)
                    : launch_fwd_s<T, D, HOOK, false, kNoDrop, true>(maps, p, s);
   }
-  constexpr bool kFew = HOOK == kHookScoresAny;
-  return split ? launch_fwd_s<T, D, HOOK, true, kNoDrop, kFew>(maps, p, s)
-               : launch_fwd_s<T, D, HOOK, false, kNoDrop, kFew>(maps, p, s);
+  return split ? launch_fwd_s<T, D, HOOK, true>(maps, p, s) : launch_fwd_s<T, D, HOOK, false>(maps, p, s);
 }
 
 template <typename T, int D>
