@@ -62,7 +62,10 @@ PyObject* call(PyObject*, PyObject* const* a, Py_ssize_t n) {
   double sm_scale = 1.0 / std::sqrt((double)D);
   if (a[5] != Py_None) {
     sm_scale = PyFloat_AsDouble(a[5]);
-    if (sm_scale == -1.0 && PyErr_Occurred()) return nullptr;
+    if (sm_scale == -1.0 && PyErr_Occurred()) {  // what Python's float() takes, or refuses in words of its own
+      PyErr_Clear();
+      Py_RETURN_NONE;
+    }
   }
   const long split = PyLong_AsLong(a[6]);
   if (split == -1 && PyErr_Occurred()) return nullptr;

@@ -72,6 +72,9 @@ def test_what_is_not_plain_goes_the_long_way():
     for other in (wide[..., 1:65], wide[..., :64].transpose(2, 3), q.float(), q.cpu(), q[:, :, :0], q[0], q.bfloat16(), q[..., :32],
                   q[:, :3], torch.nn.Parameter(q).as_subclass(type("T", (torch.Tensor,), {}))):
         assert call(other, k, v) is None
+    assert torch.equal(F.attention(q, k, v, True, "0.25"), F.attention(q, k, v, True, 0.25))  # what float() takes
+    with pytest.raises(ValueError, match="could not convert"):
+        F.attention(q, k, v, True, "a quarter")
     with pytest.raises(TypeError, match="float16 or bfloat16"):
         F.attention_with_row_sum(q.float(), k.float(), v.float())
     with pytest.raises(AssertionError):
