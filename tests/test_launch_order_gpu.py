@@ -1,0 +1,51 @@
+"""Launches whose order or overlap is chosen by their size: key-major softmax sums of heads whose last CTA has few keys, and
+the column sums' reduce that begins before the forward pass has ended."""
+import pytest
+import torch
+
+import flash_attn_with_score_b200 as F
+from oracle import oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("N", [257, 384, 385, 513, 640, 641])  # last CTA of 1 to 256 keys: the first ones come last up to 128
+@pytest.mark.parametrize("B,H,Hk,M,D", [(2, 6, 2, 300, 64), (1, 8, 8, 129, 128), (3, 4, 4, 1, 32)])
+def test_softmax_sums_of_a_few_last_keys(N, B, H, Hk, M, D):
+    g = torch.Generator(device="cuda").manual_seed(N + M)
+    q, k, v = [torch.randn(B, h, s, D, device="cuda", generator=g).half() for h, s in ((H, M), (Hk, N), (Hk, N))]
+    w = ((q.double() @ k.double().repeat_interleave(H // Hk, 1).mT) * D ** -0.5).softmax(-1)
+    _, got = F.attention_with_softmax_col_sum(q, k, v, False, per_q_head=True)
+    assert F.last_backend() == "tcgen05"
+    ok, viol = orc.check_sum(got.cpu(), w.sum(-2).float().cpu())
+    assert ok, viol
+    S = N + 40  # the same over the keys before a split, from the queries behind it
+    q, k, v = [torch.randn(B, h, S, D, device="cuda", generator=g).half() for h in (H, Hk, Hk)]
+    w = ((q.double() @ k.double().repeat_interleave(H // Hk, 1).mT) * D ** -0.5).softmax(-1)
+    _, got = F.attention_cross_token_softmax_sum(q, k, v, N, False, per_q_head=True)
+    ok, viol = orc.check_sum(got.cpu(), w[:, :, N:, :N].sum(-2).float().cpu())
+    assert ok, viol
+    assert F.device_status() == 0
+
+
+@pytest.mark.parametrize("B,H,Hk,S,D", [(1, 8, 8, 512, 64), (1, 16, 4, 300, 128), (1, 37, 37, 512, 64), (1, 38, 19, 512, 64)])
+def test_keys_written_just_before_the_column_sums(B, H, Hk, S, D):
+    """148 CTAs of 128 rows or fewer, whose reduce reads the keys early, and more: keys that the kernel before the call wrote,
+    and writes again right behind it."""
+    g = torch.Generator(device="cuda").manual_seed(S)
+    q, v = [torch.randn(B, h, S, D, device="cuda", generator=g).half() for h in (H, Hk)]
+    keys = [torch.randn(B, Hk, S, D, device="cuda", generator=g).half() for _ in range(4)]
+    want = []
+    for x in keys:
+        want.append(F.attention_with_col_sum(q, x, v, True)[1])
+        torch.cuda.synchronize()
+    k = torch.zeros_like(keys[0])
+    for _ in range(5):
+        got = []
+        for x in keys:
+            k.copy_(x)
+            got.append(F.attention_with_col_sum(q, k, v, True)[1])
+            k.fill_(float("nan"))
+        for x, y in zip(got, want):
+            assert torch.equal(x, y)
+    assert F.device_status() == 0

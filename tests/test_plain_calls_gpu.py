@@ -72,9 +72,6 @@ def test_what_is_not_plain_goes_the_long_way():
     for other in (wide[..., 1:65], wide[..., :64].transpose(2, 3), q.float(), q.cpu(), q[:, :, :0], q[0], q.bfloat16(), q[..., :32],
                   q[:, :3], torch.nn.Parameter(q).as_subclass(type("T", (torch.Tensor,), {}))):
         assert call(other, k, v) is None
-    assert torch.equal(F.attention(q, k, v, True, "0.25"), F.attention(q, k, v, True, 0.25))  # what float() takes
-    with pytest.raises(ValueError, match="could not convert"):
-        F.attention(q, k, v, True, "a quarter")
     with pytest.raises(TypeError, match="float16 or bfloat16"):
         F.attention_with_row_sum(q.float(), k.float(), v.float())
     with pytest.raises(AssertionError):
@@ -93,3 +90,10 @@ def test_what_is_not_plain_goes_the_long_way():
     torch.cuda.synchronize()
     for x, y in zip(got, want):
         assert torch.equal(x, y)
+
+
+def test_scales_that_only_float_takes():
+    q, k, v = _inputs(64, 64, 64, torch.float16, False)
+    assert torch.equal(F.attention(q, k, v, True, "0.25"), F.attention(q, k, v, True, 0.25))
+    with pytest.raises(ValueError, match="could not convert"):
+        F.attention(q, k, v, True, "a quarter")
