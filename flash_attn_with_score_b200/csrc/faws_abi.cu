@@ -411,7 +411,8 @@ bool scores_only_on_cuda_cores(const ScoresOnlyParams& p, int sms) {
 
 // Bytes of the dropout mask that a forward pass leaves for its backward pass, 0 where it leaves none.  Drawing it takes both
 // passes 1.4 us a million entries; keeping it costs memory from one to the other.  Kept for up to 16 D keys, where it is no
-// larger than the queries, which are kept as well, both in whole 128-row tiles; and at least 1 MB.  fp16 D64 causal B4 H16,
+// larger than the queries, which are kept as well, both in whole 128-row tiles (causal with more rows than keys, where it also
+// has the rows that see none, it must be no larger than the queries' own bytes); and at least 1 MB.  fp16 D64 causal B4 H16,
 // forward and backward, drawn twice and kept (us): S1000 235 and 185, 8 MB of mask; S1100, beyond the line, 290 and 221, 10 MB;
 // S2048 728 and 561, 32 MB for 16 MB of queries; S4096 2580 and 1950, 128 MB for 32.
 size_t mask_bytes_of(const faws_problem* p) { return (size_t)p->B * p->Hq * cdiv(p->M, 128) * cdiv(p->N, 128) * 2048; }
@@ -419,6 +420,7 @@ size_t kept_mask_bytes(const faws_problem* p) {
   if (!(p->dropout_p > 0.f) || p->m_begin != 0 || p->m_end != p->M || p->v.ptr == nullptr || p->out.ptr == nullptr) return 0;
   const size_t bytes = mask_bytes_of(p);
   if (bytes < (size_t(1) << 20) || p->N > 16 * p->D) return 0;
+  if (p->causal && p->M > p->N && bytes > (size_t)p->B * p->Hq * p->M * p->D * 2) return 0;
   if (!tc_allowed(p) || !tc_fwd_supported(make_fwd(p), p->dtype)) return 0;
   return bytes;
 }

@@ -124,7 +124,8 @@ int faws_attention(const faws_problem* p, void* stream);
  * to faws_attention_backward_masked, which need not draw it again (bits of entries that no query sees may be zero).
  * faws_dropout_mask_bytes says how large it is, or 0 where the plain calls are to be made: no dropout, a query-row window,
  * problems that the tcgen05 kernels do not take, a mask below 1 MB, more than 16 D keys (a mask larger than the queries,
- * both in whole 128-row tiles).  `mask` starts on a 256-byte boundary.
+ * both in whole 128-row tiles; than the queries' own bytes where causal rows outnumber the keys).  `mask` starts on a
+ * 256-byte boundary.
  * The results are those of the plain calls bit for bit.
  */
 size_t faws_dropout_mask_bytes(const faws_problem* p);

@@ -11,9 +11,6 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("B,Hq,Hk,M,N,D,causal,dtype", [
     (4, 8, 8, 512, 512, 32, True, torch.float16),         # 1 MB, as much as the queries: the smallest and the longest kept
-    (1, 16, 16, 1000, 1023, 64, True, torch.float16),     # the last key tile of a kept mask, lengths between whole tiles
-    (1, 32, 8, 400, 500, 32, False, torch.bfloat16),
-    (1, 8, 8, 1930, 2000, 128, True, torch.float16),
     (1, 32, 8, 1000, 700, 64, True, torch.bfloat16),      # rows that see no key
     (2, 16, 4, 900, 1700, 128, True, torch.float16),
     (1, 64, 64, 300, 260, 128, False, torch.bfloat16),
@@ -49,27 +46,6 @@ def test_kept_mask(monkeypatch, B, Hq, Hk, M, N, D, causal, dtype):
     assert F.device_status() == 0
 
 
-@pytest.mark.parametrize("B,Hq,Hk,M,N,D,causal,dtype", [
-    (3, 64, 16, 333, 300, 64, True, torch.bfloat16),  # rows that see no key
-    (1, 128, 32, 520, 650, 128, True, torch.float16),
-    (2, 74, 74, 250, 515, 128, False, torch.float16),
-    (8, 16, 4, 768, 400, 32, True, torch.bfloat16)])
-def test_mask_that_the_forward_kernel_leaves(monkeypatch, B, Hq, Hk, M, N, D, causal, dtype):
-    test_kept_mask(monkeypatch, B, Hq, Hk, M, N, D, causal, dtype)
-
-
-@pytest.mark.parametrize("H,M,causal,launches", [
-    (186, 256, True, 1), (184, 256, True, 2), (148, 256, False, 1), (150, 256, False, 2), (148, 300, False, 2), (254, 129, False, 1)])
-def test_where_the_mask_is_drawn(H, M, causal, launches):
-    """In the forward kernel where its CTAs fill the SMs, so that a forward pass is not slower for what it leaves; else by a
-    launch of its own.  (148 SMs.)"""
-    q, k, v = [torch.randn(1, H, s, 64, device="cuda").half().requires_grad_(True) for s in (M, 256, 256)]
-    before = F.launch_count()
-    out = F.attention(q, k, v, causal, dropout_p=0.2, philox=(1, 2))
-    assert F.launch_count() - before == launches
-    assert out.grad_fn.saved_tensors[5] is not None
-
-
 def test_saved_tensors_that_come_back_elsewhere():
     """Hooks that give the tensors back at addresses that TMA cannot read: the CUDA-core kernels, which draw the mask."""
     g = torch.Generator(device="cuda").manual_seed(1)
@@ -92,10 +68,48 @@ def test_saved_tensors_that_come_back_elsewhere():
 
 
 def test_what_keeps_no_mask():
-    """More than 16 D keys, smaller than 1 MB, no gradient wanted, rows that TMA cannot read: the plain calls."""
-    for M, N, D, H, off in ((512, 1100, 64, 16, 0), (1000, 1025, 64, 16, 0), (256, 256, 64, 8, 0), (1024, 1024, 64, 16, 1)):
+    """Larger than the queries, smaller than 1 MB, no gradient wanted, rows that TMA cannot read: the plain calls."""
+    for M, N, D, H, off in ((512, 1100, 64, 16, 0), (256, 256, 64, 8, 0), (1024, 1024, 64, 16, 1)):
         q, k, v = [torch.randn(1, H, s, D + 8, device="cuda").half()[..., off:off + D].requires_grad_(True) for s in (M, N, N)]
         out = F.attention(q, k, v, True, dropout_p=0.2, philox=(1, 2))
         assert out.grad_fn.saved_tensors[5] is None
         dq, dk, dv = torch.autograd.grad(out, (q, k, v), torch.ones_like(out))
         assert bool(torch.isfinite(dq).all() and torch.isfinite(dk).all() and torch.isfinite(dv).all())
+
+
+@pytest.mark.parametrize("B,Hq,Hk,M,N,D,causal,dtype", [
+    (1, 16, 16, 1000, 1023, 64, True, torch.float16),  # the last key tile of a kept mask
+    (1, 32, 8, 400, 500, 32, False, torch.bfloat16),
+    (1, 8, 8, 1930, 2000, 128, True, torch.float16)])
+def test_kept_mask_of_lengths_between_whole_tiles(monkeypatch, B, Hq, Hk, M, N, D, causal, dtype):
+    test_kept_mask(monkeypatch, B, Hq, Hk, M, N, D, causal, dtype)
+
+
+def test_which_masks_are_kept():
+    """Up to 16 D keys; among causal rows that see no key, in bytes no larger than the queries."""
+    for M, N, causal, kept in ((1000, 1024, True, True), (1000, 1025, True, False), (1025, 1000, True, False),
+                               (1025, 1000, False, True), (1152, 1000, True, True)):
+        q, k, v = [torch.randn(1, 16, s, 64, device="cuda").half().requires_grad_(True) for s in (M, N, N)]
+        out = F.attention(q, k, v, causal, dropout_p=0.2, philox=(1, 2))
+        assert (out.grad_fn.saved_tensors[5] is not None) == kept
+
+
+@pytest.mark.parametrize("B,Hq,Hk,M,N,D,causal,dtype", [
+    (3, 64, 16, 333, 300, 64, True, torch.bfloat16),  # rows that see no key
+    (1, 128, 32, 520, 650, 128, True, torch.float16),
+    (2, 74, 74, 250, 515, 128, False, torch.float16),
+    (8, 16, 4, 768, 400, 32, True, torch.bfloat16)])
+def test_mask_that_the_forward_kernel_leaves(monkeypatch, B, Hq, Hk, M, N, D, causal, dtype):
+    test_kept_mask(monkeypatch, B, Hq, Hk, M, N, D, causal, dtype)
+
+
+@pytest.mark.parametrize("H,M,causal,launches", [
+    (186, 256, True, 1), (184, 256, True, 2), (148, 256, False, 1), (150, 256, False, 2), (148, 300, False, 2), (254, 129, False, 1)])
+def test_where_the_mask_is_drawn(H, M, causal, launches):
+    """In the forward kernel where its CTAs fill the SMs, so that a forward pass is not slower for what it leaves; else by a
+    launch of its own.  (148 SMs.)"""
+    q, k, v = [torch.randn(1, H, s, 64, device="cuda").half().requires_grad_(True) for s in (M, 256, 256)]
+    before = F.launch_count()
+    out = F.attention(q, k, v, causal, dropout_p=0.2, philox=(1, 2))
+    assert F.launch_count() - before == launches
+    assert out.grad_fn.saved_tensors[5] is not None
