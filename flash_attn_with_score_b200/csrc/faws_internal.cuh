@@ -105,6 +105,7 @@ struct FwdParams {
   DropoutParams drop;
   uint32_t* drop_mask;   // tcgen05 attention(): the mask in memory (mask_word), or null
   int mask_drawn;        // launch_dropout_mask has drawn it; 0: the forward kernel draws it and leaves it there
+  int early_tiles;       // tcgen05 score launches: the first tiles fetched into L2 before the wait on the previous kernel
 };
 
 // Raw column sums are linear in q: for a 128 x 128 (query tile, key tile) pair in which every

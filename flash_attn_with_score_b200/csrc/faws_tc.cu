@@ -326,6 +326,17 @@ tc_fwd_kernel(const __grid_constant__ TcMaps maps, const FwdParams p, const __gr
     prefetch_tmap(&maps.v);
     prefetch_tmap(&maps.o);
     if constexpr (HOOK == kHookScores || HOOK == kHookScores16) prefetch_tmap(&maps.st);
+    // The first tiles on their way into L2 while the kernel before this one still drains: behind a launch that writes
+    // scores, whose stores keep DRAM busy, the first loads take 3 us (0.8 us otherwise).  The launcher says where.
+    if (kStoreHook && p.early_tiles && nt > 0) {
+      for (int t = 0; t < L::kQTiles; ++t)
+        for (int c = 0; c < D / 64; ++c) tma_prefetch_4d(&maps.q, c * 64, r_tile_of[t] - p.m_begin, h, b);
+      for (int idx = 0; idx < min(nt, 2); ++idx)
+        for (int c = 0; c < D / 64; ++c) {
+          tma_prefetch_4d(&maps.k, c * 64, tile_of(idx) * BN, hk, b);
+          tma_prefetch_4d(&maps.v, c * 64, tile_of(idx) * BN, hk, b);
+        }
+    }
   }
   if (threadIdx.x == 0) {
     mbar_init(&bars->q_full, 1);
@@ -1644,6 +1655,12 @@ cudaError_t launch_fwd_s(const TcMaps& maps, const FwdParams& p, cudaStream_t s)
   pp.fill_ctas = ((HOOK == kHookScores || HOOK == kHookScores16 || HOOK == kHookScoresAny) && p.causal &&
                    p.p_seq + std::min(p.m_begin + BM, p.m_end) < p.N) ? 1 : 0;
   const int nslots = pp.fill_ctas ? 2 * ncb : ncb;
+  // The first tiles fetched into L2 before the wait on the previous kernel: 65 to 740 CTAs of 256 rows per 148 SMs gain, calls
+  // back to back, the same build with and without (fp16 D128 causal: H32 S1024 36.7 and 35.5 us, H44 S768 30.7 and 29.5, H96
+  // S1024 100.6 and 100.1; bf16 Hq28 Hk4 S1531 77.7 and 77.0, H32 S2752 199.9 and 198.1).  Not for half a wave or less, which
+  // does not keep DRAM busy (H24 S768, 72 CTAs, 18.1 and 18.2), nor for five key tiles or fewer, whose CTAs of later waves pay for
+  // it (B6 H32 S368 16-bit scores 45.5 and 46.3, B10 Hq32 Hk8 S576 full 108.3 and 109.7; though B7 H12 S448 27.4 and 26.6).
+  pp.early_tiles = p.N > 5 * BN && 2LL * p.B * p.Hq * ((p.m_end - p.m_begin + 255) / 256) >= sm_count();
   // the causal round-robin walk (down from the CTA's last key tile) is the reverse order: take its cheaper index form
   if (pp.schedule == kRoundRobin && pp.causal) pp.schedule = kReverse;
   if (pp.n_splits < 1) pp.n_splits = 1;

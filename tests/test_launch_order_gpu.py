@@ -1,5 +1,5 @@
-"""Launches whose order or overlap is chosen by their size: key-major softmax sums of heads whose last CTA has few keys, and
-the column sums' reduce that begins before the forward pass has ended."""
+"""Launches whose order or overlap is chosen by their size: key-major softmax sums of heads whose last CTA has few keys, the
+column sums' reduce that begins before the forward pass has ended, and score launches that fetch their first tiles into L2."""
 import pytest
 import torch
 
@@ -49,3 +49,32 @@ def test_keys_written_just_before_the_column_sums(B, H, Hk, S, D):
         for x, y in zip(got, want):
             assert torch.equal(x, y)
     assert F.device_status() == 0
+
+
+@pytest.mark.parametrize("H,M,N,D,causal", [(64, 300, 640, 64, True), (64, 300, 641, 64, True), (37, 300, 644, 128, False),
+                                            (36, 300, 644, 128, False), (40, 512, 1024, 128, True), (300, 100, 700, 32, True)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16], ids=["fp32", "fp16"])
+def test_inputs_written_just_before_the_scores(H, M, N, D, causal, dtype):
+    """More than five key tiles and half a 256-row CTA per SM or more, and fewer: inputs that the kernels before the call wrote,
+    and write again right behind it."""
+    g = torch.Generator(device="cuda").manual_seed(N + H)
+    sets = [[torch.randn(1, H, s, D, device="cuda", generator=g).half() for s in (M, N, N)] for _ in range(3)]
+    want = []
+    for x in sets:
+        want.append(F.attention_with_scores(*x, causal, scores_dtype=dtype))
+        torch.cuda.synchronize()
+        ref = (x[0].float() @ x[1].float().mT) * D ** -0.5
+        if causal:
+            ref = ref.masked_fill(~torch.ones(M, N, dtype=torch.bool, device="cuda").tril(N - M), float("-inf"))
+        ok, err = orc.check_out(want[-1][0].cpu(), (ref.softmax(-1) @ x[2].float()).cpu())
+        assert ok, err
+    now = [torch.zeros_like(t) for t in sets[0]]
+    for _ in range(3):
+        for x, y in zip(sets, want):
+            for t, u in zip(now, x):
+                t.copy_(u)
+            got = F.attention_with_scores(*now, causal, scores_dtype=dtype)
+            for t in now:
+                t.fill_(float("nan"))
+            assert torch.equal(got[0], y[0]) and torch.equal(got[1], y[1])
+    assert F.last_backend() == "tcgen05" and F.device_status() == 0
