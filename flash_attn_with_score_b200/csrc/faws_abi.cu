@@ -197,7 +197,11 @@ int raw_col_sums(const faws_problem* p, float* sum_out, int per_q_head, void* ws
   // Launched over the forward pass where that has a CTA per SM at most: set-up and key rows are in place when it ends (fp16
   // H8 S512 D64 causal 14.1 -> 13.1 us, Hq16 Hk4 S300 15.8 -> 14.6).  With more of them its CTAs take room and bandwidth from
   // the forward pass's last ones (Hq28 Hk4 S4096 D128 120 -> 124).
-  r.overlap = (long long)p->B * p->Hq * cdiv(p->M, kTcBlockM) <= device_sms();
+  const int sms = device_sms();
+  r.overlap = (long long)p->B * p->Hq * cdiv(p->M, kTcBlockM) <= sms;
+  // Two of its CTAs per SM, three for more blocks of small head dims than that (fp16 causal D32, two and three: B13 H12 S1235,
+  // 1560 blocks, 135.3 and 132.7 us; H32 S2755, 704, 108.3 and 107.1; B3 H8 S640, 120, 15.7 and 16.1).
+  r.resident = p->D <= 32 && (long long)p->B * (per_q_head ? p->Hq : p->Hk) * cdiv(r.n_end, 128) > 3LL * sms ? 3 : 2;
   if (launch_reduce_partials(r, p->dtype, s) != cudaSuccess) return FAWS_ECUDA;
   return FAWS_OK;
 }

@@ -159,6 +159,7 @@ struct ReducePartialParams {
   int64_t k_sb, k_sh, k_ss;
   float sm_scale;
   int overlap;           // the launch may begin while the forward pass drains
+  int resident;          // CTAs of the linear form per SM: 2 or 3
 };
 
 // Backward pass of attention(): inputs q, k, v, out, dout, L; outputs dq (B,Hq,M,D), dk, dv (B,Hk,N,D).

@@ -78,3 +78,22 @@ def test_inputs_written_just_before_the_scores(H, M, N, D, causal, dtype):
                 t.fill_(float("nan"))
             assert torch.equal(got[0], y[0]) and torch.equal(got[1], y[1])
     assert F.last_backend() == "tcgen05" and F.device_status() == 0
+
+
+@pytest.mark.parametrize("B,H,Hk,S,D,causal", [(8, 28, 28, 270, 32, True), (5, 28, 28, 385, 16, False), (2, 28, 4, 270, 32, True),
+                                               (4, 28, 28, 512, 32, False), (1, 8, 8, 1029, 64, True)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_column_sums_of_two_and_three_reduce_ctas(B, H, Hk, S, D, causal, dtype):
+    """Small head dims, more key tiles than three per SM and fewer (444 of them); sums of 1 to 9 terms a thread group."""
+    g = torch.Generator(device="cuda").manual_seed(S + H)
+    q, k, v = [torch.randn(B, h, S, D, device="cuda", generator=g).to(dtype) for h in (H, Hk, Hk)]
+    s = (q.double() @ k.double().repeat_interleave(H // Hk, 1).mT) * D ** -0.5
+    if causal:
+        s = s.tril()
+    for per_head in (False, True):
+        _, got = F.attention_with_col_sum(q, k, v, causal, per_q_head=per_head)
+        assert F.last_backend() == "tcgen05"
+        want = s.sum(-2) if per_head else s.sum(-2).view(B, Hk, H // Hk, S).sum(2)
+        ok, viol = orc.check_sum(got.cpu(), want.float().cpu())
+        assert ok, viol
+    assert F.device_status() == 0
