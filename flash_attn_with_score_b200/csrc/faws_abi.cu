@@ -199,9 +199,10 @@ int raw_col_sums(const faws_problem* p, float* sum_out, int per_q_head, void* ws
   // the forward pass's last ones (Hq28 Hk4 S4096 D128 120 -> 124).
   const int sms = device_sms();
   r.overlap = (long long)p->B * p->Hq * cdiv(p->M, kTcBlockM) <= sms;
-  // Two of its CTAs per SM, three for more blocks of small head dims than that (fp16 causal D32, two and three: B13 H12 S1235,
-  // 1560 blocks, 135.3 and 132.7 us; H32 S2755, 704, 108.3 and 107.1; B3 H8 S640, 120, 15.7 and 16.1).
-  r.resident = p->D <= 32 && (long long)p->B * (per_q_head ? p->Hq : p->Hk) * cdiv(r.n_end, 128) > 3LL * sms ? 3 : 2;
+  // Its CTAs per SM: two where all of them run at once so, else three (fp16 causal, two and three: B4 H32 S384 D64, 384 blocks,
+  // 32.3 and 30.7 us; B13 H12 S1235 D32, 1560, 135.3 and 132.7; H12 S786 D128, 84, 25.6 and 26.7; bf16 H32 S2048 D128, 512, 58.6
+  // and 61.0, but fp16 S8192, 2048, 593.4 and 591.6).
+  r.resident = (long long)p->B * (per_q_head ? p->Hq : p->Hk) * cdiv(r.n_end, 128) > 2LL * sms ? 3 : 2;
   if (launch_reduce_partials(r, p->dtype, s) != cudaSuccess) return FAWS_ECUDA;
   return FAWS_OK;
 }

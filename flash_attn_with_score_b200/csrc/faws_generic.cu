@@ -530,8 +530,7 @@ __device__ __forceinline__ float sum_dealt_pairs(const float* base, int64_t head
 }
 
 // CTAS: resident per SM.  Two leave 64 registers, and no spill code (24 / 44 bytes of it in fp16, 36 / 108 in bf16 with three):
-// whole operator, 42 shapes, 1.014 in the geometric mean, 0.98 to 1.13 (bf16 B16 H4 S200 D64 full 15.9 -> 14.1 us, H32 S2048
-// D128 causal 61.0 -> 58.6).  Many blocks at head dim 32 lose: raw_col_sums says which are launched so.
+// bf16 B16 H4 S200 D64 full 15.9 -> 14.1 us, B6 H8 S174 D64 causal 12.4 -> 11.7, whole operator.  raw_col_sums chooses.
 template <typename T, int CTAS>
 __global__ void __launch_bounds__(128 * kLinGroups, CTAS) reduce_colsum_lin_kernel(ReducePartialParams p) {
   constexpr int kRowsPerWarp = 128 / (4 * kLinGroups);

@@ -84,7 +84,7 @@ def test_inputs_written_just_before_the_scores(H, M, N, D, causal, dtype):
                                                (4, 28, 28, 512, 32, False), (1, 8, 8, 1029, 64, True)])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_column_sums_of_two_and_three_reduce_ctas(B, H, Hk, S, D, causal, dtype):
-    """Small head dims, more key tiles than three per SM and fewer (444 of them); sums of 1 to 9 terms a thread group."""
+    """More key tiles of output heads than two per SM (296 of them) and fewer; sums of 1 to 9 terms a thread group."""
     g = torch.Generator(device="cuda").manual_seed(S + H)
     q, k, v = [torch.randn(B, h, S, D, device="cuda", generator=g).to(dtype) for h in (H, Hk, Hk)]
     s = (q.double() @ k.double().repeat_interleave(H // Hk, 1).mT) * D ** -0.5
