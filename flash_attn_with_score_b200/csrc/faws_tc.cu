@@ -1655,12 +1655,14 @@ cudaError_t launch_fwd_s(const TcMaps& maps, const FwdParams& p, cudaStream_t s)
   pp.fill_ctas = ((HOOK == kHookScores || HOOK == kHookScores16 || HOOK == kHookScoresAny) && p.causal &&
                    p.p_seq + std::min(p.m_begin + BM, p.m_end) < p.N) ? 1 : 0;
   const int nslots = pp.fill_ctas ? 2 * ncb : ncb;
-  // The first tiles fetched into L2 before the wait on the previous kernel: 65 to 740 CTAs of 256 rows per 148 SMs gain, calls
-  // back to back, the same build with and without (fp16 D128 causal: H32 S1024 36.7 and 35.5 us, H44 S768 30.7 and 29.5, H96
-  // S1024 100.6 and 100.1; bf16 Hq28 Hk4 S1531 77.7 and 77.0, H32 S2752 199.9 and 198.1).  Not for half a wave or less, which
-  // does not keep DRAM busy (H24 S768, 72 CTAs, 18.1 and 18.2), nor for five key tiles or fewer, whose CTAs of later waves pay for
-  // it (B6 H32 S368 16-bit scores 45.5 and 46.3, B10 Hq32 Hk8 S576 full 108.3 and 109.7; though B7 H12 S448 27.4 and 26.6).
-  pp.early_tiles = p.N > 5 * BN && 2LL * p.B * p.Hq * ((p.m_end - p.m_begin + 255) / 256) >= sm_count();
+  // The first tiles fetched into L2 before the wait on the previous kernel (calls back to back, the same build without and
+  // with, 320 shapes): six key tiles or more gain from half a wave of 256-row CTAs on (fp16 D128 causal H32 S1024 36.7 and
+  // 35.5 us, H44 S768 30.7 and 29.5; bf16 Hq28 Hk4 S1531 77.7 and 77.0, H32 S2752 199.9 and 198.1; H24 S768, 72 CTAs, 18.1 and
+  // 18.2), four and five from a whole one (bf16 B7 H12 S448 27.4 and 26.6, 0.6 % in the mean of 30); shorter CTAs pay for it
+  // (B14 Hq12 Hk3 S192 D32 17.9 and 18.5; B6 H32 S368 16-bit scores 45.5 and 46.3; 1 % in the mean of 100).
+  const int key_tiles = (p.N + BN - 1) / BN;
+  const long long ctas256 = (long long)p.B * p.Hq * ((p.m_end - p.m_begin + 255) / 256);
+  pp.early_tiles = key_tiles > 5 ? 2 * ctas256 >= sm_count() : key_tiles > 3 && ctas256 >= sm_count();
   // the causal round-robin walk (down from the CTA's last key tile) is the reverse order: take its cheaper index form
   if (pp.schedule == kRoundRobin && pp.causal) pp.schedule = kReverse;
   if (pp.n_splits < 1) pp.n_splits = 1;
@@ -1728,7 +1730,10 @@ cudaError_t launch_fwd_h(const TcMaps& maps, const FwdParams& p, cudaStream_t s)
   // 148 CTAs, 19.1 and 15.8), but for three key tiles, which two warpgroups share badly, when nearly every SM has one
   // (D128 S384 H40 13.3 and 12.0, H44 13.2 and 13.2, H49 13.2 and 14.1).
   if constexpr (HOOK != kHookScores16 && HOOK != kHookScoresAny) {
-    // dropout: 256-row CTAs only (the mask generation, not the chain of key tiles, bounds what draws it)
+    // Dropout: 256-row CTAs only.  Where the kernel draws the mask, that bounds it and not the chain of key tiles.  Where it reads
+    // the mask there is no instance of 128-row CTAs, which would suit fewer of them than SMs (fp16 causal, mask kernel and
+    // forward pass, 256 and 128 rows: B1 H16 S1000 D64 39.6 and 30.8 us, H8 S1900 D128 63.5 and 48.9; B2 H20 S1000 D64 60.1 and
+    // 61.5, B4 H16 S300 25.0 and 26.1).
     if constexpr (HOOK == kHookNone) {
       if (p.drop_mask != nullptr)
         return p.mask_drawn ? launch_fwd_s<T, D, HOOK, false, kReadMask>(maps, p, s)
