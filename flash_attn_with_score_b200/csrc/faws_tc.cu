@@ -1656,13 +1656,14 @@ cudaError_t launch_fwd_s(const TcMaps& maps, const FwdParams& p, cudaStream_t s)
                    p.p_seq + std::min(p.m_begin + BM, p.m_end) < p.N) ? 1 : 0;
   const int nslots = pp.fill_ctas ? 2 * ncb : ncb;
   // The first tiles fetched into L2 before the wait on the previous kernel (calls back to back, the same build without and
-  // with, 320 shapes): six key tiles or more gain from half a wave of 256-row CTAs on (fp16 D128 causal H32 S1024 36.7 and
+  // with, 580 shapes): six key tiles or more gain from half a wave of 256-row CTAs on (fp16 D128 causal H32 S1024 36.7 and
   // 35.5 us, H44 S768 30.7 and 29.5; bf16 Hq28 Hk4 S1531 77.7 and 77.0, H32 S2752 199.9 and 198.1; H24 S768, 72 CTAs, 18.1 and
-  // 18.2), four and five from a whole one (bf16 B7 H12 S448 27.4 and 26.6, 0.6 % in the mean of 30); shorter CTAs pay for it
-  // (B14 Hq12 Hk3 S192 D32 17.9 and 18.5; B6 H32 S368 16-bit scores 45.5 and 46.3; 1 % in the mean of 100).
+  // 18.2), four and five from three quarters (B4 Hq16 Hk8 S453 26.8 and 26.3, B7 H12 S448 27.4 and 26.6), one and two from a
+  // whole one if the inputs are other ones than the last call's (B9 Hq32 Hk8 S192 32.0 and 31.5, 0.4 % in the mean; with the
+  // same ones again, which L2 holds, -1 %).  Three lose (B3 H28 S352 22.6 and 23.2, 1 % in the mean of 60 either way).
   const int key_tiles = (p.N + BN - 1) / BN;
   const long long ctas256 = (long long)p.B * p.Hq * ((p.m_end - p.m_begin + 255) / 256);
-  pp.early_tiles = key_tiles > 5 ? 2 * ctas256 >= sm_count() : key_tiles > 3 && ctas256 >= sm_count();
+  pp.early_tiles = key_tiles != 3 && 4 * ctas256 >= (key_tiles > 5 ? 2LL : key_tiles > 3 ? 3LL : 4LL) * sm_count();
   // the causal round-robin walk (down from the CTA's last key tile) is the reverse order: take its cheaper index form
   if (pp.schedule == kRoundRobin && pp.causal) pp.schedule = kReverse;
   if (pp.n_splits < 1) pp.n_splits = 1;
@@ -1750,7 +1751,10 @@ cudaError_t launch_fwd_h(const TcMaps& maps, const FwdParams& p, cudaStream_t s)
                            (odd_f32 ? 3 * ctas128 > 5LL * sm_count()
                                     : ctas128 > ((p.N + BN - 1) / BN == 3 ? sm_count() * 7 / 8 : sm_count()));
   // Without a mask 256-row CTAs take some 1.65 times as long as 128-row ones, so whole waves decide (D128 full, 256 and 128
-  // rows: H24 S1531, 144 and 288 CTAs, 76.1 and 97.6 us; H28, 168 and 336, 147 and 129).
+  // rows: H24 S1531, 144 and 288 CTAs, 76.1 and 97.6 us; H28, 168 and 336, 147 and 129).  Over 156 odd shapes of 1 to 2.9 CTAs of
+  // 128 rows per SM, D 32 to 128, what both rules take is 0.5 % behind the better of the two in the mean; the worst: one row
+  // beyond a 256-row CTA (causal H84 S257 27.2 us, 22.3 with 128 rows), causal just above the line (H32 S1021 D64 49.1 and 45.7),
+  // full just above one wave (H26 S641 D32 34.3 and 32.3, H15 S1163 D128 58.7 and 56.3).
   const long long ctas256 = (long long)((p.m_end - p.m_begin + 255) / 256) * p.Hq * p.B;
   const bool fewer_waves = odd_f32 && !p.causal &&
                            5 * ((ctas256 + sm_count() - 1) / sm_count()) <= 3 * ((ctas128 + sm_count() - 1) / sm_count());

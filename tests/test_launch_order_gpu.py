@@ -53,11 +53,12 @@ def test_keys_written_just_before_the_column_sums(B, H, Hk, S, D):
 
 @pytest.mark.parametrize("H,M,N,D,causal", [(64, 300, 640, 64, True), (64, 300, 641, 64, True), (37, 300, 644, 128, False),
                                             (36, 300, 644, 128, False), (40, 512, 1024, 128, True), (300, 100, 700, 32, True),
-                                            (148, 200, 385, 64, True), (148, 200, 384, 64, False), (147, 200, 640, 64, True)])
+                                            (111, 200, 385, 64, True), (148, 200, 384, 64, False), (110, 200, 640, 64, True), (148, 100, 256, 128, False),
+                                            (147, 90, 130, 128, True)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16], ids=["fp32", "fp16"])
 def test_inputs_written_just_before_the_scores(H, M, N, D, causal, dtype):
-    """More than five key tiles and half a 256-row CTA per SM, four and a whole one, and fewer: inputs that the kernels before
-    the call wrote, and write again right behind it."""
+    """Key tiles and CTAs on either side of the lines: inputs that the kernels before the call wrote, and write again right
+    behind it."""
     g = torch.Generator(device="cuda").manual_seed(N + H)
     sets = [[torch.randn(1, H, s, D, device="cuda", generator=g).half() for s in (M, N, N)] for _ in range(3)]
     want = []
